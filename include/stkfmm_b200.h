@@ -219,6 +219,17 @@ int stk_p2p_lists_aux(int ukernel, int precision, int n_trg_box, const int *trg_
 int stk_gemm_3xtf32(int M, int N, int K, const float *d_A, int lda, const float *d_B, int ldb, float *d_C, int ldc,
                     int beta, void *stream);
 
+/* ---- FP64 products on the int8 tensor cores (the far field's translations) -----
+ * No reference counterpart.  C[m + n ldc] (beta 0: =, 1: +=) sum_k A[m lda + k]
+ * B[n ldb + k] for m < M, n < N, FP64 in and out: every row of A and B scaled by a
+ * power of two and split into seven balanced base-256 digits, 34 exact integer
+ * products on the sm_100a tensor cores (tcgen05 kind::i8), put together in FP64.
+ * Error below ~2^-56 |a||b| per element (row norms), less than an FP64 sum's
+ * rounding.  A row with an infinity or NaN gives NaN.  Device pointers; the call
+ * allocates its scratch and waits for the result.  STK_ERR_NOT_SUPPORTED off sm_100. */
+int stk_gemm_f64_i8(int M, int N, int K, const double *d_A, int lda, const double *d_B, int ldb, double *d_C, int ldc,
+                    int beta, void *stream);
+
 /* ---- reusable asynchronous list plan -----------------------------------------
  * Replaces, for a list evaluated many times, the per-(target box, source box)
  * ker_poten calls that PVFMM's list loops make at every evaluation

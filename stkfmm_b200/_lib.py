@@ -48,6 +48,8 @@ SIGNATURES = [
                                               c_void_p, c_int, c_void_p]),
     ("stk_gemm_3xtf32", c_int, [c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int,
                                 c_void_p]),
+    ("stk_gemm_f64_i8", c_int, [c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int,
+                                c_void_p]),
     ("stk_p2p_plan_create", c_void_p, [c_int, P_i, P_i, P_i, P_i, c_int, P_i, P_i, c_int, c_int, c_double, P_i]),
     ("stk_p2p_plan_execute", c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                      c_void_p]),

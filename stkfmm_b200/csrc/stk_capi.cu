@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "../../include/stkfmm_b200.h"
+#include "stk_i8gemm.cuh"
 #include "stk_kernel_table.hpp"
 #include "stk_p2p.cuh"
 #include "stk_tree.hpp"
@@ -376,6 +377,46 @@ extern "C" int stk_gemm_3xtf32(int M, int N, int K, const float *d_A, int lda, c
         rc = STK_ERR_CUDA;
     if (!rc && e) rc = STK_ERR_CUDA;
     cudaStreamSynchronize(s);
+    cudaFree(buf);
+    cudaGetLastError();
+    return rc;
+}
+
+// FP64 product on the int8 tensor cores, for direct use and tests
+extern "C" int stk_gemm_f64_i8(int M, int N, int K, const double *d_A, int lda, const double *d_B, int ldb, double *d_C,
+                               int ldc, int beta, void *stream) {
+    if (M < 0 || N < 0 || K < 0 || (beta != 0 && beta != 1)) return STK_ERR_INVALID_ARG;
+    if (M == 0 || N == 0 || K == 0) return STK_OK;
+    if (!d_A || !d_B || !d_C || lda < K || ldb < K || ldc < M) return STK_ERR_INVALID_ARG;
+    int ndev = 0;
+    if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
+        cudaGetLastError();
+        return STK_ERR_NO_DEVICE;
+    }
+    if (!umma_available()) return STK_ERR_NOT_SUPPORTED;
+    cudaStream_t s = (cudaStream_t)stream;
+    const int nkb = i8_kblocks(K);
+    const size_t ba = i8_bytes(M, nkb), bb = i8_bytes(N, nkb);
+    const size_t sa = sizeof(double) * i8_pad_rows(M), sb = sizeof(double) * i8_pad_rows(N);
+    uint8_t *buf = nullptr;
+    const size_t np = (size_t)i8_gemm_parts(M, N, nkb), pb = np > 1 ? sizeof(double) * np * M * N : 0;
+    if (cudaMalloc(&buf, ba + bb + sa + sb + pb + 64) != cudaSuccess) {
+        cudaGetLastError();
+        return STK_ERR_CUDA;
+    }
+    uint8_t *da = buf, *db = da + ba;
+    double *fa = reinterpret_cast<double *>(db + bb), *fb = fa + sa / sizeof(double);
+    double *parts = pb ? fb + sb / sizeof(double) : nullptr;
+    int *err = reinterpret_cast<int *>(reinterpret_cast<uint8_t *>(fb) + sb + pb);
+    int rc = STK_OK, e = 0;
+    if (cudaMemsetAsync(err, 0, sizeof(int), s) != cudaSuccess ||
+        i8_digits(d_A, lda, nullptr, M, K, nkb, nullptr, da, fa, s) != cudaSuccess ||
+        i8_digits(d_B, ldb, nullptr, N, K, nkb, nullptr, db, fb, s) != cudaSuccess ||
+        i8_gemm(M, N, I8Operand{da, fa, nkb}, I8Operand{db, fb, nkb}, 1.0, beta, d_C, ldc, nullptr, parts, err,
+                s) != cudaSuccess ||
+        cudaMemcpyAsync(&e, err, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess)
+        rc = STK_ERR_CUDA;
+    if (cudaStreamSynchronize(s) != cudaSuccess || e) rc = STK_ERR_CUDA;
     cudaFree(buf);
     cudaGetLastError();
     return rc;

@@ -452,7 +452,20 @@ __global__ void to_float_kernel(const double *__restrict__ a, long long n, float
         b[i] = (float)a[i];
 }
 
-constexpr int kM2LChunk = 256;  // pairs (columns) per batched-GEMM problem of the M2L
+// Pairs (columns) of one offset per problem of the chunked M2L: one tensor-core tile wide.
+// Small trees pad every offset's last chunk (Stokes, 32k points: 92 k columns for 56 k pairs
+// at 256 wide, 72 k at 128).
+constexpr int kM2LChunk = 128;
+static_assert(kM2LChunk == kI8Rows, "a chunk is one row block of the int8 path");
+
+// out[i] = up[idx[i]], out[n + i] = down[idx[i]]
+__global__ void gather_scales_kernel(const double *__restrict__ up, const double *__restrict__ down,
+                                     const int *__restrict__ idx, long long n, double *__restrict__ out) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        out[i] = up[idx[i]];
+        out[n + i] = down[idx[i]];
+    }
+}
 
 // X[r + k j] = phi_hat[r + k gsrc[j]], or 0 for a padding column (gsrc[j] < 0)
 template <class T>
@@ -902,6 +915,112 @@ int build_m2l_lowrank(FarField &F, const std::vector<double> &unit, const double
     return STK_OK;
 }
 
+// ---- FP64 products on the int8 tensor cores ---------------------------------------
+// Operator digits, built with the operators and shared with them.
+int build_i8_operators(FarField &F, cudaStream_t s) {
+    F.i8 = F.i8_pq = false;
+    const char *env = getenv("STKFMM_F64_I8");
+    if ((env && env[0] == '0') || !umma_available()) return STK_OK;
+    const int N = F.n * F.ke, k = F.m2l_rank;
+    // column-major M x K operators: row m's values are ld apart
+    auto op = [&](I8Buf &b, const DevBuf &src, int M, int K) -> int {
+        int rc = b.reserve(M, K);
+        if (!rc) rc = b.reserve_kscale(K);
+        if (rc) return rc;
+        FCUDA(i8_column_scales((const double *)src.ptr, M, M, K, b.up(), b.down(), s));
+        FCUDA(i8_digits_trans((const double *)src.ptr, M, M, K, b.nkb, b.down(), b.digits(), b.scales(), s));
+        return STK_OK;
+    };
+    int rc = op(F.i8_uc2ue, F.uc2ue, N, N);
+    if (!rc) rc = op(F.i8_dc2de, F.dc2de, N, N);
+    if (!rc) rc = op(F.i8_m2m, F.m2m, N, 8 * N);
+    if (!rc) rc = op(F.i8_l2l, F.l2l, 8 * N, N);
+    if (!rc) rc = op(F.i8_vt, F.m2l_vt, k, N);
+    if (!rc) rc = op(F.i8_e, F.m2l_e, N, k);
+    if (rc) return rc;
+    F.i8 = true;
+    // the factors of every offset, within 8 GiB
+    const int nslot = (int)F.m2l_r.size(), kb = (k + kI8Rows - 1) / kI8Rows;
+    F.i8_q_blk.assign(nslot, 0);
+    int qb = 0;
+    for (int sl = 0; sl < nslot; sl++) {
+        F.i8_q_blk[sl] = qb;
+        qb += (F.m2l_r[sl] + kI8Rows - 1) / kI8Rows;
+    }
+    const size_t bytes = i8_bytes((long long)qb * kI8Rows, i8_kblocks(k)) +
+                         i8_bytes((long long)nslot * kb * kI8Rows, i8_kblocks(F.m2l_rmax));
+    if (bytes > (8ull << 30)) return STK_OK;
+    // scales along K: of Q over all offsets (one set of k), of P_d per offset (rmax each)
+    const int rmax = F.m2l_rmax;
+    rc = F.i8_q.reserve((long long)qb * kI8Rows, k);
+    if (!rc) rc = F.i8_p.reserve((long long)nslot * kb * kI8Rows, rmax);
+    if (!rc) rc = F.i8_q.reserve_kscale(k);
+    if (!rc) rc = F.i8_p.reserve_kscale(nslot * rmax);
+    DevBuf mag;
+    if (!rc) rc = mag.reserve(sizeof(unsigned long long) * k);
+    if (rc) return rc;
+    long long qcols = 0;
+    for (int sl = 0; sl < nslot; sl++) qcols += F.m2l_r[sl];
+    FCUDA(i8_row_scales((const double *)F.m2l_q.ptr, k, qcols, k, (unsigned long long *)mag.ptr, F.i8_q.up(),
+                        F.i8_q.down(), s));
+    for (int sl = 0; sl < nslot; sl++) {
+        const double *Q = (const double *)F.m2l_q.ptr + F.m2l_pq_off[sl], *P = (const double *)F.m2l_p.ptr + F.m2l_pq_off[sl];
+        const size_t ks = (size_t)sl * rmax;
+        FCUDA(i8_digits(Q, k, nullptr, F.m2l_r[sl], k, F.i8_q.nkb, F.i8_q.down(), F.i8_q.digits(F.i8_q_blk[sl]),
+                        F.i8_q.scales(F.i8_q_blk[sl]), s));
+        FCUDA(i8_column_scales(P, k, k, F.m2l_r[sl], F.i8_p.up() + ks, F.i8_p.down() + ks, s));
+        FCUDA(i8_digits_trans(P, k, k, F.m2l_r[sl], F.i8_p.nkb, F.i8_p.down() + ks, F.i8_p.digits((long long)sl * kb),
+                              F.i8_p.scales((long long)sl * kb), s));
+    }
+    F.i8_pq = true;
+    return STK_OK;
+}
+
+// Whether an M x N x K product is faster on the int8 tensor cores than as a cuBLAS DGEMM.
+// Measured on B200: a 128 x 128 output tile costs 1.3 us per 32 of K and ~5 us beside, 148
+// tiles at a time (100 TFLOP/s of FP64 work on full waves); the digits of the right-hand
+// operand ~8 us and 15 bytes a value, a sum over K parts ~5 us.  A DGEMM runs at ~28 TFLOP/s,
+// splitting K where the output is small, in no less than ~15 us.
+bool i8_wins(int M, int N, int K) {
+    const int nkb = i8_kblocks(K), np = i8_gemm_parts(M, N, nkb);
+    const double tiles = std::ceil((double)M / kI8Rows) * std::ceil((double)N / kI8Rows) * np;
+    const double i8_us = 8.0 + (double)N * K * 15.0 / 3e6 + (np > 1 ? 5.0 : 0.0) +
+                         std::ceil(tiles / 148.0) * (1.45 * ((nkb + np - 1) / np) + 5.0);
+    return i8_us < std::max(15.0, 2.0 * M * N * K / 28e6);
+}
+
+// C[:, col(j)] (add = 0: =, 1: +=) alpha A X[:, idx(j)] for j < m: A column-major M x K
+// (and as digits), X columns of K values, idx / cols null for the identity.  Y, Xg: scratch of
+// the cuBLAS path (M x m, K x m).
+int far_product(FarField &F, const DevBuf &A, const I8Buf &A8, int M, int K, const double *X, const int *idx, int m,
+                double alpha, int add, double *C, const int *cols, double *Xg, double *Y, cudaStream_t s) {
+    if (m <= 0) return STK_OK;
+    if (F.i8 && i8_wins(M, m, K)) {
+        const int np = i8_gemm_parts(M, m, i8_kblocks(K));
+        int rc = F.i8_b.reserve(m, K);
+        if (!rc && np > 1) rc = F.i8_parts.reserve(sizeof(double) * (size_t)np * M * m);
+        if (rc) return rc;
+        t_launches += np > 1 ? 3 : 2;
+        FCUDA(i8_digits(X, K, idx, m, K, F.i8_b.nkb, A8.up(), F.i8_b.digits(), F.i8_b.scales(), s));
+        FCUDA(i8_gemm(M, m, A8.op(), F.i8_b.op(), alpha, add, C, M, cols, np > 1 ? (double *)F.i8_parts.ptr : nullptr,
+                      (int *)F.tc_err.ptr, s));
+        return STK_OK;
+    }
+    const double zero = 0.0, one = 1.0;
+    if (idx) {
+        const int rc = gather_cols(X, idx, m, K, Xg, s);
+        if (rc) return rc;
+        X = Xg;
+    }
+    if (!cols) {
+        FBLAS(cublasDgemm(F.blas, CUBLAS_OP_N, CUBLAS_OP_N, M, m, K, &alpha, (const double *)A.ptr, M, X, K,
+                          add ? &one : &zero, C, M));
+        return STK_OK;
+    }
+    FBLAS(cublasDgemm(F.blas, CUBLAS_OP_N, CUBLAS_OP_N, M, m, K, &alpha, (const double *)A.ptr, M, X, K, &zero, Y, M));
+    return scatter_cols(Y, cols, m, M, 1.0, add, C, s);
+}
+
 // Build the level-independent operators for (m2x, p).
 int build_operators(FarField &F, cudaStream_t s) {
     const int n = F.n, N = F.n * F.ke;
@@ -1027,6 +1146,7 @@ int build_operators(FarField &F, cudaStream_t s) {
     FBLAS(cublasDgemm(F.blas, CUBLAS_OP_N, CUBLAS_OP_T, N, k, N, &one, (const double *)F.dc2de.ptr, N,
                       (const double *)VTu.ptr, N, &zero, (double *)F.m2l_e.ptr, N));
     rc = build_m2l_lowrank(F, unit, (const double *)VTu.ptr, (const double *)VTv.ptr, offset_matrix, K, T, s);
+    if (!rc) rc = build_i8_operators(F, s);
     if (rc) return rc;
     FCUDA(cudaStreamSynchronize(s));
     return STK_OK;
@@ -1212,6 +1332,17 @@ void share_operators(FarField &dst, const FarField &src) {
     dst.m2l_q32.share(src.m2l_q32);
     dst.m2l_vt.share(src.m2l_vt);
     dst.m2l_e.share(src.m2l_e);
+    dst.i8 = src.i8;
+    dst.i8_pq = src.i8_pq;
+    dst.i8_q_blk = src.i8_q_blk;
+    dst.i8_uc2ue.share(src.i8_uc2ue);
+    dst.i8_dc2de.share(src.i8_dc2de);
+    dst.i8_m2m.share(src.i8_m2m);
+    dst.i8_l2l.share(src.i8_l2l);
+    dst.i8_vt.share(src.i8_vt);
+    dst.i8_e.share(src.i8_e);
+    dst.i8_q.share(src.i8_q);
+    dst.i8_p.share(src.i8_p);
 }
 
 // an event recorded on s after the work queued so far (the entry's build)
@@ -1244,7 +1375,6 @@ static int setup_m2l_chunks_tc(FarField &F, const std::vector<int> &chunk_slot, 
     if (!rc) rc = F.tcc_q_lo.reserve(sizeof(float) * (size_t)qrows * k4);
     if (!rc) rc = F.tcc_pt_hi.reserve(sizeof(float) * (size_t)nslot * k * rmax);
     if (!rc) rc = F.tcc_pt_lo.reserve(sizeof(float) * (size_t)nslot * k * rmax);
-    if (!rc && !F.tc_err.ptr) rc = F.tc_err.reserve(sizeof(int) * 4);
     if (rc) return rc;
     // Q_d (k x r_d column-major, offsets back to back) read as qrows K-major rows of k
     tc_rows_kernel<<<grid_for(qrows * k4), 256, 0, s>>>((const double *)F.m2l_q.ptr, k, qrows, k4,
@@ -1256,7 +1386,6 @@ static int setup_m2l_chunks_tc(FarField &F, const std::vector<int> &chunk_slot, 
             (float *)F.tcc_pt_hi.ptr + (size_t)sl * k * rmax, (float *)F.tcc_pt_lo.ptr + (size_t)sl * k * rmax);
         FCUDA(cudaGetLastError());
     }
-    FCUDA(cudaMemsetAsync(F.tc_err.ptr, 0, sizeof(int) * 4, s));
     // tile tables, group by group
     const int nc = F.m2l_chunks, gc = F.m2l_group_chunks, ngroups = (nc + gc - 1) / gc;
     std::vector<GroupTile> t1, t2;
@@ -1292,6 +1421,57 @@ static int setup_m2l_chunks_tc(FarField &F, const std::vector<int> &chunk_slot, 
     return STK_OK;
 }
 
+// The same two stages for the FP64 path on the int8 tensor cores: Z_c = Q_d^T X_c and
+// Y_c = P_d Z_c in FP64, the digits of Z formed between the two launches.  The digits of
+// phi_hat are formed once per node and gathered by the first launch itself.
+static int setup_m2l_chunks_i8(FarField &F, const std::vector<int> &chunk_slot, const std::vector<int> &gsrc, int nn,
+                               cudaStream_t s) {
+    // Bases of up to two row blocks (laplace_p) have offsets of rank ~50: most of a 128-row tile
+    // is padding and a tile's drain takes longer than its products.  LapPGrad, 1M points, p = 10
+    // (k = 240, 1.26M pairs): M2L 4.76 ms here, 4.31 ms as batched DGEMMs; with few chunks the
+    // DGEMMs' many launches cost more (4k points: 0.17 against 0.28 ms).
+    F.i8_chunks = F.i8_pq && F.m2l_chunks > 0 && (F.m2l_rank > 2 * kI8Rows || F.m2l_chunks <= 1024);
+    if (!F.i8_chunks) return STK_OK;
+    const int k = F.m2l_rank, kb = (k + kI8Rows - 1) / kI8Rows, rmax = F.m2l_rmax;
+    const int nc = F.m2l_chunks, gc = F.m2l_group_chunks, ngroups = (nc + gc - 1) / gc;
+    std::vector<I8Tile> t1, t2;
+    std::vector<int> rank(nc), valid(nc);  // a chunk's real columns come first
+    F.i8_t1_off.assign(ngroups + 1, 0);
+    F.i8_t2_off.assign(ngroups + 1, 0);
+    for (int g = 0; g < ngroups; g++) {
+        F.i8_t1_off[g] = (int)t1.size();
+        F.i8_t2_off[g] = (int)t2.size();
+        for (int c = g * gc; c < std::min(nc, (g + 1) * gc); c++) {
+            const int sl = chunk_slot[c], r = F.m2l_r[sl], ci = c - g * gc;
+            const long long col = (long long)ci * kM2LChunk;
+            rank[c] = r;
+            int nv = 0;
+            while (nv < kM2LChunk && gsrc[(size_t)c * kM2LChunk + nv] >= 0) nv++;
+            valid[c] = nv;
+            for (int m0 = 0; m0 < r; m0 += kI8Rows)
+                t1.push_back(I8Tile{F.i8_q_blk[sl] + m0 / kI8Rows, ci, i8_kblocks(k), std::min(kI8Rows, r - m0), nv,
+                                    rmax, col * rmax + m0});
+            for (int m0 = 0; m0 < k; m0 += kI8Rows)
+                t2.push_back(I8Tile{sl * kb + m0 / kI8Rows, ci, i8_kblocks(r), std::min(kI8Rows, k - m0), nv, k,
+                                    col * k + m0});
+        }
+    }
+    F.i8_t1_off[ngroups] = (int)t1.size();
+    F.i8_t2_off[ngroups] = (int)t2.size();
+    const long long gcols = (long long)gc * kM2LChunk;
+    int rc = F.i8_z.reserve(gcols, rmax);
+    // digits of phi_hat, one row per node
+    F.i8_x.nkb = i8_kblocks(k);
+    if (!rc) rc = F.i8_x.dig.reserve(i8_row_bytes(nn, F.i8_x.nkb));
+    if (!rc) rc = F.i8_x.scale.reserve(sizeof(double) * (size_t)nn);
+    if (!rc) rc = F.i8_valid.upload(valid.data(), sizeof(int) * nc, s);
+    if (!rc) rc = F.i8_rank.upload(rank.data(), sizeof(int) * nc, s);
+    if (!rc) rc = F.i8_slot.upload(chunk_slot.data(), sizeof(int) * nc, s);
+    if (!rc) rc = F.i8_tiles1.upload(t1.data(), sizeof(I8Tile) * t1.size(), s);
+    if (!rc) rc = F.i8_tiles2.upload(t2.data(), sizeof(I8Tile) * t2.size(), s);
+    return rc;
+}
+
 // Dense M2L of the complete levels (M2LDenseLevel).  A level l >= 4 qualifies
 // when all 8^l boxes are present and its V lists hold at least 70% of 189 pairs
 // per box (periodic and deep uniform levels); the stacked factors and the work
@@ -1299,6 +1479,7 @@ static int setup_m2l_chunks_tc(FarField &F, const std::vector<int> &chunk_slot, 
 // 1e5 pairs) stay on the chunked path, so small trees build no stacked factors.
 // STKFMM_M2L_DENSE=0 turns it off.
 static int setup_m2l_dense(FarField &F, const Octree &T, int nslot, cudaStream_t s) {
+    F.dn_i8 = false;
     F.dense.clear();
     const char *env = getenv("STKFMM_M2L_DENSE");
     if (env && env[0] == '0') return STK_OK;
@@ -1413,6 +1594,19 @@ static int setup_m2l_dense(FarField &F, const Octree &T, int nslot, cudaStream_t
                                                                        (long long)k * qs_total,
                                                                        (float *)F.dn_qs32.ptr);
     FCUDA(cudaGetLastError());
+    // digits of the stacked factors for the FP64 path (int8 tensor cores) and of one level's
+    // operands, within 16 GiB
+    const int kb = (k + kI8Rows - 1) / kI8Rows;
+    int rcc_all = 1, qb = 0;
+    for (int b = 0; b < 64; b++) rcc_all = std::max(rcc_all, F.dn_rcc[b]);
+    for (int cs = 0; cs < 8; cs++) {
+        F.dn_q8_blk[cs] = qb;
+        qb += (F.dn_rs[cs] + kI8Rows - 1) / kI8Rows;
+    }
+    const size_t dig_bytes = i8_bytes((long long)qb * kI8Rows, i8_kblocks(k)) +
+                             i8_bytes(64LL * kb * kI8Rows, i8_kblocks(rcc_all)) +
+                             i8_bytes(nmax, i8_kblocks(k)) + i8_bytes(nmax, i8_kblocks(rcc_all));
+    F.dn_i8 = F.i8_pq && dig_bytes <= (16ull << 30);
     // tensor-core operands of the mixed path (3xTF32 hi / lo, K-major rows of a multiple
     // of 4 floats): Qs_c'^T per source type and Pv_{c,c'}^T per block, within 4 GiB
     F.tc = false;
@@ -1433,7 +1627,6 @@ static int setup_m2l_dense(FarField &F, const Octree &T, int nslot, cudaStream_t
             if (!rc) rc = F.tc_qa_lo.reserve(sizeof(float) * std::max<size_t>(qa, 4));
             if (!rc) rc = F.tc_pa_hi.reserve(sizeof(float) * std::max<size_t>(pa, 4));
             if (!rc) rc = F.tc_pa_lo.reserve(sizeof(float) * std::max<size_t>(pa, 4));
-            if (!rc) rc = F.tc_err.reserve(sizeof(int) * 4);
             if (rc) return rc;
             for (int cs = 0; cs < 8; cs++)
                 if (F.dn_rs[cs])
@@ -1446,12 +1639,11 @@ static int setup_m2l_dense(FarField &F, const Octree &T, int nslot, cudaStream_t
                         (const double *)F.dn_pv.ptr + F.dn_pv_off[c], k, F.dn_rv[c], (F.dn_rv[c] + 3) / 4 * 4,
                         (float *)F.tc_pa_hi.ptr + F.tc_pa_off[c], (float *)F.tc_pa_lo.ptr + F.tc_pa_off[c]);
             FCUDA(cudaGetLastError());
-            FCUDA(cudaMemsetAsync(F.tc_err.ptr, 0, sizeof(int) * 4, s));
             F.tc = true;
         }
     }
     // per block row: its slot index and its row in Z_c'
-    std::vector<int> rowq, srow;
+    std::vector<int> rowq, srow, pcol;  // pcol: the block row's column of all P_d (rmax per offset)
     for (int b = 0; b < 64; b++) {
         F.dn_row_off[b] = rowq.size();
         const int cs = b % 8;
@@ -1460,12 +1652,41 @@ static int setup_m2l_dense(FarField &F, const Octree &T, int nslot, cudaStream_t
             for (int i = 0; i < F.m2l_rt[sl]; i++) {
                 rowq.push_back(q);
                 srow.push_back(rows_s[(size_t)cs * nslot + sl] + i);
+                pcol.push_back(sl * F.m2l_rmax + i);
             }
         }
+        while (rowq.size() % 4) {  // the digit kernel reads the tables four at a time
+            rowq.push_back(0);
+            srow.push_back(0);
+            pcol.push_back(0);
+        }
     }
+    F.dn_rows = rowq.size();
     rc = F.dn_rowq.upload(rowq.data(), sizeof(int) * rowq.size(), s);
     if (!rc) rc = F.dn_srow.upload(srow.data(), sizeof(int) * srow.size(), s);
     if (rc) return rc;
+    if (F.dn_i8) {
+        rc = F.dn_q8.reserve((long long)std::max(qb, 1) * kI8Rows, k);
+        if (!rc) rc = F.dn_p8.reserve(64LL * kb * kI8Rows, rcc_all);
+        if (!rc) rc = F.dn_phi8.reserve(nmax, k);
+        if (!rc) rc = F.dn_zc8.reserve(nmax, rcc_all);
+        // the scales along K of every block row: those of its offset's P_d
+        DevBuf ksrc;
+        if (!rc) rc = F.dn_ks.reserve(sizeof(double) * 2 * F.dn_rows);
+        if (!rc) rc = ksrc.upload(pcol.data(), sizeof(int) * pcol.size(), s);
+        if (rc) return rc;
+        gather_scales_kernel<<<grid_for((long long)F.dn_rows), 256, 0, s>>>(
+            F.i8_p.up(), F.i8_p.down(), (const int *)ksrc.ptr, (long long)F.dn_rows, (double *)F.dn_ks.ptr);
+        FCUDA(cudaGetLastError());
+        for (int cs = 0; cs < 8; cs++)
+            FCUDA(i8_digits((const double *)F.dn_qs.ptr + F.dn_qs_off[cs], k, nullptr, F.dn_rs[cs], k, F.dn_q8.nkb,
+                            F.i8_q.down(), F.dn_q8.digits(F.dn_q8_blk[cs]), F.dn_q8.scales(F.dn_q8_blk[cs]), s));
+        for (int b = 0; b < 64; b++)
+            FCUDA(i8_digits_trans((const double *)F.dn_pv.ptr + F.dn_pv_off[b / 8] + (size_t)k * F.dn_pstart[b], k,
+                                  F.dn_rcc[b] ? k : 0, F.dn_rcc[b], F.dn_p8.nkb,
+                                  (const double *)F.dn_ks.ptr + F.dn_rows + F.dn_row_off[b],
+                                  F.dn_p8.digits((long long)b * kb), F.dn_p8.scales((long long)b * kb), s));
+    }
     // per level: nodes in type order and the (c, c') source tables
     std::vector<int> qidx((size_t)64 * nslot, -1);
     for (int b = 0; b < 64; b++)
@@ -1501,7 +1722,24 @@ static int setup_m2l_dense(FarField &F, const Octree &T, int nslot, cudaStream_t
                 tab[D->tab_off[b] + (size_t)pos[t - b0] * F.dn_q[b] + q] = pos[a - b0];
                 D->pairs++;
             }
+        // int8 path: the output tiles of one source type's products, all (owned) target types
+        std::vector<I8Tile> t8;
+        for (int cs = 0; cs < 8; cs++) {
+            D->tiles8_off[cs] = (int)t8.size();
+            for (int c = 0; c < 8; c++) {
+                const int b = 8 * c + cs;
+                if (!F.dn_rcc[b] || !F.dn_own[c]) continue;
+                for (int nt = 0; nt < n8 / kI8Rows; nt++)
+                    for (int mt = 0; mt < kb; mt++) {
+                        const long long col = (long long)c * n8 + nt * kI8Rows;
+                        t8.push_back(I8Tile{b * kb + mt, (int)(col / kI8Rows), i8_kblocks(F.dn_rcc[b]),
+                                            std::min(kI8Rows, k - mt * kI8Rows), kI8Rows, k, col * k + mt * kI8Rows});
+                    }
+            }
+        }
+        D->tiles8_off[8] = (int)t8.size();
         rc = D->d_nodes.upload(nodes.data(), sizeof(int) * nodes.size(), s);
+        if (!rc && F.dn_i8) rc = D->d_tiles8.upload(t8.data(), sizeof(I8Tile) * t8.size(), s);
         if (!rc) rc = D->d_tab.upload(tab.data(), sizeof(int) * tab.size(), s);
         if (rc) return rc;
         F.dense.push_back(std::move(D));
@@ -1635,6 +1873,12 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
     }
     const Octree &T = kd->tree;
     const int nn = T.num_nodes(), n = F.n, N = n * ke;
+    // set by a tensor-core product whose pipeline wait gave up
+    if (!F.tc_err.ptr) {
+        rc = F.tc_err.reserve(sizeof(int) * 4);
+        if (rc) return rc;
+        FCUDA(cudaMemsetAsync(F.tc_err.ptr, 0, sizeof(int) * 4, s));
+    }
     std::vector<double> unit = unit_surface(p);
     rc = upload_points(F.unit_surf, unit, s);
     // node levels and centres on the device
@@ -1970,6 +2214,7 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
         if (!rc) rc = F.d_m2l_ptr32[4].upload(c2f.data(), sizeof(void *) * nc, s);
         if (rc) return rc;
         rc = setup_m2l_chunks_tc(F, chunk_slot, nslot, s);
+        if (!rc) rc = setup_m2l_chunks_i8(F, chunk_slot, gsrc, nn, s);
         if (rc) return rc;
         F.m2l_flops = 0;
         for (int c = 0; c < nc; c++) F.m2l_flops += 4.0 * k * F.m2l_r[chunk_slot[c]] * kM2LChunk;
@@ -1982,6 +2227,24 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
         int maxm = 0;
         for (int l = 0; l <= T.depth(); l++) maxm = std::max(maxm, F.parent_off[l + 1] - F.parent_off[l]);
         maxm = std::max(maxm, std::max(ms, mx));
+        if (F.i8) {  // the largest right-hand operand of far_product
+            auto shape = [&](int M, int m, int K) {
+                if (rc || m <= 0 || !i8_wins(M, m, K)) return;
+                const int np = i8_gemm_parts(M, m, i8_kblocks(K));
+                rc = F.i8_b.reserve(m, K);
+                if (!rc && np > 1) rc = F.i8_parts.reserve(sizeof(double) * (size_t)np * M * m);
+            };
+            for (int l = 0; l <= T.depth(); l++) {
+                const int m = F.parent_off[l + 1] - F.parent_off[l];
+                shape(N, m, 8 * N);
+                shape(8 * N, m, N);
+                shape(N, F.s2m_level_off[l + 1] - F.s2m_level_off[l], N);
+                shape(N, F.s2l_level_off[l + 1] - F.s2l_level_off[l], N);
+            }
+            shape(k, nn, N);
+            shape(N, nn, k);
+            if (rc) return rc;
+        }
         rc = F.tmp0.reserve(sizeof(double) * (size_t)std::max(maxm, 1) * N);
         if (!rc) rc = F.tmp1.reserve(sizeof(double) * (size_t)std::max(maxm, 1) * N);
         if (rc) return rc;
@@ -2064,6 +2327,50 @@ static int m2l_dense_level_tc(FarField &F, const M2LDenseLevel &D, const double 
     return scatter_cols<float>(psi, nodes, n, k, 1.0, 1, psi_hat, s);
 }
 
+// The FP64 dense M2L of one complete level on the int8 tensor cores (stk_i8gemm.cu), source
+// type by source type: Z = Qs_c'^T Phi_c' (FP64), the digits of its gathered rows for all
+// targets at once (the scale of a target's row is that of one source type's block), and one
+// grouped launch Psi_c += Pv_{c,c'} Zc over the target types c -- 8 x 160 tiles at level 5 and
+// p = 8 where one target type's 160 would leave 136 of 148 SMs idle in the second wave.
+// RPY PXYZ, 2M points (p = 8): M2L 62.8 ms with cuBLAS DGEMMs (29.9 TFLOP/s).
+static int m2l_dense_level_i8(FarField &F, const M2LDenseLevel &D, const double *phi_hat, double *psi_hat,
+                              cudaStream_t s) {
+    const int k = F.m2l_rank, n8 = D.n8, n = 8 * n8;
+    const int *nodes = (const int *)D.d_nodes.ptr;
+    double *psi = (double *)F.dn_psi.ptr, *Z = (double *)F.dn_z.ptr;
+    int *err = (int *)F.tc_err.ptr;
+    t_launches++;
+    FCUDA(i8_digits(phi_hat, k, nodes, n, k, F.dn_phi8.nkb, F.i8_q.up(), F.dn_phi8.digits(), F.dn_phi8.scales(), s));
+    FCUDA(cudaMemsetAsync(psi, 0, sizeof(double) * (size_t)k * n, s));
+    for (int cs = 0; cs < 8; cs++) {
+        const int rs = F.dn_rs[cs], nt = D.tiles8_off[cs + 1] - D.tiles8_off[cs];
+        if (!rs || !nt) continue;
+        t_launches += 3;
+        FCUDA(i8_gemm(rs, n8, F.dn_q8.op(F.dn_q8_blk[cs]), F.dn_phi8.op((long long)cs * n8 / kI8Rows), 1.0, 0, Z, rs,
+                      nullptr, nullptr, err, s));
+        I8Gather g{};
+        g.z = Z;
+        g.ldz = rs;
+        g.tab = (const int *)D.d_tab.ptr;
+        g.rowq = (const int *)F.dn_rowq.ptr;
+        g.srow = (const int *)F.dn_srow.ptr;
+        g.kscale = (const double *)F.dn_ks.ptr;
+        while ((1 << g.lg) < n8) g.lg++;
+        for (int c = 0; c < 8; c++) {
+            const int b = 8 * c + cs;
+            g.tab_off[c] = (long long)D.tab_off[b];
+            g.row_off[c] = (long long)F.dn_row_off[b];
+            g.nq[c] = F.dn_q[b];
+            g.K[c] = F.dn_own[c] ? F.dn_rcc[b] : 0;
+        }
+        FCUDA(i8_digits_gather(g, F.dn_zc8.nkb, F.dn_zc8.digits(), F.dn_zc8.scales(), s));
+        // source types in a fixed order: deterministic
+        FCUDA(i8_grouped(F.dn_p8.op(), F.dn_zc8.op(), (const I8Tile *)D.d_tiles8.ptr + D.tiles8_off[cs], nt, 1, psi, err,
+                         s));
+    }
+    return scatter_cols<double>(psi, nodes, n, k, 1.0, 1, psi_hat, s);
+}
+
 // Dense M2L of one complete level: psi_hat[:, t] += sum over the level's V-list
 // pairs, by box parity type (M2LDenseLevel), in T = double (FP64) or float (mixed).
 template <class T>
@@ -2080,6 +2387,8 @@ static int m2l_dense_level(FarField &F, const M2LDenseLevel &D, const double *ph
     const int *nodes = (const int *)D.d_nodes.ptr;
     if constexpr (std::is_same<T, float>::value) {
         if (F.tc) return m2l_dense_level_tc(F, D, phi_hat, psi_hat, s);
+    } else {
+        if (F.dn_i8) return m2l_dense_level_i8(F, D, phi_hat, psi_hat, s);
     }
     int rc = gather_cols<double, T>(phi_hat, nodes, n, k, phi, s);
     if (rc) return rc;
@@ -2167,9 +2476,8 @@ int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const dou
                 t_launches++;
                 alpha = 1.0;
             }
-            FBLAS(cublasDgemm(F.blas, CUBLAS_OP_N, CUBLAS_OP_N, N, m, n * kc, &alpha, (const double *)F.uc2ue.ptr, N,
-                              (const double *)F.check.ptr + (size_t)a * n * kc, n * kc, &zero, Y, N));
-            int rc = scatter_cols(Y, (const int *)F.d_s2m_nodes.ptr + a, m, N, 1.0, 0, phi, s);
+            int rc = far_product(F, F.uc2ue, F.i8_uc2ue, N, n * kc, (const double *)F.check.ptr + (size_t)a * n * kc,
+                                 nullptr, m, alpha, 0, phi, (const int *)F.d_s2m_nodes.ptr + a, X, Y, s);
             if (rc) return rc;
         }
     }
@@ -2180,9 +2488,7 @@ int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const dou
         const int a = F.parent_off[l], m = F.parent_off[l + 1] - a;
         if (m == 0) continue;
         const double *Xc = phi + (size_t)T.level_begin[l + 1] * N;
-        FBLAS(cublasDgemm(F.blas, CUBLAS_OP_N, CUBLAS_OP_N, N, m, 8 * N, &one, (const double *)F.m2m.ptr, N, Xc, 8 * N,
-                          &zero, Y, N));
-        int rc = scatter_cols(Y, d_parents + a, m, N, 1.0, 0, phi, s);
+        int rc = far_product(F, F.m2m, F.i8_m2m, N, 8 * N, Xc, nullptr, m, 1.0, 0, phi, d_parents + a, nullptr, Y, s);
         if (rc) return rc;
     }
 
@@ -2195,8 +2501,11 @@ int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const dou
     // solves are much larger than the fields they stand for.  FP32-accurate products
     // (3xTF32 on the tensor cores) raised the mixed Stokes FMM's error from 2.8e-7 to
     // 5.2e-7 (V^T phi alone) and 7.3e-7 (both); p = 8, 12000 clustered points.
-    FBLAS(cublasDgemm(F.blas, CUBLAS_OP_N, CUBLAS_OP_N, k, nn, N, &one, (const double *)F.m2l_vt.ptr, k, phi, N,
-                      &zero, phi_hat, k));
+    {
+        const int rc = far_product(F, F.m2l_vt, F.i8_vt, k, N, phi, nullptr, nn, 1.0, 0, phi_hat, nullptr, nullptr,
+                                   nullptr, s);
+        if (rc) return rc;
+    }
     // gather the sources of every (offset, chunk) column, one batched GEMM over the
     // chunks, then each target sums its columns in offset order (deterministic)
     FCUDA(cudaMemsetAsync(psi_hat, 0, sizeof(double) * (size_t)nn * k, s));
@@ -2241,6 +2550,29 @@ int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const dou
             FCUDA(cudaGetLastError());
             continue;
         }
+        if (!mixed && F.i8_chunks) {
+            const int g = c0 / gc;
+            int *err = (int *)F.tc_err.ptr;
+            t_launches += 2;
+            if (c0 == 0) {
+                FCUDA(i8_digits_rows(phi_hat, k, nn, k, F.i8_x.nkb, F.i8_q.up(), (uint8_t *)F.i8_x.dig.ptr,
+                                     (double *)F.i8_x.scale.ptr, s));
+                t_launches++;
+            }
+            FCUDA(i8_grouped_gather(F.i8_q.op(), I8Rows{(const uint8_t *)F.i8_x.dig.ptr, (const double *)F.i8_x.scale.ptr, F.i8_x.nkb},
+                                    gsrc, (const I8Tile *)F.i8_tiles1.ptr + F.i8_t1_off[g],
+                                    F.i8_t1_off[g + 1] - F.i8_t1_off[g], 0, (double *)F.m2l_z.ptr, err, s));
+            FCUDA(i8_digits_blocks((const double *)F.m2l_z.ptr, rmax, ncol, (const int *)F.i8_rank.ptr + c0,
+                                   (const int *)F.i8_valid.ptr + c0, F.i8_z.nkb,
+                                   F.i8_p.up(), (const int *)F.i8_slot.ptr + c0, rmax, F.i8_z.digits(),
+                                   F.i8_z.scales(), s));
+            FCUDA(i8_grouped(F.i8_p.op(), F.i8_z.op(), (const I8Tile *)F.i8_tiles2.ptr + F.i8_t2_off[g],
+                             F.i8_t2_off[g + 1] - F.i8_t2_off[g], 0, (double *)F.m2l_y.ptr, err, s));
+            m2l_reduce_kernel<double><<<grid_for((long long)nn * k), 256, 0, s>>>(
+                (const double *)F.m2l_y.ptr, gbeg, gend, (const int *)F.d_m2l_red_col.ptr, nn, k, col0, psi_hat);
+            FCUDA(cudaGetLastError());
+            continue;
+        }
         if (mixed)
             m2l_gather_kernel<float><<<gg, 256, 0, s>>>(phi_hat, gsrc, k, ncol, (float *)F.m2l_x.ptr);
         else
@@ -2273,8 +2605,11 @@ int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const dou
                                            : m2l_dense_level<double>(F, *Dp, phi_hat, psi_hat, s);
         if (rcd) return rcd;
     }
-    FBLAS(cublasDgemm(F.blas, CUBLAS_OP_N, CUBLAS_OP_N, N, nn, k, &one, (const double *)F.m2l_e.ptr, N, psi_hat, k,
-                      &one, psi, N));
+    {
+        const int rc = far_product(F, F.m2l_e, F.i8_e, N, k, psi_hat, nullptr, nn, 1.0, 1, psi, nullptr, nullptr,
+                                   nullptr, s);
+        if (rc) return rc;
+    }
     // triply periodic: the root's far images (FP64)
     if (F.periodic && (!F.split || f->shard_rank == 0))
         FBLAS(cublasDgemv(F.blas, CUBLAS_OP_N, N, N, &one, (const double *)F.m2c_op.ptr, N, phi, 1, &one, psi, 1));
@@ -2308,9 +2643,8 @@ int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const dou
                     t_launches++;
                     alpha = 1.0;
                 }
-                FBLAS(cublasDgemm(F.blas, CUBLAS_OP_N, CUBLAS_OP_N, N, m, n * kc, &alpha, (const double *)F.dc2de.ptr,
-                                  N, (const double *)F.dcheck.ptr + (size_t)a * n * kc, n * kc, &zero, Y, N));
-                int rc = scatter_cols(Y, (const int *)F.d_s2l_nodes.ptr + a, m, N, 1.0, 1, psi, s);
+                int rc = far_product(F, F.dc2de, F.i8_dc2de, N, n * kc, (const double *)F.dcheck.ptr + (size_t)a * n * kc,
+                                     nullptr, m, alpha, 1, psi, (const int *)F.d_s2l_nodes.ptr + a, X, Y, s);
                 if (rc) return rc;
             }
     }
@@ -2322,10 +2656,9 @@ int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const dou
     for (int l = 1; l <= T.depth(); l++) {
         const int a = F.parent_off[l - 1], m = F.parent_off[l] - a;
         if (m == 0) continue;
-        int rc = gather_cols(psi, d_parents + a, m, N, X, s);
+        int rc = far_product(F, F.l2l, F.i8_l2l, 8 * N, N, psi, d_parents + a, m, 1.0, 1,
+                             psi + (size_t)T.level_begin[l] * N, nullptr, X, nullptr, s);
         if (rc) return rc;
-        FBLAS(cublasDgemm(F.blas, CUBLAS_OP_N, CUBLAS_OP_N, 8 * N, m, N, &one, (const double *)F.l2l.ptr, 8 * N, X, N,
-                          &one, psi + (size_t)T.level_begin[l] * N, 8 * N));
     }
 
     // ---- evaluation at the targets: L2T and M2T (W list) ----
@@ -2384,12 +2717,12 @@ int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const dou
 }
 
 int farfield_status(KernelData *kd) {
-    if (!kd->far || !(kd->far->tc || kd->far->tcc) || !kd->far->tc_err.ptr) return STK_OK;
+    if (!kd->far || !(kd->far->tc || kd->far->tcc || kd->far->i8) || !kd->far->tc_err.ptr) return STK_OK;
     int e = 0;
     if (cudaMemcpy(&e, kd->far->tc_err.ptr, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return STK_ERR_CUDA;
     if (e == 0) return STK_OK;
     cudaMemset(kd->far->tc_err.ptr, 0, sizeof(int));
-    fprintf(stderr, "stkfmm_b200: a tensor-core M2L GEMM stopped at a pipeline wait (code %d)\n", e);
+    fprintf(stderr, "stkfmm_b200: a tensor-core GEMM stopped at a pipeline wait (code %d)\n", e);
     return STK_ERR_CUDA;
 }
 

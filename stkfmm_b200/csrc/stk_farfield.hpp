@@ -15,6 +15,7 @@
 #include <cusolverDn.h>
 
 #include "stk_handle.hpp"
+#include "stk_i8gemm.cuh"
 #include "stk_kernel_table.hpp"
 #include "stk_p2p.cuh"
 #include "stk_tree.hpp"
@@ -54,7 +55,38 @@ struct M2LDenseLevel {
     DevBuf d_nodes;              // 8 n8 node ids, type-major (type c: [c n8, (c+1) n8))
     DevBuf d_tab;                // per (c, c'): n8 x nq source positions within type c' (-1: no pair)
     std::vector<size_t> tab_off;  // [8 c + c'] start in d_tab
+    DevBuf d_tiles8;             // int8 path: per source type its output tiles, all target types
+    int tiles8_off[9] = {};
     long long pairs = 0;
+};
+
+// Digits of an FP64 operand for the int8 tensor cores (stk_i8gemm.cuh).
+struct I8Buf {
+    DevBuf dig, scale;
+    DevBuf kscale;  // operators: up[0 .. kn), down[0 .. kn) (i8_column_scales)
+    int nkb = 0, kn = 0;
+    int reserve_kscale(int K) {
+        kn = K;
+        return kscale.reserve(sizeof(double) * 2 * (size_t)K);
+    }
+    double *up() const { return (double *)kscale.ptr; }
+    double *down() const { return (double *)kscale.ptr + kn; }
+    int reserve(long long rows, int K) {
+        nkb = i8_kblocks(K);
+        const int rc = dig.reserve(i8_bytes(rows, nkb));
+        return rc ? rc : scale.reserve(sizeof(double) * (size_t)i8_pad_rows(rows));
+    }
+    uint8_t *digits(long long blk = 0) const { return (uint8_t *)dig.ptr + (size_t)blk * nkb * kI8BlockBytes; }
+    double *scales(long long blk = 0) const { return (double *)scale.ptr + (size_t)blk * kI8Rows; }
+    // from row block blk on
+    I8Operand op(long long blk = 0) const { return {digits(blk), scales(blk), nkb}; }
+    void share(const I8Buf &o) {
+        dig.share(o.dig);
+        scale.share(o.scale);
+        kscale.share(o.kscale);
+        nkb = o.nkb;
+        kn = o.kn;
+    }
 };
 
 struct FarField {
@@ -85,6 +117,17 @@ struct FarField {
     DevBuf m2l_vt;              // V^T: k x (n ke)
     DevBuf m2l_e;               // DC2DE U: (n ke) x k
     std::vector<int> m2l_slot;  // offset code (0..342) -> block, -1 for adjacent offsets
+    // the same operators as digits: the FP64 products run on the int8 tensor cores
+    // (i8; STKFMM_F64_I8=0 or no sm_100 leaves them to cuBLAS)
+    bool i8 = false;
+    I8Buf i8_uc2ue, i8_dc2de, i8_m2m, i8_l2l, i8_vt, i8_e;
+    // chunked M2L: Q_d^T (r_d rows, from row block i8_q_blk[slot]) and P_d (k rows, from row
+    // block slot * ceil(k / 128)); i8_pq: they fit their budget
+    bool i8_pq = false;
+    I8Buf i8_q, i8_p;
+    std::vector<int> i8_q_blk;
+    I8Buf i8_b;       // digits of the right-hand operand of one product
+    DevBuf i8_parts;  // outputs of a product's K parts
     // periodic (PXY, PXYZ): DC2DE M2C of the root (far images, max |s| >= 2)
     bool periodic = false;
     int m2c_p = 0, m2c_m2x = -1, m2c_pbc = 0, m2c_ff = -1;  // what m2c_op was built for (m2c_ff: far field on)
@@ -128,6 +171,12 @@ struct FarField {
     long long tcc_q_rows = 0;
     DevBuf tcc_tiles1, tcc_tiles2;
     std::vector<int> tcc_t1_off, tcc_t2_off;  // per group: its tiles in the arrays above
+    // the FP64 path's chunked M2L on the int8 tensor cores: per chunk its rank, real columns and slot, and per group
+    // of columns the output tiles of both stages
+    bool i8_chunks = false;
+    I8Buf i8_x, i8_z;
+    DevBuf i8_rank, i8_valid, i8_slot, i8_tiles1, i8_tiles2;
+    std::vector<int> i8_t1_off, i8_t2_off;
     double m2l_flops = 0;                   // flops of one M2L (both stages, padded ranks and chunks)
     double m2l_flops_alg = 0;               // the same at the true ranks over the real pairs, plus the
                                             // two basis products (V^T phi, (DC2DE U) psi_hat)
@@ -143,6 +192,14 @@ struct FarField {
     DevBuf dn_rowq, dn_srow;                // per block row: its slot index q, its row in Z_c'
     size_t dn_row_off[64] = {};
     DevBuf dn_phi, dn_psi, dn_z, dn_zc;     // per-level work buffers (FP64 or FP32)
+    // FP64 path on the int8 tensor cores (dn_i8): Qs_c'^T from row block dn_q8_blk[c'], the
+    // blocks Pv_{c,c'} from row block (8 c + c') ceil(k / 128); per level the digits of Phi and
+    // of the gathered Z of one source type, and per source type the output tiles of all targets
+    bool dn_i8 = false;
+    I8Buf dn_q8, dn_p8, dn_phi8, dn_zc8;
+    DevBuf dn_ks;                           // scales along K per block row: up, then down
+    size_t dn_rows = 0;                     // entries of dn_rowq / dn_srow
+    int dn_q8_blk[8] = {};
     // mixed path on the tensor cores (stk_umma.cu): 3xTF32 hi / lo operands, K-major
     bool tc = false;
     DevBuf tc_qa_hi, tc_qa_lo;              // Qs_c'^T per source type: dn_rs[c'] rows of k4 floats

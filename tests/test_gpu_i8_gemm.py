@@ -1,0 +1,83 @@
+"""GPU: FP64 products on the int8 tensor cores (stk_gemm_f64_i8) against long-double sums.
+
+Tolerance.  A row is rounded to 2^-56 of its scale 2^e <= 2 max|x| at each value, and the digit
+products i + j >= 8 are dropped, about sqrt(5 K) 73^2 256^4 of 2^110 (a scaled product of the largest
+values): with normal values, max|x| < 5 rms, the whole is below 2^-55 |a||b|.  C's elements are
+|a||b| / sqrt(K) on average, and the result is rounded to FP64 (2^-53 in all, with the two
+conversions): relative L2 below 2^-53 (1 + sqrt(K) / 4)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def torch_cuda():
+    import torch
+    assert torch.cuda.is_available(), "GPU tests need a CUDA device"
+    return torch
+
+
+def product(torch, A, B, C=None):
+    """C (+)= A B^T through the C ABI; returns M x N."""
+    from stkfmm_b200 import lib
+    M, K = A.shape
+    N = B.shape[0]
+    a, b = torch.as_tensor(A, device="cuda"), torch.as_tensor(B, device="cuda")
+    out = torch.as_tensor(np.zeros((N, M)) if C is None else np.ascontiguousarray(C.T), device="cuda")
+    rc = lib().stk_gemm_f64_i8(M, N, K, a.data_ptr(), K, b.data_ptr(), K, out.data_ptr(), M, 0 if C is None else 1,
+                               torch.cuda.current_stream().cuda_stream)
+    assert rc == 0, rc
+    torch.cuda.synchronize()
+    return out.cpu().numpy().T
+
+
+# one block; ragged M, N, K; several K blocks; more tiles than one CTA's turn; two K segments
+@pytest.mark.parametrize("M,N,K", [(128, 128, 32), (1, 1, 1), (129, 257, 33), (37, 5, 640), (300, 200, 100),
+                                   (3000, 2000, 64), (130, 70, 16384), (130, 70, 16385), (64, 40, 33000)])
+def test_matches_long_double(torch_cuda, M, N, K):
+    rng = np.random.default_rng(M + 7 * N + 13 * K)
+    A, B = rng.normal(size=(M, K)), rng.normal(size=(N, K))
+    A *= np.exp2(rng.integers(-40, 40, size=(M, 1)))  # every row its own scale
+    C0 = rng.normal(size=(M, N)) * np.abs(A).max(1, keepdims=True)
+    got = product(torch_cuda, A, B)
+    sub = slice(0, M, max(1, M // 150)), slice(0, N, max(1, N // 150))
+    ref = A[sub[0]].astype(np.longdouble) @ B[sub[1]].astype(np.longdouble).T
+    rows = np.abs(A[sub[0]]).max(1, keepdims=True)
+    err = np.linalg.norm(((got[sub] - ref) / rows).astype(float)) / np.linalg.norm((ref / rows).astype(float))
+    assert err < 2.0 ** -53 * (1 + np.sqrt(K) / 4), err
+    # += adds the same product, rounded once more
+    both = product(torch_cuda, A, B, C0)
+    np.testing.assert_allclose(both, C0 + got, rtol=0, atol=float(2.0 ** -51 * np.abs(C0 + got).max()))
+    np.testing.assert_array_equal(got, product(torch_cuda, A, B))  # integer sums: the same bits again
+
+
+def test_digits_at_the_ends_of_their_range(torch_cuda):
+    """Values whose digits are all extreme (the int32 sums' bound), powers of two, exact integers, and
+    the smallest and largest magnitudes."""
+    K = 16384
+    for top in (np.nextafter(1.0, 0.0), 1.0, 127 / 128, np.nextafter(127 / 128, 0.0), 0.5):
+        big = np.full((2, K), top)
+        big[1] *= -1
+        got = product(torch_cuda, big, big)
+        assert np.allclose(got, K * top * top * np.array([[1, -1], [-1, 1]]), rtol=2.0 ** -50, atol=0), top
+    rng = np.random.default_rng(3)
+    ints = rng.integers(-2 ** 20, 2 ** 20, size=(140, 200)).astype(float)
+    np.testing.assert_array_equal(product(torch_cuda, ints, ints), ints @ ints.T)
+    for s in (2.0 ** -1000, 2.0 ** -1060, 2.0 ** 1000):
+        x = ints[:5, :64] * s
+        np.testing.assert_allclose(product(torch_cuda, x, ints[:5, :64] / 2 ** 20), (x / 2.0 ** 20) @ ints[:5, :64].T,
+                                   rtol=1e-14, atol=0 if s > 1e-305 else 2.0 ** -1000)
+
+
+def test_zero_and_non_finite_rows(torch_cuda):
+    rng = np.random.default_rng(4)
+    A, B = rng.normal(size=(6, 70)), rng.normal(size=(9, 70))
+    A[1] = 0.0
+    A[2, 3], A[3, 69], B[4, 0] = np.inf, np.nan, -np.inf
+    got = product(torch_cuda, A, B)
+    bad = np.zeros((6, 9), bool)
+    bad[2:4] = bad[:, 4] = True
+    assert not np.isfinite(got[bad]).any()
+    np.testing.assert_allclose(got[~bad], (A @ B.T)[~bad], rtol=0, atol=1e-13)
+    assert (got[1, ~bad[1]] == 0).all()
