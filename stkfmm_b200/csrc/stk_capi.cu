@@ -115,9 +115,10 @@ extern "C" int stk_ukernel_aux_dim(int uk) { return (uk < 0 || uk >= UK_COUNT) ?
 // ---------------------------------------------------------------------------
 // direct sum on device pointers
 // ---------------------------------------------------------------------------
+// add = 0: d_out = sum, 1: +=
 static int direct_device(int uk, int nsrc, const double *d_src, const double *d_val, int ntrg, const double *d_trg,
                          double *d_out, int prec, cudaStream_t stream, Workspace &ws,
-                         const double *d_trg_aux = nullptr) {
+                         const double *d_trg_aux = nullptr, int add = 1) {
     if (uk < 0 || uk >= UK_COUNT || nsrc < 0 || ntrg < 0) return STK_ERR_INVALID_ARG;
     if (prec != PREC_FP64 && prec != PREC_MIXED) return STK_ERR_INVALID_ARG;
     if (nsrc == 0 || ntrg == 0) return STK_OK;
@@ -125,45 +126,21 @@ static int direct_device(int uk, int nsrc, const double *d_src, const double *d_
     if ((uk_tvdim_host(uk) > 0) != (d_trg_aux != nullptr)) return STK_ERR_INVALID_ARG;
     int rc = ws.ensure_device();
     if (rc) return rc;
-    if ((rc = ws.begin(stream))) return rc;
-    const int sd = uk_sdim_host(uk);
-    const int rs = uk_record_stride(uk);
-    // source records
-    double *rec = ws.buf<double>(Workspace::kRec, (size_t)nsrc * rs);
-    if (!rec) return STK_ERR_CUDA;
-    STK_CUDA(launch_pack_records(nsrc, nullptr, d_src, d_val, sd, nullptr, 0, rs, rec, stream));
-    // work list: 64-target chunks x source chunks
-    std::vector<WorkItem> items;
-    std::vector<int> sbeg, send, ent;
-    build_direct_items(ntrg, nsrc, ws.num_sms(), items, sbeg, send, ent);
-    int *d_sbeg = ws.buf<int>(Workspace::kSrcBeg, sbeg.size());
-    int *d_send = ws.buf<int>(Workspace::kSrcEnd, send.size());
-    int *d_ent = ws.buf<int>(Workspace::kEnt, ent.size());
-    WorkItem *d_items = ws.buf<WorkItem>(Workspace::kItems, items.size());
-    if (!d_sbeg || !d_send || !d_ent || !d_items) return STK_ERR_CUDA;
-    STK_CUDA(cudaMemcpyAsync(d_sbeg, sbeg.data(), sbeg.size() * sizeof(int), cudaMemcpyHostToDevice, stream));
-    STK_CUDA(cudaMemcpyAsync(d_send, send.data(), send.size() * sizeof(int), cudaMemcpyHostToDevice, stream));
-    STK_CUDA(cudaMemcpyAsync(d_ent, ent.data(), ent.size() * sizeof(int), cudaMemcpyHostToDevice, stream));
-    STK_CUDA(cudaMemcpyAsync(d_items, items.data(), items.size() * sizeof(WorkItem), cudaMemcpyHostToDevice, stream));
     ListP2PArgs a{};
-    a.src_rec = rec;
-    a.src_box_begin = d_sbeg;
-    a.src_box_end = d_send;
-    a.list_ent = d_ent;
-    a.items = d_items;
-    a.n_items = (int)items.size();
-    a.counter = ws.counter();
+    a.src_xyz = d_src;
+    a.src_val = d_val;
+    a.nsrc = nsrc;
+    a.ntrg = ntrg;
+    direct_chunks(uk, prec, ntrg, nsrc, ws.num_sms(), a.src_chunk, a.n_chunk);
+    if ((rc = ws.begin(stream))) return rc;
+    if (a.n_chunk > 1 && !(a.parts = ws.buf<double>(Workspace::kParts, (size_t)a.n_chunk * ntrg * uk_tdim_host(uk))))
+        return STK_ERR_CUDA;
     a.trg_xyz = d_trg;
     a.trg_out = d_out;
     a.box_centre = nullptr;  // per-item origin: the item's first target
-    a.period = 1.0;
-    a.atomic_out = sbeg.size() > 1 ? 1 : 0;
     a.trg_aux = d_trg_aux;
-    STK_CUDA(launch_list_p2p(uk, prec, a, ws.num_sms(), stream));
-    // the host vectors may die at return: copies from pageable memory have been
-    // staged by the time cudaMemcpyAsync returns, so no host wait is needed
-    if ((rc = ws.end(stream))) return rc;
-    return STK_OK;
+    STK_CUDA(launch_direct_p2p(uk, prec, a, add, ws.num_sms(), stream));
+    return ws.end(stream);
 }
 
 extern "C" int stk_ukernel_direct_device(int ukernel, int nsrc, const double *d_src_coord, const double *d_src_value,
@@ -204,9 +181,9 @@ extern "C" int stk_evaluate_kernel_device(unsigned kernel, unsigned ppkernel, in
                          (cudaStream_t)stream, Workspace::thread_local_ws());
 }
 
-// Host-array direct sum for micro-kernel uk (accumulate).  Targets are sorted in
-// Morton order before upload so that 64-target items are compact (tight local
-// origins for the mixed path); results are scattered back to the caller's order.
+// Host-array direct sum for micro-kernel uk (accumulate).  Mixed precision: the targets are
+// sorted in Morton order before upload so that 64-target items are compact (tight local
+// origins); results are scattered back to the caller's order.
 static int direct_host(int uk, int nsrc, const double *src, const double *val, int ntrg, const double *trg,
                        double *out, int prec) {
     if (uk < 0 || uk >= UK_COUNT || nsrc < 0 || ntrg < 0 || uk_tvdim_host(uk) > 0) return STK_ERR_INVALID_ARG;
@@ -217,26 +194,43 @@ static int direct_host(int uk, int nsrc, const double *src, const double *val, i
     int rc = ws.ensure_device();
     if (rc) return rc;
     cudaStream_t s = ws.stream();
-    const int sd = uk_sdim_host(uk), td = uk_tdim_host(uk);
+    const size_t sd = uk_sdim_host(uk), td = uk_tdim_host(uk);
     std::vector<int> order;
     std::vector<double> trg_sorted;
-    morton_order(trg, ntrg, order, trg_sorted);
-    double *d_src = ws.buf<double>(Workspace::kHostSrc, (size_t)nsrc * 3);
-    double *d_val = ws.buf<double>(Workspace::kHostVal, (size_t)nsrc * sd);
-    double *d_trg = ws.buf<double>(Workspace::kHostTrg, (size_t)ntrg * 3);
-    double *d_out = ws.buf<double>(Workspace::kHostOut, (size_t)ntrg * td);
-    if (!d_src || !d_val || !d_trg || !d_out) return STK_ERR_CUDA;
-    STK_CUDA(cudaMemcpyAsync(d_src, src, sizeof(double) * 3 * nsrc, cudaMemcpyHostToDevice, s));
-    STK_CUDA(cudaMemcpyAsync(d_val, val, sizeof(double) * sd * nsrc, cudaMemcpyHostToDevice, s));
-    STK_CUDA(cudaMemcpyAsync(d_trg, trg_sorted.data(), sizeof(double) * 3 * ntrg, cudaMemcpyHostToDevice, s));
-    STK_CUDA(cudaMemsetAsync(d_out, 0, sizeof(double) * td * ntrg, s));
-    rc = direct_device(uk, nsrc, d_src, d_val, ntrg, d_trg, d_out, prec, s, ws);
+    if (prec == PREC_MIXED) {
+        morton_order(trg, ntrg, order, trg_sorted);
+        trg = trg_sorted.data();
+    }
+    // sources, values and targets as one device array; through one pinned buffer and one copy
+    // while they fit its bound (a call of a few hundred points is mostly copies: three pageable
+    // ones took ~25 us more)
+    const size_t ns3 = 3 * (size_t)nsrc, nv = sd * nsrc, nt3 = 3 * (size_t)ntrg, no = td * ntrg;
+    double *d_in = ws.buf<double>(Workspace::kHostIn, ns3 + nv + nt3);
+    double *d_out = ws.buf<double>(Workspace::kHostOut, no);
+    if (!d_in || !d_out) return STK_ERR_CUDA;
+    double *pin = static_cast<double *>(ws.pinned((ns3 + nv + nt3 + no) * sizeof(double)));
+    if (pin) {
+        std::memcpy(pin, src, ns3 * sizeof(double));
+        std::memcpy(pin + ns3, val, nv * sizeof(double));
+        std::memcpy(pin + ns3 + nv, trg, nt3 * sizeof(double));
+        STK_CUDA(cudaMemcpyAsync(d_in, pin, (ns3 + nv + nt3) * sizeof(double), cudaMemcpyHostToDevice, s));
+    } else {
+        STK_CUDA(cudaMemcpyAsync(d_in, src, ns3 * sizeof(double), cudaMemcpyHostToDevice, s));
+        STK_CUDA(cudaMemcpyAsync(d_in + ns3, val, nv * sizeof(double), cudaMemcpyHostToDevice, s));
+        STK_CUDA(cudaMemcpyAsync(d_in + ns3 + nv, trg, nt3 * sizeof(double), cudaMemcpyHostToDevice, s));
+    }
+    rc = direct_device(uk, nsrc, d_in, d_in + ns3, ntrg, d_in + ns3 + nv, d_out, prec, s, ws, nullptr, 0);
     if (rc) return rc;
-    std::vector<double> res((size_t)ntrg * td);
-    STK_CUDA(cudaMemcpyAsync(res.data(), d_out, sizeof(double) * td * ntrg, cudaMemcpyDeviceToHost, s));
+    std::vector<double> res(pin ? 0 : no);
+    double *r = pin ? pin + ns3 + nv + nt3 : res.data();
+    STK_CUDA(cudaMemcpyAsync(r, d_out, no * sizeof(double), cudaMemcpyDeviceToHost, s));
     STK_CUDA(cudaStreamSynchronize(s));
-    for (int i = 0; i < ntrg; i++)
-        for (int k = 0; k < td; k++) out[(size_t)order[i] * td + k] += res[(size_t)i * td + k];
+    if (order.empty()) {
+        for (size_t i = 0; i < no; i++) out[i] += r[i];
+    } else {
+        for (int i = 0; i < ntrg; i++)
+            for (size_t k = 0; k < td; k++) out[(size_t)order[i] * td + k] += r[(size_t)i * td + k];
+    }
     return STK_OK;
 }
 

@@ -35,6 +35,7 @@
 //    MUFU rsqrt + one Newton step; each tile's FP32 partial sums are added into
 //    Kahan-compensated FP32 accumulators.
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 #include "stk_p2p.cuh"
@@ -165,9 +166,19 @@ template <int RS> struct RawStride {
     static constexpr int value = ((RS / 2) & 1) ? RS : RS + 2;
 };
 
-template <int UK, bool MIXED>
+// One component of a source record from the caller's own arrays (8 bytes, no alignment
+// beyond a double's).
+__device__ __forceinline__ void cp_async8(void *smem, const void *gmem) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+
+// DIRECT: a direct sum (launch_direct_p2p).  Item it is targets [64 c, ...) against source chunk
+// k, c the fast index: the warps of an SM read the same sources.  Sources come straight from
+// the caller's arrays, and there are no lists to read or to set up.
+template <int UK, bool MIXED, bool DIRECT>
 __global__ void __launch_bounds__(Cta<MIXED>::threads, MinBlocks<UK, MIXED>::value)
-    list_p2p_kernel(const ListP2PArgs a) {
+    list_p2p_kernel(const __grid_constant__ ListP2PArgs a) {
     constexpr int kWarpsPerCta = Cta<MIXED>::warps;
     using K = Uk<UK>;
     constexpr int TDIM = K::TDIM;
@@ -201,12 +212,25 @@ __global__ void __launch_bounds__(Cta<MIXED>::threads, MinBlocks<UK, MIXED>::val
     int *s_src = sg_src[wid];
     int *s_code = sg_code[wid];
 
-    for (;;) {
+    for (int turn = 0;; turn++) {
         int it = 0;
-        if (lane == 0) it = (int)atomicAdd(a.counter, 1u);
-        it = __shfl_sync(kFull, it, 0);
-        if (it >= a.n_items) break;
-        const WorkItem w = a.items[it];
+        WorkItem w;
+        if constexpr (DIRECT) {
+            it = (turn * gridDim.x + blockIdx.x) * kWarpsPerCta + wid;  // equal items: dealt in turn
+            if (it >= a.n_items) break;
+            const int nc = (a.ntrg + 63) >> 6, c = it % nc;
+            w.trg_box = c;
+            w.t0 = 64 * c;
+            w.nt = min(64, a.ntrg - w.t0);
+            w.glog = w.nt > 32 ? 0 : min(5, __clz(w.nt - 1) - 26);  // 2^glog <= 64 / nt
+            w.e0 = it / nc;
+            w.e1 = w.e0 + 1;
+        } else {
+            if (lane == 0) it = (int)atomicAdd(a.counter, 1u);
+            it = __shfl_sync(kFull, it, 0);
+            if (it >= a.n_items) break;
+            w = a.items[it];
+        }
         // the host sizes glog for 64 slots; 4 slots per lane give twice the lanes per target
         const int glog = TPL == 4 ? min(5, w.glog + 1) : w.glog;
         const int g = 1 << glog;
@@ -311,7 +335,7 @@ __global__ void __launch_bounds__(Cta<MIXED>::threads, MinBlocks<UK, MIXED>::val
         for (int ec = w.e0; ec < w.e1; ec += 32) {
             const int ne = min(32, w.e1 - ec);
             int sz = 0, sbeg = 0, code = kShiftNoneCode;
-            if (lane < ne) {
+            if constexpr (!DIRECT) if (lane < ne) {
                 const int ent = a.list_ent[ec + lane];
                 const int sb = ent >> 5;
                 code = ent & 31;
@@ -321,19 +345,25 @@ __global__ void __launch_bounds__(Cta<MIXED>::threads, MinBlocks<UK, MIXED>::val
                 // unless the lists guarantee coincidence only in the unshifted own box)
                 if (!a.coincident_own_box || sb == w.trg_box || code != kShiftNoneCode) code |= kMayCoincide;
             }
-            int incl = sz;
+            int total;
+            if constexpr (DIRECT) {
+                sbeg = w.e0 * a.src_chunk;
+                total = min(a.src_chunk, a.nsrc - sbeg);
+            } else {
+                int incl = sz;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(kFull, incl, o);
-                if (lane >= o) incl += v;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(kFull, incl, o);
+                    if (lane >= o) incl += v;
+                }
+                total = __shfl_sync(kFull, incl, 31);
+                __syncwarp();  // the previous chunk's segment table is no longer read
+                s_end[lane] = lane < ne ? incl : 0x7fffffff;
+                s_src[lane] = sbeg - (incl - sz);
+                s_code[lane] = code;
+                __syncwarp();
+                if (total == 0) continue;
             }
-            const int total = __shfl_sync(kFull, incl, 31);
-            __syncwarp();  // the previous chunk's segment table is no longer read
-            s_end[lane] = lane < ne ? incl : 0x7fffffff;
-            s_src[lane] = sbeg - (incl - sz);
-            s_code[lane] = code;
-            __syncwarp();
-            if (total == 0) continue;
 
             // per-lane cursor into the segment table; positions only grow
             int seg = 0;
@@ -344,7 +374,16 @@ __global__ void __launch_bounds__(Cta<MIXED>::threads, MinBlocks<UK, MIXED>::val
             // or nothing past the stream's end; one commit group per call either way,
             // so every lane counts the same groups
             auto fetch = [&](int p, int z, int &zs) {
-                if (p < total) {
+                if constexpr (DIRECT) {
+                    if (p < total) {
+                        const double *x = a.src_xyz + 3 * (size_t)(sbeg + p), *v = a.src_val + (size_t)K::SDIM * (sbeg + p);
+                        double *dst = traw[wid][z][lane];
+#pragma unroll
+                        for (int q = 0; q < 3; q++) cp_async8(dst + q, x + q);
+#pragma unroll
+                        for (int q = 0; q < K::SDIM; q++) cp_async8(dst + 3 + q, v + q);
+                    }
+                } else if (p < total) {
                     while (p >= s_end[seg]) seg++;
                     const double *src = a.src_rec + (size_t)(s_src[seg] + p) * RS;
                     double *dst = traw[wid][z][lane];
@@ -379,13 +418,17 @@ __global__ void __launch_bounds__(Cta<MIXED>::threads, MinBlocks<UK, MIXED>::val
                         x[0] = rn[0];
                         x[1] = rn[1];
                         x[2] = rn[2];
-                        const int cdf = s_code[zseg[0]];
-                        may_coincide = cdf & kMayCoincide;
-                        const int cd = cdf & 31;
-                        if (cd != kShiftNoneCode) {  // periodic image
-                            x[0] += (cd % 3 - 1) * a.period;
-                            x[1] += ((cd / 3) % 3 - 1) * a.period;
-                            x[2] += (cd / 9 - 1) * a.period;
+                        if constexpr (DIRECT) {
+                            may_coincide = 1;
+                        } else {
+                            const int cdf = s_code[zseg[0]];
+                            may_coincide = cdf & kMayCoincide;
+                            const int cd = cdf & 31;
+                            if (cd != kShiftNoneCode) {  // periodic image
+                                x[0] += (cd % 3 - 1) * a.period;
+                                x[1] += ((cd / 3) % 3 - 1) * a.period;
+                                x[2] += (cd / 9 - 1) * a.period;
+                            }
                         }
                         K::stage(rn + 3, v);
                     } else {
@@ -512,10 +555,14 @@ STK_UNROLL(STK_P2P_UNROLL_FP64)
             for (int h = 0; h < TPL; h++) {
                 if (!act[h]) continue;
                 double *dst = a.trg_out + (size_t)tt[h] * TDIM;
+                if constexpr (DIRECT)
+                    if (a.parts) dst = a.parts + ((size_t)w.e0 * a.ntrg + tt[h]) * TDIM;
 #pragma unroll
                 for (int k = 0; k < TDIM; k++) {
                     const double val = K::SCALE * K::comp_scale(k) * o[h][k];
-                    if (a.atomic_out)
+                    if (DIRECT && !a.atomic_out)  // atomic_out: add (to the caller's values)
+                        dst[k] = val;
+                    else if (!DIRECT && a.atomic_out)
                         atomicAdd(dst + k, val);
                     else
                         dst[k] += val;
@@ -525,28 +572,51 @@ STK_UNROLL(STK_P2P_UNROLL_FP64)
     }
 }
 
-template <int UK, bool MIXED>
-cudaError_t launch_impl(const ListP2PArgs &a, int num_sms, cudaStream_t stream) {
+// resident CTAs per SM of a kernel instance
+template <int UK, bool MIXED, bool DIRECT> cudaError_t occupancy(int &n) {
     static int blocks_per_sm = 0;
     if (blocks_per_sm == 0) {
-        cudaError_t err =
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, list_p2p_kernel<UK, MIXED>,
-                                                          Cta<MIXED>::threads, 0);
+        int v = 0;
+        const cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, list_p2p_kernel<UK, MIXED, DIRECT>,
+                                                                              Cta<MIXED>::threads, 0);
         if (err != cudaSuccess) return err;
-        if (blocks_per_sm < 1) blocks_per_sm = 1;
+        blocks_per_sm = std::max(v, 1);
     }
+    n = blocks_per_sm;
+    return cudaSuccess;
+}
+
+template <int UK, bool MIXED, bool DIRECT>
+cudaError_t launch_impl(const ListP2PArgs &a, int num_sms, cudaStream_t stream) {
+    int blocks_per_sm = 1;
+    cudaError_t err = occupancy<UK, MIXED, DIRECT>(blocks_per_sm);
+    if (err != cudaSuccess) return err;
     constexpr int kWarpsPerCta = Cta<MIXED>::warps;
     long long want = ((long long)a.n_items + kWarpsPerCta - 1) / kWarpsPerCta;
     int grid = (int)std::max(1LL, std::min<long long>((long long)num_sms * blocks_per_sm, want));
-    cudaError_t err = cudaMemsetAsync(a.counter, 0, sizeof(unsigned int), stream);
-    if (err != cudaSuccess) return err;
-    list_p2p_kernel<UK, MIXED><<<grid, Cta<MIXED>::threads, 0, stream>>>(a);
+    if (!DIRECT && (err = cudaMemsetAsync(a.counter, 0, sizeof(unsigned int), stream)) != cudaSuccess) return err;
+    list_p2p_kernel<UK, MIXED, DIRECT><<<grid, Cta<MIXED>::threads, 0, stream>>>(a);
     return cudaGetLastError();
 }
 
-template <int UK>
-cudaError_t launch_prec(int prec, const ListP2PArgs &a, int num_sms, cudaStream_t stream) {
-    return prec == PREC_MIXED ? launch_impl<UK, true>(a, num_sms, stream) : launch_impl<UK, false>(a, num_sms, stream);
+// f(integral_constant<int, UK>) for the micro-kernel uk
+template <int UK = 0, class F> cudaError_t with_uk(int uk, const F &f) {
+    if constexpr (UK < UK_COUNT) {
+        if (uk == UK) return f(std::integral_constant<int, UK>());
+        return with_uk<UK + 1>(uk, f);
+    } else {
+        return cudaErrorInvalidValue;
+    }
+}
+
+// out[i] (=|+=) the chunks' sums, in order
+__global__ void sum_chunks_kernel(const double *__restrict__ parts, int n_chunk, long long n, int add,
+                                  double *__restrict__ out) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        double v = parts[i];
+        for (int k = 1; k < n_chunk; k++) v += parts[k * n + i];
+        out[i] = add ? out[i] + v : v;
+    }
 }
 
 __global__ void pack_records_kernel(int n, const int *__restrict__ perm, const double *__restrict__ xyz,
@@ -587,42 +657,70 @@ int uk_record_stride(int uk) { return (3 + uk_sdim(uk) + 1) & ~1; }
 
 cudaError_t launch_list_p2p(int uk, int prec, const ListP2PArgs &a, int num_sms, cudaStream_t stream) {
     if (a.n_items <= 0) return cudaSuccess;
-    switch (uk) {
-    case UK_LAPLACE_P: return launch_prec<UK_LAPLACE_P>(prec, a, num_sms, stream);
-    case UK_LAPLACE_PGRAD: return launch_prec<UK_LAPLACE_PGRAD>(prec, a, num_sms, stream);
-    case UK_LAPLACE_DIPOLEP: return launch_prec<UK_LAPLACE_DIPOLEP>(prec, a, num_sms, stream);
-    case UK_LAPLACE_DIPOLEPGRAD: return launch_prec<UK_LAPLACE_DIPOLEPGRAD>(prec, a, num_sms, stream);
-    case UK_STOKES_VEL: return launch_prec<UK_STOKES_VEL>(prec, a, num_sms, stream);
-    case UK_RPY_U: return launch_prec<UK_RPY_U>(prec, a, num_sms, stream);
-    case UK_RPY_ULAPU: return launch_prec<UK_RPY_ULAPU>(prec, a, num_sms, stream);
-    case UK_STK_ULAPU: return launch_prec<UK_STK_ULAPU>(prec, a, num_sms, stream);
-    case UK_STOKES_REGVEL: return launch_prec<UK_STOKES_REGVEL>(prec, a, num_sms, stream);
-    case UK_STOKES_PVEL: return launch_prec<UK_STOKES_PVEL>(prec, a, num_sms, stream);
-    case UK_STOKES_DOUBLEPVEL: return launch_prec<UK_STOKES_DOUBLEPVEL>(prec, a, num_sms, stream);
-    case UK_LAPLACE_SLDL_PGRAD: return launch_prec<UK_LAPLACE_SLDL_PGRAD>(prec, a, num_sms, stream);
-    case UK_STOKES_SLDL_PVEL: return launch_prec<UK_STOKES_SLDL_PVEL>(prec, a, num_sms, stream);
-    case UK_LAPLACE_SLDL_P: return launch_prec<UK_LAPLACE_SLDL_P>(prec, a, num_sms, stream);
-    case UK_LAPLACE_PGRADGRAD: return launch_prec<UK_LAPLACE_PGRADGRAD>(prec, a, num_sms, stream);
-    case UK_LAPLACE_DIPOLEPGRADGRAD: return launch_prec<UK_LAPLACE_DIPOLEPGRADGRAD>(prec, a, num_sms, stream);
-    case UK_LAPLACE_QUADP: return launch_prec<UK_LAPLACE_QUADP>(prec, a, num_sms, stream);
-    case UK_LAPLACE_QUADPGRADGRAD: return launch_prec<UK_LAPLACE_QUADPGRADGRAD>(prec, a, num_sms, stream);
-    case UK_STOKES_PVELGRAD: return launch_prec<UK_STOKES_PVELGRAD>(prec, a, num_sms, stream);
-    case UK_STOKES_DOUBLEPVELGRAD: return launch_prec<UK_STOKES_DOUBLEPVELGRAD>(prec, a, num_sms, stream);
-    case UK_STOKES_PVELLAPLACIAN: return launch_prec<UK_STOKES_PVELLAPLACIAN>(prec, a, num_sms, stream);
-    case UK_STOKES_DOUBLELAPLACIAN: return launch_prec<UK_STOKES_DOUBLELAPLACIAN>(prec, a, num_sms, stream);
-    case UK_STOKES_TRACTION: return launch_prec<UK_STOKES_TRACTION>(prec, a, num_sms, stream);
-    case UK_STOKES_DOUBLETRACTION: return launch_prec<UK_STOKES_DOUBLETRACTION>(prec, a, num_sms, stream);
-    case UK_STOKES_REGFTVEL: return launch_prec<UK_STOKES_REGFTVEL>(prec, a, num_sms, stream);
-    case UK_STOKES_REGFTVELOMEGA: return launch_prec<UK_STOKES_REGFTVELOMEGA>(prec, a, num_sms, stream);
-    case UK_STOKES_VELOMEGA: return launch_prec<UK_STOKES_VELOMEGA>(prec, a, num_sms, stream);
-    case UK_REGVEL_ADJ_SRC:
-        if (!a.trg_aux) return cudaErrorInvalidValue;
-        return launch_prec<UK_REGVEL_ADJ_SRC>(prec, a, num_sms, stream);
-    case UK_REGVEL_ADJ_TRG:
-        if (!a.trg_aux) return cudaErrorInvalidValue;
-        return launch_prec<UK_REGVEL_ADJ_TRG>(prec, a, num_sms, stream);
-    default: return cudaErrorInvalidValue;
+    if (uk >= 0 && uk < UK_COUNT && uk_tvdim(uk) > 0 && !a.trg_aux) return cudaErrorInvalidValue;
+    return with_uk(uk, [&](auto id) {
+        constexpr int UK = decltype(id)::value;
+        return prec == PREC_MIXED ? launch_impl<UK, true, false>(a, num_sms, stream)
+                                  : launch_impl<UK, false, false>(a, num_sms, stream);
+    });
+}
+
+// FP64: chunks so that the equal items fill whole turns of the resident warps.  An item costs
+// its sources plus ~40 more (first tile's latency, output), so many short items only pay where
+// the targets alone leave warps idle: 300 x 400 points run as 65 items of 32 sources.
+// Mixed: at least 256 sources per item, as its Kahan sums are formed per item.
+void direct_chunks(int uk, int prec, int ntrg, int nsrc, int num_sms, int &chunk, int &n_chunk) {
+    const long long nc = std::max(1, (ntrg + 63) / 64);
+    num_sms = std::max(num_sms, 1);
+    if (prec == PREC_MIXED) {
+        n_chunk = (int)std::max(1LL, ((long long)num_sms * 64 + nc - 1) / nc);
+        n_chunk = std::min(n_chunk, std::max(1, nsrc / 256));
+        chunk = ((nsrc + n_chunk - 1) / n_chunk + 31) / 32 * 32;
+        n_chunk = (nsrc + chunk - 1) / chunk;
+        return;
     }
+    int per_sm = 8;
+    with_uk(uk, [&](auto id) { return occupancy<decltype(id)::value, false, true>(per_sm); });
+    const double slots = (double)num_sms * per_sm;
+    double best = 0.0;
+    chunk = (nsrc + 31) / 32 * 32;
+    n_chunk = 1;
+    // up to eight turns of the warps, tiles of 32 sources
+    const long long most = std::min<long long>((nsrc + 31) / 32, std::max<long long>(1, (long long)(8 * slots) / nc));
+    for (long long n = 1; n <= most; n = n < 64 ? n + 1 : n + n / 16) {
+        const int c = (int)((((nsrc + n - 1) / n) + 31) / 32 * 32);
+        const long long k = (nsrc + c - 1) / c;
+        const double items = (double)nc * k;
+        // useful share of the time: ragged sources, ragged last turn, cost per item
+        const double eff = (double)nsrc / ((double)k * c) * items / (std::ceil(items / slots) * slots) * c / (c + 40.0);
+        if (eff > best * 1.001) {
+            best = eff;
+            chunk = c;
+            n_chunk = (int)k;
+        }
+    }
+}
+
+cudaError_t launch_direct_p2p(int uk, int prec, const ListP2PArgs &args, int add, int num_sms, cudaStream_t stream) {
+    if (args.nsrc <= 0 || args.ntrg <= 0) return cudaSuccess;
+    if (uk < 0 || uk >= UK_COUNT || (uk_tvdim(uk) > 0) != (args.trg_aux != nullptr)) return cudaErrorInvalidValue;
+    const bool split = args.n_chunk > 1;
+    const long long items = (long long)((args.ntrg + 63) / 64) * args.n_chunk;
+    if ((split && !args.parts) || items > 0x7fffffffll) return cudaErrorInvalidValue;
+    ListP2PArgs a = args;
+    a.n_items = (int)items;
+    if (!split) a.parts = nullptr;
+    a.atomic_out = !split && add;
+    cudaError_t e = with_uk(uk, [&](auto id) {
+        constexpr int UK = decltype(id)::value;
+        return prec == PREC_MIXED ? launch_impl<UK, true, true>(a, num_sms, stream)
+                                  : launch_impl<UK, false, true>(a, num_sms, stream);
+    });
+    if (e != cudaSuccess || !split) return e;
+    const long long n = (long long)a.ntrg * uk_tdim(uk);
+    sum_chunks_kernel<<<(int)std::min<long long>((n + 255) / 256, 148 * 16), 256, 0, stream>>>(a.parts, a.n_chunk, n, add,
+                                                                                             a.trg_out);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_pack_records(int n, const int *perm, const double *xyz, const double *v1, int d1,

@@ -39,6 +39,11 @@ struct ListP2PArgs {
                                // entry of the target's own box (lists of one octree over both
                                // point sets); the mixed path then skips the coincidence mask
                                // elsewhere.  0: every pair is masked.
+    // direct sums only (launch_direct_p2p): all sources against all targets
+    const double *src_xyz, *src_val;  // 3 and SDIM doubles per source
+    int nsrc, ntrg;
+    int src_chunk, n_chunk;  // source points per chunk (a multiple of 32), chunks
+    double *parts;           // outputs of each chunk, ntrg x TDIM each (null: one chunk, added to trg_out)
 };
 
 // Record stride (doubles) for a micro-kernel: 3 coordinates + SDIM values,
@@ -51,6 +56,15 @@ double uk_scale_host(int uk);
 
 // Launch the list kernel for micro-kernel `uk` with the given precision.
 cudaError_t launch_list_p2p(int uk, int prec, const ListP2PArgs &a, int num_sms, cudaStream_t stream);
+
+// Direct sum of all sources at all targets: items of 64 targets x one chunk of sources, which
+// the kernel derives from its block index; raw source arrays, nothing to set up.  With several
+// chunks each writes its own sums and a second kernel adds them up in order (repeats give the
+// same bits).  direct_chunks: sources per chunk (a multiple of 32) and the number of chunks.
+void direct_chunks(int uk, int prec, int ntrg, int nsrc, int num_sms, int &chunk, int &n_chunk);
+// a: src_xyz, src_val, nsrc, ntrg, src_chunk, n_chunk, parts (n_chunk > 1), trg_xyz, trg_aux and
+// trg_out; add = 0: trg_out = sum, 1: +=
+cudaError_t launch_direct_p2p(int uk, int prec, const ListP2PArgs &a, int add, int num_sms, cudaStream_t stream);
 
 // rec[i] = (xyz[perm[i]], v1[perm[i]] (d1 values), v2[perm[i]] (d2 values), 0 padding)
 // perm may be null (identity).  v2 may be null (d2 = 0).  Coordinates are

@@ -112,6 +112,24 @@ void *Workspace::raw(int slot, size_t bytes) {
     return cur_->ptr[slot];
 }
 
+void *Workspace::pinned(size_t bytes) {
+    if (bytes > kPinnedBytes) return nullptr;
+    if (pin_cap_ < bytes) {
+        size_t want = 64u << 10;
+        while (want < bytes) want *= 2;
+        if (pin_) cudaFreeHost(pin_);  // its last call has waited for its copies
+        pin_ = nullptr;
+        pin_cap_ = 0;
+        if (cudaHostAlloc(&pin_, want, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            pin_ = nullptr;
+            return nullptr;
+        }
+        pin_cap_ = want;
+    }
+    return pin_;
+}
+
 unsigned int *Workspace::counter() { return cur_ ? cur_->counter : nullptr; }
 int Workspace::num_sms() { return cur_ ? cur_->sms : 1; }
 cudaStream_t Workspace::stream() { return cur_ ? cur_->stream : nullptr; }
@@ -124,35 +142,6 @@ static inline int lanes_log2(int m) {
     int glog = 0;
     while (glog < 5 && (m << (glog + 1)) <= kItemTargets) glog++;
     return glog;
-}
-
-void build_direct_items(int ntrg, int nsrc, int num_sms, std::vector<WorkItem> &items, std::vector<int> &src_begin,
-                        std::vector<int> &src_end, std::vector<int> &ent) {
-    const int nchunk = (ntrg + kItemTargets - 1) / kItemTargets;
-    // enough items to fill every warp slot several times over, but source
-    // chunks of at least 256 points
-    const long long want_items = (long long)std::max(num_sms, 1) * 64;
-    int nsc = (int)std::max(1LL, (want_items + nchunk - 1) / nchunk);
-    nsc = std::min(nsc, std::max(1, nsrc / 256));
-    int sc = (nsrc + nsc - 1) / nsc;
-    sc = (sc + 31) / 32 * 32;
-    nsc = (nsrc + sc - 1) / sc;
-    src_begin.resize(nsc);
-    src_end.resize(nsc);
-    ent.resize(nsc);
-    for (int k = 0; k < nsc; k++) {
-        src_begin[k] = k * sc;
-        src_end[k] = std::min(nsrc, (k + 1) * sc);
-        ent[k] = (k << 5) | kShiftNone;
-    }
-    items.clear();
-    items.reserve((size_t)nchunk * nsc);
-    // full chunks first (largest cost), the ragged last chunk at the end
-    for (int c = 0; c < nchunk; c++) {
-        const int t0 = kItemTargets * c;
-        const int m = std::min(kItemTargets, ntrg - t0);
-        for (int k = 0; k < nsc; k++) items.push_back({c, t0, m, lanes_log2(m), k, k + 1});
-    }
 }
 
 void build_list_items(int n_trg_box, const int *trg_begin, const int *trg_end, const int *list_off,

@@ -18,7 +18,7 @@ namespace stk {
 // to the next thread when its thread ends and is never freed before exit.
 class Workspace {
   public:
-    enum Slot { kRec, kSrcBeg, kSrcEnd, kEnt, kItems, kHostSrc, kHostVal, kHostTrg, kHostOut, kNumSlots };
+    enum Slot { kRec, kSrcBeg, kSrcEnd, kEnt, kItems, kParts, kHostIn, kHostOut, kNumSlots };
     static Workspace &thread_local_ws();
     ~Workspace();
     int ensure_device();  // STK_OK, STK_ERR_NO_DEVICE or STK_ERR_CUDA
@@ -29,6 +29,10 @@ class Workspace {
     int begin(cudaStream_t s);
     int end(cudaStream_t s);
     template <class T> T *buf(int slot, size_t n) { return static_cast<T *>(raw(slot, n * sizeof(T))); }
+    // pinned host memory for calls that wait for their result, up to kPinnedBytes per thread
+    // (null beyond, or where none can be had)
+    static constexpr size_t kPinnedBytes = 8u << 20;
+    void *pinned(size_t bytes);
     unsigned int *counter();
     int num_sms();
     cudaStream_t stream();
@@ -45,12 +49,10 @@ class Workspace {
     };
     std::map<int, Dev> devs_;
     Dev *cur_ = nullptr;
+    void *pin_ = nullptr;
+    size_t pin_cap_ = 0;
     void *raw(int slot, size_t bytes);
 };
-
-// Direct sum as a list problem: 64-target chunks x source chunks.
-void build_direct_items(int ntrg, int nsrc, int num_sms, std::vector<WorkItem> &items, std::vector<int> &src_begin,
-                        std::vector<int> &src_end, std::vector<int> &ent);
 
 // Cost-sorted work items for an explicit list; pairs = exact (target, source point) pair count.
 // balance_warps > 0: boxes with many sources get smaller target chunks, so that no
