@@ -279,8 +279,13 @@ static int p2p_lists(int ukernel, int precision, int n_trg_box, const int *trg_b
     cudaStream_t s = (cudaStream_t)stream;
     if ((rc = ws.begin(s))) return rc;
     std::vector<WorkItem> items;
-    long long pairs = 0;
-    build_list_items(n_trg_box, trg_begin, trg_end, list_off, list_ent, src_begin, src_end, items, pairs);
+    std::vector<PartGroup> groups;
+    long long pairs = 0, slots = 0;
+    if (precision == PREC_MIXED)
+        build_list_items(n_trg_box, trg_begin, trg_end, list_off, list_ent, src_begin, src_end, items, pairs);
+    else
+        build_split_items(n_trg_box, trg_begin, trg_end, list_off, list_ent, src_begin, src_end, ws.num_sms() * 15, items,
+                          groups, slots);
     if (items.empty()) return STK_OK;
     const int sd = uk_sdim_host(ukernel), rs = uk_record_stride(ukernel);
     double *rec = ws.buf<double>(Workspace::kRec, (size_t)std::max(nsrc, 1) * rs);
@@ -288,8 +293,10 @@ static int p2p_lists(int ukernel, int precision, int n_trg_box, const int *trg_b
     int *d_send = ws.buf<int>(Workspace::kSrcEnd, n_src_box);
     int *d_ent = ws.buf<int>(Workspace::kEnt, nent);
     WorkItem *d_items = ws.buf<WorkItem>(Workspace::kItems, items.size());
-    if (!rec || !d_sbeg || !d_send || !d_ent || !d_items) return STK_ERR_CUDA;
-    STK_CUDA(launch_pack_records(nsrc, nullptr, d_src_coord, d_src_value, sd, nullptr, 0, rs, rec, s));
+    PartGroup *d_groups = ws.buf<PartGroup>(Workspace::kGroups, groups.size());
+    double *d_parts = ws.buf<double>(Workspace::kParts, (size_t)slots * uk_tdim_host(ukernel));
+    if (!rec || !d_sbeg || !d_send || !d_ent || !d_items || !d_groups || !d_parts) return STK_ERR_CUDA;
+    STK_CUDA(launch_pack_records(ukernel, nsrc, nullptr, d_src_coord, d_src_value, sd, nullptr, rec, s));
     STK_CUDA(cudaMemcpyAsync(d_sbeg, src_begin, n_src_box * sizeof(int), cudaMemcpyHostToDevice, s));
     STK_CUDA(cudaMemcpyAsync(d_send, src_end, n_src_box * sizeof(int), cudaMemcpyHostToDevice, s));
     STK_CUDA(cudaMemcpyAsync(d_ent, list_ent, nent * sizeof(int), cudaMemcpyHostToDevice, s));
@@ -299,8 +306,13 @@ static int p2p_lists(int ukernel, int precision, int n_trg_box, const int *trg_b
     a.src_box_begin = d_sbeg;
     a.src_box_end = d_send;
     a.list_ent = d_ent;
+    if (!groups.empty())
+        STK_CUDA(cudaMemcpyAsync(d_groups, groups.data(), groups.size() * sizeof(PartGroup), cudaMemcpyHostToDevice, s));
     a.items = d_items;
     a.n_items = (int)items.size();
+    a.groups = d_groups;
+    a.n_groups = (int)groups.size();
+    a.parts = d_parts;
     a.counter = ws.counter();
     a.trg_xyz = d_trg_coord;
     a.trg_out = d_trg_value;
@@ -309,7 +321,9 @@ static int p2p_lists(int ukernel, int precision, int n_trg_box, const int *trg_b
     a.atomic_out = 0;
     a.trg_aux = d_trg_aux;
     STK_CUDA(launch_list_p2p(ukernel, precision, a, ws.num_sms(), s));
-    return ws.end(s);  // queued: no host wait (see direct_device)
+    // the host vectors may die at return: copies from pageable memory have been staged by the
+    // time cudaMemcpyAsync returns, so no host wait is needed
+    return ws.end(s);
 }
 
 extern "C" int stk_p2p_lists(int ukernel, int precision, int n_trg_box, const int *trg_begin, const int *trg_end,
@@ -404,8 +418,8 @@ extern "C" int stk_gemm_f64_i8(int M, int N, int K, const double *d_A, int lda, 
     int *err = reinterpret_cast<int *>(reinterpret_cast<uint8_t *>(fb) + sb + pb);
     int rc = STK_OK, e = 0;
     if (cudaMemsetAsync(err, 0, sizeof(int), s) != cudaSuccess ||
-        i8_digits(d_A, lda, nullptr, M, K, nkb, nullptr, da, fa, s) != cudaSuccess ||
-        i8_digits(d_B, ldb, nullptr, N, K, nkb, nullptr, db, fb, s) != cudaSuccess ||
+        i8_digits(d_A, lda, nullptr, M, K, nkb, nullptr, nullptr, da, fa, s) != cudaSuccess ||
+        i8_digits(d_B, ldb, nullptr, N, K, nkb, nullptr, nullptr, db, fb, s) != cudaSuccess ||
         i8_gemm(M, N, I8Operand{da, fa, nkb}, I8Operand{db, fb, nkb}, 1.0, beta, d_C, ldc, nullptr, parts, err,
                 s) != cudaSuccess ||
         cudaMemcpyAsync(&e, err, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess)

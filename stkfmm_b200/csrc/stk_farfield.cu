@@ -406,16 +406,17 @@ __global__ void gather_cols_kernel(const TS *__restrict__ src, const int *__rest
     }
 }
 
-// dst[:, cols[j]] (= or +=) alpha src[:, j]; no two j may share a column
+// dst[:, cols[j]] (= or +=) mul[j] src[:, j] (mul null: 1); no two j may share a column
 template <class TS>
 __global__ void scatter_cols_kernel(const TS *__restrict__ src, const int *__restrict__ cols, int m, int N,
-                                    double alpha, int add, double *__restrict__ dst) {
+                                    const double *__restrict__ mul, int add, double *__restrict__ dst) {
     const long long total = (long long)m * N;
     for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
          idx += (long long)gridDim.x * blockDim.x) {
         const int j = (int)(idx / N), r = (int)(idx - (long long)j * N);
         double *d = dst + (size_t)cols[j] * N + r;
-        *d = add ? *d + alpha * (double)src[idx] : alpha * (double)src[idx];
+        const double v = (mul ? mul[j] : 1.0) * (double)src[idx];
+        *d = add ? *d + v : v;
     }
 }
 
@@ -430,10 +431,10 @@ int gather_cols(const TS *src, const int *cols, int m, int N, TD *dst, cudaStrea
 }
 
 template <class TS>
-int scatter_cols(const TS *src, const int *cols, int m, int N, double alpha, int add, double *dst, cudaStream_t s) {
+int scatter_cols(const TS *src, const int *cols, int m, int N, const double *mul, int add, double *dst, cudaStream_t s) {
     if (m <= 0) return STK_OK;
     t_launches++;
-    scatter_cols_kernel<TS><<<grid_for((long long)m * N), 256, 0, s>>>(src, cols, m, N, alpha, add, dst);
+    scatter_cols_kernel<TS><<<grid_for((long long)m * N), 256, 0, s>>>(src, cols, m, N, mul, add, dst);
     return cudaGetLastError() == cudaSuccess ? STK_OK : STK_ERR_CUDA;
 }
 
@@ -966,7 +967,7 @@ int build_i8_operators(FarField &F, cudaStream_t s) {
     for (int sl = 0; sl < nslot; sl++) {
         const double *Q = (const double *)F.m2l_q.ptr + F.m2l_pq_off[sl], *P = (const double *)F.m2l_p.ptr + F.m2l_pq_off[sl];
         const size_t ks = (size_t)sl * rmax;
-        FCUDA(i8_digits(Q, k, nullptr, F.m2l_r[sl], k, F.i8_q.nkb, F.i8_q.down(), F.i8_q.digits(F.i8_q_blk[sl]),
+        FCUDA(i8_digits(Q, k, nullptr, F.m2l_r[sl], k, F.i8_q.nkb, F.i8_q.down(), nullptr, F.i8_q.digits(F.i8_q_blk[sl]),
                         F.i8_q.scales(F.i8_q_blk[sl]), s));
         FCUDA(i8_column_scales(P, k, k, F.m2l_r[sl], F.i8_p.up() + ks, F.i8_p.down() + ks, s));
         FCUDA(i8_digits_trans(P, k, k, F.m2l_r[sl], F.i8_p.nkb, F.i8_p.down() + ks, F.i8_p.digits((long long)sl * kb),
@@ -989,11 +990,11 @@ bool i8_wins(int M, int N, int K) {
     return i8_us < std::max(15.0, 2.0 * M * N * K / 28e6);
 }
 
-// C[:, col(j)] (add = 0: =, 1: +=) alpha A X[:, idx(j)] for j < m: A column-major M x K
-// (and as digits), X columns of K values, idx / cols null for the identity.  Y, Xg: scratch of
-// the cuBLAS path (M x m, K x m).
+// C[:, col(j)] (add = 0: =, 1: +=) mul(j) A X[:, idx(j)] for j < m: A column-major M x K
+// (and as digits), X columns of K values, idx / cols null for the identity, mul powers of two
+// (null: 1, given with cols only).  Y, Xg: scratch of the cuBLAS path (M x m, K x m).
 int far_product(FarField &F, const DevBuf &A, const I8Buf &A8, int M, int K, const double *X, const int *idx, int m,
-                double alpha, int add, double *C, const int *cols, double *Xg, double *Y, cudaStream_t s) {
+                const double *mul, int add, double *C, const int *cols, double *Xg, double *Y, cudaStream_t s) {
     if (m <= 0) return STK_OK;
     if (F.i8 && i8_wins(M, m, K)) {
         const int np = i8_gemm_parts(M, m, i8_kblocks(K));
@@ -1001,8 +1002,8 @@ int far_product(FarField &F, const DevBuf &A, const I8Buf &A8, int M, int K, con
         if (!rc && np > 1) rc = F.i8_parts.reserve(sizeof(double) * (size_t)np * M * m);
         if (rc) return rc;
         t_launches += np > 1 ? 3 : 2;
-        FCUDA(i8_digits(X, K, idx, m, K, F.i8_b.nkb, A8.up(), F.i8_b.digits(), F.i8_b.scales(), s));
-        FCUDA(i8_gemm(M, m, A8.op(), F.i8_b.op(), alpha, add, C, M, cols, np > 1 ? (double *)F.i8_parts.ptr : nullptr,
+        FCUDA(i8_digits(X, K, idx, m, K, F.i8_b.nkb, A8.up(), mul, F.i8_b.digits(), F.i8_b.scales(), s));
+        FCUDA(i8_gemm(M, m, A8.op(), F.i8_b.op(), 1.0, add, C, M, cols, np > 1 ? (double *)F.i8_parts.ptr : nullptr,
                       (int *)F.tc_err.ptr, s));
         return STK_OK;
     }
@@ -1013,12 +1014,12 @@ int far_product(FarField &F, const DevBuf &A, const I8Buf &A8, int M, int K, con
         X = Xg;
     }
     if (!cols) {
-        FBLAS(cublasDgemm(F.blas, CUBLAS_OP_N, CUBLAS_OP_N, M, m, K, &alpha, (const double *)A.ptr, M, X, K,
+        FBLAS(cublasDgemm(F.blas, CUBLAS_OP_N, CUBLAS_OP_N, M, m, K, &one, (const double *)A.ptr, M, X, K,
                           add ? &one : &zero, C, M));
         return STK_OK;
     }
-    FBLAS(cublasDgemm(F.blas, CUBLAS_OP_N, CUBLAS_OP_N, M, m, K, &alpha, (const double *)A.ptr, M, X, K, &zero, Y, M));
-    return scatter_cols(Y, cols, m, M, 1.0, add, C, s);
+    FBLAS(cublasDgemm(F.blas, CUBLAS_OP_N, CUBLAS_OP_N, M, m, K, &one, (const double *)A.ptr, M, X, K, &zero, Y, M));
+    return scatter_cols(Y, cols, m, M, mul, add, C, s);
 }
 
 // Build the level-independent operators for (m2x, p).
@@ -1235,10 +1236,15 @@ int setup_pass(ListPass &P, int uk, const std::vector<int> &tb, const std::vecto
                int shard_rank = 0, int shard_n = 1) {
     P.uk = uk;
     std::vector<WorkItem> items;
+    std::vector<PartGroup> groups;
+    long long slots = 0;
     build_list_items((int)tb.size(), tb.data(), te.data(), off.data(), ent.data(), h_src_beg, h_src_end, items,
                      P.pairs, balance_warps, shard_rank, shard_n);
     P.n_items = (int)items.size();
-    int rc = P.items.upload(items.data(), items.size() * sizeof(WorkItem), s);
+    int rc = P.items[1].upload(items, groups, 0, s);
+    build_split_items((int)tb.size(), tb.data(), te.data(), off.data(), ent.data(), h_src_beg, h_src_end,
+                      balance_warps * 5 / 4, items, groups, slots, shard_rank, shard_n);
+    if (!rc) rc = P.items[0].upload(items, groups, slots, s);
     if (!rc) rc = P.ent.upload(ent.data(), ent.size() * sizeof(int), s);
     if (!rc && own_src) rc = P.src_beg.upload(h_src_beg, sizeof(int) * n_src_box, s);
     if (!rc && own_src) rc = P.src_end.upload(h_src_end, sizeof(int) * n_src_box, s);
@@ -1247,16 +1253,17 @@ int setup_pass(ListPass &P, int uk, const std::vector<int> &tb, const std::vecto
 }
 
 int run_pass(const ListPass &P, int prec, const double *rec, const int *src_beg, const int *src_end,
-             const double *trg_xyz, double *out, unsigned int *counter, int sms, cudaStream_t s) {
-    if (P.n_items == 0) return STK_OK;
-    t_launches++;
+             const double *trg_xyz, double *out, unsigned int *counter, DevBuf &parts, int sms, cudaStream_t s) {
+    const ItemList &il = P.items[prec];
+    if (il.n_items == 0) return STK_OK;
+    t_launches += il.n_groups ? 2 : 1;
     ListP2PArgs a{};
     a.src_rec = rec;
     a.src_box_begin = src_beg;
     a.src_box_end = src_end;
     a.list_ent = (const int *)P.ent.ptr;
-    a.items = (const WorkItem *)P.items.ptr;
-    a.n_items = P.n_items;
+    const int rc = il.args(a, parts, uk_tdim_host(P.uk));
+    if (rc) return rc;
     a.counter = counter;
     a.trg_xyz = trg_xyz;
     a.trg_out = out;
@@ -1680,7 +1687,7 @@ static int setup_m2l_dense(FarField &F, const Octree &T, int nslot, cudaStream_t
         FCUDA(cudaGetLastError());
         for (int cs = 0; cs < 8; cs++)
             FCUDA(i8_digits((const double *)F.dn_qs.ptr + F.dn_qs_off[cs], k, nullptr, F.dn_rs[cs], k, F.dn_q8.nkb,
-                            F.i8_q.down(), F.dn_q8.digits(F.dn_q8_blk[cs]), F.dn_q8.scales(F.dn_q8_blk[cs]), s));
+                            F.i8_q.down(), nullptr, F.dn_q8.digits(F.dn_q8_blk[cs]), F.dn_q8.scales(F.dn_q8_blk[cs]), s));
         for (int b = 0; b < 64; b++)
             FCUDA(i8_digits_trans((const double *)F.dn_pv.ptr + F.dn_pv_off[b / 8] + (size_t)k * F.dn_pstart[b], k,
                                   F.dn_rcc[b] ? k : 0, F.dn_rcc[b], F.dn_p8.nkb,
@@ -1903,11 +1910,16 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
     if (!rc) rc = F.psi_hat.reserve(sizeof(double) * (size_t)nn * F.m2l_rank);
     if (rc) return rc;
 
-    auto by_level = [&](std::vector<int> &nodes, std::vector<int> &off) {
-        std::stable_sort(nodes.begin(), nodes.end(), [&](int a, int b) { return T.level[a] < T.level[b]; });
-        off.assign(T.depth() + 2, 0);
-        for (int b : nodes) off[T.level[b] + 1]++;
-        for (int l = 0; l <= T.depth(); l++) off[l + 1] += off[l];
+    // levels of a compact node list, and 2^-level
+    auto levels_of = [&](const std::vector<int> &nodes, DevBuf &lev, DevBuf &mul) -> int {
+        std::vector<int> l(nodes.size());
+        std::vector<double> m(nodes.size());
+        for (size_t i = 0; i < nodes.size(); i++) {
+            l[i] = T.level[nodes[i]];
+            m[i] = std::ldexp(1.0, -l[i]);
+        }
+        const int r = lev.upload(l.data(), sizeof(int) * l.size(), s);
+        return r ? r : mul.upload(m.data(), sizeof(double) * m.size(), s);
     };
     std::vector<double> ctr(3 * (size_t)nn);
     for (int i = 0; i < nn; i++) T.centre(i, &ctr[3 * (size_t)i]);
@@ -1926,9 +1938,9 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
     F.s2m_nodes.clear();
     for (int b : T.leaves)
         if (T.src_count(b) > 0) F.s2m_nodes.push_back(b);
-    by_level(F.s2m_nodes, F.s2m_level_off);
     const int ms = (int)F.s2m_nodes.size();
     rc = F.d_s2m_nodes.upload(F.s2m_nodes.data(), sizeof(int) * ms, s);
+    if (!rc) rc = levels_of(F.s2m_nodes, F.s2m_lev, F.s2m_mul);
     if (!rc) rc = F.uc_xyz.reserve(sizeof(double) * 3 * (size_t)std::max(ms, 1) * n);
     if (!rc) rc = F.check.reserve(sizeof(double) * (size_t)std::max(ms, 1) * n * kc);
     if (rc) return rc;
@@ -1998,9 +2010,9 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
     F.s2l_nodes.clear();
     for (int b = 0; b < nn; b++)
         if (T.X.off[b + 1] > T.X.off[b] && !x_direct(b)) F.s2l_nodes.push_back(b);
-    by_level(F.s2l_nodes, F.s2l_level_off);
     const int mx = (int)F.s2l_nodes.size();
     rc = F.d_s2l_nodes.upload(F.s2l_nodes.data(), sizeof(int) * mx, s);
+    if (!rc) rc = levels_of(F.s2l_nodes, F.s2l_lev, F.s2l_mul);
     if (!rc) rc = F.dc_xyz.reserve(sizeof(double) * 3 * (size_t)std::max(mx, 1) * n);
     if (!rc) rc = F.dcheck.reserve(sizeof(double) * (size_t)std::max(mx, 1) * n * kc);
     if (rc) return rc;
@@ -2052,6 +2064,20 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
                 if (!w_direct(T.W.ent[e] >> 5)) went.push_back(T.W.ent[e]);
         }
         woff[nn] = (int)went.size();
+        // the nodes whose surfaces are sources
+        std::vector<int> l2t_nodes, m2t_nodes;
+        for (int e : lent) l2t_nodes.push_back(e >> 5);
+        std::vector<char> seen(nn, 0);
+        for (int e : went)
+            if (!seen[e >> 5]) {
+                seen[e >> 5] = 1;
+                m2t_nodes.push_back(e >> 5);
+            }
+        F.n_l2t = (int)l2t_nodes.size();
+        F.n_m2t = (int)m2t_nodes.size();
+        rc = F.d_l2t_nodes.upload(l2t_nodes.data(), sizeof(int) * l2t_nodes.size(), s);
+        if (!rc) rc = F.d_m2t_nodes.upload(m2t_nodes.data(), sizeof(int) * m2t_nodes.size(), s);
+        if (rc) return rc;
         F.m2t.reset();
         F.l2t.reset();
         // target-side passes follow the handle's shard (the upward pass, S2L and the
@@ -2081,6 +2107,17 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
     F.parent_off[T.depth() + 1] = (int)F.parents.size();
     rc = F.d_parents.upload(F.parents.data(), sizeof(int) * F.parents.size(), s);
     if (rc) return rc;
+
+    // The coarsest level whose upward densities are read (by a V list, a W list, or the periodic
+    // far images), and whose downward densities are not all zero: M2M stops and L2L starts
+    // there.  Without periodic images that is level 2 at the earliest; the products above it
+    // (N x 8N by one and by eight boxes) read whole operators for nothing.
+    F.up_top = F.down_top = F.periodic ? 0 : T.depth() + 1;
+    for (int b = 0; b < nn && !F.periodic; b++) {
+        for (int e = T.V.off[b]; e < T.V.off[b + 1]; e++) F.up_top = std::min(F.up_top, (int)T.level[T.V.ent[e] >> 5]);
+        for (int e = T.W.off[b]; e < T.W.off[b + 1]; e++) F.up_top = std::min(F.up_top, (int)T.level[T.W.ent[e] >> 5]);
+        if (T.V.off[b + 1] > T.V.off[b] || T.X.off[b + 1] > T.X.off[b]) F.down_top = std::min(F.down_top, (int)T.level[b]);
+    }
 
     // ---- M2L: V-list pairs grouped by offset ----
     {
@@ -2238,9 +2275,9 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
                 const int m = F.parent_off[l + 1] - F.parent_off[l];
                 shape(N, m, 8 * N);
                 shape(8 * N, m, N);
-                shape(N, F.s2m_level_off[l + 1] - F.s2m_level_off[l], N);
-                shape(N, F.s2l_level_off[l + 1] - F.s2l_level_off[l], N);
             }
+            shape(N, ms, N);
+            shape(N, mx, N);
             shape(k, nn, N);
             shape(N, nn, k);
             if (rc) return rc;
@@ -2324,7 +2361,7 @@ static int m2l_dense_level_tc(FarField &F, const M2LDenseLevel &D, const double 
             FCUDA(cudaEventRecord(F.tc_ev[si], F.tc_stream[si]));
             FCUDA(cudaStreamWaitEvent(s, F.tc_ev[si], 0));
         }
-    return scatter_cols<float>(psi, nodes, n, k, 1.0, 1, psi_hat, s);
+    return scatter_cols<float>(psi, nodes, n, k, nullptr, 1, psi_hat, s);
 }
 
 // The FP64 dense M2L of one complete level on the int8 tensor cores (stk_i8gemm.cu), source
@@ -2340,7 +2377,8 @@ static int m2l_dense_level_i8(FarField &F, const M2LDenseLevel &D, const double 
     double *psi = (double *)F.dn_psi.ptr, *Z = (double *)F.dn_z.ptr;
     int *err = (int *)F.tc_err.ptr;
     t_launches++;
-    FCUDA(i8_digits(phi_hat, k, nodes, n, k, F.dn_phi8.nkb, F.i8_q.up(), F.dn_phi8.digits(), F.dn_phi8.scales(), s));
+    FCUDA(i8_digits(phi_hat, k, nodes, n, k, F.dn_phi8.nkb, F.i8_q.up(), nullptr, F.dn_phi8.digits(),
+                    F.dn_phi8.scales(), s));
     FCUDA(cudaMemsetAsync(psi, 0, sizeof(double) * (size_t)k * n, s));
     for (int cs = 0; cs < 8; cs++) {
         const int rs = F.dn_rs[cs], nt = D.tiles8_off[cs + 1] - D.tiles8_off[cs];
@@ -2368,7 +2406,7 @@ static int m2l_dense_level_i8(FarField &F, const M2LDenseLevel &D, const double 
         FCUDA(i8_grouped(F.dn_p8.op(), F.dn_zc8.op(), (const I8Tile *)D.d_tiles8.ptr + D.tiles8_off[cs], nt, 1, psi, err,
                          s));
     }
-    return scatter_cols<double>(psi, nodes, n, k, 1.0, 1, psi_hat, s);
+    return scatter_cols<double>(psi, nodes, n, k, nullptr, 1, psi_hat, s);
 }
 
 // Dense M2L of one complete level: psi_hat[:, t] += sum over the level's V-list
@@ -2413,7 +2451,7 @@ static int m2l_dense_level(FarField &F, const M2LDenseLevel &D, const double *ph
                                psi + (size_t)c * n8 * k, dt, k, ct, CUBLAS_GEMM_DEFAULT));
         }
     }
-    return scatter_cols<T>(psi, nodes, n, k, 1.0, 1, psi_hat, s);
+    return scatter_cols<T>(psi, nodes, n, k, nullptr, 1, psi_hat, s);
 }
 
 int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const double *d_dl, double *trg_sorted,
@@ -2442,14 +2480,31 @@ int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const dou
         t_launches++;
         // fused check pass: SL values then DL values in one record
         const bool both = F.fused_src && k == 0 && d_dl;
-        if (launch_pack_records(ps.n, (const int *)kd->d_perm[k].ptr, (const double *)kd->d_xyz[k].ptr,
+        if (launch_pack_records(uk, ps.n, (const int *)kd->d_perm[k].ptr, (const double *)kd->d_xyz[k].ptr,
                                 k == 0 ? d_sl : d_dl, k == 0 ? ki->kdim_sl : ki->kdim_dl, both ? d_dl : nullptr,
-                                both ? ki->kdim_dl : 0, rs, (double *)F.rec_pts[k].ptr, s) != cudaSuccess)
+                                (double *)F.rec_pts[k].ptr, s) != cudaSuccess)
             return STK_ERR_CUDA;
         return STK_OK;
     };
 
-    // ---- upward pass: S2M, then check -> equivalent per level ----
+    // check potentials -> equivalent densities of m nodes of any level: the level's factor
+    // 2^-l (1 + pot_exp) goes into the products' columns (one factor) or, per component, into
+    // the check potentials
+    auto solve = [&](double *check, int m, const DevBuf &A, const I8Buf &A8, const DevBuf &lev, const DevBuf &mul,
+                     const DevBuf &nodes, int add, double *dst) -> int {
+        if (F.scaled) {
+            CompF e;
+            for (int c = 0; c < 4; c++) e.v[c] = 1.0 + F.pot_exp[c];
+            level_scale_kernel<<<grid_for((long long)m * n * kc), 256, 0, s>>>(check, m, n * kc, kc, (const int *)lev.ptr, 0,
+                                                                              e);
+            FCUDA(cudaGetLastError());
+            t_launches++;
+        }
+        return far_product(F, A, A8, N, n * kc, check, nullptr, m, F.scaled ? nullptr : (const double *)mul.ptr, add, dst,
+                           (const int *)nodes.ptr, X, Y, s);
+    };
+
+    // ---- upward pass: S2M, then check -> equivalent ----
     const int ms = (int)F.s2m_nodes.size();
     if (ms) {
         FCUDA(cudaMemsetAsync(F.check.ptr, 0, sizeof(double) * (size_t)ms * n * kc, s));
@@ -2459,36 +2514,20 @@ int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const dou
             if (!rc)
                 rc = run_pass(F.s2m[k], prec, (const double *)F.rec_pts[k].ptr, (const int *)kd->d_beg[k].ptr,
                               (const int *)kd->d_end[k].ptr, (const double *)F.uc_xyz.ptr, (double *)F.check.ptr,
-                              counter, sms, s);
+                              counter, kd->d_parts, sms, s);
             if (rc) return rc;
         }
-        for (int l = 0; l + 1 < (int)F.s2m_level_off.size(); l++) {
-            const int a = F.s2m_level_off[l], m = F.s2m_level_off[l + 1] - a;
-            if (m <= 0) continue;
-            double alpha = std::ldexp(1.0, -l);
-            if (F.scaled) {
-                // normalised check potential: 2^-l (1 + pot_exp[a]) per component
-                CompF e;
-                for (int c = 0; c < 4; c++) e.v[c] = 1.0 + F.pot_exp[c];
-                level_scale_kernel<<<grid_for((long long)m * n * kc), 256, 0, s>>>(
-                    (double *)F.check.ptr + (size_t)a * n * kc, m, n * kc, kc, nullptr, l, e);
-                FCUDA(cudaGetLastError());
-                t_launches++;
-                alpha = 1.0;
-            }
-            int rc = far_product(F, F.uc2ue, F.i8_uc2ue, N, n * kc, (const double *)F.check.ptr + (size_t)a * n * kc,
-                                 nullptr, m, alpha, 0, phi, (const int *)F.d_s2m_nodes.ptr + a, X, Y, s);
-            if (rc) return rc;
-        }
+        const int rc = solve((double *)F.check.ptr, ms, F.uc2ue, F.i8_uc2ue, F.s2m_lev, F.s2m_mul, F.d_s2m_nodes, 0, phi);
+        if (rc) return rc;
     }
     FCUDA(cudaEventRecord(kd->ph[1], s));
     // M2M, bottom up: parents of level l from the contiguous children block at level l+1
     const int *d_parents = (const int *)F.d_parents.ptr;
-    for (int l = T.depth() - 1; l >= 0; l--) {
+    for (int l = T.depth() - 1; l >= F.up_top; l--) {
         const int a = F.parent_off[l], m = F.parent_off[l + 1] - a;
         if (m == 0) continue;
         const double *Xc = phi + (size_t)T.level_begin[l + 1] * N;
-        int rc = far_product(F, F.m2m, F.i8_m2m, N, 8 * N, Xc, nullptr, m, 1.0, 0, phi, d_parents + a, nullptr, Y, s);
+        int rc = far_product(F, F.m2m, F.i8_m2m, N, 8 * N, Xc, nullptr, m, nullptr, 0, phi, d_parents + a, nullptr, Y, s);
         if (rc) return rc;
     }
 
@@ -2502,7 +2541,7 @@ int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const dou
     // (3xTF32 on the tensor cores) raised the mixed Stokes FMM's error from 2.8e-7 to
     // 5.2e-7 (V^T phi alone) and 7.3e-7 (both); p = 8, 12000 clustered points.
     {
-        const int rc = far_product(F, F.m2l_vt, F.i8_vt, k, N, phi, nullptr, nn, 1.0, 0, phi_hat, nullptr, nullptr,
+        const int rc = far_product(F, F.m2l_vt, F.i8_vt, k, N, phi, nullptr, nn, nullptr, 0, phi_hat, nullptr, nullptr,
                                    nullptr, s);
         if (rc) return rc;
     }
@@ -2606,7 +2645,7 @@ int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const dou
         if (rcd) return rcd;
     }
     {
-        const int rc = far_product(F, F.m2l_e, F.i8_e, N, k, psi_hat, nullptr, nn, 1.0, 1, psi, nullptr, nullptr,
+        const int rc = far_product(F, F.m2l_e, F.i8_e, N, k, psi_hat, nullptr, nn, nullptr, 1, psi, nullptr, nullptr,
                                    nullptr, s);
         if (rc) return rc;
     }
@@ -2625,78 +2664,55 @@ int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const dou
             if (!rc)
                 rc = run_pass(F.s2l[k], prec, (const double *)F.rec_pts[k].ptr, (const int *)kd->d_beg[k].ptr,
                               (const int *)kd->d_end[k].ptr, (const double *)F.dc_xyz.ptr, (double *)F.dcheck.ptr,
-                              counter, sms, s);
+                              counter, kd->d_parts, sms, s);
             if (rc) return rc;
             any = true;
         }
-        if (any)
-            for (int l = 0; l + 1 < (int)F.s2l_level_off.size(); l++) {
-                const int a = F.s2l_level_off[l], m = F.s2l_level_off[l + 1] - a;
-                if (m <= 0) continue;
-                double alpha = std::ldexp(1.0, -l);
-                if (F.scaled) {
-                    CompF e;
-                    for (int c = 0; c < 4; c++) e.v[c] = 1.0 + F.pot_exp[c];
-                    level_scale_kernel<<<grid_for((long long)m * n * kc), 256, 0, s>>>(
-                        (double *)F.dcheck.ptr + (size_t)a * n * kc, m, n * kc, kc, nullptr, l, e);
-                    FCUDA(cudaGetLastError());
-                    t_launches++;
-                    alpha = 1.0;
-                }
-                int rc = far_product(F, F.dc2de, F.i8_dc2de, N, n * kc, (const double *)F.dcheck.ptr + (size_t)a * n * kc,
-                                     nullptr, m, alpha, 1, psi, (const int *)F.d_s2l_nodes.ptr + a, X, Y, s);
-                if (rc) return rc;
-            }
+        if (any) {
+            const int rc = solve((double *)F.dcheck.ptr, mx, F.dc2de, F.i8_dc2de, F.s2l_lev, F.s2l_mul, F.d_s2l_nodes, 1, psi);
+            if (rc) return rc;
+        }
     }
     // split far field: every rank holds its target nodes' M2L / S2L contributions;
     // one sum over the shard group gives all ranks the whole downward densities
     if (F.split && f->allreduce(psi, (long long)nn * N, (void *)s, f->allreduce_user) != 0) return STK_ERR_CUDA;
     FCUDA(cudaEventRecord(kd->ph[4], s));
     // L2L, top down: the level-l children block of the level-(l-1) parents
-    for (int l = 1; l <= T.depth(); l++) {
+    for (int l = F.down_top + 1; l <= T.depth(); l++) {
         const int a = F.parent_off[l - 1], m = F.parent_off[l] - a;
         if (m == 0) continue;
-        int rc = far_product(F, F.l2l, F.i8_l2l, 8 * N, N, psi, d_parents + a, m, 1.0, 1,
+        int rc = far_product(F, F.l2l, F.i8_l2l, 8 * N, N, psi, d_parents + a, m, nullptr, 1,
                              psi + (size_t)T.level_begin[l] * N, nullptr, X, nullptr, s);
         if (rc) return rc;
     }
 
     // ---- evaluation at the targets: L2T and M2T (W list) ----
     const long long npts = (long long)nn * n;
-    auto pack_surface = [&](const DevBuf &xyz, const double *dens, int uk) -> int {
-        const int rs = uk_record_stride(uk);
-        int rc = F.rec_surf.reserve(sizeof(double) * (size_t)npts * rs);
+    // records of the listed nodes' surfaces, at their nodes' places; scaled kernels: back to
+    // physical densities at each node's level, component c times 2^-l den_exp[c]
+    auto pack_surface = [&](const DevBuf &xyz, const double *dens, int uk, const DevBuf &nodes, int m) -> int {
+        const int rc = F.rec_surf.reserve(sizeof(double) * (size_t)npts * uk_record_stride(uk));
         if (rc) return rc;
         t_launches++;
-        if (launch_pack_records((int)npts, nullptr, (const double *)xyz.ptr, dens, ke, nullptr, 0, rs,
-                                (double *)F.rec_surf.ptr, s) != cudaSuccess)
+        if (launch_pack_surface(uk, (const int *)nodes.ptr, m, n, (const double *)xyz.ptr, dens,
+                                F.scaled ? (const int *)F.d_level.ptr : nullptr, F.den_exp, (double *)F.rec_surf.ptr,
+                                s) != cudaSuccess)
             return STK_ERR_CUDA;
         return STK_OK;
     };
     FCUDA(cudaEventRecord(kd->ph[5], s));
     const double *trg_xyz = (const double *)kd->d_xyz[2].ptr;
-    if (F.scaled) {
-        // back to physical densities at each node's level: component c times 2^-l den_exp[c]
-        CompF e;
-        for (int c = 0; c < 4; c++) e.v[c] = F.den_exp[c];
-        level_scale_kernel<<<grid_for((long long)nn * N), 256, 0, s>>>(psi, nn, N, ke, (const int *)F.d_level.ptr, 0,
-                                                                      e);
-        level_scale_kernel<<<grid_for((long long)nn * N), 256, 0, s>>>(phi, nn, N, ke, (const int *)F.d_level.ptr, 0,
-                                                                      e);
-        FCUDA(cudaGetLastError());
-        t_launches += 2;
-    }
-    int rc = pack_surface(F.de_xyz, psi, F.l2t.uk);
+    int rc = pack_surface(F.de_xyz, psi, F.l2t.uk, F.d_l2t_nodes, F.n_l2t);
     if (!rc)
         rc = run_pass(F.l2t, prec, (const double *)F.rec_surf.ptr, (const int *)F.l2t.src_beg.ptr,
-                      (const int *)F.l2t.src_end.ptr, trg_xyz, trg_sorted, counter, sms, s);
+                      (const int *)F.l2t.src_end.ptr, trg_xyz, trg_sorted, counter, kd->d_parts, sms, s);
     if (rc) return rc;
     FCUDA(cudaEventRecord(kd->ph[6], s));
     if (F.m2t.n_items) {
-        rc = pack_surface(F.ue_xyz, phi, F.m2t.uk);
+        rc = pack_surface(F.ue_xyz, phi, F.m2t.uk, F.d_m2t_nodes, F.n_m2t);
         if (!rc)
             rc = run_pass(F.m2t, prec, (const double *)F.rec_surf.ptr, (const int *)F.m2t.src_beg.ptr,
-                          (const int *)F.m2t.src_end.ptr, trg_xyz, trg_sorted, counter, sms, s);
+                          (const int *)F.m2t.src_end.ptr, trg_xyz, trg_sorted, counter, kd->d_parts, sms, s);
         if (rc) return rc;
     }
     // periodizeFMM: PVel, PVelGrad and PVelLaplacian only (not Traction), with the

@@ -28,12 +28,13 @@ constexpr double kRad1 = 2.95;  // upward check, downward equivalent
 // One P2P evaluation over a list, with its work items resident on the device.
 struct ListPass {
     int uk = -1;
-    int n_items = 0;
+    int n_items = 0;    // 0: nothing to do (the mixed path's count)
     long long pairs = 0;
-    DevBuf items, ent, src_beg, src_end, trg_box_centre;
+    ItemList items[2];  // FP64, mixed
+    DevBuf ent, src_beg, src_end, trg_box_centre;
     void reset() {
         uk = -1;
-        n_items = 0;
+        n_items = items[0].n_items = items[1].n_items = 0;
         pairs = 0;
     }
 };
@@ -141,9 +142,12 @@ struct FarField {
     DevBuf phi_hat, psi_hat;   // compressed M2L sources / targets (nodes x k)
     DevBuf check, dcheck;      // S2M / S2L check potentials (compact)
     DevBuf rec_surf, rec_pts[2], tmp0, tmp1;
-    std::vector<int> s2m_nodes, s2l_nodes;          // compact order (sorted by level)
-    std::vector<int> s2m_level_off, s2l_level_off;  // per level start in the compact order
+    std::vector<int> s2m_nodes, s2l_nodes;          // compact order
     DevBuf d_s2m_nodes, d_s2l_nodes;
+    DevBuf s2m_lev, s2m_mul, s2l_lev, s2l_mul;      // their levels l, and 2^-l
+    int up_top = 0, down_top = 0;                   // coarsest levels of M2M's outputs, L2L's inputs
+    DevBuf d_l2t_nodes, d_m2t_nodes;                // nodes whose surfaces L2T / M2T read
+    int n_l2t = 0, n_m2t = 0;
     ListPass s2m[2], s2l[2], m2t, l2t;  // [SL, DL]
     bool fused_src = false;             // S2M / S2L as one SL+DL pass (s2m[0], s2l[0])
     int fused_check_uk = -1;

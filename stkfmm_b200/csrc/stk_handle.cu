@@ -75,6 +75,26 @@ int DevBuf::upload(const void *src, size_t n, cudaStream_t s) {
     return STK_OK;
 }
 
+int ItemList::upload(const std::vector<WorkItem> &it, const std::vector<PartGroup> &g, long long slots, cudaStream_t s) {
+    n_items = (int)it.size();
+    n_groups = (int)g.size();
+    part_targets = slots;
+    int rc = items.upload(it.data(), it.size() * sizeof(WorkItem), s);
+    if (!rc && n_groups) rc = groups.upload(g.data(), g.size() * sizeof(PartGroup), s);
+    return rc;
+}
+
+int ItemList::args(ListP2PArgs &a, DevBuf &parts, int tdim) const {
+    a.items = (const WorkItem *)items.ptr;
+    a.n_items = n_items;
+    a.groups = (const PartGroup *)groups.ptr;
+    a.n_groups = n_groups;
+    if (!n_groups) return STK_OK;
+    const int rc = parts.reserve(sizeof(double) * (size_t)part_targets * tdim);
+    a.parts = (double *)parts.ptr;
+    return rc;
+}
+
 KernelData::~KernelData() {
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
@@ -246,17 +266,21 @@ extern "C" int Stk3DFMM_setup_tree(Stk3DFMM *fmm, unsigned kernel) {
     const PointSet &tg = T.sets[2];
     kd->u_pairs[0] = kd->u_pairs[1] = 0;
     for (int k = 0; k < 2; k++) {
-        kd->n_items[k] = 0;
+        kd->u_items[k][0].n_items = kd->u_items[k][1].n_items = 0;
         if (k == 1 && (!dl || kd->fused)) continue;
         const PointSet &sp = T.sets[k];
         std::vector<WorkItem> items;
-        long long pairs = 0;
+        std::vector<PartGroup> groups;
+        long long pairs = 0, slots = 0;
         build_list_items(nn, tg.node_begin.data(), tg.node_end.data(), T.U.off.data(), T.U.ent.data(),
                          sp.node_begin.data(), sp.node_end.data(), items, pairs, fmm->sms * 12, fmm->shard_rank,
                          fmm->shard_n);
         kd->u_pairs[k] = pairs;
-        kd->n_items[k] = (int)items.size();
-        up(kd->d_items[k], items.data(), items.size() * sizeof(WorkItem));
+        if (!rc) rc = kd->u_items[k][1].upload(items, groups, 0, s);
+        build_split_items(nn, tg.node_begin.data(), tg.node_end.data(), T.U.off.data(), T.U.ent.data(),
+                          sp.node_begin.data(), sp.node_end.data(), fmm->sms * 15, items, groups, slots,
+                          fmm->shard_rank, fmm->shard_n);
+        if (!rc) rc = kd->u_items[k][0].upload(items, groups, slots, s);
     }
     if (kd->fused) kd->u_pairs[1] = kd->u_pairs[0];
     if (!rc) rc = kd->d_counter.reserve(64);
@@ -351,28 +375,23 @@ int stk::near_device(Stk3DFMM *f, KernelData *kd, const double *d_sl, const doub
         if (k == 1 && (!dl || kd->fused)) continue;
         // the FMM's near field: U list plus the W / X interactions evaluated directly
         const ListPass *fp = far ? &kd->far->near[k] : nullptr;
-        const int n_items = far ? fp->n_items : kd->n_items[k];
-        if (n_items == 0) continue;
+        const ItemList &il = far ? fp->items[f->precision] : kd->u_items[k][f->precision];
+        if (il.n_items == 0) continue;
         const int uk = kd->fused ? fused_uk(kd) : ki->slot[k == 0 ? SLOT_S2T_SL : SLOT_S2T_DL];
         const int rs = uk_record_stride(uk);
         const PointSet &sp = T.sets[k];
         rc = kd->d_rec[k].reserve(sizeof(double) * std::max(1, sp.n) * rs);
         if (rc) return rc;
         double *rec = (double *)kd->d_rec[k].ptr;
-        if (kd->fused)
-            HCUDA(launch_pack_records(sp.n, (const int *)kd->d_perm[0].ptr, (const double *)kd->d_xyz[0].ptr, d_sl,
-                                      ki->kdim_sl, d_dl, ki->kdim_dl, rs, rec, s));
-        else
-            HCUDA(launch_pack_records(sp.n, (const int *)kd->d_perm[k].ptr, (const double *)kd->d_xyz[k].ptr,
-                                      k == 0 ? d_sl : d_dl, k == 0 ? ki->kdim_sl : ki->kdim_dl, nullptr, 0, rs, rec,
-                                      s));
+        HCUDA(launch_pack_records(uk, sp.n, (const int *)kd->d_perm[k].ptr, (const double *)kd->d_xyz[k].ptr,
+                                  k == 0 ? d_sl : d_dl, k == 0 ? ki->kdim_sl : ki->kdim_dl, kd->fused ? d_dl : nullptr,
+                                  rec, s));
         ListP2PArgs a{};
         a.src_rec = rec;
         a.src_box_begin = (const int *)kd->d_beg[k].ptr;
         a.src_box_end = (const int *)kd->d_end[k].ptr;
         a.list_ent = far ? (const int *)fp->ent.ptr : (const int *)kd->d_uent.ptr;
-        a.items = far ? (const WorkItem *)fp->items.ptr : (const WorkItem *)kd->d_items[k].ptr;
-        a.n_items = n_items;
+        if ((rc = il.args(a, kd->d_parts, td))) return rc;
         a.counter = (unsigned int *)kd->d_counter.ptr;
         a.trg_xyz = (const double *)kd->d_xyz[2].ptr;
         a.trg_out = out;
@@ -382,7 +401,7 @@ int stk::near_device(Stk3DFMM *f, KernelData *kd, const double *d_sl, const doub
         // one octree holds the sources and the targets: coincident points share a leaf
         a.coincident_own_box = 1;
         HCUDA(launch_list_p2p(uk, f->precision, a, f->sms, s));
-        launches += 2;  // record packing + list kernel
+        launches += il.n_groups ? 3 : 2;  // record packing, list kernel, split sums
     }
     HCUDA(cudaEventRecord(kd->ph[0], s));
     kd->last_far = far;

@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include "stk_kernel_table.hpp"
+#include "stk_p2p.cuh"
 #include "stk_tree.hpp"
 
 namespace stk {
@@ -38,6 +39,16 @@ struct DevBuf {
 
 struct FarField;
 
+// Work items of one list pass in one precision, resident on the device.
+struct ItemList {
+    DevBuf items, groups;
+    int n_items = 0, n_groups = 0;
+    long long part_targets = 0;  // target slots of split sums
+    int upload(const std::vector<WorkItem> &it, const std::vector<PartGroup> &g, long long slots, cudaStream_t s);
+    // items, groups and the slots' buffer into the kernel's arguments (tdim components)
+    int args(ListP2PArgs &a, DevBuf &parts, int tdim) const;
+};
+
 // One activated kernel: the reference's impl::FMMData (STKFMM_impl.hpp:19-174).
 struct KernelData {
     const KernelInfo *info = nullptr;
@@ -45,9 +56,9 @@ struct KernelData {
     bool tree_ready = false;
     bool fused = false;            // SL and DL at the same points: one fused U-list pass
     long long u_pairs[2] = {0, 0}; // exact U-list (target, source point) pairs, SL and DL
-    int n_items[2] = {0, 0};
+    ItemList u_items[2][2];        // U-list items [SL, DL][FP64, mixed]
     DevBuf d_xyz[3], d_perm[3], d_beg[3], d_end[3];  // per point set: sorted coords, perm, node ranges
-    DevBuf d_centre, d_uent, d_items[2], d_counter;
+    DevBuf d_centre, d_uent, d_counter, d_parts;
     DevBuf d_val[2], d_rec[2], d_out_sorted, d_out_user, d_alpha;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;  // bracket the kernel launches of the last evaluation
     bool timed = false;

@@ -421,6 +421,8 @@ struct RowLoad {
     const double *ks;
     const int *kof, *kset, *nof;  // per 128-row block, or null
     int kld;
+    const double *rmul;
+    __device__ double mul(long long r) const { return rmul ? rmul[r] : 1.0; }
     __device__ int used_blocks(long long blk, int nkb) const { return kof ? (kof[blk] + kI8K - 1) / kI8K : nkb; }
     __device__ int len(long long r) const {
         return kof ? (r % kI8Rows < nof[r / kI8Rows] ? kof[r / kI8Rows] : 0) : K;
@@ -437,6 +439,7 @@ struct RowLoad {
 };
 struct GatherLoad {
     I8Gather g;
+    __device__ double mul(long long) const { return 1.0; }
     __device__ int used_blocks(long long blk, int) const { return (g.K[(blk * kI8Rows) >> g.lg] + kI8K - 1) / kI8K; }
     __device__ int len(long long r) const { return g.K[r >> g.lg]; }
     __device__ void load4(long long r, int k, int n, double (&v)[4]) const {
@@ -527,7 +530,7 @@ __global__ void __launch_bounds__(256) i8_digits_kernel(const __grid_constant__ 
             cluster.sync();  // everyone has read part before the next group writes it
         }
         const RowScale sc = row_scale(m);
-        if (lane == 0 && sl == 0 && (!ROWS || r < rows)) scale[r] = sc.s;
+        if (lane == 0 && sl == 0 && (!ROWS || r < rows)) scale[r] = r < rows ? sc.s * ld.mul(r) : 0.0;
         uint8_t *blk = dig + (size_t)(grp / 16) * nkb * kI8BlockBytes + (size_t)(grp % 16) * 256;
         for (int k0 = ka; k0 < kz; k0 += 128) {
             if (kz - ka > 128 || !sc.finite) {  // one turn: still in registers
@@ -582,6 +585,7 @@ struct TransLoad {
     long long ld;
     int K;
     const double *ks;
+    __device__ double mul(long long) const { return 1.0; }
     __device__ int used_blocks(long long, int nkb) const { return nkb; }
     __device__ int len(long long) const { return K; }
     __device__ void load4(long long r, int k, int n, double (&v)[4]) const {
@@ -707,17 +711,17 @@ cudaError_t i8_row_scales(const double *src, long long ld, long long rows, int K
     return cudaGetLastError();
 }
 cudaError_t i8_digits(const double *src, long long ld, const int *idx, long long rows, int K, int nkb,
-                      const double *kscale, uint8_t *dig, double *scale, cudaStream_t s) {
-    return launch_digits(RowLoad{src, ld, idx, K, kscale, nullptr, nullptr, nullptr, 0}, rows, nkb, dig, scale, s);
+                      const double *kscale, const double *rmul, uint8_t *dig, double *scale, cudaStream_t s) {
+    return launch_digits(RowLoad{src, ld, idx, K, kscale, nullptr, nullptr, nullptr, 0, rmul}, rows, nkb, dig, scale, s);
 }
 cudaError_t i8_digits_rows(const double *src, long long ld, long long rows, int K, int nkb, const double *kscale,
                            uint8_t *dig, double *scale, cudaStream_t s) {
-    return launch_digits<true>(RowLoad{src, ld, nullptr, K, kscale, nullptr, nullptr, nullptr, 0}, rows, nkb, dig, scale, s);
+    return launch_digits<true>(RowLoad{src, ld, nullptr, K, kscale, nullptr, nullptr, nullptr, 0, nullptr}, rows, nkb, dig, scale, s);
 }
 cudaError_t i8_digits_blocks(const double *src, long long ld, long long rows, const int *kof, const int *nof, int nkb,
                              const double *kscale, const int *kset, int kld, uint8_t *dig, double *scale,
                              cudaStream_t s) {
-    return launch_digits(RowLoad{src, ld, nullptr, 0, kscale, kof, kset, nof, kld}, rows, nkb, dig, scale, s);
+    return launch_digits(RowLoad{src, ld, nullptr, 0, kscale, kof, kset, nof, kld, nullptr}, rows, nkb, dig, scale, s);
 }
 cudaError_t i8_digits_trans(const double *src, long long ld, long long rows, int K, int nkb, const double *kscale,
                             uint8_t *dig, double *scale, cudaStream_t s) {

@@ -60,8 +60,9 @@ cudaError_t i8_row_scales(const double *src, long long ld, long long rows, int K
                           double *down, cudaStream_t s);
 
 // x(r, k) = src[(idx ? idx[r] : r) ld + k] kscale[k], K contiguous; idx[r] < 0 gives a zero row.
+// rmul (nullable): powers of two that multiply the rows' stored scales.
 cudaError_t i8_digits(const double *src, long long ld, const int *idx, long long rows, int K, int nkb,
-                      const double *kscale, uint8_t *dig, double *scale, cudaStream_t s);
+                      const double *kscale, const double *rmul, uint8_t *dig, double *scale, cudaStream_t s);
 // the same as gatherable rows (I8Rows)
 cudaError_t i8_digits_rows(const double *src, long long ld, long long rows, int K, int nkb, const double *kscale,
                            uint8_t *dig, double *scale, cudaStream_t s);

@@ -18,8 +18,7 @@
 // runs a one-time occupancy query (and, with lazy module loading, its module
 // load).  The cached address belongs to the device's primary context: after a
 // cudaDeviceReset of that device the entry point must not be used again in the
-// process.  Every call shares the array and leaves its contents behind: the
-// work counter that must start at zero is cleared by each call, and two calls
+// process.  Every call shares the array and leaves its contents behind: two calls
 // whose work overlaps on the GPU (different streams, or host threads, at the
 // same time) race on the array.
 #include <mutex>
@@ -66,30 +65,6 @@ int noalloc_scratch(void **out) {
     return STK_OK;
 }
 
-__host__ __device__ inline int lanes_log2(int m) {
-    int glog = 0;
-    while (glog < 5 && (m << (glog + 1)) <= kItemTargets) glog++;
-    return glog;
-}
-
-// Writes the work list of a direct sum (64-target chunks x source chunks of
-// `sc` points) into the scratch.  Same decomposition as the allocating path.
-__global__ void noalloc_direct_items_kernel(int ntrg, int nsrc, int nchunk, int nsc, int sc,
-                                           stk::WorkItem *items, int *sbeg, int *send, int *ent) {
-    const int total = nchunk * nsc;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-        const int c = i / nsc, k = i - (i / nsc) * nsc;
-        const int t0 = kItemTargets * c;
-        const int m = min(kItemTargets, ntrg - t0);
-        items[i] = stk::WorkItem{c, t0, m, lanes_log2(m), k, k + 1};
-        if (c == 0) {
-            sbeg[k] = k * sc;
-            send[k] = min(nsrc, (k + 1) * sc);
-            ent[k] = (k << 5) | stk::kShiftNone;
-        }
-    }
-}
-
 }  // namespace
 
 extern "C" int stk_ukernel_direct_device_noalloc(int ukernel, int nsrc, const double *d_src_coord,
@@ -108,7 +83,8 @@ extern "C" int stk_ukernel_direct_device_noalloc(int ukernel, int nsrc, const do
         cudaGetLastError();
         return STK_ERR_NO_DEVICE;
     }
-    // work decomposition (as the allocating direct path)
+    // The sizes this entry takes, by its interface: the records and the work list of 64-target
+    // chunks x source chunks (>= 256 points) within the scratch.
     const long long nchunk = (ntrg + kItemTargets - 1) / kItemTargets;
     const long long want_items = (long long)(sms > 0 ? sms : 1) * 64;
     long long nsc = (want_items + nchunk - 1) / nchunk;
@@ -117,49 +93,29 @@ extern "C" int stk_ukernel_direct_device_noalloc(int ukernel, int nsrc, const do
     long long sc = (nsrc + nsc - 1) / nsc;
     sc = (sc + 31) / 32 * 32;
     nsc = (nsrc + sc - 1) / sc;
-    const long long nitems = nchunk * nsc;
-    // scratch layout: counter | items | source-chunk ranges and entries | source records
-    const int rs = stk::uk_record_stride(ukernel);
-    const size_t off_items = 256;
-    const size_t off_sbeg = round_up(off_items + (size_t)nitems * sizeof(stk::WorkItem), 256);
+    const size_t off_sbeg = round_up(256 + (size_t)(nchunk * nsc) * 24, 256);
     const size_t off_send = round_up(off_sbeg + (size_t)nsc * sizeof(int), 256);
     const size_t off_ent = round_up(off_send + (size_t)nsc * sizeof(int), 256);
     const size_t off_rec = round_up(off_ent + (size_t)nsc * sizeof(int), 256);
-    const size_t need = off_rec + (size_t)nsrc * rs * sizeof(double);
+    const size_t need = off_rec + (size_t)nsrc * ((3 + sdim + 1) & ~1) * sizeof(double);
     if (need > kNoAllocScratchBytes) return STK_ERR_SIZE;  // beyond the fixed 8 MiB scratch
 
     void *base = nullptr;
     int rc = noalloc_scratch(&base);
     if (rc) return rc;
-    unsigned char *s = static_cast<unsigned char *>(base);
-    cudaStream_t st = (cudaStream_t)stream;
-    stk::WorkItem *items = reinterpret_cast<stk::WorkItem *>(s + off_items);
-    int *sbeg = reinterpret_cast<int *>(s + off_sbeg);
-    int *send = reinterpret_cast<int *>(s + off_send);
-    int *ent = reinterpret_cast<int *>(s + off_ent);
-    double *rec = reinterpret_cast<double *>(s + off_rec);
-
-    const int threads = 256;
-    const int grid = (int)((nitems + threads - 1) / threads < 1024 ? (nitems + threads - 1) / threads : 1024);
-    noalloc_direct_items_kernel<<<grid, threads, 0, st>>>(ntrg, nsrc, (int)nchunk, (int)nsc, (int)sc, items, sbeg,
-                                                          send, ent);
-    if (cudaGetLastError() != cudaSuccess) return STK_ERR_CUDA;
-    if (stk::launch_pack_records(nsrc, nullptr, d_src_coord, d_src_value, sdim, nullptr, 0, rs, rec, st) !=
-        cudaSuccess)
-        return STK_ERR_CUDA;
+    // the direct form of the list kernel reads the caller's arrays; the chunks' sums are kept in
+    // the scratch and added in order, or by atomics where they do not fit
     stk::ListP2PArgs a{};
-    a.src_rec = rec;
-    a.src_box_begin = sbeg;
-    a.src_box_end = send;
-    a.list_ent = ent;
-    a.items = items;
-    a.n_items = (int)nitems;
-    a.counter = reinterpret_cast<unsigned int *>(s);  // zeroed by the launch itself
+    a.src_xyz = d_src_coord;
+    a.src_val = d_src_value;
+    a.nsrc = nsrc;
+    a.ntrg = ntrg;
+    stk::direct_chunks(ukernel, precision, ntrg, nsrc, sms, a.src_chunk, a.n_chunk);
     a.trg_xyz = d_trg_coord;
     a.trg_out = d_trg_value;
-    a.box_centre = nullptr;
-    a.period = 1.0;
-    a.atomic_out = nsc > 1 ? 1 : 0;
-    if (stk::launch_list_p2p(ukernel, precision, a, sms, st) != cudaSuccess) return STK_ERR_CUDA;
+    const bool fits = (size_t)a.n_chunk * ntrg * tdim * sizeof(double) <= kNoAllocScratchBytes;
+    if (fits) a.parts = static_cast<double *>(base);
+    if (stk::launch_direct_p2p(ukernel, precision, a, fits ? 1 : 2, sms, (cudaStream_t)stream) != cudaSuccess)
+        return STK_ERR_CUDA;
     return STK_OK;
 }

@@ -17,14 +17,17 @@
 //    walks the concatenated stream in 32-source tiles that cross segment
 //    boundaries, so only the last tile of an item is padded (with one tile per
 //    entry, padding was ~19% of the evaluated pairs on clustered trees).
-//  * Tile staging: lane i copies the raw record of stream position i of the
-//    next tile into its own shared-memory slot with cp.async (16-byte
-//    asynchronous copies, L2 -> shared) while the current tile is consumed;
-//    then it applies the periodic image shift, computes the per-source staged
-//    values (Uk<>::stage) and writes one column of the structure-of-arrays
-//    tile (one row per component).
-//  * FP64 path: one source and two targets per step; r = x_t - (x_s + shift)
-//    formed in double exactly as the oracle forms it.
+//  * Tiles: lane i copies the record of stream position i of the next tile into
+//    its own shared-memory slot with cp.async (16-byte asynchronous copies,
+//    L2 -> shared) while the current tile is consumed.  Records carry the
+//    per-source staged values (Uk<>::stage), computed once by the pack kernel.
+//  * FP64 path: one source and two targets per step, records read as they landed
+//    (16-byte broadcast loads; a lane only adds a periodic shift to its own
+//    record); r = x_t - (x_s + shift) formed in double exactly as the oracle
+//    forms it.  Long items are split by source ranges, their sums kept apart and
+//    added in order by a second kernel (build_split_items).
+//  * Mixed path: the lane splits its landed record into a column of a
+//    structure-of-arrays tile (one row per component).
 //  * Mixed path: at staging each source coordinate, shifted to the target
 //    box's centre c in FP64, is split into FP32 hi + lo parts
 //    (x - c = hi + lo to ~2^-48 relative); targets likewise.  Per pair the
@@ -70,7 +73,9 @@ template <class K> struct NtvOf<K, std::void_t<decltype(K::NTV)>> {
 
 template <int UK> struct Rec {
     static constexpr int SDIM = Uk<UK>::SDIM;
-    static constexpr int RS = (3 + SDIM + 1) & ~1;  // doubles per global record (16-byte multiple)
+    static constexpr int RS = (3 + Uk<UK>::NV + 1) & ~1;  // doubles per global record (16-byte multiple)
+    // landing slot: a record, or a direct sum's raw values before they are staged in place
+    static constexpr int SLOT = (3 + (SDIM > Uk<UK>::NV ? SDIM : Uk<UK>::NV) + 1) & ~1;
 };
 
 // Resident CTAs per SM requested from the register allocator (1: no
@@ -186,7 +191,7 @@ __global__ void __launch_bounds__(Cta<MIXED>::threads, MinBlocks<UK, MIXED>::val
     constexpr int TV = K::TV;  // per-output-point values (adjoint kernels)
     constexpr int NTV = NtvOf<K>::value;
     constexpr int RS = Rec<UK>::RS;
-    constexpr int RSS = RawStride<RS>::value;
+    constexpr int RSS = RawStride<DIRECT ? Rec<UK>::SLOT : RS>::value;
     constexpr int TPL = TargetsPerLane<K>::value;
     constexpr bool HILO = MIXED && kMixedDisp == kDispHiLo;
     // shared tile, one row per component: coordinates (FP64, or FP32 hi x3 + lo x3)
@@ -195,9 +200,10 @@ __global__ void __launch_bounds__(Cta<MIXED>::threads, MinBlocks<UK, MIXED>::val
     using CT = typename std::conditional<HILO, float, double>::type;
     using S = typename std::conditional<MIXED, float, double>::type;
 
-    __shared__ __align__(16) CT tcoord[kWarpsPerCta][NCC][32];
-    __shared__ __align__(16) S tval[kWarpsPerCta][NV][32];
-    constexpr int DEPTH = StageDepth<RS>::value;
+    // (mixed path only: the FP64 path reads the landed records as they are)
+    __shared__ __align__(16) CT tcoord[kWarpsPerCta][MIXED ? NCC : 1][MIXED ? 32 : 1];
+    __shared__ __align__(16) S tval[kWarpsPerCta][MIXED ? NV : 1][MIXED ? 32 : 1];
+    constexpr int DEPTH = MIXED ? StageDepth<RS>::value : 2;  // FP64: one zone read, one landing
     // cp.async landing zones, one record per lane and tile in flight
     __shared__ __align__(16) double traw[kWarpsPerCta][DEPTH][32][RSS];
     // the item's list entries (up to 32 at a time) as segments of one source stream
@@ -206,8 +212,8 @@ __global__ void __launch_bounds__(Cta<MIXED>::threads, MinBlocks<UK, MIXED>::val
     __shared__ int sg_code[kWarpsPerCta][32];  // periodic shift code
     const int wid = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    CT(*mc)[32] = tcoord[wid];
-    S(*mv)[32] = tval[wid];
+    auto &mc = tcoord[wid];
+    auto &mv = tval[wid];
     int *s_end = sg_end[wid];
     int *s_src = sg_src[wid];
     int *s_code = sg_code[wid];
@@ -341,6 +347,11 @@ __global__ void __launch_bounds__(Cta<MIXED>::threads, MinBlocks<UK, MIXED>::val
                 code = ent & 31;
                 sbeg = a.src_box_begin[sb];
                 sz = a.src_box_end[sb] - sbeg;
+                if (ec + lane == w.e1 - 1) sz = min(sz, w.stop);
+                if (ec + lane == w.e0) {
+                    sbeg += w.skip;
+                    sz -= w.skip;
+                }
                 // bit 5: the segment may hold a source at a target's position (always,
                 // unless the lists guarantee coincidence only in the unshifted own box)
                 if (!a.coincident_own_box || sb == w.trg_box || code != kShiftNoneCode) code |= kMayCoincide;
@@ -393,6 +404,52 @@ __global__ void __launch_bounds__(Cta<MIXED>::threads, MinBlocks<UK, MIXED>::val
                 }
                 cp_async_commit();
             };
+            if constexpr (!MIXED) {
+                // ---- FP64: tiles are read straight from their landing zone (records carry
+                // staged values; a lane's record is broadcast to the lanes of a target group) ----
+                fetch(lane, 0, zseg[0]);
+                int zone = 0;
+                for (int p0 = 0; p0 < total; p0 += 32, zone ^= 1) {
+                    const int n = min(32, total - p0);
+                    cp_async_wait_group<0>();
+                    if (lane < n) {  // fix up this lane's own record in place
+                        double *raw = traw[wid][zone][lane];
+                        if constexpr (DIRECT) {
+                            double f[K::SDIM], v[NV];
+#pragma unroll
+                            for (int q = 0; q < K::SDIM; q++) f[q] = raw[3 + q];
+                            K::stage(f, v);
+#pragma unroll
+                            for (int q = 0; q < NV; q++) raw[3 + q] = v[q];
+                        } else {
+                            const int cd = s_code[zseg[0]] & 31;
+                            if (cd != kShiftNoneCode) {  // periodic image
+                                raw[0] += (cd % 3 - 1) * a.period;
+                                raw[1] += ((cd / 3) % 3 - 1) * a.period;
+                                raw[2] += (cd / 9 - 1) * a.period;
+                            }
+                        }
+                    }
+                    __syncwarp();  // the tile is complete, and the previous one no longer read
+                    fetch(p0 + 32 + lane, zone ^ 1, zseg[0]);
+                    const double(*tile)[RSS] = traw[wid][zone];
+STK_UNROLL(STK_P2P_UNROLL_FP64)
+                    for (int j = sub; j < n; j += g) {
+                        double rn[RS];
+#pragma unroll
+                        for (int q = 0; q < RS / 2; q++) {
+                            const double2 t2 = *reinterpret_cast<const double2 *>(&tile[j][2 * q]);
+                            rn[2 * q] = t2.x;
+                            rn[2 * q + 1] = t2.y;
+                        }
+#pragma unroll
+                        for (int h = 0; h < TPL; h++)
+                            eval(acc[h], xt[h][0] - rn[0], xt[h][1] - rn[1], xt[h][2] - rn[2], rn + 3, ta[h]);
+                    }
+                }
+                __syncwarp();  // the last tile has been read
+                continue;
+            }
 #pragma unroll
             for (int z = 0; z < DEPTH; z++) fetch(32 * z + lane, z, zseg[z]);
             int p0 = 0, zone = 0;
@@ -408,9 +465,10 @@ __global__ void __launch_bounds__(Cta<MIXED>::threads, MinBlocks<UK, MIXED>::val
                     double x[3];
                     if (lane < n) {
                         const double *raw = traw[wid][zone][lane];
-                        double rn[RS];
+                        constexpr int RR = DIRECT ? Rec<UK>::SLOT : RS;
+                        double rn[RR];
 #pragma unroll
-                        for (int q = 0; q < RS / 2; q++) {
+                        for (int q = 0; q < RR / 2; q++) {
                             const double2 t2 = *reinterpret_cast<const double2 *>(raw + 2 * q);
                             rn[2 * q] = t2.x;
                             rn[2 * q + 1] = t2.y;
@@ -430,7 +488,12 @@ __global__ void __launch_bounds__(Cta<MIXED>::threads, MinBlocks<UK, MIXED>::val
                                 x[2] += (cd / 9 - 1) * a.period;
                             }
                         }
-                        K::stage(rn + 3, v);
+                        if constexpr (DIRECT) {
+                            K::stage(rn + 3, v);
+                        } else {
+#pragma unroll
+                            for (int q = 0; q < NV; q++) v[q] = rn[3 + q];
+                        }
                     } else {
 #pragma unroll
                         for (int k = 0; k < 3; k++) x[k] = c[k] + kPadCoord;
@@ -447,7 +510,7 @@ __global__ void __launch_bounds__(Cta<MIXED>::threads, MinBlocks<UK, MIXED>::val
                         }
                     } else {
 #pragma unroll
-                        for (int k = 0; k < 3; k++) mc[k][lane] = x[k] - c[k];  // c = 0 on the FP64 path
+                        for (int k = 0; k < 3; k++) mc[k][lane] = x[k] - c[k];
                     }
 #pragma unroll
                     for (int q = 0; q < NV; q++) mv[q][lane] = (S)v[q];
@@ -516,17 +579,6 @@ STK_UNROLL(STK_P2P_UNROLL_MIXED)
                     // Kahan-compensated accumulation of the partial sums once a lane has
                     // evaluated ~32 sources since the last step (every g tiles)
                     if (++kahan_tiles >= kKahanTiles * g) kahan_step();
-                } else {
-STK_UNROLL(STK_P2P_UNROLL_FP64)
-                    for (int j = sub; j < n; j += g) {
-                        double sv[NV];
-#pragma unroll
-                        for (int q = 0; q < NV; q++) sv[q] = mv[q][j];
-                        const double sx = mc[0][j], sy = mc[1][j], sz = mc[2][j];
-#pragma unroll
-                        for (int h = 0; h < TPL; h++)
-                            eval(acc[h], xt[h][0] - sx, xt[h][1] - sy, xt[h][2] - sz, sv, ta[h]);
-                    }
                 }
             }
         }
@@ -555,14 +607,20 @@ STK_UNROLL(STK_P2P_UNROLL_FP64)
             for (int h = 0; h < TPL; h++) {
                 if (!act[h]) continue;
                 double *dst = a.trg_out + (size_t)tt[h] * TDIM;
-                if constexpr (DIRECT)
+                bool store = false;  // a part's own slot
+                if constexpr (DIRECT) {
+                    store = a.atomic_out == 0;
                     if (a.parts) dst = a.parts + ((size_t)w.e0 * a.ntrg + tt[h]) * TDIM;
+                } else if (w.part >= 0) {
+                    store = true;
+                    dst = a.parts + (size_t)(w.part + tt[h] - w.t0) * TDIM;
+                }
 #pragma unroll
                 for (int k = 0; k < TDIM; k++) {
                     const double val = K::SCALE * K::comp_scale(k) * o[h][k];
-                    if (DIRECT && !a.atomic_out)  // atomic_out: add (to the caller's values)
+                    if (store)
                         dst[k] = val;
-                    else if (!DIRECT && a.atomic_out)
+                    else if (a.atomic_out == 2)
                         atomicAdd(dst + k, val);
                     else
                         dst[k] += val;
@@ -609,29 +667,88 @@ template <int UK = 0, class F> cudaError_t with_uk(int uk, const F &f) {
     }
 }
 
+// trg_out += the parts of targets whose sources were split over items, in order
+__global__ void add_parts_kernel(const PartGroup *__restrict__ groups, int n, int d, const double *__restrict__ parts,
+                                 double *__restrict__ out) {
+    for (int i = blockIdx.x; i < n; i += gridDim.x) {
+        const PartGroup g = groups[i];
+        const int m = g.nt * d;
+        for (int j = threadIdx.x; j < m; j += blockDim.x) {
+            const double *p = parts + (size_t)g.part0 * d + j;
+            double v = 0.0;
+#pragma unroll 4
+            for (int k = 0; k < g.n_parts; k++) v += p[(size_t)k * m];
+            out[(size_t)g.t0 * d + j] += v;
+        }
+    }
+}
+
 // out[i] (=|+=) the chunks' sums, in order
 __global__ void sum_chunks_kernel(const double *__restrict__ parts, int n_chunk, long long n, int add,
                                   double *__restrict__ out) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         double v = parts[i];
+#pragma unroll 8
         for (int k = 1; k < n_chunk; k++) v += parts[k * n + i];
         out[i] = add ? out[i] + v : v;
     }
 }
 
+// One thread per source: its values staged once here instead of in every tile that reads it.
+template <int UK>
 __global__ void pack_records_kernel(int n, const int *__restrict__ perm, const double *__restrict__ xyz,
-                                    const double *__restrict__ v1, int d1, const double *__restrict__ v2, int d2,
-                                    int stride, double *__restrict__ rec) {
+                                    const double *__restrict__ v1, int d1, const double *__restrict__ v2,
+                                    double *__restrict__ rec) {
+    using K = Uk<UK>;
+    constexpr int RS = Rec<UK>::RS;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int p = perm ? perm[i] : i;
-        double *r = rec + (size_t)i * stride;
-        r[0] = xyz[3 * (size_t)i + 0];
-        r[1] = xyz[3 * (size_t)i + 1];
-        r[2] = xyz[3 * (size_t)i + 2];
-        int q = 3;
-        for (int k = 0; k < d1; k++) r[q++] = v1[(size_t)p * d1 + k];
-        for (int k = 0; k < d2; k++) r[q++] = v2[(size_t)p * d2 + k];
-        for (; q < stride; q++) r[q] = 0.0;
+        double f[K::SDIM], r[RS], v[K::NV];
+#pragma unroll
+        for (int k = 0; k < K::SDIM; k++)
+            f[k] = k < d1 ? v1[(size_t)p * d1 + k] : v2[(size_t)p * (K::SDIM - d1) + k - d1];
+        K::stage(f, v);
+#pragma unroll
+        for (int k = 0; k < 3; k++) r[k] = xyz[3 * (size_t)i + k];
+#pragma unroll
+        for (int k = 3; k < RS; k++) r[k] = k - 3 < K::NV ? v[k - 3 < K::NV ? k - 3 : 0] : 0.0;
+        double2 *o = reinterpret_cast<double2 *>(rec + (size_t)i * RS);
+#pragma unroll
+        for (int k = 0; k < RS / 2; k++) o[k] = make_double2(r[2 * k], r[2 * k + 1]);
+    }
+}
+
+struct DensExp {
+    double v[4];
+};
+
+template <int UK>
+__global__ void pack_surface_kernel(const int *__restrict__ nodes, int m, int n, const double *__restrict__ xyz,
+                                    const double *__restrict__ dens, const int *__restrict__ level, DensExp e,
+                                    double *__restrict__ rec) {
+    using K = Uk<UK>;
+    constexpr int RS = Rec<UK>::RS;
+    const long long total = (long long)m * n;
+    for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
+         idx += (long long)gridDim.x * blockDim.x) {
+        const int i = (int)(idx / n), j = (int)(idx - (long long)i * n), b = nodes[i];
+        const size_t p = (size_t)b * n + j;
+        double f[K::SDIM], r[RS], v[K::NV];
+#pragma unroll
+        for (int k = 0; k < K::SDIM; k++) f[k] = dens[p * K::SDIM + k];
+        if (level) {
+#pragma unroll
+            for (int k = 0; k < K::SDIM; k++)
+                if (e.v[k & 3] != 0.0) f[k] *= exp2(-(double)level[b] * e.v[k & 3]);
+        }
+        K::stage(f, v);
+#pragma unroll
+        for (int k = 0; k < 3; k++) r[k] = xyz[3 * p + k];
+#pragma unroll
+        for (int k = 3; k < RS; k++) r[k] = k - 3 < K::NV ? v[k - 3 < K::NV ? k - 3 : 0] : 0.0;
+        double2 *o = reinterpret_cast<double2 *>(rec + p * RS);
+#pragma unroll
+        for (int k = 0; k < RS / 2; k++) o[k] = make_double2(r[2 * k], r[2 * k + 1]);
     }
 }
 
@@ -653,16 +770,28 @@ int uk_sdim_host(int uk) { return uk_sdim(uk); }
 int uk_tdim_host(int uk) { return uk_tdim(uk); }
 int uk_tvdim_host(int uk) { return uk_tvdim(uk); }
 double uk_scale_host(int uk) { return uk_scale(uk); }
-int uk_record_stride(int uk) { return (3 + uk_sdim(uk) + 1) & ~1; }
+int uk_record_stride(int uk) {
+    int rs = 0;
+    with_uk(uk, [&](auto id) {
+        rs = Rec<decltype(id)::value>::RS;
+        return cudaSuccess;
+    });
+    return rs;
+}
 
 cudaError_t launch_list_p2p(int uk, int prec, const ListP2PArgs &a, int num_sms, cudaStream_t stream) {
     if (a.n_items <= 0) return cudaSuccess;
     if (uk >= 0 && uk < UK_COUNT && uk_tvdim(uk) > 0 && !a.trg_aux) return cudaErrorInvalidValue;
-    return with_uk(uk, [&](auto id) {
+    if (a.n_groups > 0 && (!a.groups || !a.parts)) return cudaErrorInvalidValue;
+    const cudaError_t e = with_uk(uk, [&](auto id) {
         constexpr int UK = decltype(id)::value;
         return prec == PREC_MIXED ? launch_impl<UK, true, false>(a, num_sms, stream)
                                   : launch_impl<UK, false, false>(a, num_sms, stream);
     });
+    if (e != cudaSuccess || a.n_groups == 0) return e;
+    add_parts_kernel<<<std::min(a.n_groups, 148 * 16), 128, 0, stream>>>(a.groups, a.n_groups, uk_tdim(uk), a.parts,
+                                                                         a.trg_out);
+    return cudaGetLastError();
 }
 
 // FP64: chunks so that the equal items fill whole turns of the resident warps.  An item costs
@@ -706,30 +835,49 @@ cudaError_t launch_direct_p2p(int uk, int prec, const ListP2PArgs &args, int add
     if (uk < 0 || uk >= UK_COUNT || (uk_tvdim(uk) > 0) != (args.trg_aux != nullptr)) return cudaErrorInvalidValue;
     const bool split = args.n_chunk > 1;
     const long long items = (long long)((args.ntrg + 63) / 64) * args.n_chunk;
-    if ((split && !args.parts) || items > 0x7fffffffll) return cudaErrorInvalidValue;
+    if ((split && add != 2 && !args.parts) || items > 0x7fffffffll) return cudaErrorInvalidValue;
     ListP2PArgs a = args;
     a.n_items = (int)items;
     if (!split) a.parts = nullptr;
-    a.atomic_out = !split && add;
+    a.atomic_out = split && add != 2 ? 0 : add;
+    if (add == 2) a.parts = nullptr;
     cudaError_t e = with_uk(uk, [&](auto id) {
         constexpr int UK = decltype(id)::value;
         return prec == PREC_MIXED ? launch_impl<UK, true, true>(a, num_sms, stream)
                                   : launch_impl<UK, false, true>(a, num_sms, stream);
     });
-    if (e != cudaSuccess || !split) return e;
+    if (e != cudaSuccess || !split || add == 2) return e;
     const long long n = (long long)a.ntrg * uk_tdim(uk);
     sum_chunks_kernel<<<(int)std::min<long long>((n + 255) / 256, 148 * 16), 256, 0, stream>>>(a.parts, a.n_chunk, n, add,
                                                                                              a.trg_out);
     return cudaGetLastError();
 }
 
-cudaError_t launch_pack_records(int n, const int *perm, const double *xyz, const double *v1, int d1,
-                                const double *v2, int d2, int stride, double *rec, cudaStream_t stream) {
+cudaError_t launch_pack_records(int uk, int n, const int *perm, const double *xyz, const double *v1, int d1,
+                                const double *v2, double *rec, cudaStream_t stream) {
     if (n <= 0) return cudaSuccess;
-    const int threads = 256;
-    const int grid = std::min((n + threads - 1) / threads, 148 * 16);
-    pack_records_kernel<<<grid, threads, 0, stream>>>(n, perm, xyz, v1, d1, v2, d2, stride, rec);
-    return cudaGetLastError();
+    if (uk < 0 || uk >= UK_COUNT || (d1 < uk_sdim(uk)) != (v2 != nullptr)) return cudaErrorInvalidValue;
+    return with_uk(uk, [&](auto id) {
+        const int threads = 256;
+        const int grid = std::min((n + threads - 1) / threads, 148 * 16);
+        pack_records_kernel<decltype(id)::value><<<grid, threads, 0, stream>>>(n, perm, xyz, v1, d1, v2, rec);
+        return cudaGetLastError();
+    });
+}
+
+cudaError_t launch_pack_surface(int uk, const int *nodes, int m, int n, const double *xyz, const double *dens,
+                                const int *level, const double *den_exp, double *rec, cudaStream_t stream) {
+    if (m <= 0) return cudaSuccess;
+    if (uk < 0 || uk >= UK_COUNT || uk_sdim(uk) > 4) return cudaErrorInvalidValue;
+    return with_uk(uk, [&](auto id) {
+        constexpr int UK = decltype(id)::value;
+        if constexpr (Uk<UK>::SDIM <= 4) {
+            const DensExp e = {{den_exp[0], den_exp[1], den_exp[2], den_exp[3]}};
+            const int grid = (int)std::min<long long>(((long long)m * n + 255) / 256, 148 * 16);
+            pack_surface_kernel<UK><<<grid, 256, 0, stream>>>(nodes, m, n, xyz, dens, level, e, rec);
+        }
+        return cudaGetLastError();
+    });
 }
 
 cudaError_t launch_scatter_add(int n, int d, const int *perm, const double *in, const double *alpha, double *out,

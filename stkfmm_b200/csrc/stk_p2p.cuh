@@ -18,11 +18,22 @@ struct WorkItem {
     int glog; // lanes per target = 1 << glog
     int e0;   // first list entry
     int e1;   // one past the last list entry
+    // FP64 items (build_split_items): the range of the entries' sources, from source `skip` of
+    // the first entry to source `stop` (exclusive) of the last, and where the sums of a
+    // part go (target slot in ListP2PArgs::parts; -1: added to trg_out)
+    int skip = 0, stop = 0x7fffffff;
+    int part = -1;
+};
+
+// Targets whose sources were split over several items: n_parts runs of nt target slots from
+// slot part0 on, added to trg_out in order.
+struct PartGroup {
+    int t0, nt, part0, n_parts;
 };
 
 // Device-resident description of one list evaluation.
 struct ListP2PArgs {
-    const double *src_rec;     // source records, RS doubles each: x, y, z, values..., padding
+    const double *src_rec;     // source records, RS doubles each: x, y, z, staged values..., padding
     const int *src_box_begin;  // per source box: first record
     const int *src_box_end;    // per source box: one past the last record
     const int *list_ent;       // per entry: (source box << 5) | periodic shift code (0..26, 13 = none)
@@ -39,14 +50,16 @@ struct ListP2PArgs {
                                // entry of the target's own box (lists of one octree over both
                                // point sets); the mixed path then skips the coincidence mask
                                // elsewhere.  0: every pair is masked.
+    const PartGroup *groups;   // targets with split sources, their sums in `parts`
+    int n_groups;
     // direct sums only (launch_direct_p2p): all sources against all targets
     const double *src_xyz, *src_val;  // 3 and SDIM doubles per source
     int nsrc, ntrg;
     int src_chunk, n_chunk;  // source points per chunk (a multiple of 32), chunks
-    double *parts;           // outputs of each chunk, ntrg x TDIM each (null: one chunk, added to trg_out)
+    double *parts;           // outputs of each chunk, ntrg x TDIM each (null: one chunk)
 };
 
-// Record stride (doubles) for a micro-kernel: 3 coordinates + SDIM values,
+// Record stride (doubles) for a micro-kernel: 3 coordinates + NV staged values,
 // rounded up to a 16-byte multiple.
 int uk_record_stride(int uk);
 int uk_sdim_host(int uk);
@@ -63,14 +76,18 @@ cudaError_t launch_list_p2p(int uk, int prec, const ListP2PArgs &a, int num_sms,
 // same bits).  direct_chunks: sources per chunk (a multiple of 32) and the number of chunks.
 void direct_chunks(int uk, int prec, int ntrg, int nsrc, int num_sms, int &chunk, int &n_chunk);
 // a: src_xyz, src_val, nsrc, ntrg, src_chunk, n_chunk, parts (n_chunk > 1), trg_xyz, trg_aux and
-// trg_out; add = 0: trg_out = sum, 1: +=
+// trg_out; add = 0: trg_out = sum, 1: +=, 2: += by atomics, without parts
 cudaError_t launch_direct_p2p(int uk, int prec, const ListP2PArgs &a, int add, int num_sms, cudaStream_t stream);
 
-// rec[i] = (xyz[perm[i]], v1[perm[i]] (d1 values), v2[perm[i]] (d2 values), 0 padding)
-// perm may be null (identity).  v2 may be null (d2 = 0).  Coordinates are
-// multiplied by coord_scale after subtracting coord_shift (per axis).
-cudaError_t launch_pack_records(int n, const int *perm, const double *xyz, const double *v1, int d1,
-                                const double *v2, int d2, int stride, double *rec, cudaStream_t stream);
+// Source records of micro-kernel uk: rec[i] = (xyz[i], stage(v1[perm[i]] (d1 values),
+// v2[perm[i]] (the rest of SDIM)), 0 padding); perm may be null (identity), v2 null.
+cudaError_t launch_pack_records(int uk, int n, const int *perm, const double *xyz, const double *v1, int d1,
+                                const double *v2, double *rec, cudaStream_t stream);
+
+// Records of KIFMM surfaces: for each listed node b, rec[b n + i] = (xyz[b n + i], stage(densities
+// of its point i, component c times 2^(-level[b] den_exp[c]))), i < n; level null: no factor.
+cudaError_t launch_pack_surface(int uk, const int *nodes, int m, int n, const double *xyz, const double *dens,
+                                const int *level, const double *den_exp, double *rec, cudaStream_t stream);
 
 // out[perm[i] * d + k] += alpha_k * in[i * d + k]   (alpha per component; perm may be null)
 cudaError_t launch_scatter_add(int n, int d, const int *perm, const double *in, const double *alpha,

@@ -27,9 +27,14 @@ struct stk_p2p_plan {
     int n_src_box = 0;
     double period = 1.0;
     long long pairs = 0;
-    int n_items = 0;
+    int n_items[2] = {0, 0};  // FP64 (split), mixed
+    int n_groups = 0;
+    long long part_targets = 0;
     int *d_sbeg = nullptr, *d_send = nullptr, *d_ent = nullptr;
-    stk::WorkItem *d_items = nullptr;
+    stk::WorkItem *d_items[2] = {nullptr, nullptr};
+    stk::PartGroup *d_groups = nullptr;
+    double *d_parts = nullptr;  // sums of split sources, grown to the largest micro-kernel used
+    size_t parts_cap = 0;       // doubles
     unsigned int *d_counter = nullptr;
     double *d_rec = nullptr;  // packed source records, grown to the largest record stride used
     size_t rec_cap = 0;       // doubles
@@ -37,7 +42,10 @@ struct stk_p2p_plan {
         cudaFree(d_sbeg);
         cudaFree(d_send);
         cudaFree(d_ent);
-        cudaFree(d_items);
+        cudaFree(d_items[0]);
+        cudaFree(d_items[1]);
+        cudaFree(d_groups);
+        cudaFree(d_parts);
         cudaFree(d_counter);
         cudaFree(d_rec);
     }
@@ -99,16 +107,24 @@ extern "C" stk_p2p_plan *stk_p2p_plan_create(int n_trg_box, const int *trg_begin
     p->ntrg = ntrg;
     p->n_src_box = n_src_box;
     p->period = period;
-    std::vector<stk::WorkItem> items;
-    if (n_trg_box > 0)
-        stk::build_list_items(n_trg_box, trg_begin, trg_end, list_off, list_ent, src_begin, src_end, items, p->pairs);
-    p->n_items = (int)items.size();
     const int nent = n_trg_box > 0 ? list_off[n_trg_box] : 0;
     bool ok = cudaGetDevice(&p->device) == cudaSuccess &&
               cudaDeviceGetAttribute(&p->num_sms, cudaDevAttrMultiProcessorCount, p->device) == cudaSuccess &&
               cudaMalloc(&p->d_counter, 64) == cudaSuccess && upload(&p->d_sbeg, src_begin, n_src_box) == cudaSuccess &&
-              upload(&p->d_send, src_end, n_src_box) == cudaSuccess && upload(&p->d_ent, list_ent, nent) == cudaSuccess &&
-              upload(&p->d_items, items.data(), items.size()) == cudaSuccess;
+              upload(&p->d_send, src_end, n_src_box) == cudaSuccess && upload(&p->d_ent, list_ent, nent) == cudaSuccess;
+    if (ok && n_trg_box > 0) {
+        std::vector<stk::WorkItem> items;
+        std::vector<stk::PartGroup> groups;
+        stk::build_list_items(n_trg_box, trg_begin, trg_end, list_off, list_ent, src_begin, src_end, items, p->pairs);
+        p->n_items[1] = (int)items.size();
+        ok = upload(&p->d_items[1], items.data(), items.size()) == cudaSuccess;
+        stk::build_split_items(n_trg_box, trg_begin, trg_end, list_off, list_ent, src_begin, src_end, p->num_sms * 15,
+                               items, groups, p->part_targets);
+        p->n_items[0] = (int)items.size();
+        p->n_groups = (int)groups.size();
+        ok = ok && upload(&p->d_items[0], items.data(), items.size()) == cudaSuccess &&
+             upload(&p->d_groups, groups.data(), groups.size()) == cudaSuccess;
+    }
     if (!ok) {
         cudaGetLastError();
         delete p;
@@ -137,28 +153,34 @@ extern "C" int stk_p2p_plan_execute(stk_p2p_plan *plan, int ukernel, int precisi
     if (!plan || ukernel < 0 || ukernel >= stk::UK_COUNT) return STK_ERR_INVALID_ARG;
     if (precision != stk::PREC_FP64 && precision != stk::PREC_MIXED) return STK_ERR_INVALID_ARG;
     if ((stk::uk_tvdim_host(ukernel) > 0) != (d_trg_aux != nullptr)) return STK_ERR_INVALID_ARG;
-    if (plan->n_items == 0) return STK_OK;
+    const bool mixed = precision == stk::PREC_MIXED;
+    if (plan->n_items[mixed] == 0) return STK_OK;
     if ((plan->nsrc > 0 && (!d_src_coord || !d_src_value)) || !d_trg_coord || !d_trg_value) return STK_ERR_INVALID_ARG;
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev != plan->device) return STK_ERR_INVALID_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     const int sd = stk::uk_sdim_host(ukernel), rs = stk::uk_record_stride(ukernel);
-    const size_t need = (size_t)std::max(plan->nsrc, 1) * rs;
-    if (plan->rec_cap < need) {
-        // grow the record buffer: earlier executions may still read it on any stream
-        if (plan->d_rec) {
+    // grow a buffer: earlier executions may still use it on any stream
+    auto grow = [](double **buf, size_t *cap, size_t need) {
+        if (*cap >= need) return true;
+        if (*buf) {
             cudaDeviceSynchronize();
-            cudaFree(plan->d_rec);
-            plan->d_rec = nullptr;
-            plan->rec_cap = 0;
+            cudaFree(*buf);
+            *buf = nullptr;
+            *cap = 0;
         }
-        if (cudaMalloc(&plan->d_rec, need * sizeof(double)) != cudaSuccess) {
+        if (cudaMalloc(buf, need * sizeof(double)) != cudaSuccess) {
             cudaGetLastError();
-            return STK_ERR_CUDA;
+            return false;
         }
-        plan->rec_cap = need;
-    }
-    if (stk::launch_pack_records(plan->nsrc, nullptr, d_src_coord, d_src_value, sd, nullptr, 0, rs, plan->d_rec, s) !=
+        *cap = need;
+        return true;
+    };
+    if (!grow(&plan->d_rec, &plan->rec_cap, (size_t)std::max(plan->nsrc, 1) * rs)) return STK_ERR_CUDA;
+    if (!mixed && plan->n_groups > 0 &&
+        !grow(&plan->d_parts, &plan->parts_cap, (size_t)plan->part_targets * stk::uk_tdim_host(ukernel)))
+        return STK_ERR_CUDA;
+    if (stk::launch_pack_records(ukernel, plan->nsrc, nullptr, d_src_coord, d_src_value, sd, nullptr, plan->d_rec, s) !=
         cudaSuccess)
         return STK_ERR_CUDA;
     stk::ListP2PArgs a{};
@@ -166,8 +188,13 @@ extern "C" int stk_p2p_plan_execute(stk_p2p_plan *plan, int ukernel, int precisi
     a.src_box_begin = plan->d_sbeg;
     a.src_box_end = plan->d_send;
     a.list_ent = plan->d_ent;
-    a.items = plan->d_items;
-    a.n_items = plan->n_items;
+    a.items = plan->d_items[mixed];
+    a.n_items = plan->n_items[mixed];
+    if (!mixed) {
+        a.groups = plan->d_groups;
+        a.n_groups = plan->n_groups;
+        a.parts = plan->d_parts;
+    }
     a.counter = plan->d_counter;
     a.trg_xyz = d_trg_coord;
     a.trg_out = d_trg_value;

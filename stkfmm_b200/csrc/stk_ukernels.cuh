@@ -47,6 +47,8 @@
 // and a double-layer source at the same point in one pass:
 //   laplace_pgrad + laplace_dipolepgrad, stokes_pvel + stokes_doublepvel.
 #pragma once
+#include <type_traits>
+
 #include <cuda_runtime.h>
 
 namespace stk {
@@ -329,6 +331,17 @@ template <> struct Uk<UK_RPY_ULAPU> {
         V rinv3 = rinv2 * rinv;
         V c = fmav(v[0], dx, fmav(v[1], dy, v[2] * dz)) * rinv2;
         V nc3 = c * cst<V>(-3.0);
+        if constexpr (std::is_same<V, double>::value) {
+            // u = f (1/r + a^2/3 / r^3) + r c (1/r - a^2 / r^3): three operations fewer
+            const double k3 = v[3] * rinv3, P = rinv + k3, Q = c * fma(-3.0, k3, rinv);
+            u[0] = fmav(Q, dx, fmav(v[0], P, u[0]));
+            u[1] = fmav(Q, dy, fmav(v[1], P, u[1]));
+            u[2] = fmav(Q, dz, fmav(v[2], P, u[2]));
+            u[3] = fmav(fmav(nc3, dx, v[0]), rinv3, u[3]);
+            u[4] = fmav(fmav(nc3, dy, v[1]), rinv3, u[4]);
+            u[5] = fmav(fmav(nc3, dz, v[2]), rinv3, u[5]);
+            return;
+        }
         V Cx = fmav(nc3, dx, v[0]) * rinv3;
         V Cy = fmav(nc3, dy, v[1]) * rinv3;
         V Cz = fmav(nc3, dz, v[2]) * rinv3;

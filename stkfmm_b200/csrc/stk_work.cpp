@@ -219,6 +219,119 @@ void build_list_items(int n_trg_box, const int *trg_begin, const int *trg_end, c
     items.swap(sorted);
 }
 
+// Targets of the next chunk of `left` remaining ones.  A chunk of m targets with g = 2^glog
+// lanes each goes through every source in 1/g of a turn, and every 32-source tile costs about
+// one and a half turns beside (its copy, wait and loop start): the remainder is either taken
+// whole or cut at the largest power of two, whichever is cheaper in sum.
+static int split_remainder(int left) {
+    static const std::vector<int> next = [] {
+        std::vector<int> n(kItemTargets + 1, 0);
+        std::vector<double> cost(kItemTargets + 1, 0.0);
+        for (int r = 1; r <= kItemTargets; r++) {
+            const double tile = 1.5 / 32;
+            int p = 1;
+            while (p * 2 <= r) p *= 2;
+            const double whole = 1.0 / (1 << lanes_log2(r)) + tile;
+            const double cut = p < r ? 1.0 / (1 << lanes_log2(p)) + tile + cost[r - p] : whole;
+            n[r] = cut < whole ? p : r;
+            cost[r] = std::min(cut, whole);
+        }
+        return n;
+    }();
+    return next[std::min(left, kItemTargets)];
+}
+
+void build_split_items(int n_trg_box, const int *trg_begin, const int *trg_end, const int *list_off,
+                       const int *list_ent, const int *src_begin, const int *src_end, int warps,
+                       std::vector<WorkItem> &items, std::vector<PartGroup> &groups, long long &part_targets,
+                       int shard_rank, int shard_n) {
+    items.clear();
+    groups.clear();
+    part_targets = 0;
+    struct Chunk {
+        int box, t0, nt, glog;
+        long long ns, turns;  // sources; sources a lane goes through
+    };
+    std::vector<Chunk> chunks;
+    long long total = 0;
+    for (int b = 0; b < n_trg_box; b++) {
+        const int nt = trg_end[b] - trg_begin[b];
+        if (nt <= 0) continue;
+        long long ns = 0;
+        for (int e = list_off[b]; e < list_off[b + 1]; e++) {
+            const int sb = list_ent[e] >> 5;
+            ns += src_end[sb] - src_begin[sb];
+        }
+        if (ns == 0) continue;
+        for (int t0 = trg_begin[b], left = nt; left > 0;) {
+            const int m = split_remainder(left);
+            const int glog = lanes_log2(m);
+            const long long turns = (ns + (1 << glog) - 1) >> glog;
+            chunks.push_back({b, t0, m, glog, ns, turns});
+            total += turns;
+            t0 += m;
+            left -= m;
+        }
+    }
+    if (shard_n > 1) {
+        // chunks dealt largest first to the least-loaded shard: the same assignment on every shard
+        std::vector<int> idx(chunks.size()), owner;
+        std::iota(idx.begin(), idx.end(), 0);
+        std::stable_sort(idx.begin(), idx.end(), [&](int a, int b) { return chunks[a].turns > chunks[b].turns; });
+        std::vector<double> cost;
+        for (int i : idx) cost.push_back((double)chunks[i].turns);
+        partition_lpt((int)cost.size(), cost.data(), shard_n, owner);
+        std::vector<Chunk> own;
+        total = 0;
+        for (size_t i = 0; i < idx.size(); i++)
+            if (owner[i] == shard_rank) {
+                own.push_back(chunks[idx[i]]);
+                total += own.back().turns;
+            }
+        chunks.swap(own);
+    }
+    // A quarter of a warp's share, at least 64 sources per lane (a shorter run would be mostly
+    // the first tile's latency and the output): 32k Stokes points, 128 per leaf, run as 4600
+    // items of 64 x 384 pairs instead of 4096 of 8 x 1700.
+    const long long cap = std::max(total / (4LL * std::max(warps, 1)), 64LL);
+    std::vector<std::pair<long long, int>> cost;
+    for (const Chunk &c : chunks) {
+        const int g = 1 << c.glog;
+        long long np = std::max(1LL, std::min(c.turns / std::max(cap / 2, 1LL), (c.turns + cap - 1) / cap));
+        const long long len = ((c.ns + np - 1) / np + 31) / 32 * 32;
+        np = (c.ns + len - 1) / len;
+        int e = list_off[c.box];
+        long long at = 0;  // sources of the entries before e
+        const int part0 = (int)part_targets;
+        for (long long j = 0; j < np; j++) {
+            const long long a = j * len, z = std::min(c.ns, a + len);
+            auto size = [&](int q) {
+                const int sb = list_ent[q] >> 5;
+                return (long long)(src_end[sb] - src_begin[sb]);
+            };
+            while (at + size(e) <= a) at += size(e++);  // the entry that holds source a
+            WorkItem w{c.box, c.t0, c.nt, c.glog, e, e + 1};
+            w.skip = (int)(a - at);
+            long long end = at + size(e);
+            while (end < z) end += size(w.e1++);
+            w.stop = (int)(z - (end - size(w.e1 - 1)));
+            if (np > 1) {
+                w.part = (int)part_targets;
+                part_targets += c.nt;
+            }
+            cost.push_back({(z - a) / g, (int)items.size()});
+            items.push_back(w);
+        }
+        if (np > 1) groups.push_back({c.t0, c.nt, part0, (int)np});
+    }
+    // longest first
+    std::stable_sort(cost.begin(), cost.end(), [](const auto &a, const auto &b) { return a.first > b.first; });
+    std::vector<WorkItem> sorted;
+    sorted.reserve(items.size());
+    for (const auto &c : cost) sorted.push_back(items[c.second]);
+    items.swap(sorted);
+}
+
 long long pair_sources(const WorkItem &w, const int *list_ent, const int *src_begin, const int *src_end) {
     long long ns = 0;
     for (int e = w.e0; e < w.e1; e++) {

@@ -18,7 +18,7 @@ namespace stk {
 // to the next thread when its thread ends and is never freed before exit.
 class Workspace {
   public:
-    enum Slot { kRec, kSrcBeg, kSrcEnd, kEnt, kItems, kParts, kHostIn, kHostOut, kNumSlots };
+    enum Slot { kRec, kSrcBeg, kSrcEnd, kEnt, kItems, kGroups, kParts, kHostIn, kHostOut, kNumSlots };
     static Workspace &thread_local_ws();
     ~Workspace();
     int ensure_device();  // STK_OK, STK_ERR_NO_DEVICE or STK_ERR_CUDA
@@ -62,6 +62,17 @@ class Workspace {
 void build_list_items(int n_trg_box, const int *trg_begin, const int *trg_end, const int *list_off,
                       const int *list_ent, const int *src_begin, const int *src_end, std::vector<WorkItem> &items,
                       long long &pairs, int balance_warps = 0, int shard_rank = 0, int shard_n = 1);
+
+// The FP64 path's items of the same lists: 64 targets (or the 32 / 16 / 8 / < 8 of a box's
+// remainder) against a range of the box's sources.  A box's targets whose sources take one
+// warp longer than a share of the pass on `warps` warps are split into equal runs of whole
+// 32-source tiles, their sums kept in `part_targets` target slots and added in order
+// (groups).  Splitting the sources keeps 64 targets per staged source where smaller target
+// chunks would stage every source several times.  shard_n > 1: the items of shard shard_rank.
+void build_split_items(int n_trg_box, const int *trg_begin, const int *trg_end, const int *list_off,
+                       const int *list_ent, const int *src_begin, const int *src_end, int warps,
+                       std::vector<WorkItem> &items, std::vector<PartGroup> &groups, long long &part_targets,
+                       int shard_rank = 0, int shard_n = 1);
 
 // Source points of one work item (the sum over its list entries).
 long long pair_sources(const WorkItem &w, const int *list_ent, const int *src_begin, const int *src_end);
