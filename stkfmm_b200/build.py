@@ -85,7 +85,7 @@ def build_octree(force: bool = False) -> str:
     if force or not os.path.exists(OCTREE_LIB) or os.path.getmtime(OCTREE_LIB) < _newest(deps):
         cxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else (shutil.which("g++") or "c++")
         tmp = OCTREE_LIB + ".tmp"
-        cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-I" + INCLUDE, "-o", tmp] + srcs
+        cmd = [cxx, "-O2", "-std=c++17", "-pthread", "-fPIC", "-shared", "-I" + INCLUDE, "-o", tmp] + srcs
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError("g++ failed on libstk_octree.so:\n%s%s" % (r.stdout, r.stderr))

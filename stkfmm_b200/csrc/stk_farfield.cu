@@ -1378,20 +1378,24 @@ static int setup_m2l_chunks_tc(FarField &F, const std::vector<int> &chunk_slot, 
     for (int sl = 0; sl < nslot; sl++) qrows += F.m2l_r[sl];
     const size_t bytes = 8 * ((size_t)qrows * k4 + (size_t)nslot * k * rmax);
     if (bytes > (4ull << 30)) return STK_OK;
-    int rc = F.tcc_q_hi.reserve(sizeof(float) * (size_t)qrows * k4);
-    if (!rc) rc = F.tcc_q_lo.reserve(sizeof(float) * (size_t)qrows * k4);
-    if (!rc) rc = F.tcc_pt_hi.reserve(sizeof(float) * (size_t)nslot * k * rmax);
-    if (!rc) rc = F.tcc_pt_lo.reserve(sizeof(float) * (size_t)nslot * k * rmax);
-    if (rc) return rc;
-    // Q_d (k x r_d column-major, offsets back to back) read as qrows K-major rows of k
-    tc_rows_kernel<<<grid_for(qrows * k4), 256, 0, s>>>((const double *)F.m2l_q.ptr, k, qrows, k4,
-                                                        (float *)F.tcc_q_hi.ptr, (float *)F.tcc_q_lo.ptr);
-    FCUDA(cudaGetLastError());
-    for (int sl = 0; sl < nslot; sl++) {
-        tc_trows_kernel<<<grid_for((long long)k * rmax), 256, 0, s>>>(
-            (const double *)F.m2l_p.ptr + F.m2l_pq_off[sl], k, F.m2l_r[sl], rmax,
-            (float *)F.tcc_pt_hi.ptr + (size_t)sl * k * rmax, (float *)F.tcc_pt_lo.ptr + (size_t)sl * k * rmax);
+    int rc = STK_OK;
+    if (!F.tcc_ops) {  // once per operator set, not per tree
+        rc = F.tcc_q_hi.reserve(sizeof(float) * (size_t)qrows * k4);
+        if (!rc) rc = F.tcc_q_lo.reserve(sizeof(float) * (size_t)qrows * k4);
+        if (!rc) rc = F.tcc_pt_hi.reserve(sizeof(float) * (size_t)nslot * k * rmax);
+        if (!rc) rc = F.tcc_pt_lo.reserve(sizeof(float) * (size_t)nslot * k * rmax);
+        if (rc) return rc;
+        // Q_d (k x r_d column-major, offsets back to back) read as qrows K-major rows of k
+        tc_rows_kernel<<<grid_for(qrows * k4), 256, 0, s>>>((const double *)F.m2l_q.ptr, k, qrows, k4,
+                                                            (float *)F.tcc_q_hi.ptr, (float *)F.tcc_q_lo.ptr);
         FCUDA(cudaGetLastError());
+        for (int sl = 0; sl < nslot; sl++) {
+            tc_trows_kernel<<<grid_for((long long)k * rmax), 256, 0, s>>>(
+                (const double *)F.m2l_p.ptr + F.m2l_pq_off[sl], k, F.m2l_r[sl], rmax,
+                (float *)F.tcc_pt_hi.ptr + (size_t)sl * k * rmax, (float *)F.tcc_pt_lo.ptr + (size_t)sl * k * rmax);
+            FCUDA(cudaGetLastError());
+        }
+        F.tcc_ops = true;
     }
     // tile tables, group by group
     const int nc = F.m2l_chunks, gc = F.m2l_group_chunks, ngroups = (nc + gc - 1) / gc;
@@ -1852,6 +1856,7 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
             cache_put(g_ops, key, e);
         }
         F.ops_ref = e;
+        F.tcc_ops = false;
         F.m2c_p = 0;  // the periodic operator follows the (possibly new) operators
     }
     F.periodic = f->pbc >= 1;
@@ -2130,13 +2135,14 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
         if (rc) return rc;
         std::vector<char> dense_lvl(T.depth() + 1, 0);
         for (auto &dl : F.dense) dense_lvl[dl->level] = 1;
-        std::vector<std::vector<int>> srcs(nslot), trgs(nslot);
         std::vector<long long> slot_pairs(nslot, 0);
-        for (int b = 0; b < nn; b++)
+        std::vector<int> slot(T.V.size(), -1), cnt(nslot, 0);  // per entry: its offset's slot, -1: not chunked
+        for (int b = 0; b < nn; b++) {
+            const int64_t L = 1LL << T.level[b];
+            const bool chunked = !dense_lvl[T.level[b]] && own(b);
             for (int e = T.V.off[b]; e < T.V.off[b + 1]; e++) {
                 const int a = T.V.ent[e] >> 5, code = T.V.ent[e] & 31;
                 const int sx = code % 3 - 1, sy = (code / 3) % 3 - 1, sz = code / 9 - 1;
-                const int64_t L = 1LL << T.level[b];
                 const int dx = (int)((int64_t)T.ix[a] + sx * L - T.ix[b]);
                 const int dy = (int)((int64_t)T.iy[a] + sy * L - T.iy[b]);
                 const int dz = (int)((int64_t)T.iz[a] + sz * L - T.iz[b]);
@@ -2144,36 +2150,36 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
                 const int sl = F.m2l_slot[(dx + 3) + 7 * (dy + 3) + 49 * (dz + 3)];
                 if (sl < 0) return STK_ERR_STATE;
                 slot_pairs[sl]++;
-                if (dense_lvl[T.level[b]] || !own(b)) continue;
-                srcs[sl].push_back(a);
-                trgs[sl].push_back(b);
+                if (!chunked) continue;
+                slot[e] = sl;
+                cnt[sl]++;
             }
-        // column chunks of kM2LChunk pairs of one offset; padded columns gather zeros
-        std::vector<int> gsrc, chunk_slot;
-        std::vector<std::vector<int>> cols_of(nn);  // per target node: its columns, by offset
+        }
+        // column chunks of kM2LChunk pairs of one offset, offset after offset; padded columns gather
+        // zeros
+        std::vector<int> chunk_slot, next(nslot);
         long long pairs = 0;
         for (int sl = 0; sl < nslot; sl++) {
-            const int m = (int)srcs[sl].size();
-            for (int c0 = 0; c0 < m; c0 += kM2LChunk) {
-                const int base = (int)gsrc.size();
-                chunk_slot.push_back(sl);
-                for (int i = 0; i < kM2LChunk; i++) {
-                    const bool real = c0 + i < m;
-                    gsrc.push_back(real ? srcs[sl][c0 + i] : -1);
-                    if (real) cols_of[trgs[sl][c0 + i]].push_back(base + i);
-                }
-            }
-            pairs += m;
+            next[sl] = (int)chunk_slot.size() * kM2LChunk;
+            chunk_slot.insert(chunk_slot.end(), (cnt[sl] + kM2LChunk - 1) / kM2LChunk, sl);
+            pairs += cnt[sl];
         }
         for (auto &dl : F.dense) pairs += dl->pairs;
         F.m2l_pairs = pairs;
         F.m2l_chunks = (int)chunk_slot.size();
-        F.m2l_cols = (long long)gsrc.size();
-        std::vector<int> red_off(nn + 1, 0), red_col;
+        F.m2l_cols = (long long)F.m2l_chunks * kM2LChunk;
+        // per column its source; per target node its columns, by offset
+        std::vector<int> gsrc((size_t)F.m2l_cols, -1), red_off(nn + 1, 0), red_col;
         red_col.reserve(pairs);
         for (int b = 0; b < nn; b++) {
             red_off[b] = (int)red_col.size();
-            red_col.insert(red_col.end(), cols_of[b].begin(), cols_of[b].end());
+            for (int e = T.V.off[b]; e < T.V.off[b + 1]; e++)
+                if (slot[e] >= 0) {
+                    const int c = next[slot[e]]++;
+                    gsrc[c] = T.V.ent[e] >> 5;
+                    red_col.push_back(c);
+                }
+            std::sort(red_col.begin() + red_off[b], red_col.end());
         }
         red_off[nn] = (int)red_col.size();
         const int k = F.m2l_rank;
@@ -2207,52 +2213,55 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
         if (!rc) rc = F.m2l_y.reserve(sizeof(double) * (size_t)k * gcols);
         if (!rc) rc = F.m2l_z.reserve(sizeof(double) * (size_t)rmax * gcols);
         if (rc) return rc;
-        // Per group of columns and padded rank r: two batched GEMMs over that group's
-        // chunks whose offset has rank r,
-        //   Z_c = Q_d^T X_c (r x 256),  Y_c = P_d Z_c (k x 256).
-        // Pointer arrays in (group, rank, chunk) order -- A: the offset's factor; B, C:
-        // the chunk's slot in its group -- as FP64 and FP32 views of the same buffers.
-        std::vector<int> order;
-        F.m2l_seg.clear();
-        for (int g = 0; g < ngroups; g++) {
-            const int c0 = g * gc, c1e = std::min(nc, c0 + gc);
-            std::map<int, std::vector<int>> by_rank;
-            for (int c = c0; c < c1e; c++) by_rank[F.m2l_r[chunk_slot[c]]].push_back(c);
-            for (auto &kv : by_rank) {
-                F.m2l_seg.push_back({g, kv.first, (int)order.size(), (int)kv.second.size()});
-                order.insert(order.end(), kv.second.begin(), kv.second.end());
-            }
-        }
-        std::vector<const void *> a1(nc), b1(nc), a2(nc), a1f(nc), b1f(nc), a2f(nc);
-        std::vector<void *> c1(nc), c2(nc), c1f(nc), c2f(nc);
-        for (int i = 0; i < nc; i++) {
-            const int c = order[i], sl = chunk_slot[c];
-            const size_t j = (size_t)(c % gc);  // slot within its group
-            a1[i] = (const double *)F.m2l_q.ptr + F.m2l_pq_off[sl];
-            a2[i] = (const double *)F.m2l_p.ptr + F.m2l_pq_off[sl];
-            a1f[i] = (const float *)F.m2l_q32.ptr + F.m2l_pq_off[sl];
-            a2f[i] = (const float *)F.m2l_p32.ptr + F.m2l_pq_off[sl];
-            b1[i] = (const double *)F.m2l_x.ptr + j * kM2LChunk * k;
-            b1f[i] = (const float *)F.m2l_x.ptr + j * kM2LChunk * k;
-            c1[i] = (double *)F.m2l_z.ptr + j * kM2LChunk * rmax;
-            c1f[i] = (float *)F.m2l_z.ptr + j * kM2LChunk * rmax;
-            c2[i] = (double *)F.m2l_y.ptr + j * kM2LChunk * k;
-            c2f[i] = (float *)F.m2l_y.ptr + j * kM2LChunk * k;
-        }
-        rc = F.d_m2l_ptr[0].upload(a1.data(), sizeof(void *) * nc, s);
-        if (!rc) rc = F.d_m2l_ptr[1].upload(b1.data(), sizeof(void *) * nc, s);
-        if (!rc) rc = F.d_m2l_ptr[2].upload(c1.data(), sizeof(void *) * nc, s);
-        if (!rc) rc = F.d_m2l_ptr[3].upload(a2.data(), sizeof(void *) * nc, s);
-        if (!rc) rc = F.d_m2l_ptr[4].upload(c2.data(), sizeof(void *) * nc, s);
-        if (!rc) rc = F.d_m2l_ptr32[0].upload(a1f.data(), sizeof(void *) * nc, s);
-        if (!rc) rc = F.d_m2l_ptr32[1].upload(b1f.data(), sizeof(void *) * nc, s);
-        if (!rc) rc = F.d_m2l_ptr32[2].upload(c1f.data(), sizeof(void *) * nc, s);
-        if (!rc) rc = F.d_m2l_ptr32[3].upload(a2f.data(), sizeof(void *) * nc, s);
-        if (!rc) rc = F.d_m2l_ptr32[4].upload(c2f.data(), sizeof(void *) * nc, s);
-        if (rc) return rc;
         rc = setup_m2l_chunks_tc(F, chunk_slot, nslot, s);
         if (!rc) rc = setup_m2l_chunks_i8(F, chunk_slot, gsrc, nn, s);
         if (rc) return rc;
+        F.m2l_seg.clear();
+        if (!F.tcc || !F.i8_chunks) {
+            // Per group of columns and padded rank r: two batched GEMMs over that group's
+            // chunks whose offset has rank r,
+            //   Z_c = Q_d^T X_c (r x 256),  Y_c = P_d Z_c (k x 256).
+            // Pointer arrays in (group, rank, chunk) order -- A: the offset's factor; B, C:
+            // the chunk's slot in its group -- as FP64 and FP32 views of the same buffers.
+            std::vector<int> order;
+            F.m2l_seg.clear();
+            for (int g = 0; g < ngroups; g++) {
+                const int c0 = g * gc, c1e = std::min(nc, c0 + gc);
+                std::map<int, std::vector<int>> by_rank;
+                for (int c = c0; c < c1e; c++) by_rank[F.m2l_r[chunk_slot[c]]].push_back(c);
+                for (auto &kv : by_rank) {
+                    F.m2l_seg.push_back({g, kv.first, (int)order.size(), (int)kv.second.size()});
+                    order.insert(order.end(), kv.second.begin(), kv.second.end());
+                }
+            }
+            std::vector<const void *> a1(nc), b1(nc), a2(nc), a1f(nc), b1f(nc), a2f(nc);
+            std::vector<void *> c1(nc), c2(nc), c1f(nc), c2f(nc);
+            for (int i = 0; i < nc; i++) {
+                const int c = order[i], sl = chunk_slot[c];
+                const size_t j = (size_t)(c % gc);  // slot within its group
+                a1[i] = (const double *)F.m2l_q.ptr + F.m2l_pq_off[sl];
+                a2[i] = (const double *)F.m2l_p.ptr + F.m2l_pq_off[sl];
+                a1f[i] = (const float *)F.m2l_q32.ptr + F.m2l_pq_off[sl];
+                a2f[i] = (const float *)F.m2l_p32.ptr + F.m2l_pq_off[sl];
+                b1[i] = (const double *)F.m2l_x.ptr + j * kM2LChunk * k;
+                b1f[i] = (const float *)F.m2l_x.ptr + j * kM2LChunk * k;
+                c1[i] = (double *)F.m2l_z.ptr + j * kM2LChunk * rmax;
+                c1f[i] = (float *)F.m2l_z.ptr + j * kM2LChunk * rmax;
+                c2[i] = (double *)F.m2l_y.ptr + j * kM2LChunk * k;
+                c2f[i] = (float *)F.m2l_y.ptr + j * kM2LChunk * k;
+            }
+            rc = F.d_m2l_ptr[0].upload(a1.data(), sizeof(void *) * nc, s);
+            if (!rc) rc = F.d_m2l_ptr[1].upload(b1.data(), sizeof(void *) * nc, s);
+            if (!rc) rc = F.d_m2l_ptr[2].upload(c1.data(), sizeof(void *) * nc, s);
+            if (!rc) rc = F.d_m2l_ptr[3].upload(a2.data(), sizeof(void *) * nc, s);
+            if (!rc) rc = F.d_m2l_ptr[4].upload(c2.data(), sizeof(void *) * nc, s);
+            if (!rc) rc = F.d_m2l_ptr32[0].upload(a1f.data(), sizeof(void *) * nc, s);
+            if (!rc) rc = F.d_m2l_ptr32[1].upload(b1f.data(), sizeof(void *) * nc, s);
+            if (!rc) rc = F.d_m2l_ptr32[2].upload(c1f.data(), sizeof(void *) * nc, s);
+            if (!rc) rc = F.d_m2l_ptr32[3].upload(a2f.data(), sizeof(void *) * nc, s);
+            if (!rc) rc = F.d_m2l_ptr32[4].upload(c2f.data(), sizeof(void *) * nc, s);
+            if (rc) return rc;
+        }
         F.m2l_flops = 0;
         for (int c = 0; c < nc; c++) F.m2l_flops += 4.0 * k * F.m2l_r[chunk_slot[c]] * kM2LChunk;
         F.m2l_flops_alg = 4.0 * (double)k * N * nn;

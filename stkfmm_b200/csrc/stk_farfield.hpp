@@ -170,7 +170,7 @@ struct FarField {
     // Q_d^T of every offset as K-major rows (sum_d r_d rows of k4 floats), P_d^T per offset
     // (k rows of rmax floats each, offset after offset), and per group of columns the tiles
     // of both stages (Z = Q_d^T X into split Z, Y = P_d Z)
-    bool tcc = false;
+    bool tcc = false, tcc_ops = false;  // in use; the operands are built
     DevBuf tcc_q_hi, tcc_q_lo, tcc_pt_hi, tcc_pt_lo;
     long long tcc_q_rows = 0;
     DevBuf tcc_tiles1, tcc_tiles2;

@@ -3,8 +3,12 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
+#include <exception>
+#include <mutex>
 #include <numeric>
-#include <unordered_set>
+#include <system_error>
+#include <thread>
 
 namespace stk {
 
@@ -36,6 +40,129 @@ inline uint64_t node_key(int l, uint64_t x, uint64_t y, uint64_t z) { return (1U
 }  // namespace
 
 uint64_t morton_key(double x, double y, double z) { return interleave(quantize(x), quantize(y), quantize(z)); }
+
+void parallel_ranges(size_t n, size_t grain, const std::function<void(size_t, size_t)> &f) {
+    const size_t hw = std::max(1u, std::thread::hardware_concurrency());
+    const size_t nt = std::min<size_t>({hw, 16, n / std::max<size_t>(grain, 1)});
+    if (nt < 2) {
+        f(0, n);
+        return;
+    }
+    std::vector<std::thread> th;
+    std::vector<std::exception_ptr> err(nt);
+    auto run = [&](size_t i) {
+        try {
+            f(n * i / nt, n * (i + 1) / nt);
+        } catch (...) {
+            err[i] = std::current_exception();
+        }
+    };
+    th.reserve(nt);
+    size_t started = 1;
+    try {
+        for (; started < nt; started++) th.emplace_back(run, started);
+    } catch (const std::system_error &) {  // no more threads: the rest runs here
+    }
+    run(0);
+    for (size_t i = started; i < nt; i++) run(i);
+    for (auto &t : th) t.join();
+    for (auto &e : err)
+        if (e) std::rethrow_exception(e);
+}
+
+// Least-significant-digit radix sort of the leading 32 bits, 8 bits a pass (a Morton key of 10
+// of its 20 levels: few keys agree that far), then the runs of equal leading bits by the whole
+// key.  Every range of the keys counts its digits, and the counts of all ranges in digit order are
+// where each range writes: equal keys keep their order on any number of threads.
+void sort_keys(std::vector<uint64_t> &keys, std::vector<int> &perm) {
+    const size_t n = keys.size();
+    perm.resize(n);
+    std::iota(perm.begin(), perm.end(), 0);
+    if (n < 2) return;
+    constexpr int kBits = 8, kBins = 1 << kBits, kTop = 28;  // four passes, from bit 28 of 60
+    std::vector<uint64_t> keys2(n);
+    std::vector<int> perm2(n);
+    const size_t nr = n < (1u << 18) ? 1 : std::min<size_t>(16, n >> 16);  // ranges
+    std::vector<size_t> count(nr * kBins);
+    for (int shift = kTop; shift < 60; shift += kBits) {
+        auto begin = [&](size_t r) { return n * r / nr; };
+        parallel_ranges(nr, 1, [&](size_t r0, size_t r1) {
+            for (size_t r = r0; r < r1; r++) {
+                size_t *c = &count[r * kBins];
+                std::fill(c, c + kBins, (size_t)0);
+                for (size_t i = begin(r); i < begin(r + 1); i++) c[(keys[i] >> shift) & (kBins - 1)]++;
+            }
+        });
+        size_t at = 0;
+        bool one = false;  // every key has the same digit
+        for (int d = 0; d < kBins; d++) {
+            const size_t from = at;
+            for (size_t r = 0; r < nr; r++) {
+                const size_t c = count[r * kBins + d];
+                count[r * kBins + d] = at;
+                at += c;
+            }
+            one = one || at - from == n;
+        }
+        if (one) continue;
+        parallel_ranges(nr, 1, [&](size_t r0, size_t r1) {
+            for (size_t r = r0; r < r1; r++) {
+                size_t *c = &count[r * kBins];
+                for (size_t i = begin(r); i < begin(r + 1); i++) {
+                    const size_t to = c[(keys[i] >> shift) & (kBins - 1)]++;
+                    keys2[to] = keys[i];
+                    perm2[to] = perm[i];
+                }
+            }
+        });
+        keys.swap(keys2);
+        perm.swap(perm2);
+    }
+    std::vector<std::pair<uint64_t, int>> run;
+    for (size_t i = 0; i < n;) {
+        size_t j = i + 1;
+        bool sorted = true;
+        for (; j < n && (keys[j] >> kTop) == (keys[i] >> kTop); j++) sorted = sorted && keys[j - 1] <= keys[j];
+        if (!sorted) {
+            run.clear();
+            for (size_t q = i; q < j; q++) run.push_back({keys[q], perm[q]});  // perm ascends within equal keys
+            std::sort(run.begin(), run.end());
+            for (size_t q = i; q < j; q++) {
+                keys[q] = run[q - i].first;
+                perm[q] = run[q - i].second;
+            }
+        }
+        i = j;
+    }
+}
+
+namespace {
+
+// keys, permutation and coordinates of a point set in Morton order; false: a point outside [0,1)
+bool sort_points(const double *xyz, int n, PointSet &ps) {
+    ps.n = n;
+    ps.key.resize(n);
+    std::vector<char> bad(1, 0);
+    parallel_ranges(n, 32768, [&](size_t a, size_t z) {
+        for (size_t i = a; i < z; i++) {
+            const double *p = xyz + 3 * i;
+            if (!(p[0] >= 0.0 && p[0] < 1.0 && p[1] >= 0.0 && p[1] < 1.0 && p[2] >= 0.0 && p[2] < 1.0)) {
+                __atomic_store_n(&bad[0], 1, __ATOMIC_RELAXED);
+                return;
+            }
+            ps.key[i] = morton_key(p[0], p[1], p[2]);
+        }
+    });
+    if (bad[0]) return false;
+    sort_keys(ps.key, ps.perm);
+    ps.xyz.resize(3 * (size_t)n);
+    parallel_ranges(n, 32768, [&](size_t a, size_t z) {
+        for (size_t i = a; i < z; i++) std::memcpy(&ps.xyz[3 * i], xyz + 3 * (size_t)ps.perm[i], 3 * sizeof(double));
+    });
+    return true;
+}
+
+}  // namespace
 
 double Octree::side(int i) const { return std::ldexp(1.0, -level[i]); }
 
@@ -79,14 +206,8 @@ std::string Octree::build(const double *pts, int n, int max_pts, int max_depth, 
     if (pbc_ < 0 || pbc_ > 3) return "pbc must be 0..3";
     pbc = pbc_;
     max_depth = std::max(0, std::min(max_depth, kMaxDepth));
-    std::vector<uint64_t> keys(n);
-    for (int i = 0; i < n; i++) {
-        const double *p = pts + 3 * (size_t)i;
-        for (int k = 0; k < 3; k++)
-            if (!(p[k] >= 0.0 && p[k] < 1.0)) return "tree point outside the unit box after scaling";
-        keys[i] = morton_key(p[0], p[1], p[2]);
-    }
-    std::sort(keys.begin(), keys.end());
+    if (!sort_points(pts, n, tree_)) return "tree point outside the unit box after scaling";
+    const std::vector<uint64_t> &keys = tree_.key;
 
     level.assign(1, 0);
     parent.assign(1, -1);
@@ -136,32 +257,34 @@ std::string Octree::assign(int set, const double *xyz, int n) {
     if (set < 0 || set > 2) return "invalid point set";
     if (n < 0 || (n > 0 && !xyz)) return "invalid points";
     PointSet &ps = sets[set];
-    ps.n = n;
-    std::vector<uint64_t> keys(n);
-    for (int i = 0; i < n; i++) {
-        const double *p = xyz + 3 * (size_t)i;
-        for (int k = 0; k < 3; k++)
-            if (!(p[k] >= 0.0 && p[k] < 1.0)) return "point outside the unit box after scaling";
-        keys[i] = morton_key(p[0], p[1], p[2]);
+    // the tree points themselves (sources and targets at the same points): sorted already.  The
+    // coordinates in the caller's order are compared through the permutation.
+    bool same = n == tree_.n && n > 0;
+    if (same) {
+        std::vector<char> differ(1, 0);
+        parallel_ranges(n, 65536, [&](size_t a, size_t z) {
+            for (size_t i = a; i < z; i++)
+                if (std::memcmp(&tree_.xyz[3 * i], xyz + 3 * (size_t)tree_.perm[i], 3 * sizeof(double))) {
+                    __atomic_store_n(&differ[0], 1, __ATOMIC_RELAXED);
+                    return;
+                }
+        });
+        same = !differ[0];
     }
-    ps.perm.resize(n);
-    std::iota(ps.perm.begin(), ps.perm.end(), 0);
-    std::stable_sort(ps.perm.begin(), ps.perm.end(), [&](int a, int b) { return keys[a] < keys[b]; });
-    ps.xyz.resize(3 * (size_t)n);
-    ps.key.resize(n);
-    for (int i = 0; i < n; i++) {
-        const int p = ps.perm[i];
-        ps.key[i] = keys[p];
-        for (int k = 0; k < 3; k++) ps.xyz[3 * (size_t)i + k] = xyz[3 * (size_t)p + k];
-    }
+    if (same)
+        ps = tree_;
+    else if (!sort_points(xyz, n, ps))
+        return "point outside the unit box after scaling";
     const int nn = num_nodes();
     ps.node_begin.resize(nn);
     ps.node_end.resize(nn);
-    for (int i = 0; i < nn; i++) {
+    for (int i = 0; i < nn; i++) {  // within the parent's range
         const uint64_t lo = key_lo_[i];
         const uint64_t hi = lo + (1ULL << (3 * (kMaxDepth - level[i])));
-        ps.node_begin[i] = (int)(std::lower_bound(ps.key.begin(), ps.key.end(), lo) - ps.key.begin());
-        ps.node_end[i] = (int)(std::lower_bound(ps.key.begin(), ps.key.end(), hi) - ps.key.begin());
+        const auto b = ps.key.begin() + (i ? ps.node_begin[parent[i]] : 0);
+        const auto e = i ? ps.key.begin() + ps.node_end[parent[i]] : ps.key.end();
+        ps.node_begin[i] = (int)(std::lower_bound(b, e, lo) - ps.key.begin());
+        ps.node_end[i] = (int)(std::lower_bound(b, e, hi) - ps.key.begin());
     }
     return "";
 }
@@ -208,16 +331,23 @@ void Octree::build_lists() {
                 }
     };
 
-    for (int b : leaves) {
+    // every entry once, in ascending order
+    auto finish = [](std::vector<int> &x) {
+        std::sort(x.begin(), x.end());
+        x.erase(std::unique(x.begin(), x.end()), x.end());
+    };
+    // nodes are independent of each other (U, W, V): spread over the host's threads
+    constexpr size_t kGrain = 128;
+    parallel_ranges(leaves.size(), kGrain, [&](size_t first, size_t last) {
+    std::vector<int> stack;
+    for (size_t li = first; li < last; li++) {
+        const int b = leaves[li];
         if (trg_count(b) == 0) continue;
-        std::unordered_set<long long> seenU, seenW;
         auto addU = [&](int node, int code) {
-            if (src_count(node) == 0) return;
-            if (seenU.insert((long long)node * 32 + code).second) Ul[b].push_back((node << 5) | code);
+            if (src_count(node) > 0) Ul[b].push_back((node << 5) | code);
         };
         auto addW = [&](int node, int code) {
-            if (src_count(node) == 0) return;
-            if (seenW.insert((long long)node * 32 + code).second) Wl[b].push_back((node << 5) | code);
+            if (src_count(node) > 0) Wl[b].push_back((node << 5) | code);
         };
         neighbours(b, [&](int node, int code, const int64_t *p, int l) {
             if (node >= 0) {
@@ -225,7 +355,7 @@ void Octree::build_lists() {
                     addU(node, code);
                     return;
                 }
-                std::vector<int> stack(1, node);
+                stack.assign(1, node);
                 while (!stack.empty()) {
                     const int m = stack.back();
                     stack.pop_back();
@@ -249,12 +379,14 @@ void Octree::build_lists() {
                 if (a >= 0) addU(a, code);
             }
         });
-        std::sort(Ul[b].begin(), Ul[b].end());
-        std::sort(Wl[b].begin(), Wl[b].end());
+        finish(Ul[b]);
+        finish(Wl[b]);
     }
+    });
 
     // V: children of the parent's colleagues that are not adjacent
-    for (int b = 1; b < nn; b++) {
+    parallel_ranges(nn, kGrain, [&](size_t first, size_t last) {
+    for (int b = std::max(1, (int)first); b < (int)last; b++) {
         if (trg_count(b) == 0) continue;
         const int P = parent[b];
         neighbours(P, [&](int node, int code, const int64_t *, int) {
@@ -266,17 +398,23 @@ void Octree::build_lists() {
         });
         std::sort(Vl[b].begin(), Vl[b].end());
     }
+    });
 
     // X: the W relation seen from the source side.  For every leaf a with
     // sources, the nodes with targets that are descendants of a's colleagues,
     // not adjacent to a, with a parent adjacent to a, gain a (with the inverse
     // shift).  Walking from the source leaves also covers source leaves that hold
     // no targets, which have no W list of their own.
-    for (int a : leaves) {
+    std::mutex x_mutex;
+    parallel_ranges(leaves.size(), kGrain, [&](size_t first, size_t last) {
+    std::vector<std::pair<int, int>> found;  // (node, entry)
+    std::vector<int> stack;
+    for (size_t li = first; li < last; li++) {
+        const int a = leaves[li];
         if (src_count(a) == 0) continue;
         neighbours(a, [&](int node, int code, const int64_t *, int) {
             if (node < 0 || is_leaf(node)) return;
-            std::vector<int> stack(1, node);
+            stack.assign(1, node);
             while (!stack.empty()) {
                 const int m = stack.back();
                 stack.pop_back();
@@ -285,16 +423,16 @@ void Octree::build_lists() {
                     if (adjacent(c, code, a)) {
                         if (!is_leaf(c)) stack.push_back(c);
                     } else {
-                        Xl[c].push_back((a << 5) | shift_negate(code));
+                        found.push_back({c, (a << 5) | shift_negate(code)});
                     }
                 }
             }
         });
     }
-    for (auto &x : Xl) {
-        std::sort(x.begin(), x.end());
-        x.erase(std::unique(x.begin(), x.end()), x.end());
-    }
+    std::lock_guard<std::mutex> lock(x_mutex);
+    for (const auto &f : found) Xl[f.first].push_back(f.second);
+    });
+    for (auto &x : Xl) finish(x);
 
     U = to_csr(Ul);
     V = to_csr(Vl);

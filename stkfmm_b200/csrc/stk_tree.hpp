@@ -17,6 +17,7 @@
 //     recorded as an image shift code per entry.
 #pragma once
 #include <cstdint>
+#include <functional>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -84,11 +85,20 @@ class Octree {
   private:
     std::unordered_map<uint64_t, int> lookup_;
     std::vector<uint64_t> key_lo_;                  // Morton key of each node's lower corner (max depth)
+    PointSet tree_;                                 // the tree points, sorted
     int find(int l, int64_t x, int64_t y, int64_t z) const;
     bool adjacent(int a, int shift, int b) const;
 };
 
 uint64_t morton_key(double x, double y, double z);
+
+// perm = the indices of n keys in ascending order, equal keys in their given order; the keys
+// (Morton keys, below 2^60) come back sorted.
+void sort_keys(std::vector<uint64_t> &keys, std::vector<int> &perm);
+
+// f(begin, end) over [0, n) in contiguous ranges on several host threads; one call on this
+// thread where n holds fewer than two ranges of `grain`, or where threads cannot be had.
+void parallel_ranges(size_t n, size_t grain, const std::function<void(size_t, size_t)> &f);
 
 // Longest-processing-time assignment: items (in the given order, largest first)
 // each go to the part with the smallest load so far; ties to the lowest part.

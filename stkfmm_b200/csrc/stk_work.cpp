@@ -357,9 +357,7 @@ void morton_order(const double *xyz, int n, std::vector<int> &order, std::vector
         for (int k = 0; k < 3; k++) u[k] = std::min(std::max((xyz[3 * (size_t)i + k] - lo[k]) * inv, 0.0), 0.999999999);
         key[i] = morton_key(u[0], u[1], u[2]);
     }
-    order.resize(n);
-    std::iota(order.begin(), order.end(), 0);
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return key[a] < key[b]; });
+    sort_keys(key, order);
     sorted.resize(3 * (size_t)n);
     for (int i = 0; i < n; i++)
         for (int k = 0; k < 3; k++) sorted[3 * (size_t)i + k] = xyz[3 * (size_t)order[i] + k];
