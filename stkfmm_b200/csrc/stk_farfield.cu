@@ -1229,11 +1229,14 @@ int build_periodic(FarField &F, int pbc, int far_field, cudaStream_t s) {
 
 // Set up one list pass: target boxes with contiguous target ranges, list entries
 // over source boxes.  src_beg / src_end are device arrays owned elsewhere when
-// own_src is false.
+// own_src is false.  check: the pass's outputs are check potentials (S2M, S2L), which the
+// pseudo-inverses amplify by up to 1e8 in directions that barely reach the targets: one order
+// of summation in both precisions keeps their rounding, and so the FMM's (a reordered S2M
+// moves a Stokes FMM by 2e-10), and splitting their short source lists gained nothing.
 int setup_pass(ListPass &P, int uk, const std::vector<int> &tb, const std::vector<int> &te,
                const std::vector<int> &off, const std::vector<int> &ent, const int *h_src_beg, const int *h_src_end,
-               int n_src_box, bool own_src, const std::vector<double> &centres, int balance_warps, cudaStream_t s,
-               int shard_rank = 0, int shard_n = 1) {
+               int n_src_box, bool own_src, const std::vector<double> &centres, int balance_warps, bool check,
+               cudaStream_t s, int shard_rank = 0, int shard_n = 1) {
     P.uk = uk;
     std::vector<WorkItem> items;
     std::vector<PartGroup> groups;
@@ -1242,9 +1245,13 @@ int setup_pass(ListPass &P, int uk, const std::vector<int> &tb, const std::vecto
                      P.pairs, balance_warps, shard_rank, shard_n);
     P.n_items = (int)items.size();
     int rc = P.items[1].upload(items, groups, 0, s);
-    build_split_items((int)tb.size(), tb.data(), te.data(), off.data(), ent.data(), h_src_beg, h_src_end,
-                      balance_warps * 5 / 4, items, groups, slots, shard_rank, shard_n);
-    if (!rc) rc = P.items[0].upload(items, groups, slots, s);
+    if (check) {
+        if (!rc) P.items[0].share(P.items[1]);
+    } else {
+        build_split_items((int)tb.size(), tb.data(), te.data(), off.data(), ent.data(), h_src_beg, h_src_end,
+                          balance_warps * 5 / 4, items, groups, slots, shard_rank, shard_n);
+        if (!rc) rc = P.items[0].upload(items, groups, slots, s);
+    }
     if (!rc) rc = P.ent.upload(ent.data(), ent.size() * sizeof(int), s);
     if (!rc && own_src) rc = P.src_beg.upload(h_src_beg, sizeof(int) * n_src_box, s);
     if (!rc && own_src) rc = P.src_end.upload(h_src_end, sizeof(int) * n_src_box, s);
@@ -1970,7 +1977,7 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
             F.s2m[k].reset();
             if (uk < 0 || T.sets[k].n == 0) continue;
             rc = setup_pass(F.s2m[k], uk, tb, te, off, ent, T.sets[k].node_begin.data(), T.sets[k].node_end.data(),
-                            nn, false, cc, bw, s);
+                            nn, false, cc, bw, true, s);
             if (rc) return rc;
         }
     }
@@ -2005,7 +2012,7 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
             F.near[k].reset();
             if (T.sets[k].n == 0 || ki->slot[k == 0 ? SLOT_S2T_SL : SLOT_S2T_DL] < 0) continue;
             rc = setup_pass(F.near[k], ki->slot[k == 0 ? SLOT_S2T_SL : SLOT_S2T_DL], tg.node_begin, tg.node_end, noff,
-                            nent, T.sets[k].node_begin.data(), T.sets[k].node_end.data(), nn, false, ctr, bw, s,
+                            nent, T.sets[k].node_begin.data(), T.sets[k].node_end.data(), nn, false, ctr, bw, false, s,
                             f->shard_rank, f->shard_n);
             if (rc) return rc;
         }
@@ -2043,7 +2050,7 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
             F.s2l[k].reset();
             if (uk < 0 || T.sets[k].n == 0) continue;
             rc = setup_pass(F.s2l[k], uk, tb, te, off, ent, T.sets[k].node_begin.data(), T.sets[k].node_end.data(),
-                            nn, false, cc, bw, s);
+                            nn, false, cc, bw, true, s);
             if (rc) return rc;
         }
     }
@@ -2088,10 +2095,10 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
         // target-side passes follow the handle's shard (the upward pass, S2L and the
         // M2L are computed in full on every shard)
         rc = setup_pass(F.m2t, ki->slot[SLOT_M2T], tg.node_begin, tg.node_end, woff, went, sb.data(), se.data(), nn,
-                        true, ctr, bw, s, f->shard_rank, f->shard_n);
+                        true, ctr, bw, false, s, f->shard_rank, f->shard_n);
         if (!rc)
             rc = setup_pass(F.l2t, ki->slot[SLOT_L2T], tg.node_begin, tg.node_end, loff, lent, sb.data(), se.data(),
-                            nn, true, ctr, bw, s, f->shard_rank, f->shard_n);
+                            nn, true, ctr, bw, false, s, f->shard_rank, f->shard_n);
         if (rc) return rc;
     }
 

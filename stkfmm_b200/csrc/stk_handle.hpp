@@ -45,6 +45,13 @@ struct ItemList {
     int n_items = 0, n_groups = 0;
     long long part_targets = 0;  // target slots of split sums
     int upload(const std::vector<WorkItem> &it, const std::vector<PartGroup> &g, long long slots, cudaStream_t s);
+    void share(const ItemList &o) {
+        items.share(o.items);
+        groups.share(o.groups);
+        n_items = o.n_items;
+        n_groups = o.n_groups;
+        part_targets = o.part_targets;
+    }
     // items, groups and the slots' buffer into the kernel's arguments (tdim components)
     int args(ListP2PArgs &a, DevBuf &parts, int tdim) const;
 };
