@@ -667,19 +667,50 @@ template <int UK = 0, class F> cudaError_t with_uk(int uk, const F &f) {
     }
 }
 
-// trg_out += the parts of targets whose sources were split over items, in order
-__global__ void add_parts_kernel(const PartGroup *__restrict__ groups, int n, int d, const double *__restrict__ parts,
-                                 double *__restrict__ out) {
+// trg_out += the parts of targets whose sources were split over items: blockIdx.y takes columns of
+// the groups blockIdx.x, ....  Groups of many parts (a leaf with a long list: hundreds) are summed
+// in eight runs of parts side by side, 32 columns per CTA, the runs' sums then in order: as one
+// chain of all parts per thread, the longest groups took 140 us of a 131k-point wall evaluation.
+// The order depends on the lists alone, so repeats give the same bits.
+constexpr int kPartThreads = 256, kPartRuns = 8, kPartWide = kPartThreads / kPartRuns;
+
+__global__ void __launch_bounds__(kPartThreads)
+    add_parts_kernel(const PartGroup *__restrict__ groups, int n, int d, const double *__restrict__ parts,
+                     double *__restrict__ out) {
+    __shared__ double red[kPartRuns][kPartWide];
+    const int run = threadIdx.x / kPartWide, jj = threadIdx.x - run * kPartWide;
     for (int i = blockIdx.x; i < n; i += gridDim.x) {
         const PartGroup g = groups[i];
         const int m = g.nt * d;
-        for (int j = threadIdx.x; j < m; j += blockDim.x) {
-            const double *p = parts + (size_t)g.part0 * d + j;
-            double v = 0.0;
+        const double *p = parts + (size_t)g.part0 * d;
+        double *o = out + (size_t)g.t0 * d;
+        if (g.n_parts <= 2 * kPartRuns) {
+            const int j = blockIdx.y * kPartThreads + threadIdx.x;
+            if (j < m) {
+                double v = 0.0;
 #pragma unroll 4
-            for (int k = 0; k < g.n_parts; k++) v += p[(size_t)k * m];
-            out[(size_t)g.t0 * d + j] += v;
+                for (int k = 0; k < g.n_parts; k++) v += p[(size_t)k * m + j];
+                o[j] += v;
+            }
+            continue;
         }
+        const int j = blockIdx.y * kPartWide + jj;
+        if (blockIdx.y * kPartWide >= m) continue;
+        const int k0 = (int)((long long)g.n_parts * run / kPartRuns), k1 = (int)((long long)g.n_parts * (run + 1) / kPartRuns);
+        double v = 0.0;
+        if (j < m) {
+#pragma unroll 8
+            for (int k = k0; k < k1; k++) v += p[(size_t)k * m + j];
+        }
+        red[run][jj] = v;
+        __syncthreads();
+        if (run == 0 && j < m) {
+            double t = 0.0;
+#pragma unroll
+            for (int r = 0; r < kPartRuns; r++) t += red[r][jj];
+            o[j] += t;
+        }
+        __syncthreads();
     }
 }
 
@@ -789,7 +820,8 @@ cudaError_t launch_list_p2p(int uk, int prec, const ListP2PArgs &a, int num_sms,
                                   : launch_impl<UK, false, false>(a, num_sms, stream);
     });
     if (e != cudaSuccess || a.n_groups == 0) return e;
-    add_parts_kernel<<<std::min(a.n_groups, 148 * 16), 128, 0, stream>>>(a.groups, a.n_groups, uk_tdim(uk), a.parts,
+    const int d = uk_tdim(uk);
+    add_parts_kernel<<<dim3(std::min(a.n_groups, 148 * 8), (64 * d + kPartWide - 1) / kPartWide), kPartThreads, 0, stream>>>(a.groups, a.n_groups, d, a.parts,
                                                                          a.trg_out);
     return cudaGetLastError();
 }
