@@ -549,8 +549,8 @@ __global__ void tc_trows_kernel(const double *__restrict__ src, int k, int R, in
     }
 }
 
-// phi_hat columns cols[j] (k values each, FP64) as K-major rows of ld floats, split;
-// cols[j] < 0 (chunk padding) gives a zero row
+// phi_hat columns cols[j] (cols null: j; k values each, FP64) as K-major rows of ld floats,
+// split; cols[j] < 0 (chunk padding) gives a zero row
 __global__ void tc_gather_cols_kernel(const double *__restrict__ src, const int *__restrict__ cols, long long n,
                                       int k, int ld, float *__restrict__ hi, float *__restrict__ lo) {
     const long long total = n * ld;
@@ -558,7 +558,7 @@ __global__ void tc_gather_cols_kernel(const double *__restrict__ src, const int 
          idx += (long long)gridDim.x * blockDim.x) {
         const long long j = idx / ld;
         const int r = (int)(idx - j * ld);
-        const int c = cols[j];
+        const long long c = cols ? cols[j] : j;
         float h = 0.f, l = 0.f;
         if (r < k && c >= 0) tf32_hilo(src[(size_t)c * k + r], h, l);
         hi[idx] = h;
@@ -2216,7 +2216,7 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
         if (rc) return rc;
         const int rmax = F.m2l_rmax;
         // k4 (not k) per column: the tensor-core path keeps split FP32 rows of k4 floats here
-        rc = F.m2l_x.reserve(sizeof(double) * (size_t)((k + 3) / 4 * 4) * gcols);
+        rc = F.m2l_x.reserve(sizeof(double) * (size_t)((k + 3) / 4 * 4) * std::max<size_t>(gcols, nn));
         if (!rc) rc = F.m2l_y.reserve(sizeof(double) * (size_t)k * gcols);
         if (!rc) rc = F.m2l_z.reserve(sizeof(double) * (size_t)rmax * gcols);
         if (rc) return rc;
@@ -2582,19 +2582,30 @@ int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const dou
         const cublasComputeType_t ct = mixed ? CUBLAS_COMPUTE_32F : CUBLAS_COMPUTE_64F;
         DevBuf *P = mixed ? F.d_m2l_ptr32 : F.d_m2l_ptr;
         if (mixed && F.tcc) {
-            // tensor cores: split gather, Z = Q_d^T X (split), Y = P_d Z, in two grouped launches
+            // tensor cores, two grouped launches: Z = Q_d^T X (split), then Y = P_d Z.  Where Q_d fits
+            // one 128-row tile, X's columns are gathered by the first launch from the nodes' split
+            // phi_hat (LapPGrad, 1M points, p = 10: M2L 3.14 -> 2.82 ms, writing X out took 0.87);
+            // with two or three tiles per chunk, each of which would gather them again, X is written
+            // out (Stokes, 32k points, p = 8: 0.58 against 0.60 ms gathered).
             const int g = c0 / gc, k4 = (k + 3) / 4 * 4;
-            float *xh = (float *)F.m2l_x.ptr, *xl = xh + (size_t)ncol * k4;
+            const bool gather = rmax <= 128;
+            const long long nx = gather ? nn : ncol;
+            float *xh = (float *)F.m2l_x.ptr, *xl = xh + (size_t)nx * k4;
             float *zh = (float *)F.m2l_z.ptr, *zl = zh + (size_t)ncol * rmax;
             int *err = (int *)F.tc_err.ptr;
-            t_launches += 3;
-            tc_gather_cols_kernel<<<grid_for(ncol * k4), 256, 0, s>>>(phi_hat, gsrc, ncol, k, k4, xh, xl);
-            FCUDA(cudaGetLastError());
-            FCUDA(umma_grouped_3xtf32(Tf32Rows{(const float *)F.tcc_q_hi.ptr, (const float *)F.tcc_q_lo.ptr,
-                                               (int)F.tcc_q_rows, k, k4},
-                                      Tf32Rows{xh, xl, (int)ncol, k, k4},
-                                      (const GroupTile *)F.tcc_tiles1.ptr + F.tcc_t1_off[g],
-                                      F.tcc_t1_off[g + 1] - F.tcc_t1_off[g], zh, zl, err, s));
+            const Tf32Rows q{(const float *)F.tcc_q_hi.ptr, (const float *)F.tcc_q_lo.ptr, (int)F.tcc_q_rows, k, k4};
+            const GroupTile *t1 = (const GroupTile *)F.tcc_tiles1.ptr + F.tcc_t1_off[g];
+            const int n1 = F.tcc_t1_off[g + 1] - F.tcc_t1_off[g];
+            t_launches += 2;
+            if (!gather || c0 == 0) {
+                t_launches++;
+                tc_gather_cols_kernel<<<grid_for(nx * k4), 256, 0, s>>>(phi_hat, gather ? nullptr : gsrc, nx, k, k4, xh, xl);
+                FCUDA(cudaGetLastError());
+            }
+            if (gather)
+                FCUDA(umma_grouped_gather_3xtf32(q, Tf32Rows{xh, xl, nn, k, k4}, gsrc, t1, n1, zh, zl, err, s));
+            else
+                FCUDA(umma_grouped_3xtf32(q, Tf32Rows{xh, xl, (int)ncol, k, k4}, t1, n1, zh, zl, err, s));
             FCUDA(umma_grouped_3xtf32(Tf32Rows{(const float *)F.tcc_pt_hi.ptr, (const float *)F.tcc_pt_lo.ptr,
                                                (int)F.m2l_r.size() * k, rmax, rmax},
                                       Tf32Rows{zh, zl, (int)ncol, rmax, rmax},

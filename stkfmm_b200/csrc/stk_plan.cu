@@ -160,7 +160,9 @@ extern "C" int stk_p2p_plan_execute(stk_p2p_plan *plan, int ukernel, int precisi
     if (cudaGetDevice(&dev) != cudaSuccess || dev != plan->device) return STK_ERR_INVALID_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     const int sd = stk::uk_sdim_host(ukernel), rs = stk::uk_record_stride(ukernel);
-    // grow a buffer: earlier executions may still use it on any stream
+    // grow a buffer: earlier executions may still use it on any stream; at least eight doubles
+    // per source and per split target slot, so that a forward pass and its adjoints (3 and 7
+    // components) allocate once
     auto grow = [](double **buf, size_t *cap, size_t need) {
         if (*cap >= need) return true;
         if (*buf) {
@@ -176,9 +178,10 @@ extern "C" int stk_p2p_plan_execute(stk_p2p_plan *plan, int ukernel, int precisi
         *cap = need;
         return true;
     };
-    if (!grow(&plan->d_rec, &plan->rec_cap, (size_t)std::max(plan->nsrc, 1) * rs)) return STK_ERR_CUDA;
+    if (!grow(&plan->d_rec, &plan->rec_cap, (size_t)std::max(plan->nsrc, 1) * std::max(rs, 8)))
+        return STK_ERR_CUDA;
     if (!mixed && plan->n_groups > 0 &&
-        !grow(&plan->d_parts, &plan->parts_cap, (size_t)plan->part_targets * stk::uk_tdim_host(ukernel)))
+        !grow(&plan->d_parts, &plan->parts_cap, (size_t)plan->part_targets * std::max(stk::uk_tdim_host(ukernel), 8)))
         return STK_ERR_CUDA;
     if (stk::launch_pack_records(ukernel, plan->nsrc, nullptr, d_src_coord, d_src_value, sd, nullptr, plan->d_rec, s) !=
         cudaSuccess)

@@ -73,6 +73,15 @@ struct Bars {
     uint32_t tmem;
 };
 
+// four rows (any) x 32 FP32 of a map whose boxes are one row high
+__device__ __forceinline__ void tma_gather4(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0, int4 r) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, "
+        "%5, %6, %7}], [%2];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(r.x), "r"(r.y), "r"(r.z), "r"(r.w)
+        : "memory");
+}
+
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0, int c1) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
@@ -139,6 +148,7 @@ struct TileSpec {
 
 // One GEMM C = A B^T over (gx = ceil(M/128)) x ceil(N/128) tiles.
 struct DenseJob {
+    static constexpr bool kGather = false;
     int M, N, K, ldc, beta, gx, ntiles;
     float *C;
     __device__ TileSpec tile(int i) const { return {(i % gx) * kBM, (i / gx) * kBN, K}; }
@@ -156,11 +166,15 @@ struct DenseJob {
     }
 };
 
-// Many small GEMMs in one launch: tile i is described by tiles[i].
-struct GroupJob {
+// Many small GEMMs in one launch: tile i is described by tiles[i].  GATHER: row n of a tile's B
+// block is row rows[b_row + n] of B (zero where that is negative).
+template <bool GATHER> struct GroupJob {
+    static constexpr bool kGather = GATHER;
     const GroupTile *tiles;
     int ntiles;
     float *C, *C_lo;
+    const int *rows;
+    int b_rows;  // rows of B: beyond it the copies fill zeros
     __device__ TileSpec tile(int i) const {
         const GroupTile &g = tiles[i];
         return {g.a_row, g.b_row, g.K};
@@ -230,7 +244,42 @@ __global__ void __launch_bounds__(kThreads, 1)
 
     if (warp == 0) {
         // ---- TMA producer ----
-        if (lane == 0) {
+        if constexpr (Job::kGather) {
+            // the whole warp: lane i copies rows 4 i .. 4 i + 3 of the tile's B block
+            long long g = 0;
+            for (int t = blockIdx.x; t < job.ntiles && ok; t += gridDim.x) {
+                const TileSpec ts = job.tile(t);
+                int4 r = reinterpret_cast<const int4 *>(job.rows + ts.b_row)[lane];
+                r.x = r.x < 0 ? job.b_rows : r.x;
+                r.y = r.y < 0 ? job.b_rows : r.y;
+                r.z = r.z < 0 ? job.b_rows : r.z;
+                r.w = r.w < 0 ? job.b_rows : r.w;
+                const int nkb = (ts.K + kBK - 1) / kBK;
+                for (int kb = 0; kb < nkb; kb++, g++) {
+                    const int s = (int)(g % kStages);
+                    const uint32_t ph = (uint32_t)(g / kStages) & 1u;
+                    if (!__all_sync(0xffffffffu, mbar_wait(saddr(&bars->empty[s]), ph ^ 1u))) {
+                        ok = false;
+                        break;
+                    }
+                    const uint32_t fb = saddr(&bars->full[s]);
+                    const uint32_t st = saddr(tiles + s * kStageBytes);
+                    if (lane == 0) {
+                        mbar_expect_tx(fb, kStageBytes);
+                        tma_load_2d(st, &mAh, fb, kb * kBK, ts.a_row);
+                        tma_load_2d(st + kTileBytes, &mAl, fb, kb * kBK, ts.a_row);
+                    }
+                    __syncwarp();
+                    tma_gather4(st + 2 * kTileBytes + lane * 512, &mBh, fb, kb * kBK, r);
+                    tma_gather4(st + 3 * kTileBytes + lane * 512, &mBl, fb, kb * kBK, r);
+                }
+            }
+            if (!ok && lane == 0) {
+                atomicExch(err, 1);
+                if (g > 0) mbar_wait(saddr(&bars->full[(g - 1) % kStages]), (uint32_t)((g - 1) / kStages) & 1u);
+            }
+            __syncwarp();
+        } else if (lane == 0) {
             long long g = 0;  // K-blocks issued so far
             for (int t = blockIdx.x; t < job.ntiles && ok; t += gridDim.x) {
                 const TileSpec ts = job.tile(t);
@@ -384,12 +433,12 @@ EncodeTiledFn encode_fn() {
 }
 
 // rows x K FP32, row pitch ld floats; boxes of 128 rows x 32 K, 128-byte swizzle
-bool encode(CUtensorMap *m, const float *base, int rows, int K, int ld) {
+bool encode(CUtensorMap *m, const float *base, int rows, int K, int ld, int box_rows = kBM) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return false;
     const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
     const cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
-    const cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)kBM};
+    const cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)box_rows};
     const cuuint32_t estr[2] = {1, 1};
     return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(base), dims, strides, box, estr,
               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -462,10 +511,29 @@ cudaError_t umma_grouped_3xtf32(Tf32Rows A, Tf32Rows B, const GroupTile *tiles, 
     if (!encode(&mah, A.hi, A.rows, A.k, A.ld) || !encode(&mal, A.lo, A.rows, A.k, A.ld) ||
         !encode(&mbh, B.hi, B.rows, B.k, B.ld) || !encode(&mbl, B.lo, B.rows, B.k, B.ld))
         return cudaErrorInvalidValue;
-    const cudaError_t ae = smem_attr<GroupJob>();
+    const cudaError_t ae = smem_attr<GroupJob<false>>();
     if (ae != cudaSuccess) return ae;
-    umma_3xtf32_kernel<GroupJob><<<std::min(ntiles, sm_count()), kThreads, kSmemBytes, s>>>(
-        mah, mal, mbh, mbl, GroupJob{tiles, ntiles, C, C_lo}, err);
+    umma_3xtf32_kernel<GroupJob<false>><<<std::min(ntiles, sm_count()), kThreads, kSmemBytes, s>>>(
+        mah, mal, mbh, mbl, GroupJob<false>{tiles, ntiles, C, C_lo, nullptr, 0}, err);
+    return cudaGetLastError();
+}
+
+cudaError_t umma_grouped_gather_3xtf32(Tf32Rows A, Tf32Rows B, const int *rows, const GroupTile *tiles, int ntiles,
+                                       float *C, float *C_lo, int *err, cudaStream_t s) {
+    if (ntiles <= 0) return cudaSuccess;
+    auto aligned = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+    if (!A.hi || !A.lo || !B.hi || !B.lo || !rows || !tiles || !C || !err || A.ld % 4 || B.ld % 4 || A.k > A.ld ||
+        B.k > B.ld || A.k <= 0 || B.k <= 0 || A.rows <= 0 || B.rows <= 0 || !aligned(A.hi) || !aligned(A.lo) ||
+        !aligned(B.hi) || !aligned(B.lo) || !aligned(rows))
+        return cudaErrorInvalidValue;
+    CUtensorMap mah, mal, mbh, mbl;
+    if (!encode(&mah, A.hi, A.rows, A.k, A.ld) || !encode(&mal, A.lo, A.rows, A.k, A.ld) ||
+        !encode(&mbh, B.hi, B.rows, B.k, B.ld, 1) || !encode(&mbl, B.lo, B.rows, B.k, B.ld, 1))
+        return cudaErrorInvalidValue;
+    const cudaError_t ae = smem_attr<GroupJob<true>>();
+    if (ae != cudaSuccess) return ae;
+    umma_3xtf32_kernel<GroupJob<true>><<<std::min(ntiles, sm_count()), kThreads, kSmemBytes, s>>>(
+        mah, mal, mbh, mbl, GroupJob<true>{tiles, ntiles, C, C_lo, rows, B.rows}, err);
     return cudaGetLastError();
 }
 

@@ -45,6 +45,12 @@ struct GroupTile {
 cudaError_t umma_grouped_3xtf32(Tf32Rows A, Tf32Rows B, const GroupTile *tiles, int ntiles, float *C, float *C_lo,
                                 int *err, cudaStream_t s);
 
+// The same with gathered B rows: row n of a tile's B block is row rows[b_row + n] of B, zero where
+// that is negative (b_row a multiple of 128, rows 16-byte aligned).  The rows come by four-row
+// gather copies (TMA tile::gather4), 64 per K-block.
+cudaError_t umma_grouped_gather_3xtf32(Tf32Rows A, Tf32Rows B, const int *rows, const GroupTile *tiles, int ntiles,
+                                       float *C, float *C_lo, int *err, cudaStream_t s);
+
 // v = hi + lo to ~2^-24 relative with both parts exact in TF32: hi = v rounded to
 // TF32 (to nearest, ties away), lo = (v - hi) rounded to TF32 (v - hi is exact in FP32)
 __device__ __forceinline__ void tf32_split_value(float v, float &hi, float &lo) {
