@@ -133,8 +133,10 @@ static int direct_device(int uk, int nsrc, const double *d_src, const double *d_
     a.ntrg = ntrg;
     direct_chunks(uk, prec, ntrg, nsrc, ws.num_sms(), a.src_chunk, a.n_chunk);
     if ((rc = ws.begin(stream))) return rc;
-    if (a.n_chunk > 1 && !(a.parts = ws.buf<double>(Workspace::kParts, (size_t)a.n_chunk * ntrg * uk_tdim_host(uk))))
-        return STK_ERR_CUDA;
+    if (a.n_chunk > 1 && !(a.parts = ws.buf<double>(Workspace::kParts, (size_t)a.n_chunk * ntrg * uk_tdim_host(uk)))) {
+        a.n_chunk = 1;  // no memory for the chunks' sums: one chunk of all sources
+        a.src_chunk = (nsrc + 31) / 32 * 32;
+    }
     a.trg_xyz = d_trg;
     a.trg_out = d_out;
     a.box_centre = nullptr;  // per-item origin: the item's first target
@@ -286,6 +288,11 @@ static int p2p_lists(int ukernel, int precision, int n_trg_box, const int *trg_b
     else
         build_split_items(n_trg_box, trg_begin, trg_end, list_off, list_ent, src_begin, src_end, ws.num_sms() * 15, items,
                           groups, slots);
+    double *d_parts = groups.empty() ? nullptr : ws.buf<double>(Workspace::kParts, (size_t)slots * uk_tdim_host(ukernel));
+    if (!groups.empty() && !d_parts) {  // no memory for split sums: items that split no sources
+        groups.clear();
+        build_list_items(n_trg_box, trg_begin, trg_end, list_off, list_ent, src_begin, src_end, items, pairs);
+    }
     if (items.empty()) return STK_OK;
     const int sd = uk_sdim_host(ukernel), rs = uk_record_stride(ukernel);
     double *rec = ws.buf<double>(Workspace::kRec, (size_t)std::max(nsrc, 1) * rs);
@@ -294,8 +301,7 @@ static int p2p_lists(int ukernel, int precision, int n_trg_box, const int *trg_b
     int *d_ent = ws.buf<int>(Workspace::kEnt, nent);
     WorkItem *d_items = ws.buf<WorkItem>(Workspace::kItems, items.size());
     PartGroup *d_groups = ws.buf<PartGroup>(Workspace::kGroups, groups.size());
-    double *d_parts = ws.buf<double>(Workspace::kParts, (size_t)slots * uk_tdim_host(ukernel));
-    if (!rec || !d_sbeg || !d_send || !d_ent || !d_items || !d_groups || !d_parts) return STK_ERR_CUDA;
+    if (!rec || !d_sbeg || !d_send || !d_ent || !d_items || !d_groups) return STK_ERR_CUDA;
     STK_CUDA(launch_pack_records(ukernel, nsrc, nullptr, d_src_coord, d_src_value, sd, nullptr, rec, s));
     STK_CUDA(cudaMemcpyAsync(d_sbeg, src_begin, n_src_box * sizeof(int), cudaMemcpyHostToDevice, s));
     STK_CUDA(cudaMemcpyAsync(d_send, src_end, n_src_box * sizeof(int), cudaMemcpyHostToDevice, s));

@@ -938,7 +938,10 @@ int build_i8_operators(FarField &F, cudaStream_t s) {
     if (!rc) rc = op(F.i8_l2l, F.l2l, 8 * N, N);
     if (!rc) rc = op(F.i8_vt, F.m2l_vt, k, N);
     if (!rc) rc = op(F.i8_e, F.m2l_e, N, k);
-    if (rc) return rc;
+    if (rc) {  // no memory for them: the products stay with cuBLAS
+        for (I8Buf *b : {&F.i8_uc2ue, &F.i8_dc2de, &F.i8_m2m, &F.i8_l2l, &F.i8_vt, &F.i8_e}) b->release();
+        return STK_OK;
+    }
     F.i8 = true;
     // the factors of every offset, within 8 GiB
     const int nslot = (int)F.m2l_r.size(), kb = (k + kI8Rows - 1) / kI8Rows;
@@ -959,7 +962,11 @@ int build_i8_operators(FarField &F, cudaStream_t s) {
     if (!rc) rc = F.i8_p.reserve_kscale(nslot * rmax);
     DevBuf mag;
     if (!rc) rc = mag.reserve(sizeof(unsigned long long) * k);
-    if (rc) return rc;
+    if (rc) {
+        F.i8_q.release();
+        F.i8_p.release();
+        return STK_OK;
+    }
     long long qcols = 0;
     for (int sl = 0; sl < nslot; sl++) qcols += F.m2l_r[sl];
     FCUDA(i8_row_scales((const double *)F.m2l_q.ptr, k, qcols, k, (unsigned long long *)mag.ptr, F.i8_q.up(),
@@ -996,11 +1003,9 @@ bool i8_wins(int M, int N, int K) {
 int far_product(FarField &F, const DevBuf &A, const I8Buf &A8, int M, int K, const double *X, const int *idx, int m,
                 const double *mul, int add, double *C, const int *cols, double *Xg, double *Y, cudaStream_t s) {
     if (m <= 0) return STK_OK;
-    if (F.i8 && i8_wins(M, m, K)) {
-        const int np = i8_gemm_parts(M, m, i8_kblocks(K));
-        int rc = F.i8_b.reserve(m, K);
-        if (!rc && np > 1) rc = F.i8_parts.reserve(sizeof(double) * (size_t)np * M * m);
-        if (rc) return rc;
+    const int np = i8_gemm_parts(M, m, i8_kblocks(K));
+    if (F.i8 && i8_wins(M, m, K) && !F.i8_b.reserve(m, K) &&
+        !(np > 1 && F.i8_parts.reserve(sizeof(double) * (size_t)np * M * m))) {
         t_launches += np > 1 ? 3 : 2;
         FCUDA(i8_digits(X, K, idx, m, K, F.i8_b.nkb, A8.up(), mul, F.i8_b.digits(), F.i8_b.scales(), s));
         FCUDA(i8_gemm(M, m, A8.op(), F.i8_b.op(), 1.0, add, C, M, cols, np > 1 ? (double *)F.i8_parts.ptr : nullptr,
@@ -1261,16 +1266,14 @@ int setup_pass(ListPass &P, int uk, const std::vector<int> &tb, const std::vecto
 
 int run_pass(const ListPass &P, int prec, const double *rec, const int *src_beg, const int *src_end,
              const double *trg_xyz, double *out, unsigned int *counter, DevBuf &parts, int sms, cudaStream_t s) {
-    const ItemList &il = P.items[prec];
-    if (il.n_items == 0) return STK_OK;
-    t_launches += il.n_groups ? 2 : 1;
+    if (P.items[prec].n_items == 0) return STK_OK;
     ListP2PArgs a{};
     a.src_rec = rec;
     a.src_box_begin = src_beg;
     a.src_box_end = src_end;
     a.list_ent = (const int *)P.ent.ptr;
-    const int rc = il.args(a, parts, uk_tdim_host(P.uk));
-    if (rc) return rc;
+    list_args(P.items, prec, uk_tdim_host(P.uk), parts, a);
+    t_launches += a.n_groups ? 2 : 1;
     a.counter = counter;
     a.trg_xyz = trg_xyz;
     a.trg_out = out;
@@ -1477,12 +1480,12 @@ static int setup_m2l_chunks_i8(FarField &F, const std::vector<int> &chunk_slot, 
     F.i8_t1_off[ngroups] = (int)t1.size();
     F.i8_t2_off[ngroups] = (int)t2.size();
     const long long gcols = (long long)gc * kM2LChunk;
-    int rc = F.i8_z.reserve(gcols, rmax);
-    // digits of phi_hat, one row per node
+    // digits of phi_hat, one row per node; without memory for the digits the chunks stay with cuBLAS
     F.i8_x.nkb = i8_kblocks(k);
-    if (!rc) rc = F.i8_x.dig.reserve(i8_row_bytes(nn, F.i8_x.nkb));
-    if (!rc) rc = F.i8_x.scale.reserve(sizeof(double) * (size_t)nn);
-    if (!rc) rc = F.i8_valid.upload(valid.data(), sizeof(int) * nc, s);
+    F.i8_chunks = !(F.i8_z.reserve(gcols, rmax) || F.i8_x.dig.reserve(i8_row_bytes(nn, F.i8_x.nkb)) ||
+                    F.i8_x.scale.reserve(sizeof(double) * (size_t)nn));
+    if (!F.i8_chunks) return STK_OK;
+    int rc = F.i8_valid.upload(valid.data(), sizeof(int) * nc, s);
     if (!rc) rc = F.i8_rank.upload(rank.data(), sizeof(int) * nc, s);
     if (!rc) rc = F.i8_slot.upload(chunk_slot.data(), sizeof(int) * nc, s);
     if (!rc) rc = F.i8_tiles1.upload(t1.data(), sizeof(I8Tile) * t1.size(), s);
@@ -1624,7 +1627,9 @@ static int setup_m2l_dense(FarField &F, const Octree &T, int nslot, cudaStream_t
     const size_t dig_bytes = i8_bytes((long long)qb * kI8Rows, i8_kblocks(k)) +
                              i8_bytes(64LL * kb * kI8Rows, i8_kblocks(rcc_all)) +
                              i8_bytes(nmax, i8_kblocks(k)) + i8_bytes(nmax, i8_kblocks(rcc_all));
-    F.dn_i8 = F.i8_pq && dig_bytes <= (16ull << 30);
+    F.dn_i8 = F.i8_pq && dig_bytes <= (16ull << 30) &&
+              !(F.dn_q8.reserve((long long)std::max(qb, 1) * kI8Rows, k) || F.dn_p8.reserve(64LL * kb * kI8Rows, rcc_all) ||
+                F.dn_phi8.reserve(nmax, k) || F.dn_zc8.reserve(nmax, rcc_all));
     // tensor-core operands of the mixed path (3xTF32 hi / lo, K-major rows of a multiple
     // of 4 floats): Qs_c'^T per source type and Pv_{c,c'}^T per block, within 4 GiB
     F.tc = false;
@@ -1684,13 +1689,9 @@ static int setup_m2l_dense(FarField &F, const Octree &T, int nslot, cudaStream_t
     if (!rc) rc = F.dn_srow.upload(srow.data(), sizeof(int) * srow.size(), s);
     if (rc) return rc;
     if (F.dn_i8) {
-        rc = F.dn_q8.reserve((long long)std::max(qb, 1) * kI8Rows, k);
-        if (!rc) rc = F.dn_p8.reserve(64LL * kb * kI8Rows, rcc_all);
-        if (!rc) rc = F.dn_phi8.reserve(nmax, k);
-        if (!rc) rc = F.dn_zc8.reserve(nmax, rcc_all);
         // the scales along K of every block row: those of its offset's P_d
         DevBuf ksrc;
-        if (!rc) rc = F.dn_ks.reserve(sizeof(double) * 2 * F.dn_rows);
+        rc = F.dn_ks.reserve(sizeof(double) * 2 * F.dn_rows);
         if (!rc) rc = ksrc.upload(pcol.data(), sizeof(int) * pcol.size(), s);
         if (rc) return rc;
         gather_scales_kernel<<<grid_for((long long)F.dn_rows), 256, 0, s>>>(
@@ -2282,10 +2283,10 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
         maxm = std::max(maxm, std::max(ms, mx));
         if (F.i8) {  // the largest right-hand operand of far_product
             auto shape = [&](int M, int m, int K) {
-                if (rc || m <= 0 || !i8_wins(M, m, K)) return;
+                if (m <= 0 || !i8_wins(M, m, K)) return;
                 const int np = i8_gemm_parts(M, m, i8_kblocks(K));
-                rc = F.i8_b.reserve(m, K);
-                if (!rc && np > 1) rc = F.i8_parts.reserve(sizeof(double) * (size_t)np * M * m);
+                F.i8_b.reserve(m, K);  // far_product goes to cuBLAS without
+                if (np > 1) F.i8_parts.reserve(sizeof(double) * (size_t)np * M * m);
             };
             for (int l = 0; l <= T.depth(); l++) {
                 const int m = F.parent_off[l + 1] - F.parent_off[l];
@@ -2296,7 +2297,6 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
             shape(N, mx, N);
             shape(k, nn, N);
             shape(N, nn, k);
-            if (rc) return rc;
         }
         rc = F.tmp0.reserve(sizeof(double) * (size_t)std::max(maxm, 1) * N);
         if (!rc) rc = F.tmp1.reserve(sizeof(double) * (size_t)std::max(maxm, 1) * N);

@@ -70,6 +70,11 @@ struct I8Buf {
         kn = K;
         return kscale.reserve(sizeof(double) * 2 * (size_t)K);
     }
+    void release() {
+        dig.release();
+        scale.release();
+        kscale.release();
+    }
     double *up() const { return (double *)kscale.ptr; }
     double *down() const { return (double *)kscale.ptr + kn; }
     int reserve(long long rows, int K) {

@@ -15,6 +15,7 @@
 #include <map>
 #include <memory>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/stkfmm_b200.h"
@@ -84,15 +85,14 @@ int ItemList::upload(const std::vector<WorkItem> &it, const std::vector<PartGrou
     return rc;
 }
 
-int ItemList::args(ListP2PArgs &a, DevBuf &parts, int tdim) const {
-    a.items = (const WorkItem *)items.ptr;
-    a.n_items = n_items;
-    a.groups = (const PartGroup *)groups.ptr;
-    a.n_groups = n_groups;
-    if (!n_groups) return STK_OK;
-    const int rc = parts.reserve(sizeof(double) * (size_t)part_targets * tdim);
+void list_args(const ItemList (&lists)[2], int prec, int tdim, DevBuf &parts, ListP2PArgs &a) {
+    const ItemList *il = &lists[prec];
+    if (il->n_groups && parts.reserve(sizeof(double) * (size_t)il->part_targets * tdim)) il = &lists[1];
+    a.items = (const WorkItem *)il->items.ptr;
+    a.n_items = il->n_items;
+    a.groups = (const PartGroup *)il->groups.ptr;
+    a.n_groups = il->n_groups;
     a.parts = (double *)parts.ptr;
-    return rc;
 }
 
 KernelData::~KernelData() {
@@ -375,8 +375,8 @@ int stk::near_device(Stk3DFMM *f, KernelData *kd, const double *d_sl, const doub
         if (k == 1 && (!dl || kd->fused)) continue;
         // the FMM's near field: U list plus the W / X interactions evaluated directly
         const ListPass *fp = far ? &kd->far->near[k] : nullptr;
-        const ItemList &il = far ? fp->items[f->precision] : kd->u_items[k][f->precision];
-        if (il.n_items == 0) continue;
+        const ItemList(&lists)[2] = far ? fp->items : std::as_const(kd->u_items[k]);
+        if (lists[f->precision].n_items == 0) continue;
         const int uk = kd->fused ? fused_uk(kd) : ki->slot[k == 0 ? SLOT_S2T_SL : SLOT_S2T_DL];
         const int rs = uk_record_stride(uk);
         const PointSet &sp = T.sets[k];
@@ -391,7 +391,7 @@ int stk::near_device(Stk3DFMM *f, KernelData *kd, const double *d_sl, const doub
         a.src_box_begin = (const int *)kd->d_beg[k].ptr;
         a.src_box_end = (const int *)kd->d_end[k].ptr;
         a.list_ent = far ? (const int *)fp->ent.ptr : (const int *)kd->d_uent.ptr;
-        if ((rc = il.args(a, kd->d_parts, td))) return rc;
+        list_args(lists, f->precision, td, kd->d_parts, a);
         a.counter = (unsigned int *)kd->d_counter.ptr;
         a.trg_xyz = (const double *)kd->d_xyz[2].ptr;
         a.trg_out = out;
@@ -401,7 +401,7 @@ int stk::near_device(Stk3DFMM *f, KernelData *kd, const double *d_sl, const doub
         // one octree holds the sources and the targets: coincident points share a leaf
         a.coincident_own_box = 1;
         HCUDA(launch_list_p2p(uk, f->precision, a, f->sms, s));
-        launches += il.n_groups ? 3 : 2;  // record packing, list kernel, split sums
+        launches += a.n_groups ? 3 : 2;  // record packing, list kernel, split sums
     }
     HCUDA(cudaEventRecord(kd->ph[0], s));
     kd->last_far = far;

@@ -52,9 +52,12 @@ struct ItemList {
         n_groups = o.n_groups;
         part_targets = o.part_targets;
     }
-    // items, groups and the slots' buffer into the kernel's arguments (tdim components)
-    int args(ListP2PArgs &a, DevBuf &parts, int tdim) const;
 };
+
+// The items of a pass [FP64, mixed] for `prec`, its groups and the slots' buffer into the kernel's
+// arguments (tdim components).  Without memory for the slots an FP64 pass takes the mixed
+// path's items, which split no sources.
+void list_args(const ItemList (&lists)[2], int prec, int tdim, DevBuf &parts, ListP2PArgs &a);
 
 // One activated kernel: the reference's impl::FMMData (STKFMM_impl.hpp:19-174).
 struct KernelData {

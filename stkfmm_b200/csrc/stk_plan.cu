@@ -33,10 +33,9 @@ struct stk_p2p_plan {
     int *d_sbeg = nullptr, *d_send = nullptr, *d_ent = nullptr;
     stk::WorkItem *d_items[2] = {nullptr, nullptr};
     stk::PartGroup *d_groups = nullptr;
-    double *d_parts = nullptr;  // sums of split sources, grown to the largest micro-kernel used
-    size_t parts_cap = 0;       // doubles
+    double *d_parts[2] = {nullptr, nullptr};  // sums of split sources, 8 and 16 doubles per slot
     unsigned int *d_counter = nullptr;
-    double *d_rec = nullptr;  // packed source records, grown to the largest record stride used
+    double *d_rec = nullptr;  // packed source records, grown to the largest record stride used (at least 8)
     size_t rec_cap = 0;       // doubles
     ~stk_p2p_plan() {
         cudaFree(d_sbeg);
@@ -45,7 +44,8 @@ struct stk_p2p_plan {
         cudaFree(d_items[0]);
         cudaFree(d_items[1]);
         cudaFree(d_groups);
-        cudaFree(d_parts);
+        cudaFree(d_parts[0]);
+        cudaFree(d_parts[1]);
         cudaFree(d_counter);
         cudaFree(d_rec);
     }
@@ -160,29 +160,45 @@ extern "C" int stk_p2p_plan_execute(stk_p2p_plan *plan, int ukernel, int precisi
     if (cudaGetDevice(&dev) != cudaSuccess || dev != plan->device) return STK_ERR_INVALID_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     const int sd = stk::uk_sdim_host(ukernel), rs = stk::uk_record_stride(ukernel);
-    // grow a buffer: earlier executions may still use it on any stream; at least eight doubles
-    // per source and per split target slot, so that a forward pass and its adjoints (3 and 7
-    // components) allocate once
-    auto grow = [](double **buf, size_t *cap, size_t need) {
-        if (*cap >= need) return true;
-        if (*buf) {
+    // records, at least eight doubles each where they can be had, so that a forward pass and its
+    // adjoints (3 to 5 staged values) allocate once
+    const size_t n = std::max(plan->nsrc, 1), need = n * rs;
+    if (plan->rec_cap < need) {
+        // grow the record buffer: earlier executions may still read it on any stream
+        if (plan->d_rec) {
             cudaDeviceSynchronize();
-            cudaFree(*buf);
-            *buf = nullptr;
-            *cap = 0;
+            cudaFree(plan->d_rec);
+            plan->d_rec = nullptr;
+            plan->rec_cap = 0;
         }
-        if (cudaMalloc(buf, need * sizeof(double)) != cudaSuccess) {
+        size_t cap = n * std::max(rs, 8);
+        if (cudaMalloc(&plan->d_rec, cap * sizeof(double)) != cudaSuccess) {
             cudaGetLastError();
-            return false;
+            cap = need;
+            if (cudaMalloc(&plan->d_rec, cap * sizeof(double)) != cudaSuccess) {
+                cudaGetLastError();
+                return STK_ERR_CUDA;
+            }
         }
-        *cap = need;
-        return true;
-    };
-    if (!grow(&plan->d_rec, &plan->rec_cap, (size_t)std::max(plan->nsrc, 1) * std::max(rs, 8)))
-        return STK_ERR_CUDA;
-    if (!mixed && plan->n_groups > 0 &&
-        !grow(&plan->d_parts, &plan->parts_cap, (size_t)plan->part_targets * std::max(stk::uk_tdim_host(ukernel), 8)))
-        return STK_ERR_CUDA;
+        plan->rec_cap = cap;
+    }
+    // The split sums' slots: one buffer for up to eight components and one beyond, each allocated
+    // once and kept, so that a captured execution keeps its buffer; during a capture, too (relaxed:
+    // an allocation is no part of the stream's work).  Without memory for them the mixed path's
+    // items are taken, which split no sources.
+    const int td = stk::uk_tdim_host(ukernel);
+    double **parts = &plan->d_parts[td > 8];
+    int list = mixed;
+    if (!mixed && plan->n_groups > 0 && !*parts) {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (cudaMalloc(parts, (size_t)plan->part_targets * (td > 8 ? 16 : 8) * sizeof(double)) != cudaSuccess) {
+            cudaGetLastError();
+            *parts = nullptr;
+            list = 1;
+        }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+    }
     if (stk::launch_pack_records(ukernel, plan->nsrc, nullptr, d_src_coord, d_src_value, sd, nullptr, plan->d_rec, s) !=
         cudaSuccess)
         return STK_ERR_CUDA;
@@ -191,12 +207,12 @@ extern "C" int stk_p2p_plan_execute(stk_p2p_plan *plan, int ukernel, int precisi
     a.src_box_begin = plan->d_sbeg;
     a.src_box_end = plan->d_send;
     a.list_ent = plan->d_ent;
-    a.items = plan->d_items[mixed];
-    a.n_items = plan->n_items[mixed];
-    if (!mixed) {
+    a.items = plan->d_items[list];
+    a.n_items = plan->n_items[list];
+    if (list == 0) {
         a.groups = plan->d_groups;
         a.n_groups = plan->n_groups;
-        a.parts = plan->d_parts;
+        a.parts = *parts;
     }
     a.counter = plan->d_counter;
     a.trg_xyz = d_trg_coord;

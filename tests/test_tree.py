@@ -157,3 +157,24 @@ def test_empty_sets():
     t = Octree(pts, 8, 0, sl=np.zeros((0, 3)), trg=pts)
     off, ent = t.list("U")
     assert len(ent) == 0
+
+
+@pytest.mark.parametrize("dup,n", [(1, 1), (1, 2), (3, 5), (1, 3000), (40, 4000), (1, 70000)])
+def test_point_order_is_a_stable_morton_sort(dup, n):
+    """Points in Morton order, those of one key (equal points, dup copies of each) in the caller's
+    order; a set equal to the tree's points and one that differs in its last point agree but there."""
+    rng = np.random.default_rng(n)
+    pts = np.concatenate([clustered_points(rng, (n + dup - 1) // dup, nclusters=4, sigma=1e-4)] * dup)[:n]
+    pts = pts[rng.permutation(n)]
+    other = pts.copy()
+    other[-1] = 0.0  # the first key of all
+    t = Octree(pts, 30, 0, sl=pts, dl=other, trg=pts)
+    q = np.floor(pts * 2.0 ** 20).astype(np.int64)
+    key = np.zeros(n, dtype=np.int64)
+    for b in range(20):
+        for d in range(3):
+            key |= (q[:, d] >> b & 1) << (3 * b + d)
+    perm = t.point_set(0)[0]
+    np.testing.assert_array_equal(perm, np.argsort(key, kind="stable"))
+    np.testing.assert_array_equal(t.point_set(2)[0], perm)
+    np.testing.assert_array_equal(t.point_set(1)[0], np.concatenate([[n - 1], perm[perm != n - 1]]))
