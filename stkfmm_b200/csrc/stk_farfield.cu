@@ -1378,7 +1378,8 @@ int record_built(FarField &e, cudaStream_t s) {
 // Every tile is 128 x 128 (rows of the factor x columns of the chunk) over the whole K.
 // The operands (~8 (sum_d r_d k + nslot k rmax) bytes) must fit in 4 GiB, else the
 // SIMT path stays; STKFMM_M2L_TC=0 turns both tensor-core paths off.
-static int setup_m2l_chunks_tc(FarField &F, const std::vector<int> &chunk_slot, int nslot, cudaStream_t s) {
+static int setup_m2l_chunks_tc(FarField &F, const std::vector<int> &chunk_slot, const std::vector<int> &valid, int nslot,
+                               cudaStream_t s) {
     F.tcc = false;
     const char *env_tc = getenv("STKFMM_M2L_TC");
     if ((env_tc && env_tc[0] == '0') || !umma_available() || F.m2l_chunks == 0) return STK_OK;
@@ -1419,16 +1420,14 @@ static int setup_m2l_chunks_tc(FarField &F, const std::vector<int> &chunk_slot, 
             const int sl = chunk_slot[c], r = F.m2l_r[sl];
             const long long col = (long long)(c - g * gc) * kM2LChunk;  // first column within the group
             const int qrow0 = (int)(F.m2l_pq_off[sl] / (size_t)k);
-            for (int nt = 0; nt < kM2LChunk / 128; nt++) {
-                const long long cn = col + 128LL * nt;
-                for (int m0 = 0; m0 < r; m0 += 128) {
-                    const int mv = std::min(128, r - m0);
-                    t1.push_back(GroupTile{qrow0 + m0, (int)cn, k, mv, mv, 128, rmax, 0, cn * rmax + m0});
-                }
-                for (int m0 = 0; m0 < k; m0 += 128) {
-                    const int mv = std::min(128, k - m0);
-                    t2.push_back(GroupTile{sl * k + m0, (int)cn, r, mv, mv, 128, k, 0, cn * k + m0});
-                }
+            static_assert(kM2LChunk == 128, "a chunk is one tile wide");
+            for (int m0 = 0; m0 < r; m0 += 128) {
+                const int mv = std::min(128, r - m0);
+                t1.push_back(GroupTile{qrow0 + m0, (int)col, k, mv, mv, valid[c], rmax, 0, col * rmax + m0});
+            }
+            for (int m0 = 0; m0 < k; m0 += 128) {
+                const int mv = std::min(128, k - m0);
+                t2.push_back(GroupTile{sl * k + m0, (int)col, r, mv, mv, valid[c], k, 0, col * k + m0});
             }
         }
     }
@@ -1445,7 +1444,7 @@ static int setup_m2l_chunks_tc(FarField &F, const std::vector<int> &chunk_slot, 
 // The same two stages for the FP64 path on the int8 tensor cores: Z_c = Q_d^T X_c and
 // Y_c = P_d Z_c in FP64, the digits of Z formed between the two launches.  The digits of
 // phi_hat are formed once per node and gathered by the first launch itself.
-static int setup_m2l_chunks_i8(FarField &F, const std::vector<int> &chunk_slot, const std::vector<int> &gsrc, int nn,
+static int setup_m2l_chunks_i8(FarField &F, const std::vector<int> &chunk_slot, const std::vector<int> &valid, int nn,
                                cudaStream_t s) {
     // Bases of up to two row blocks (laplace_p) have offsets of rank ~50: most of a 128-row tile
     // is padding and a tile's drain takes longer than its products.  LapPGrad, 1M points, p = 10
@@ -1456,19 +1455,16 @@ static int setup_m2l_chunks_i8(FarField &F, const std::vector<int> &chunk_slot, 
     const int k = F.m2l_rank, kb = (k + kI8Rows - 1) / kI8Rows, rmax = F.m2l_rmax;
     const int nc = F.m2l_chunks, gc = F.m2l_group_chunks, ngroups = (nc + gc - 1) / gc;
     std::vector<I8Tile> t1, t2;
-    std::vector<int> rank(nc), valid(nc);  // a chunk's real columns come first
+    std::vector<int> rank(nc);
     F.i8_t1_off.assign(ngroups + 1, 0);
     F.i8_t2_off.assign(ngroups + 1, 0);
     for (int g = 0; g < ngroups; g++) {
         F.i8_t1_off[g] = (int)t1.size();
         F.i8_t2_off[g] = (int)t2.size();
         for (int c = g * gc; c < std::min(nc, (g + 1) * gc); c++) {
-            const int sl = chunk_slot[c], r = F.m2l_r[sl], ci = c - g * gc;
+            const int sl = chunk_slot[c], r = F.m2l_r[sl], ci = c - g * gc, nv = valid[c];
             const long long col = (long long)ci * kM2LChunk;
             rank[c] = r;
-            int nv = 0;
-            while (nv < kM2LChunk && gsrc[(size_t)c * kM2LChunk + nv] >= 0) nv++;
-            valid[c] = nv;
             for (int m0 = 0; m0 < r; m0 += kI8Rows)
                 t1.push_back(I8Tile{F.i8_q_blk[sl] + m0 / kI8Rows, ci, i8_kblocks(k), std::min(kI8Rows, r - m0), nv,
                                     rmax, col * rmax + m0});
@@ -2221,8 +2217,11 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
         if (!rc) rc = F.m2l_y.reserve(sizeof(double) * (size_t)k * gcols);
         if (!rc) rc = F.m2l_z.reserve(sizeof(double) * (size_t)rmax * gcols);
         if (rc) return rc;
-        rc = setup_m2l_chunks_tc(F, chunk_slot, nslot, s);
-        if (!rc) rc = setup_m2l_chunks_i8(F, chunk_slot, gsrc, nn, s);
+        std::vector<int> valid(nc);  // a chunk's columns come first
+        for (int c = 0; c < nc; c++)
+            while (valid[c] < kM2LChunk && gsrc[(size_t)c * kM2LChunk + valid[c]] >= 0) valid[c]++;
+        rc = setup_m2l_chunks_tc(F, chunk_slot, valid, nslot, s);
+        if (!rc) rc = setup_m2l_chunks_i8(F, chunk_slot, valid, nn, s);
         if (rc) return rc;
         F.m2l_seg.clear();
         if (!F.tcc || !F.i8_chunks) {

@@ -5,9 +5,8 @@
 //           and one of the B block's into a 4-stage shared-memory ring;
 //   warp 1  TMEM owner and MMA issuer: tcgen05.mma kind::i8, M = 128, N = 128, K = 32;
 //   warps 2-17 drain: tcgen05.ld, the digit groups put together in int64, then FP64;
-//   warps 18, 19 (gathered columns only) fetch B's rows in 16-byte asynchronous copies, the
-//           224 bytes of a row and K block by neighbouring lanes, two stages in flight
-//           before a stage is handed on.
+//   warps 18, 19 (gathered columns only) fetch B's rows in 16-byte asynchronous copies, eight
+//           lanes per row, two stages in flight before a stage is handed on.
 // The eight digit groups i + j = 0 .. 7 need 8 x 128 TMEM columns and there are 512, so a
 // tile takes two passes over K: groups 0-3 (planes 0-3 of both operands, 10 products per K
 // block) drained into an int64 per output, then groups 4-7 (all planes, 24 products).
@@ -18,7 +17,6 @@
 // Every mbarrier wait has an iteration limit: on expiry the kernel records an error code,
 // stops issuing work, waits (bounded) for what it issued, frees its TMEM and returns.
 #include <algorithm>
-#include <mutex>
 #include <type_traits>
 
 #include <cooperative_groups.h>
@@ -42,13 +40,13 @@ constexpr int kDrainCols = kBN / (kDrainWarps / 4);
 constexpr int kGatherWarps = 2;
 template <class Job> constexpr int kThreads = 32 * (2 + kDrainWarps + (Job::kGather ? kGatherWarps : 0));
 constexpr uint32_t kTmemCols = 512;
-constexpr int kSmemBytes = kStages * kStageBytes + 1536 /* barriers, gathered rows */ + 128 /* alignment */;
+constexpr int kSmemBytes = kStages * kStageBytes + 2304 /* barriers, column scales */ + 128 /* alignment */;
 static_assert(kSmemBytes <= 232448, "shared memory of one CTA");
 
 struct Bars {
     unsigned long long full[kStages], empty[kStages], accf, acce;
     uint32_t tmem;
-    int rows[2][kBN];  // gathered rows of this tile and the next
+    double col_scale[2][kBN / kDrainCols][kDrainCols];
 };
 
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
@@ -68,16 +66,17 @@ __device__ __forceinline__ uint64_t plane_desc(uint32_t addr) {
     return d;
 }
 
-// instruction descriptor: D S32, A and B S8, both K-major, M = 128, N = 128
-constexpr uint32_t kIdesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kBN >> 3) << 17) |
-                            ((uint32_t)(kBM >> 4) << 24);
+// instruction descriptor: D S32, A and B S8, both K-major, M = 128, N columns (a multiple of 16)
+__device__ __forceinline__ uint32_t idesc_i8(int N) {
+    return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+}
 
-__device__ __forceinline__ void mma_i8(uint32_t d, uint64_t a, uint64_t b, uint32_t acc) {
+__device__ __forceinline__ void mma_i8(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
-        "l"(a), "l"(b), "r"(kIdesc), "r"(acc)
+        "l"(a), "l"(b), "r"(idesc), "r"(acc)
         : "memory");
 }
 
@@ -227,7 +226,9 @@ __global__ void __launch_bounds__(kThreads<Job>, 1)
         if (lane == 0) {
             unsigned g = 0, a = 0;  // stages consumed, accumulations started
             for (int t = blockIdx.x; t < job.ntiles && ok; t += gridDim.x) {
-                const int nkb = job.tile(t).nkb;
+                const auto ts = job.tile(t);
+                const int nkb = ts.nkb;
+                const uint32_t idesc = idesc_i8((max(ts.n_valid, 1) + 15) & ~15);
                 for (int k0 = 0; k0 < nkb && ok; k0 += kI8MaxSegment) {
                     const int n = min(nkb - k0, kI8MaxSegment);
                     for (int pass = 0; pass < 2 && ok; pass++, a++) {
@@ -252,13 +253,14 @@ __global__ void __launch_bounds__(kThreads<Job>, 1)
                                 for (int gr = 0; gr < 4; gr++)
 #pragma unroll
                                     for (int i = 0; i <= gr; i++)
-                                        mma_i8(tmem + gr * kBN, da + i * step, db + (gr - i) * step, i ? 1u : first);
+                                        mma_i8(tmem + gr * kBN, da + i * step, db + (gr - i) * step, idesc,
+                                               i ? 1u : first);
                             } else {
 #pragma unroll
                                 for (int gr = 4; gr < 8; gr++)
 #pragma unroll
                                     for (int i = gr > 6; i <= min(gr, 6); i++)
-                                        mma_i8(tmem + (gr - 4) * kBN, da + i * step, db + (gr - i) * step,
+                                        mma_i8(tmem + (gr - 4) * kBN, da + i * step, db + (gr - i) * step, idesc,
                                                i > (gr > 6) ? 1u : first);
                             }
                             mma_commit(saddr(&bars->empty[s]));
@@ -281,24 +283,26 @@ __global__ void __launch_bounds__(kThreads<Job>, 1)
     } else if (Job::kGather && warp >= 2 + kDrainWarps) {
         // ---- gathered columns ----
         if constexpr (Job::kGather) {
-            const int tid = (warp - 2 - kDrainWarps) * 32 + lane;
-            constexpr int kN = 32 * kGatherWarps;
-            unsigned g = 0;
-            int buf = 0;
-            auto fetch = [&](auto planes, uint32_t dst, const uint8_t *src, const int *rows, int n, size_t pitch) {
-                constexpr int kPieces = 2 * decltype(planes)::value;  // of 16 bytes per row
-                for (int i = tid; i < n * kPieces; i += kN) {
-                    const int r = i / kPieces, j = i - r * kPieces;
-                    cp_async16(dst + (j >> 1) * kI8PlaneBytes + (r >> 3) * 256 + (j & 1) * 128 + (r & 7) * 16,
-                               src + rows[r] * pitch + j * 16);
-                }
+            // A copy instruction takes four 16-byte pieces of eight rows: the eight rows of a piece are
+            // one core matrix, 128 bytes of shared memory without bank conflicts (the MMAs alone
+            // read close to what it can give).  A thread keeps the numbers of its 16 rows of the
+            // tile, so that a copy is an address and an instruction.
+            constexpr int kTurns = kBN / 8;
+            static_assert(kGatherWarps == 2 && kI8Planes == 7, "14 pieces: 4 + 4 of planes 0-3, 3 + 3 of the others");
+            const int w = warp - 2 - kDrainWarps, r = lane & 7, q = lane >> 3;
+            const int j = 4 * w + q, j2 = 8 + 3 * w + q;
+            auto place = [&](int piece) {
+                return (uint32_t)(kI8BlockBytes + (piece >> 1) * kI8PlaneBytes + (piece & 1) * 128 + r * 16);
             };
+            const uint32_t d = place(j), d2 = place(j2);
+            unsigned g = 0;
             const size_t pitch = (size_t)B.nkb * (kI8Planes * kI8K);
-            for (int t = blockIdx.x; t < job.ntiles && ok; t += gridDim.x, buf ^= 1) {
+            for (int t = blockIdx.x; t < job.ntiles && ok; t += gridDim.x) {
                 const auto ts = job.tile(t);
-                int *rows = bars->rows[buf];
-                for (int i = tid; i < ts.n_valid; i += kN) rows[i] = job.rows[ts.b_blk * kBN + i];
-                asm volatile("bar.sync 1, %0;" ::"n"(kN) : "memory");
+                const int turns = (ts.n_valid - r + 7) >> 3;
+                int row[kTurns];
+#pragma unroll
+                for (int i = 0; i < kTurns; i++) row[i] = i < turns ? job.rows[ts.b_blk * kBN + r + 8 * i] : 0;
                 for (int k0 = 0; k0 < ts.nkb && ok; k0 += kI8MaxSegment) {
                     const int k1 = min(ts.nkb, k0 + kI8MaxSegment);
                     for (int pass = 0; pass < 2 && ok; pass++)
@@ -308,12 +312,16 @@ __global__ void __launch_bounds__(kThreads<Job>, 1)
                                 ok = false;
                                 break;
                             }
-                            const uint32_t dst = saddr(ring + s * kStageBytes) + kI8BlockBytes;
+                            const uint32_t st = saddr(ring + s * kStageBytes);
                             const uint8_t *src = B.dig + (size_t)kb * (kI8Planes * kI8K);
-                            if (pass == 0)
-                                fetch(std::integral_constant<int, 4>(), dst, src, rows, ts.n_valid, pitch);
-                            else
-                                fetch(std::integral_constant<int, kI8Planes>(), dst, src, rows, ts.n_valid, pitch);
+#pragma unroll
+                            for (int i = 0; i < kTurns; i++)
+                                if (i < turns) cp_async16(st + d + i * 256, src + row[i] * pitch + j * 16);
+                            if (pass == 1 && q < 3) {
+#pragma unroll
+                                for (int i = 0; i < kTurns; i++)
+                                    if (i < turns) cp_async16(st + d2 + i * 256, src + row[i] * pitch + j2 * 16);
+                            }
                             cp_async_commit();
                             if (g >= 2) {  // the stage issued two before has landed
                                 cp_async_wait<2>();
@@ -336,10 +344,19 @@ __global__ void __launch_bounds__(kThreads<Job>, 1)
         const int row = q * 32 + lane;
         const uint32_t tb = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0;
         unsigned a = 0;  // accumulations drained so far
+        int buf = 0;
         for (int t = blockIdx.x; t < job.ntiles && ok; t += gridDim.x) {
             const auto ts = job.tile(t);
             const bool mine = row < ts.m_valid;
             const double sa = mine ? job.alpha * A.scale[ts.a_blk * kBM + row] : 0.0;
+            // the columns' scales into shared memory while the MMAs run (read per column inside the
+            // drain they cost it its length again: L2 latency, twice for gathered columns); the
+            // four warps of these columns write the same values, and none is two tiles ahead
+            static_assert(kDrainCols == 32, "a lane per column");
+            double *sn = bars->col_scale[buf][c0 / kDrainCols];
+            buf ^= 1;
+            sn[lane] = c0 + lane < ts.n_valid ? job.scale(B.scale, ts, c0 + lane) : 0.0;
+            __syncwarp();
             for (int k0 = 0; k0 < ts.nkb && ok; k0 += kI8MaxSegment) {
                 const bool add = job.add || k0 > 0;
                 // groups 0-3: hi = sum_g acc_g 256^(3 - g)
@@ -390,7 +407,7 @@ __global__ void __launch_bounds__(kThreads<Job>, 1)
                         if (mine && n < ts.n_valid) {
                             const double v = fma((double)hi[c + j], 4294967296.0, (double)lo);
                             double *p = job.at(pc, ts, n);
-                            const double r = v * job.scale(B.scale, ts, n) * sa;
+                            const double r = v * sn[c + j] * sa;
                             *p = add ? *p + r : r;
                         }
                         pc += step;
@@ -678,11 +695,8 @@ int sm_count() {
 }
 
 template <class Job> cudaError_t launch_gemm(const I8Operand &A, const I8Operand &B, const Job &job, int *err, cudaStream_t s) {
-    static std::once_flag once;
-    static cudaError_t e = cudaSuccess;
-    std::call_once(once, [] {
-        e = cudaFuncSetAttribute(i8_gemm_kernel<Job>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    });
+    // for the current device
+    const cudaError_t e = cudaFuncSetAttribute(i8_gemm_kernel<Job>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
     if (e != cudaSuccess) return e;
     i8_gemm_kernel<Job><<<std::min(job.ntiles, sm_count()), kThreads<Job>, kSmemBytes, s>>>(A, B, job, err);
     return cudaGetLastError();

@@ -102,16 +102,17 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
     return d;
 }
 
-// instruction descriptor: D FP32, A and B TF32, both K-major, M = 128, N = 128
-constexpr uint32_t kIdesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(kBN >> 3) << 17) |
-                            ((uint32_t)(kBM >> 4) << 24);
+// instruction descriptor: D FP32, A and B TF32, both K-major, M = 128, N columns (a multiple of 16)
+__device__ __forceinline__ uint32_t idesc_tf32(int N) {
+    return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+}
 
-__device__ __forceinline__ void mma_tf32(uint32_t d, uint64_t a, uint64_t b, uint32_t acc) {
+__device__ __forceinline__ void mma_tf32(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(d),
-        "l"(a), "l"(b), "r"(kIdesc), "r"(acc), "r"(0), "r"(0), "r"(0), "r"(0)
+        "l"(a), "l"(b), "r"(idesc), "r"(acc), "r"(0), "r"(0), "r"(0), "r"(0)
         : "memory");
 }
 
@@ -143,7 +144,7 @@ __device__ __forceinline__ void tmem_ld32_nowait(uint32_t taddr, uint32_t (&r)[3
 // columns [0, 128) rows b_row .. b_row + 127 of B (tensor-map coordinates), summed
 // over k < K (K-blocks of 32; the maps zero-fill beyond their inner extent).
 struct TileSpec {
-    int a_row, b_row, K;
+    int a_row, b_row, K, n_valid;
 };
 
 // One GEMM C = A B^T over (gx = ceil(M/128)) x ceil(N/128) tiles.
@@ -151,7 +152,7 @@ struct DenseJob {
     static constexpr bool kGather = false;
     int M, N, K, ldc, beta, gx, ntiles;
     float *C;
-    __device__ TileSpec tile(int i) const { return {(i % gx) * kBM, (i / gx) * kBN, K}; }
+    __device__ TileSpec tile(int i) const { return {(i % gx) * kBM, (i / gx) * kBN, K, min(kBN, N - (i / gx) * kBN)}; }
     __device__ void store(int, const TileSpec &t, int row, const float (&acc)[kBN]) const {
         const int m = t.a_row + row;
         if (m >= M) return;
@@ -177,7 +178,7 @@ template <bool GATHER> struct GroupJob {
     int b_rows;  // rows of B: beyond it the copies fill zeros
     __device__ TileSpec tile(int i) const {
         const GroupTile &g = tiles[i];
-        return {g.a_row, g.b_row, g.K};
+        return {g.a_row, g.b_row, g.K, g.n_valid};
     }
     __device__ void store(int i, const TileSpec &, int row, const float (&acc)[kBN]) const {
         const GroupTile &g = tiles[i];
@@ -245,11 +246,13 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (warp == 0) {
         // ---- TMA producer ----
         if constexpr (Job::kGather) {
-            // the whole warp: lane i copies rows 4 i .. 4 i + 3 of the tile's B block
+            // the whole warp: lane i copies rows 4 i .. 4 i + 3 of the tile's B block, up to n_valid
             long long g = 0;
             for (int t = blockIdx.x; t < job.ntiles && ok; t += gridDim.x) {
                 const TileSpec ts = job.tile(t);
-                int4 r = reinterpret_cast<const int4 *>(job.rows + ts.b_row)[lane];
+                const int nl = (ts.n_valid + 3) >> 2;
+                int4 r = make_int4(0, 0, 0, 0);
+                if (lane < nl) r = reinterpret_cast<const int4 *>(job.rows + ts.b_row)[lane];
                 r.x = r.x < 0 ? job.b_rows : r.x;
                 r.y = r.y < 0 ? job.b_rows : r.y;
                 r.z = r.z < 0 ? job.b_rows : r.z;
@@ -265,13 +268,15 @@ __global__ void __launch_bounds__(kThreads, 1)
                     const uint32_t fb = saddr(&bars->full[s]);
                     const uint32_t st = saddr(tiles + s * kStageBytes);
                     if (lane == 0) {
-                        mbar_expect_tx(fb, kStageBytes);
+                        mbar_expect_tx(fb, 2 * kTileBytes + nl * 1024);
                         tma_load_2d(st, &mAh, fb, kb * kBK, ts.a_row);
                         tma_load_2d(st + kTileBytes, &mAl, fb, kb * kBK, ts.a_row);
                     }
                     __syncwarp();
-                    tma_gather4(st + 2 * kTileBytes + lane * 512, &mBh, fb, kb * kBK, r);
-                    tma_gather4(st + 3 * kTileBytes + lane * 512, &mBl, fb, kb * kBK, r);
+                    if (lane < nl) {
+                        tma_gather4(st + 2 * kTileBytes + lane * 512, &mBh, fb, kb * kBK, r);
+                        tma_gather4(st + 3 * kTileBytes + lane * 512, &mBl, fb, kb * kBK, r);
+                    }
                 }
             }
             if (!ok && lane == 0) {
@@ -311,7 +316,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (lane == 0) {
             long long g = 0;  // K-blocks committed so far
             for (int t = blockIdx.x; t < job.ntiles && ok; t += gridDim.x) {
-                const int nkb = (job.tile(t).K + kBK - 1) / kBK;
+                const TileSpec ts = job.tile(t);
+                const int nkb = (ts.K + kBK - 1) / kBK;
+                const uint32_t idesc = idesc_tf32((max(ts.n_valid, 1) + 15) & ~15);
                 for (int kb = 0; kb < nkb; kb++) {
                     const int s = (int)(g % kStages), b = (int)(g % kAccBufs);
                     if (!mbar_wait(saddr(&bars->acce[b]), ((uint32_t)(g / kAccBufs) & 1u) ^ 1u) ||
@@ -329,9 +336,9 @@ __global__ void __launch_bounds__(kThreads, 1)
                         const uint64_t bh = smem_desc(st + 2 * kTileBytes + off),
                                        bl = smem_desc(st + 3 * kTileBytes + off);
                         // small terms first; the block's first product overwrites the buffer
-                        mma_tf32(d, al, bh, ks > 0 ? 1u : 0u);
-                        mma_tf32(d, ah, bl, 1u);
-                        mma_tf32(d, ah, bh, 1u);
+                        mma_tf32(d, al, bh, idesc, ks > 0 ? 1u : 0u);
+                        mma_tf32(d, ah, bl, idesc, 1u);
+                        mma_tf32(d, ah, bh, idesc, 1u);
                     }
                     mma_commit(saddr(&bars->empty[s]));  // the stage is free once these MMAs are done
                     mma_commit(saddr(&bars->accf[b]));   // the accumulator is ready
@@ -366,6 +373,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if constexpr (kLdCols == 64) {
 #pragma unroll
                     for (int c = 0; c < kBN / 64; c++) {
+                        if (c * 64 >= ts.n_valid) break;
                         uint32_t r0[32], r1[32];
                         tmem_ld32_nowait(tb + (uint32_t)(c * 64), r0);
                         tmem_ld32_nowait(tb + (uint32_t)(c * 64 + 32), r1);
@@ -379,6 +387,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 } else {
 #pragma unroll
                     for (int c = 0; c < kBN / 32; c++) {
+                        if (c * 32 >= ts.n_valid) break;
                         uint32_t r[32];
                         tmem_ld32(tb + (uint32_t)(c * 32), r);
 #pragma unroll
@@ -456,14 +465,9 @@ int sm_count() {
     return n > 0 ? n : 1;
 }
 
-// opt-in to the pipeline's dynamic shared memory, once per kernel instance
+// opt-in to the pipeline's dynamic shared memory, for the current device
 template <class Job> cudaError_t smem_attr() {
-    static std::once_flag once;
-    static cudaError_t e = cudaSuccess;
-    std::call_once(once, [] {
-        e = cudaFuncSetAttribute(umma_3xtf32_kernel<Job>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    });
-    return e;
+    return cudaFuncSetAttribute(umma_3xtf32_kernel<Job>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
 }
 
 }  // namespace
