@@ -345,19 +345,27 @@ __global__ void __launch_bounds__(kThreads<Job>, 1)
         const uint32_t tb = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0;
         unsigned a = 0;  // accumulations drained so far
         int buf = 0;
-        for (int t = blockIdx.x; t < job.ntiles && ok; t += gridDim.x) {
+        // scales of this thread's row and of column c0 + lane of a tile, read a tile ahead (read at
+        // the tile's start they took 3000 clocks, two dependent L2 latencies and a third for gathered
+        // columns; read per column inside the drain, its length again)
+        double sa = 0.0, sb = 0.0;
+        static_assert(kDrainCols == 32, "a lane per column");
+        auto read_scales = [&](int t) {
+            if (t >= job.ntiles) return;
             const auto ts = job.tile(t);
-            const bool mine = row < ts.m_valid;
-            const double sa = mine ? job.alpha * A.scale[ts.a_blk * kBM + row] : 0.0;
-            // the columns' scales into shared memory while the MMAs run (read per column inside the
-            // drain they cost it its length again: L2 latency, twice for gathered columns); the
-            // four warps of these columns write the same values, and none is two tiles ahead
-            static_assert(kDrainCols == 32, "a lane per column");
+            sa = row < ts.m_valid ? job.alpha * A.scale[ts.a_blk * kBM + row] : 0.0;
+            sb = c0 + lane < ts.n_valid ? job.scale(B.scale, ts, c0 + lane) : 0.0;
+        };
+        read_scales(blockIdx.x);
+        for (int t = blockIdx.x; t < job.ntiles && ok; t += gridDim.x) {
+            const int nkb = job.tile(t).nkb;
+            const double sr = sa;
+            // the four warps of these columns write the same values, and none is two tiles ahead
             double *sn = bars->col_scale[buf][c0 / kDrainCols];
             buf ^= 1;
-            sn[lane] = c0 + lane < ts.n_valid ? job.scale(B.scale, ts, c0 + lane) : 0.0;
+            sn[lane] = sb;
             __syncwarp();
-            for (int k0 = 0; k0 < ts.nkb && ok; k0 += kI8MaxSegment) {
+            for (int k0 = 0; k0 < nkb && ok; k0 += kI8MaxSegment) {
                 const bool add = job.add || k0 > 0;
                 // groups 0-3: hi = sum_g acc_g 256^(3 - g)
                 if (!__all_sync(0xffffffffu, mbar_wait(saddr(&bars->accf), a & 1u))) {
@@ -383,14 +391,14 @@ __global__ void __launch_bounds__(kThreads<Job>, 1)
                 __syncwarp();
                 if (lane == 0) mbar_arrive(saddr(&bars->acce));
                 a++;
+                if (k0 + kI8MaxSegment >= nkb) read_scales(t + gridDim.x);
                 // groups 4-7: lo = sum_g acc_g 256^(7 - g); value = hi 2^32 + lo
                 if (!__all_sync(0xffffffffu, mbar_wait(saddr(&bars->accf), a & 1u))) {
                     ok = false;
                     break;
                 }
                 tc_fence_after();
-                double *pc = job.first(ts, c0) + row;
-                const long long step = job.step(ts);
+                // first all values, so that the next tile's MMAs run while these are scaled and stored
 #pragma unroll
                 for (int c = 0; c < kDrainCols; c += 4) {
                     int g4[4], g5[4], g6[4], g7[4];
@@ -403,20 +411,28 @@ __global__ void __launch_bounds__(kThreads<Job>, 1)
                     for (int j = 0; j < 4; j++) {
                         const long long lo = (long long)g4[j] * (1 << 24) + (long long)g5[j] * (1 << 16) +
                                              (long long)g6[j] * (1 << 8) + (long long)g7[j];
-                        const int n = c0 + c + j;
-                        if (mine && n < ts.n_valid) {
-                            const double v = fma((double)hi[c + j], 4294967296.0, (double)lo);
-                            double *p = job.at(pc, ts, n);
-                            const double r = v * sn[c + j] * sa;
-                            *p = add ? *p + r : r;
-                        }
-                        pc += step;
+                        hi[c + j] = __double_as_longlong(fma((double)hi[c + j], 4294967296.0, (double)lo));
                     }
                 }
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(saddr(&bars->acce));
                 a++;
+                asm volatile("" ::: "memory");  // the tile is read again: kept, it would spill
+                const auto ts = job.tile(t);
+                double *pc = job.first(ts, c0) + row;
+                const long long step = job.step(ts);
+#pragma unroll
+                for (int c = 0; c < kDrainCols; c++) {
+                    // four columns at a time: pointers and scales of all 32 at once would spill
+                    if (c % 4 == 0) asm volatile("" : "+l"(pc)::"memory");
+                    if (row < ts.m_valid && c0 + c < ts.n_valid) {
+                        double *p = job.at(pc, ts, c0 + c);
+                        const double v = __longlong_as_double(hi[c]) * sn[c] * sr;
+                        *p = add ? *p + v : v;
+                    }
+                    pc += step;
+                }
             }
         }
         if (!ok && lane == 0) atomicExch(err, 13);
