@@ -3,17 +3,22 @@
 // Pipeline of one CTA (persistent: 128 x 128 output tiles in turn):
 //   warp 0  producer: per K block (32 values) one bulk copy of the A block's digit planes
 //           and one of the B block's into a 4-stage shared-memory ring;
-//   warp 1  TMEM owner and MMA issuer: tcgen05.mma kind::i8, M = 128, N = 128, K = 32;
+//   warp 1  TMEM owner and MMA issuer: tcgen05.mma kind::i8, M = 128, K = 32, N the tile's
+//           columns rounded up to 16 (partly filled M2L chunks hold 82 on average);
 //   warps 2-17 drain: tcgen05.ld, the digit groups put together in int64, then FP64;
-//   warps 18, 19 (gathered columns only) fetch B's rows in 16-byte asynchronous copies, eight
-//           lanes per row, two stages in flight before a stage is handed on.
+//   warps 18, 19 (gathered columns only) fetch B's rows in 16-byte asynchronous copies, two
+//           stages in flight before a stage is handed on.
 // The eight digit groups i + j = 0 .. 7 need 8 x 128 TMEM columns and there are 512, so a
 // tile takes two passes over K: groups 0-3 (planes 0-3 of both operands, 10 products per K
 // block) drained into an int64 per output, then groups 4-7 (all planes, 24 products).
-// What bounds it: shared memory.  Per K block the 34 MMAs read 8 KB each and the copies
-// write 88 KB, 360 KB against ~128 bytes per clock, 2800 clocks for 34 x 64 clocks of MMA
-// at the nominal rate.  128 x 64 tiles (all groups resident, one pass) would read 6 KB per
-// MMA of half the work.
+// What bounds it (M = 636, N = 32768, K = 3584, B200): 1.55 ms, 97 TFLOP/s of FP64 work (cuBLAS:
+// 29.9); tensor pipe active 71% at 1.64 GHz (power), L2 7.1 TB/s.  By shared memory alone, the
+// 34 MMAs of a K block read 8 KB each and the copies write 88 KB: 2800 clocks for 34 x 64 of MMA.
+// 128 x 64 tiles (all groups resident, one pass) would read 6 KB per MMA of half the work; CTA
+// pairs (256 x 128 tiles, 2110 clocks by the same count) measured 1.71 ms.
+// Short K (M2L's P_d, 4 K blocks): the chain of the two passes, 18000 clocks a tile, 5900 of
+// them MMA: the second pass's MMAs 6200, the drains 1800 and 6000, the wait for the first 2000;
+// a third of the L2 traffic less (blocks kept for the second pass, used rows only) changed nothing.
 // Every mbarrier wait has an iteration limit: on expiry the kernel records an error code,
 // stops issuing work, waits (bounded) for what it issued, frees its TMEM and returns.
 #include <algorithm>
