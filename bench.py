@@ -815,6 +815,8 @@ def cpu_baseline(ul, pts, q, d, pairs, target_seconds=15.0):
     bounded sample."""
     from oracle import oracle as O
     O.build()
+    if not O.ref_simd_available():
+        return {"unavailable": "oracle/_ref was not built (reference tree absent where the library was built)"}
     cores = os.cpu_count() or 1
     w = cpu_full_prepare(ul, pts, q, d)
     cpu_full_step(w)  # thread pool and pages warm
