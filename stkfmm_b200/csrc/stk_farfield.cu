@@ -1000,11 +1000,11 @@ bool i8_wins(int M, int N, int K) {
 // C[:, col(j)] (add = 0: =, 1: +=) mul(j) A X[:, idx(j)] for j < m: A column-major M x K
 // (and as digits), X columns of K values, idx / cols null for the identity, mul powers of two
 // (null: 1, given with cols only).  Y, Xg: scratch of the cuBLAS path (M x m, K x m).
-int far_product(FarField &F, const DevBuf &A, const I8Buf &A8, int M, int K, const double *X, const int *idx, int m,
+int far_product(FarField &F, bool i8, const DevBuf &A, const I8Buf &A8, int M, int K, const double *X, const int *idx, int m,
                 const double *mul, int add, double *C, const int *cols, double *Xg, double *Y, cudaStream_t s) {
     if (m <= 0) return STK_OK;
     const int np = i8_gemm_parts(M, m, i8_kblocks(K));
-    if (F.i8 && i8_wins(M, m, K) && !F.i8_b.reserve(m, K) &&
+    if (i8 && i8_wins(M, m, K) && !F.i8_b.reserve(m, K) &&
         !(np > 1 && F.i8_parts.reserve(sizeof(double) * (size_t)np * M * m))) {
         t_launches += np > 1 ? 3 : 2;
         FCUDA(i8_digits(X, K, idx, m, K, F.i8_b.nkb, A8.up(), mul, F.i8_b.digits(), F.i8_b.scales(), s));
@@ -1947,6 +1947,10 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
     F.s2m_nodes.clear();
     for (int b : T.leaves)
         if (T.src_count(b) > 0) F.s2m_nodes.push_back(b);
+    auto by_level = [&](std::vector<int> &v) {
+        std::stable_sort(v.begin(), v.end(), [&](int a, int b) { return T.level[a] < T.level[b]; });
+    };
+    by_level(F.s2m_nodes);
     const int ms = (int)F.s2m_nodes.size();
     rc = F.d_s2m_nodes.upload(F.s2m_nodes.data(), sizeof(int) * ms, s);
     if (!rc) rc = levels_of(F.s2m_nodes, F.s2m_lev, F.s2m_mul);
@@ -2019,6 +2023,7 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
     F.s2l_nodes.clear();
     for (int b = 0; b < nn; b++)
         if (T.X.off[b + 1] > T.X.off[b] && !x_direct(b)) F.s2l_nodes.push_back(b);
+    by_level(F.s2l_nodes);
     const int mx = (int)F.s2l_nodes.size();
     rc = F.d_s2l_nodes.upload(F.s2l_nodes.data(), sizeof(int) * mx, s);
     if (!rc) rc = levels_of(F.s2l_nodes, F.s2l_lev, F.s2l_mul);
@@ -2483,6 +2488,12 @@ int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const dou
     double *phi = (double *)F.phi.ptr, *psi = (double *)F.psi.ptr;
     double *X = (double *)F.tmp0.ptr, *Y = (double *)F.tmp1.ptr;
     t_launches = 0;
+    // The mixed path rounds the densities to FP32 after the FP64 products.  Those of the Stokes
+    // translations are larger than the fields they stand for by orders of magnitude, and
+    // products that round differently, however well, move the mixed result by up to 3.5e-8 (Stokes
+    // wall, 100k points; within its 3e-7 error, but no longer the same numbers); laplace_p's
+    // by 6e-13.  So the mixed path takes the int8 products for laplace_p alone.
+    const bool i8 = F.i8 && (prec == PREC_FP64 || F.ke == 1);
     FCUDA(cudaMemsetAsync(phi, 0, sizeof(double) * (size_t)nn * N, s));
     FCUDA(cudaMemsetAsync(psi, 0, sizeof(double) * (size_t)nn * N, s));
 
@@ -2505,8 +2516,9 @@ int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const dou
     // check potentials -> equivalent densities of m nodes of any level: the level's factor
     // 2^-l (1 + pot_exp) goes into the products' columns (one factor) or, per component, into
     // the check potentials
-    auto solve = [&](double *check, int m, const DevBuf &A, const I8Buf &A8, const DevBuf &lev, const DevBuf &mul,
+    auto solve = [&](double *check, const std::vector<int> &host_nodes, const DevBuf &A, const I8Buf &A8, const DevBuf &lev, const DevBuf &mul,
                      const DevBuf &nodes, int add, double *dst) -> int {
+        const int m = (int)host_nodes.size();
         if (F.scaled) {
             CompF e;
             for (int c = 0; c < 4; c++) e.v[c] = 1.0 + F.pot_exp[c];
@@ -2515,8 +2527,15 @@ int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const dou
             FCUDA(cudaGetLastError());
             t_launches++;
         }
-        return far_product(F, A, A8, N, n * kc, check, nullptr, m, F.scaled ? nullptr : (const double *)mul.ptr, add, dst,
-                           (const int *)nodes.ptr, X, Y, s);
+        // one product over the levels, or (the mixed path's rounding, see i8) one per level
+        for (int a = 0, b; a < m; a = b) {
+            for (b = i8 ? m : a + 1; b < m && T.level[host_nodes[b]] == T.level[host_nodes[a]]; b++) {}
+            const int rc = far_product(F, i8, A, A8, N, n * kc, check + (size_t)a * n * kc, nullptr, b - a,
+                                       F.scaled ? nullptr : (const double *)mul.ptr + a, add, dst,
+                                       (const int *)nodes.ptr + a, X, Y, s);
+            if (rc) return rc;
+        }
+        return STK_OK;
     };
 
     // ---- upward pass: S2M, then check -> equivalent ----
@@ -2532,7 +2551,7 @@ int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const dou
                               counter, kd->d_parts, sms, s);
             if (rc) return rc;
         }
-        const int rc = solve((double *)F.check.ptr, ms, F.uc2ue, F.i8_uc2ue, F.s2m_lev, F.s2m_mul, F.d_s2m_nodes, 0, phi);
+        const int rc = solve((double *)F.check.ptr, F.s2m_nodes, F.uc2ue, F.i8_uc2ue, F.s2m_lev, F.s2m_mul, F.d_s2m_nodes, 0, phi);
         if (rc) return rc;
     }
     FCUDA(cudaEventRecord(kd->ph[1], s));
@@ -2542,7 +2561,7 @@ int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const dou
         const int a = F.parent_off[l], m = F.parent_off[l + 1] - a;
         if (m == 0) continue;
         const double *Xc = phi + (size_t)T.level_begin[l + 1] * N;
-        int rc = far_product(F, F.m2m, F.i8_m2m, N, 8 * N, Xc, nullptr, m, nullptr, 0, phi, d_parents + a, nullptr, Y, s);
+        int rc = far_product(F, i8, F.m2m, F.i8_m2m, N, 8 * N, Xc, nullptr, m, nullptr, 0, phi, d_parents + a, nullptr, Y, s);
         if (rc) return rc;
     }
 
@@ -2556,7 +2575,7 @@ int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const dou
     // (3xTF32 on the tensor cores) raised the mixed Stokes FMM's error from 2.8e-7 to
     // 5.2e-7 (V^T phi alone) and 7.3e-7 (both); p = 8, 12000 clustered points.
     {
-        const int rc = far_product(F, F.m2l_vt, F.i8_vt, k, N, phi, nullptr, nn, nullptr, 0, phi_hat, nullptr, nullptr,
+        const int rc = far_product(F, i8, F.m2l_vt, F.i8_vt, k, N, phi, nullptr, nn, nullptr, 0, phi_hat, nullptr, nullptr,
                                    nullptr, s);
         if (rc) return rc;
     }
@@ -2671,7 +2690,7 @@ int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const dou
         if (rcd) return rcd;
     }
     {
-        const int rc = far_product(F, F.m2l_e, F.i8_e, N, k, psi_hat, nullptr, nn, nullptr, 1, psi, nullptr, nullptr,
+        const int rc = far_product(F, i8, F.m2l_e, F.i8_e, N, k, psi_hat, nullptr, nn, nullptr, 1, psi, nullptr, nullptr,
                                    nullptr, s);
         if (rc) return rc;
     }
@@ -2695,7 +2714,7 @@ int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const dou
             any = true;
         }
         if (any) {
-            const int rc = solve((double *)F.dcheck.ptr, mx, F.dc2de, F.i8_dc2de, F.s2l_lev, F.s2l_mul, F.d_s2l_nodes, 1, psi);
+            const int rc = solve((double *)F.dcheck.ptr, F.s2l_nodes, F.dc2de, F.i8_dc2de, F.s2l_lev, F.s2l_mul, F.d_s2l_nodes, 1, psi);
             if (rc) return rc;
         }
     }
@@ -2707,7 +2726,7 @@ int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const dou
     for (int l = F.down_top + 1; l <= T.depth(); l++) {
         const int a = F.parent_off[l - 1], m = F.parent_off[l] - a;
         if (m == 0) continue;
-        int rc = far_product(F, F.l2l, F.i8_l2l, 8 * N, N, psi, d_parents + a, m, nullptr, 1,
+        int rc = far_product(F, i8, F.l2l, F.i8_l2l, 8 * N, N, psi, d_parents + a, m, nullptr, 1,
                              psi + (size_t)T.level_begin[l] * N, nullptr, X, nullptr, s);
         if (rc) return rc;
     }

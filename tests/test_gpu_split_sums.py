@@ -127,3 +127,16 @@ def test_fp64_fmm_int8_products(torch_cuda, monkeypatch, kernel, p, max_pts):
         noise[mode] = rel_l2(r3 / 3.0, res[mode])
     assert noise["1"] < 2.0 * noise["0"] + 1e-14, noise
     assert rel_l2(res["1"], res["0"]) < 4.0 * noise["0"] + 1e-14, (rel_l2(res["1"], res["0"]), noise)
+
+
+@pytest.mark.parametrize("kernel,max_pts", [(2, 40), (16, 60), (128, 60)])
+def test_mixed_fmm_keeps_its_fp64_products(torch_cuda, monkeypatch, kernel, max_pts):
+    """The mixed path of the Stokes translations rounds to FP32 after its FP64 products and stays with
+    cuBLAS for them: the same numbers with the int8 products on and off (a rebuilt operator set, 1e-13
+    as for any two handles that built their own)."""
+    pts, slv, dlv, td = fmm_case(kernel, 9000, seed=80 + kernel)
+    res = {}
+    for mode in ("0", "1"):
+        monkeypatch.setenv("STKFMM_F64_I8", mode)
+        _, res[mode] = run_fmm(kernel, 8, max_pts, pts, slv, dlv, td, prec=1)
+    assert rel_l2(res["1"], res["0"]) < 1e-13
