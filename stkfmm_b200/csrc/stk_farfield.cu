@@ -2516,8 +2516,8 @@ int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const dou
     // check potentials -> equivalent densities of m nodes of any level: the level's factor
     // 2^-l (1 + pot_exp) goes into the products' columns (one factor) or, per component, into
     // the check potentials
-    auto solve = [&](double *check, const std::vector<int> &host_nodes, const DevBuf &A, const I8Buf &A8, const DevBuf &lev, const DevBuf &mul,
-                     const DevBuf &nodes, int add, double *dst) -> int {
+    auto solve = [&](double *check, const std::vector<int> &host_nodes, const DevBuf &A, const I8Buf &A8,
+                     const DevBuf &lev, const DevBuf &mul, const DevBuf &nodes, int add, double *dst) -> int {
         const int m = (int)host_nodes.size();
         if (F.scaled) {
             CompF e;
