@@ -411,7 +411,7 @@ extern "C" int stk_gemm_f64_i8(int M, int N, int K, const double *d_A, int lda, 
     cudaStream_t s = (cudaStream_t)stream;
     const int nkb = i8_kblocks(K);
     const size_t ba = i8_bytes(M, nkb), bb = i8_bytes(N, nkb);
-    const size_t sa = sizeof(double) * i8_pad_rows(M), sb = sizeof(double) * i8_pad_rows(N);
+    const size_t sa = sizeof(int) * i8_pad_rows(M), sb = sizeof(int) * i8_pad_rows(N);  // multiples of 512 bytes
     uint8_t *buf = nullptr;
     const size_t np = (size_t)i8_gemm_parts(M, N, nkb), pb = np > 1 ? sizeof(double) * np * M * N : 0;
     if (cudaMalloc(&buf, ba + bb + sa + sb + pb + 64) != cudaSuccess) {
@@ -419,14 +419,14 @@ extern "C" int stk_gemm_f64_i8(int M, int N, int K, const double *d_A, int lda, 
         return STK_ERR_CUDA;
     }
     uint8_t *da = buf, *db = da + ba;
-    double *fa = reinterpret_cast<double *>(db + bb), *fb = fa + sa / sizeof(double);
-    double *parts = pb ? fb + sb / sizeof(double) : nullptr;
+    int *fa = reinterpret_cast<int *>(db + bb), *fb = fa + sa / sizeof(int);
+    double *parts = pb ? reinterpret_cast<double *>(reinterpret_cast<uint8_t *>(fb) + sb) : nullptr;
     int *err = reinterpret_cast<int *>(reinterpret_cast<uint8_t *>(fb) + sb + pb);
     int rc = STK_OK, e = 0;
     if (cudaMemsetAsync(err, 0, sizeof(int), s) != cudaSuccess ||
         i8_digits(d_A, lda, nullptr, M, K, nkb, nullptr, nullptr, da, fa, s) != cudaSuccess ||
         i8_digits(d_B, ldb, nullptr, N, K, nkb, nullptr, nullptr, db, fb, s) != cudaSuccess ||
-        i8_gemm(M, N, I8Operand{da, fa, nkb}, I8Operand{db, fb, nkb}, 1.0, beta, d_C, ldc, nullptr, parts, err,
+        i8_gemm(M, N, I8Operand{da, fa, nkb}, I8Operand{db, fb, nkb}, beta, d_C, ldc, nullptr, parts, err,
                 s) != cudaSuccess ||
         cudaMemcpyAsync(&e, err, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess)
         rc = STK_ERR_CUDA;

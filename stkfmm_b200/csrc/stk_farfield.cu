@@ -460,8 +460,8 @@ constexpr int kM2LChunk = 128;
 static_assert(kM2LChunk == kI8Rows, "a chunk is one row block of the int8 path");
 
 // out[i] = up[idx[i]], out[n + i] = down[idx[i]]
-__global__ void gather_scales_kernel(const double *__restrict__ up, const double *__restrict__ down,
-                                     const int *__restrict__ idx, long long n, double *__restrict__ out) {
+__global__ void gather_scales_kernel(const int *__restrict__ up, const int *__restrict__ down,
+                                     const int *__restrict__ idx, long long n, int *__restrict__ out) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         out[i] = up[idx[i]];
         out[n + i] = down[idx[i]];
@@ -961,7 +961,7 @@ int build_i8_operators(FarField &F, cudaStream_t s) {
     if (!rc) rc = F.i8_q.reserve_kscale(k);
     if (!rc) rc = F.i8_p.reserve_kscale(nslot * rmax);
     DevBuf mag;
-    if (!rc) rc = mag.reserve(sizeof(unsigned long long) * k);
+    if (!rc) rc = mag.reserve(sizeof(unsigned) * k);
     if (rc) {
         F.i8_q.release();
         F.i8_p.release();
@@ -969,7 +969,7 @@ int build_i8_operators(FarField &F, cudaStream_t s) {
     }
     long long qcols = 0;
     for (int sl = 0; sl < nslot; sl++) qcols += F.m2l_r[sl];
-    FCUDA(i8_row_scales((const double *)F.m2l_q.ptr, k, qcols, k, (unsigned long long *)mag.ptr, F.i8_q.up(),
+    FCUDA(i8_row_scales((const double *)F.m2l_q.ptr, k, qcols, k, (unsigned *)mag.ptr, F.i8_q.up(),
                         F.i8_q.down(), s));
     for (int sl = 0; sl < nslot; sl++) {
         const double *Q = (const double *)F.m2l_q.ptr + F.m2l_pq_off[sl], *P = (const double *)F.m2l_p.ptr + F.m2l_pq_off[sl];
@@ -1008,7 +1008,7 @@ int far_product(FarField &F, bool i8, const DevBuf &A, const I8Buf &A8, int M, i
         !(np > 1 && F.i8_parts.reserve(sizeof(double) * (size_t)np * M * m))) {
         t_launches += np > 1 ? 3 : 2;
         FCUDA(i8_digits(X, K, idx, m, K, F.i8_b.nkb, A8.up(), mul, F.i8_b.digits(), F.i8_b.scales(), s));
-        FCUDA(i8_gemm(M, m, A8.op(), F.i8_b.op(), 1.0, add, C, M, cols, np > 1 ? (double *)F.i8_parts.ptr : nullptr,
+        FCUDA(i8_gemm(M, m, A8.op(), F.i8_b.op(), add, C, M, cols, np > 1 ? (double *)F.i8_parts.ptr : nullptr,
                       (int *)F.tc_err.ptr, s));
         return STK_OK;
     }
@@ -1479,7 +1479,7 @@ static int setup_m2l_chunks_i8(FarField &F, const std::vector<int> &chunk_slot, 
     // digits of phi_hat, one row per node; without memory for the digits the chunks stay with cuBLAS
     F.i8_x.nkb = i8_kblocks(k);
     F.i8_chunks = !(F.i8_z.reserve(gcols, rmax) || F.i8_x.dig.reserve(i8_row_bytes(nn, F.i8_x.nkb)) ||
-                    F.i8_x.scale.reserve(sizeof(double) * (size_t)nn));
+                    F.i8_x.scale.reserve(sizeof(int) * (size_t)nn));
     if (!F.i8_chunks) return STK_OK;
     int rc = F.i8_valid.upload(valid.data(), sizeof(int) * nc, s);
     if (!rc) rc = F.i8_rank.upload(rank.data(), sizeof(int) * nc, s);
@@ -1687,11 +1687,11 @@ static int setup_m2l_dense(FarField &F, const Octree &T, int nslot, cudaStream_t
     if (F.dn_i8) {
         // the scales along K of every block row: those of its offset's P_d
         DevBuf ksrc;
-        rc = F.dn_ks.reserve(sizeof(double) * 2 * F.dn_rows);
+        rc = F.dn_ks.reserve(sizeof(int) * 2 * F.dn_rows);
         if (!rc) rc = ksrc.upload(pcol.data(), sizeof(int) * pcol.size(), s);
         if (rc) return rc;
         gather_scales_kernel<<<grid_for((long long)F.dn_rows), 256, 0, s>>>(
-            F.i8_p.up(), F.i8_p.down(), (const int *)ksrc.ptr, (long long)F.dn_rows, (double *)F.dn_ks.ptr);
+            F.i8_p.up(), F.i8_p.down(), (const int *)ksrc.ptr, (long long)F.dn_rows, (int *)F.dn_ks.ptr);
         FCUDA(cudaGetLastError());
         for (int cs = 0; cs < 8; cs++)
             FCUDA(i8_digits((const double *)F.dn_qs.ptr + F.dn_qs_off[cs], k, nullptr, F.dn_rs[cs], k, F.dn_q8.nkb,
@@ -1699,7 +1699,7 @@ static int setup_m2l_dense(FarField &F, const Octree &T, int nslot, cudaStream_t
         for (int b = 0; b < 64; b++)
             FCUDA(i8_digits_trans((const double *)F.dn_pv.ptr + F.dn_pv_off[b / 8] + (size_t)k * F.dn_pstart[b], k,
                                   F.dn_rcc[b] ? k : 0, F.dn_rcc[b], F.dn_p8.nkb,
-                                  (const double *)F.dn_ks.ptr + F.dn_rows + F.dn_row_off[b],
+                                  (const int *)F.dn_ks.ptr + F.dn_rows + F.dn_row_off[b],
                                   F.dn_p8.digits((long long)b * kb), F.dn_p8.scales((long long)b * kb), s));
     }
     // per level: nodes in type order and the (c, c') source tables
@@ -2404,7 +2404,7 @@ static int m2l_dense_level_i8(FarField &F, const M2LDenseLevel &D, const double 
         const int rs = F.dn_rs[cs], nt = D.tiles8_off[cs + 1] - D.tiles8_off[cs];
         if (!rs || !nt) continue;
         t_launches += 3;
-        FCUDA(i8_gemm(rs, n8, F.dn_q8.op(F.dn_q8_blk[cs]), F.dn_phi8.op((long long)cs * n8 / kI8Rows), 1.0, 0, Z, rs,
+        FCUDA(i8_gemm(rs, n8, F.dn_q8.op(F.dn_q8_blk[cs]), F.dn_phi8.op((long long)cs * n8 / kI8Rows), 0, Z, rs,
                       nullptr, nullptr, err, s));
         I8Gather g{};
         g.z = Z;
@@ -2412,7 +2412,7 @@ static int m2l_dense_level_i8(FarField &F, const M2LDenseLevel &D, const double 
         g.tab = (const int *)D.d_tab.ptr;
         g.rowq = (const int *)F.dn_rowq.ptr;
         g.srow = (const int *)F.dn_srow.ptr;
-        g.kscale = (const double *)F.dn_ks.ptr;
+        g.kexp = (const int *)F.dn_ks.ptr;
         while ((1 << g.lg) < n8) g.lg++;
         for (int c = 0; c < 8; c++) {
             const int b = 8 * c + cs;
@@ -2640,10 +2640,10 @@ int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const dou
             t_launches += 2;
             if (c0 == 0) {
                 FCUDA(i8_digits_rows(phi_hat, k, nn, k, F.i8_x.nkb, F.i8_q.up(), (uint8_t *)F.i8_x.dig.ptr,
-                                     (double *)F.i8_x.scale.ptr, s));
+                                     (int *)F.i8_x.scale.ptr, s));
                 t_launches++;
             }
-            FCUDA(i8_grouped_gather(F.i8_q.op(), I8Rows{(const uint8_t *)F.i8_x.dig.ptr, (const double *)F.i8_x.scale.ptr, F.i8_x.nkb},
+            FCUDA(i8_grouped_gather(F.i8_q.op(), I8Rows{(const uint8_t *)F.i8_x.dig.ptr, (const int *)F.i8_x.scale.ptr, F.i8_x.nkb},
                                     gsrc, (const I8Tile *)F.i8_tiles1.ptr + F.i8_t1_off[g],
                                     F.i8_t1_off[g + 1] - F.i8_t1_off[g], 0, (double *)F.m2l_z.ptr, err, s));
             FCUDA(i8_digits_blocks((const double *)F.m2l_z.ptr, rmax, ncol, (const int *)F.i8_rank.ptr + c0,

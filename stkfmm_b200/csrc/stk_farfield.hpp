@@ -64,26 +64,26 @@ struct M2LDenseLevel {
 // Digits of an FP64 operand for the int8 tensor cores (stk_i8gemm.cuh).
 struct I8Buf {
     DevBuf dig, scale;
-    DevBuf kscale;  // operators: up[0 .. kn), down[0 .. kn) (i8_column_scales)
+    DevBuf kscale;  // operators: exponents up[0 .. kn), down[0 .. kn) (i8_column_scales)
     int nkb = 0, kn = 0;
     int reserve_kscale(int K) {
         kn = K;
-        return kscale.reserve(sizeof(double) * 2 * (size_t)K);
+        return kscale.reserve(sizeof(int) * 2 * (size_t)K);
     }
     void release() {
         dig.release();
         scale.release();
         kscale.release();
     }
-    double *up() const { return (double *)kscale.ptr; }
-    double *down() const { return (double *)kscale.ptr + kn; }
+    int *up() const { return (int *)kscale.ptr; }
+    int *down() const { return (int *)kscale.ptr + kn; }
     int reserve(long long rows, int K) {
         nkb = i8_kblocks(K);
         const int rc = dig.reserve(i8_bytes(rows, nkb));
-        return rc ? rc : scale.reserve(sizeof(double) * (size_t)i8_pad_rows(rows));
+        return rc ? rc : scale.reserve(sizeof(int) * (size_t)i8_pad_rows(rows));
     }
     uint8_t *digits(long long blk = 0) const { return (uint8_t *)dig.ptr + (size_t)blk * nkb * kI8BlockBytes; }
-    double *scales(long long blk = 0) const { return (double *)scale.ptr + (size_t)blk * kI8Rows; }
+    int *scales(long long blk = 0) const { return (int *)scale.ptr + (size_t)blk * kI8Rows; }
     // from row block blk on
     I8Operand op(long long blk = 0) const { return {digits(blk), scales(blk), nkb}; }
     void share(const I8Buf &o) {
@@ -206,7 +206,7 @@ struct FarField {
     // of the gathered Z of one source type, and per source type the output tiles of all targets
     bool dn_i8 = false;
     I8Buf dn_q8, dn_p8, dn_phi8, dn_zc8;
-    DevBuf dn_ks;                           // scales along K per block row: up, then down
+    DevBuf dn_ks;                           // exponents along K per block row: up, then down
     size_t dn_rows = 0;                     // entries of dn_rowq / dn_srow
     int dn_q8_blk[8] = {};
     // mixed path on the tensor cores (stk_umma.cu): 3xTF32 hi / lo operands, K-major

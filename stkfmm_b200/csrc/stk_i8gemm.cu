@@ -45,14 +45,18 @@ constexpr int kDrainCols = kBN / (kDrainWarps / 4);
 constexpr int kGatherWarps = 2;
 template <class Job> constexpr int kThreads = 32 * (2 + kDrainWarps + (Job::kGather ? kGatherWarps : 0));
 constexpr uint32_t kTmemCols = 512;
-constexpr int kSmemBytes = kStages * kStageBytes + 2304 /* barriers, column scales */ + 128 /* alignment */;
+constexpr int kBarBytes = 2944;  // barriers, column scales
+constexpr int kSmemBytes = kStages * kStageBytes + kBarBytes + 128 /* alignment */;
 static_assert(kSmemBytes <= 232448, "shared memory of one CTA");
 
 struct Bars {
     unsigned long long full[kStages], empty[kStages], accf, acce;
     uint32_t tmem;
     double col_scale[2][kBN / kDrainCols][kDrainCols];
+    short col_rest[2][kBN / kDrainCols][kDrainCols];
+    double ones[kDrainCols];
 };
+static_assert(sizeof(Bars) <= kBarBytes, "Bars fit their place");
 
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
@@ -111,7 +115,6 @@ struct DenseJob {
     static constexpr bool kGather = false;
     int M, N, add, gm, gn, ntiles, seg_kb, nkb;  // K part p: blocks [p seg_kb, ...)
     bool m_fast;
-    double alpha;
     double *C;
     long long ldc, part_ld;  // elements between the parts' outputs
     const int *cols;
@@ -133,14 +136,13 @@ struct DenseJob {
         return cols ? p + (size_t)cols[t.b_blk * kBN + n] * ldc : p;
     }
     __device__ long long step(const Tile &) const { return cols ? 0 : ldc; }
-    __device__ double scale(const double *sb, const Tile &t, int n) const { return sb[t.b_blk * kBN + n]; }
+    __device__ int scale(const int *sb, const Tile &t, int n) const { return sb[t.b_blk * kBN + n]; }
 };
 
 template <bool GATHER> struct GroupJob {
     static constexpr bool kGather = GATHER;
     const I8Tile *tiles;
     int ntiles, add;
-    double alpha;
     double *C;
     const int *rows;  // gathered columns
     struct Tile {
@@ -154,11 +156,26 @@ template <bool GATHER> struct GroupJob {
     __device__ double *first(const Tile &t, int c0) const { return t.c + (size_t)c0 * t.ldc; }
     __device__ double *at(double *p, const Tile &, int) const { return p; }
     __device__ long long step(const Tile &t) const { return t.ldc; }
-    __device__ double scale(const double *sb, const Tile &t, int n) const {
+    __device__ int scale(const int *sb, const Tile &t, int n) const {
         const int c = t.b_blk * kBN + n;
         return sb[GATHER ? rows[c] : c];
     }
 };
+
+__device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }  // normal range only
+
+// A scale 2^e as a factor of up to 2^+-500, so that a sum of digit products (below 2^88) takes two
+// of them without leaving the range of a double, and the exponent that is left (rare)
+constexpr int kCoreExp = 500;
+__device__ __forceinline__ double core_scale(int e) {
+    return e == kI8NonFinite ? __longlong_as_double(0x7ff8000000000000ll) : pow2(min(max(e, -kCoreExp), kCoreExp));
+}
+__device__ __forceinline__ int rest_exp(int e) {
+    return e == kI8NonFinite ? 0 : e - min(max(e, -kCoreExp), kCoreExp);
+}
+// v 2^r; a rest has the sign of its factor's exponent, so that v, which has been multiplied by both
+// factors, is out of range only where v 2^r is
+__device__ __forceinline__ double scale_rest(double v, int r) { return v * pow2(r >> 1) * pow2(r - (r >> 1)); }
 
 template <class Job>
 __global__ void __launch_bounds__(kThreads<Job>, 1)
@@ -178,6 +195,7 @@ __global__ void __launch_bounds__(kThreads<Job>, 1)
         mbar_init(saddr(&bars->acce), kDrainWarps);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    if (threadIdx.x < kDrainCols) bars->ones[threadIdx.x] = 1.0;
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(&bars->tmem)),
                      "r"(kTmemCols)
@@ -353,22 +371,24 @@ __global__ void __launch_bounds__(kThreads<Job>, 1)
         // scales of this thread's row and of column c0 + lane of a tile, read a tile ahead (read at
         // the tile's start they took 3000 clocks, two dependent L2 latencies and a third for gathered
         // columns; read per column inside the drain, its length again)
-        double sa = 0.0, sb = 0.0;
+        int ea = 0, eb = 0;
         static_assert(kDrainCols == 32, "a lane per column");
         auto read_scales = [&](int t) {
             if (t >= job.ntiles) return;
             const auto ts = job.tile(t);
-            sa = row < ts.m_valid ? job.alpha * A.scale[ts.a_blk * kBM + row] : 0.0;
-            sb = c0 + lane < ts.n_valid ? job.scale(B.scale, ts, c0 + lane) : 0.0;
+            ea = row < ts.m_valid ? A.scale[ts.a_blk * kBM + row] : 0;
+            eb = c0 + lane < ts.n_valid ? job.scale(B.scale, ts, c0 + lane) : 0;
         };
         read_scales(blockIdx.x);
         for (int t = blockIdx.x; t < job.ntiles && ok; t += gridDim.x) {
             const int nkb = job.tile(t).nkb;
-            const double sr = sa;
+            const double sr = core_scale(ea);
             // the four warps of these columns write the same values, and none is two tiles ahead
             double *sn = bars->col_scale[buf][c0 / kDrainCols];
             buf ^= 1;
-            sn[lane] = sb;
+            sn[lane] = core_scale(eb);
+            bars->col_rest[buf ^ 1][c0 / kDrainCols][lane] = (short)rest_exp(eb);
+            const bool wide = __any_sync(0xffffffffu, rest_exp(ea) | rest_exp(eb));
             __syncwarp();
             for (int k0 = 0; k0 < nkb && ok; k0 += kI8MaxSegment) {
                 const bool add = job.add || k0 > 0;
@@ -427,13 +447,28 @@ __global__ void __launch_bounds__(kThreads<Job>, 1)
                 const auto ts = job.tile(t);
                 double *pc = job.first(ts, c0) + row;
                 const long long step = job.step(ts);
+                const double *fn = sn;
+                double fr = sr;
+                if (wide) {
+                    // scales at the ends of the range (rare): all of it here, so that the stores below
+                    // stay as they are (a predicate in them cost 4 to 12 % of a short product)
+                    const short *rn = bars->col_rest[buf ^ 1][c0 / kDrainCols];
+                    const int ra = row < ts.m_valid ? rest_exp(A.scale[ts.a_blk * kBM + row]) : 0;
+#pragma unroll
+                    for (int c = 0; c < kDrainCols; c++) {
+                        hi[c] = __double_as_longlong(scale_rest(__longlong_as_double(hi[c]) * sn[c] * sr, ra + rn[c]));
+                        asm volatile("" ::: "memory");
+                    }
+                    fn = bars->ones;
+                    fr = 1.0;
+                }
 #pragma unroll
                 for (int c = 0; c < kDrainCols; c++) {
                     // four columns at a time: pointers and scales of all 32 at once would spill
                     if (c % 4 == 0) asm volatile("" : "+l"(pc)::"memory");
                     if (row < ts.m_valid && c0 + c < ts.n_valid) {
                         double *p = job.at(pc, ts, c0 + c);
-                        const double v = __longlong_as_double(hi[c]) * sn[c] * sr;
+                        const double v = __longlong_as_double(hi[c]) * fn[c] * fr;
                         *p = add ? *p + v : v;
                     }
                     pc += step;
@@ -450,82 +485,88 @@ __global__ void __launch_bounds__(kThreads<Job>, 1)
 }
 
 // ---- FP64 rows -> digit blocks ---------------------------------------------------
-// Source of four consecutive K values of a row (values beyond K are zero).
+// Source of four consecutive K values of a row (values beyond K are zero) and their exponents.
 struct RowLoad {
     const double *src;
     long long ld;
     const int *idx;
     int K;
-    const double *ks;
+    const int *ks;
     const int *kof, *kset, *nof;  // per 128-row block, or null
     int kld;
     const double *rmul;
-    __device__ double mul(long long r) const { return rmul ? rmul[r] : 1.0; }
+    __device__ int mul(long long r) const { return rmul ? ((__double2hiint(rmul[r]) >> 20) & 0x7ff) - 1023 : 0; }
     __device__ int used_blocks(long long blk, int nkb) const { return kof ? (kof[blk] + kI8K - 1) / kI8K : nkb; }
     __device__ int len(long long r) const {
         return kof ? (r % kI8Rows < nof[r / kI8Rows] ? kof[r / kI8Rows] : 0) : K;
     }
-    __device__ void load4(long long r, int k, int n, double (&v)[4]) const {
+    __device__ void load4(long long r, int k, int n, double (&v)[4], int (&e)[4]) const {
         const long long i = idx ? idx[r] : r;
-        const double *f = ks && kset ? ks + (size_t)kset[r / kI8Rows] * kld : ks;
+        const int *f = ks && kset ? ks + (size_t)kset[r / kI8Rows] * kld : ks;
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             v[q] = i >= 0 && k + q < n ? src[i * ld + k + q] : 0.0;
-            if (f && k + q < n) v[q] *= f[k + q];
+            e[q] = f && k + q < n ? f[k + q] : 0;
         }
     }
 };
 struct GatherLoad {
     I8Gather g;
-    __device__ double mul(long long) const { return 1.0; }
+    __device__ int mul(long long) const { return 0; }
     __device__ int used_blocks(long long blk, int) const { return (g.K[(blk * kI8Rows) >> g.lg] + kI8K - 1) / kI8K; }
     __device__ int len(long long r) const { return g.K[r >> g.lg]; }
-    __device__ void load4(long long r, int k, int n, double (&v)[4]) const {
+    __device__ void load4(long long r, int k, int n, double (&v)[4], int (&e)[4]) const {
         const int c = (int)(r >> g.lg);
         const int *t = g.tab + g.tab_off[c] + (r & ((1ll << g.lg) - 1)) * g.nq[c];
         // the tables are padded to multiples of 4
         const int4 q4 = *reinterpret_cast<const int4 *>(g.rowq + g.row_off[c] + k);
         const int4 s4 = *reinterpret_cast<const int4 *>(g.srow + g.row_off[c] + k);
+        const int4 e4 = *reinterpret_cast<const int4 *>(g.kexp + g.row_off[c] + k);
         const int rq[4] = {q4.x, q4.y, q4.z, q4.w}, sr[4] = {s4.x, s4.y, s4.z, s4.w};
+        e[0] = e4.x, e[1] = e4.y, e[2] = e4.z, e[3] = e4.w;
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             v[q] = 0.0;
             if (k + q < n) {
                 const int pos = t[rq[q]];
-                if (pos >= 0) v[q] = g.z[(size_t)pos * g.ldz + sr[q]] * g.kscale[g.row_off[c] + k + q];
+                if (pos >= 0) v[q] = g.z[(size_t)pos * g.ldz + sr[q]];
             }
         }
     }
 };
 
-// magnitude bits of four values, NaN above infinity above every finite value
-__device__ __forceinline__ unsigned long long mag(double x) {
-    return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
+// Magnitude of x 2^ke (|ke| <= kI8KExp) in an order-preserving integer: exponent and six leading
+// fraction bits of x, the exponent shifted by ke and made positive; 0 for zero, kMagNonFinite
+// for an infinity or NaN.  (x 2^ke itself may leave the range of a double.)
+constexpr unsigned kMagNonFinite = 0x7fffffffu;
+constexpr int kMagBias = 2048;
+__device__ __forceinline__ unsigned mag(double x, int ke) {
+    const unsigned t = ((unsigned)__double2hiint(x) & 0x7fffffffu) >> 14;  // exponent, 6 bits
+    if (t >= 0x7ffu << 6) return kMagNonFinite;
+    return x == 0.0 ? 0u : max(t, 1u << 6) + ((unsigned)(ke + kMagBias) << 6);
 }
 
-// the multipliers that take values below 127/128 2^e to integers below 127 2^48, whose top
-// digit is at most 127 (two, so that no factor overflows for the smallest e), and the stored
-// scale 2^(e - 35)
+// the exponent that takes a row's values, below 127/128 2^e, to integers below 127 2^48, whose
+// top digit is at most 127, and the stored scale's exponent
 struct RowScale {
-    double f1, f2, s;
+    int up, s;
     bool finite;
 };
-__device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }  // normal range only
-__device__ __forceinline__ RowScale row_scale(unsigned long long m) {
-    const int E = (int)(m >> 52);
-    if (E == 0x7ff) return {0.0, 0.0, __longlong_as_double(0x7ff8000000000000ll), false};
-    if (m == 0) return {0.0, 0.0, 0.0, true};
-    const int top6 = (int)(m >> 46) & 0x3f;             // leading fraction bits: all ones from 127/128 2^e
-    const int e = (E ? E : 1) - 1022 + (top6 == 0x3f);  // |x| < 127/128 2^e
-    const int up = 55 - e;                              // up to 55 + 1021
-    const int u1 = min(up, 1000);
-    return {pow2(u1), pow2(up - u1), pow2(max(e - 35, -1022)), true};
+__device__ __forceinline__ RowScale row_scale(unsigned m) {
+    if (m == kMagNonFinite) return {0, kI8NonFinite, false};
+    if (m == 0) return {0, 0, true};
+    const int e = (int)(m >> 6) - kMagBias - 1022 + ((m & 0x3f) == 0x3f);  // |x| < 127/128 2^e
+    return {55 - e, e - 35, true};
 }
 
-// seven balanced base-256 digits of x, as the bytes of a' + 128 (256^7 - 1) / 255, each
-// with its top bit flipped (digit = byte - 128); byte 6 is the most significant
-__device__ __forceinline__ unsigned long long digits(double x, const RowScale &sc) {
-    const long long v = __double2ll_rn(x * sc.f1 * sc.f2);
+// seven balanced base-256 digits of x 2^t, |x 2^t| < 127 2^48, as the bytes of a' + 128 (256^7 - 1)
+// / 255, each with its top bit flipped (digit = byte - 128); byte 6 is the most significant.
+// t = f + ke + rest, f + ke within +-1000: the first factor takes x to where rest (zero but at the
+// ends of the range) can neither over- nor underflow what the digits hold.
+__device__ __forceinline__ unsigned long long digits(double x, int e, int rest) {
+    double y = x * pow2(e);
+    if (rest) y *= pow2(rest);
+    const long long v = __double2ll_rn(y);
     return (unsigned long long)(v + 0x0080808080808080ll) ^ 0x0080808080808080ull;
 }
 
@@ -538,11 +579,11 @@ __device__ __forceinline__ unsigned long long digits(double x, const RowScale &s
 template <class Load, bool ROWS>
 __global__ void __launch_bounds__(256) i8_digits_kernel(const __grid_constant__ Load ld, long long rows, long long groups,
                                                         int nkb, int slice, uint8_t *__restrict__ dig,
-                                                        double *__restrict__ scale) {
+                                                        int *__restrict__ scale) {
     // [plane][16-value core][row][16 bytes], cores padded by one row against bank conflicts
     constexpr int kCore = 9 * 16;
     __shared__ __align__(16) uint8_t tile[kI8Planes][8][kCore];
-    __shared__ unsigned long long part[8];  // this CTA's largest magnitudes
+    __shared__ unsigned part[8];  // this CTA's largest magnitudes
     cg::cluster_group cluster = cg::this_cluster();
     const int nsl = (int)cluster.num_blocks(), sl = (int)cluster.block_rank();
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -552,15 +593,15 @@ __global__ void __launch_bounds__(256) i8_digits_kernel(const __grid_constant__ 
         const int n = r < rows ? min(ld.len(r), nkb * kI8K) : 0;
         // the row block's K blocks in use (the whole pitch, or fewer where K goes by blocks)
         const int kz = min(min(nkb, ld.used_blocks(grp / 16, nkb)) * kI8K, ka + slice);
-        unsigned long long m = 0;
+        unsigned m = 0;
         double v[4] = {0.0, 0.0, 0.0, 0.0};
+        int e[4] = {0, 0, 0, 0};
         for (int k = ka + 4 * lane; k < min(n, kz); k += 128) {
-            ld.load4(r, k, n, v);
+            ld.load4(r, k, n, v, e);
 #pragma unroll
-            for (int q = 0; q < 4; q++) m = max(m, mag(v[q]));
+            for (int q = 0; q < 4; q++) m = max(m, mag(v[q], e[q]));
         }
-#pragma unroll
-        for (int o = 16; o; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+        m = __reduce_max_sync(0xffffffffu, m);
         if (nsl > 1) {
             if (lane == 0) part[w] = m;
             cluster.sync();
@@ -568,18 +609,19 @@ __global__ void __launch_bounds__(256) i8_digits_kernel(const __grid_constant__ 
             cluster.sync();  // everyone has read part before the next group writes it
         }
         const RowScale sc = row_scale(m);
-        if (lane == 0 && sl == 0 && (!ROWS || r < rows)) scale[r] = r < rows ? sc.s * ld.mul(r) : 0.0;
+        if (lane == 0 && sl == 0 && (!ROWS || r < rows)) scale[r] = r < rows ? sc.s + (sc.finite ? ld.mul(r) : 0) : 0;
+        const int up = min(max(sc.up, -900), 900), rest = sc.up - up;
         uint8_t *blk = dig + (size_t)(grp / 16) * nkb * kI8BlockBytes + (size_t)(grp % 16) * 256;
         for (int k0 = ka; k0 < kz; k0 += 128) {
             if (kz - ka > 128 || !sc.finite) {  // one turn: still in registers
 #pragma unroll
-                for (int q = 0; q < 4; q++) v[q] = 0.0;
-                if (sc.finite && k0 + 4 * lane < n) ld.load4(r, k0 + 4 * lane, n, v);
+                for (int q = 0; q < 4; q++) v[q] = 0.0, e[q] = 0;
+                if (sc.finite && k0 + 4 * lane < n) ld.load4(r, k0 + 4 * lane, n, v, e);
             }
             unsigned lo[4], hi[4];
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                const unsigned long long d = digits(v[q], sc);
+                const unsigned long long d = digits(v[q], up + e[q], rest);
                 lo[q] = (unsigned)d;
                 hi[q] = (unsigned)(d >> 32);
             }
@@ -622,32 +664,33 @@ struct TransLoad {
     const double *src;
     long long ld;
     int K;
-    const double *ks;
-    __device__ double mul(long long) const { return 1.0; }
+    const int *ks;
+    __device__ int mul(long long) const { return 0; }
     __device__ int used_blocks(long long, int nkb) const { return nkb; }
     __device__ int len(long long) const { return K; }
-    __device__ void load4(long long r, int k, int n, double (&v)[4]) const {
+    __device__ void load4(long long r, int k, int n, double (&v)[4], int (&e)[4]) const {
 #pragma unroll
-        for (int q = 0; q < 4; q++) v[q] = k + q < n ? src[(k + q) * ld + r] * (ks ? ks[k + q] : 1.0) : 0.0;
+        for (int q = 0; q < 4; q++) {
+            v[q] = k + q < n ? src[(k + q) * ld + r] : 0.0;
+            e[q] = ks && k + q < n ? ks[k + q] : 0;
+        }
     }
 };
 
-// up = 2^e > the magnitude m (1 for zero), down = 1 / up; both kept in the normal range
-__device__ __forceinline__ void k_scale(unsigned long long m, double &up, double &down) {
-    const int E = (int)(m >> 52);
-    const int e = m == 0 ? 0 : min(max(E - 1022, -1000), 1000);
-    up = pow2(e);
-    down = pow2(-e);
+// 2^up > the magnitude m (0 for zero or a non-finite one), down = -up
+__device__ __forceinline__ void k_scale(unsigned m, int &up, int &down) {
+    const int e = m == 0 || m == kMagNonFinite ? 0 : (int)(m >> 6) - kMagBias - 1022;
+    up = min(max(e, -kI8KExp), kI8KExp);
+    down = -up;
 }
 
 __global__ void __launch_bounds__(256) column_scales_kernel(const double *__restrict__ src, long long ld, long long rows,
-                                                            int K, double *__restrict__ up, double *__restrict__ down) {
-    __shared__ unsigned long long red[8];
+                                                            int K, int *__restrict__ up, int *__restrict__ down) {
+    __shared__ unsigned red[8];
     for (int k = blockIdx.x; k < K; k += gridDim.x) {
-        unsigned long long m = 0;
-        for (long long r = threadIdx.x; r < rows; r += 256) m = max(m, mag(src[(size_t)k * ld + r]));
-#pragma unroll
-        for (int o = 16; o; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+        unsigned m = 0;
+        for (long long r = threadIdx.x; r < rows; r += 256) m = max(m, mag(src[(size_t)k * ld + r], 0));
+        m = __reduce_max_sync(0xffffffffu, m);
         if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -659,22 +702,21 @@ __global__ void __launch_bounds__(256) column_scales_kernel(const double *__rest
 }
 
 __global__ void row_mag_kernel(const double *__restrict__ src, long long ld, long long rows, int K,
-                               unsigned long long *__restrict__ out) {
+                               unsigned *__restrict__ out) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= K) return;
-    unsigned long long m = 0;
-    for (long long r = blockIdx.y; r < rows; r += gridDim.y) m = max(m, mag(src[r * ld + k]));
+    unsigned m = 0;
+    for (long long r = blockIdx.y; r < rows; r += gridDim.y) m = max(m, mag(src[r * ld + k], 0));
     atomicMax(out + k, m);
 }
 
-__global__ void row_scales_kernel(const unsigned long long *__restrict__ m, int K, double *__restrict__ up,
-                                  double *__restrict__ down) {
+__global__ void row_scales_kernel(const unsigned *__restrict__ m, int K, int *__restrict__ up, int *__restrict__ down) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k < K) k_scale(m[k], up[k], down[k]);
 }
 
 template <bool ROWS = false, class Load>
-cudaError_t launch_digits(const Load &ld, long long rows, int nkb, uint8_t *dig, double *scale, cudaStream_t s) {
+cudaError_t launch_digits(const Load &ld, long long rows, int nkb, uint8_t *dig, int *scale, cudaStream_t s) {
     if (rows <= 0 || nkb <= 0) return cudaSuccess;
     const long long groups = (ROWS ? rows + 7 : i8_pad_rows(rows)) / 8;
     // slices of at least 512 values until ~4 CTAs per SM run
@@ -729,40 +771,39 @@ bool operand_ok(const I8Operand &o) {
 
 }  // namespace
 
-cudaError_t i8_column_scales(const double *src, long long ld, long long rows, int K, double *up, double *down,
+cudaError_t i8_column_scales(const double *src, long long ld, long long rows, int K, int *up, int *down,
                              cudaStream_t s) {
     if (K <= 0) return cudaSuccess;
     column_scales_kernel<<<std::min(K, 148 * 8), 256, 0, s>>>(src, ld, rows, K, up, down);
     return cudaGetLastError();
 }
-cudaError_t i8_row_scales(const double *src, long long ld, long long rows, int K, unsigned long long *mag, double *up,
-                          double *down, cudaStream_t s) {
+cudaError_t i8_row_scales(const double *src, long long ld, long long rows, int K, unsigned *mag, int *up, int *down,
+                          cudaStream_t s) {
     if (K <= 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(mag, 0, sizeof(unsigned long long) * K, s);
+    cudaError_t e = cudaMemsetAsync(mag, 0, sizeof(unsigned) * K, s);
     if (e != cudaSuccess) return e;
     const dim3 grid((K + 255) / 256, (unsigned)std::max<long long>(1, std::min<long long>(rows, 512)));
     row_mag_kernel<<<grid, 256, 0, s>>>(src, ld, rows, K, mag);
     row_scales_kernel<<<(K + 255) / 256, 256, 0, s>>>(mag, K, up, down);
     return cudaGetLastError();
 }
-cudaError_t i8_digits(const double *src, long long ld, const int *idx, long long rows, int K, int nkb,
-                      const double *kscale, const double *rmul, uint8_t *dig, double *scale, cudaStream_t s) {
-    return launch_digits(RowLoad{src, ld, idx, K, kscale, nullptr, nullptr, nullptr, 0, rmul}, rows, nkb, dig, scale, s);
+cudaError_t i8_digits(const double *src, long long ld, const int *idx, long long rows, int K, int nkb, const int *kexp,
+                      const double *rmul, uint8_t *dig, int *scale, cudaStream_t s) {
+    return launch_digits(RowLoad{src, ld, idx, K, kexp, nullptr, nullptr, nullptr, 0, rmul}, rows, nkb, dig, scale, s);
 }
-cudaError_t i8_digits_rows(const double *src, long long ld, long long rows, int K, int nkb, const double *kscale,
-                           uint8_t *dig, double *scale, cudaStream_t s) {
-    return launch_digits<true>(RowLoad{src, ld, nullptr, K, kscale, nullptr, nullptr, nullptr, 0, nullptr}, rows, nkb, dig, scale, s);
+cudaError_t i8_digits_rows(const double *src, long long ld, long long rows, int K, int nkb, const int *kexp,
+                           uint8_t *dig, int *scale, cudaStream_t s) {
+    return launch_digits<true>(RowLoad{src, ld, nullptr, K, kexp, nullptr, nullptr, nullptr, 0, nullptr}, rows, nkb, dig, scale, s);
 }
 cudaError_t i8_digits_blocks(const double *src, long long ld, long long rows, const int *kof, const int *nof, int nkb,
-                             const double *kscale, const int *kset, int kld, uint8_t *dig, double *scale,
-                             cudaStream_t s) {
-    return launch_digits(RowLoad{src, ld, nullptr, 0, kscale, kof, kset, nof, kld, nullptr}, rows, nkb, dig, scale, s);
+                             const int *kexp, const int *kset, int kld, uint8_t *dig, int *scale, cudaStream_t s) {
+    return launch_digits(RowLoad{src, ld, nullptr, 0, kexp, kof, kset, nof, kld, nullptr}, rows, nkb, dig, scale, s);
 }
-cudaError_t i8_digits_trans(const double *src, long long ld, long long rows, int K, int nkb, const double *kscale,
-                            uint8_t *dig, double *scale, cudaStream_t s) {
-    return launch_digits(TransLoad{src, ld, K, kscale}, rows, nkb, dig, scale, s);
+cudaError_t i8_digits_trans(const double *src, long long ld, long long rows, int K, int nkb, const int *kexp,
+                            uint8_t *dig, int *scale, cudaStream_t s) {
+    return launch_digits(TransLoad{src, ld, K, kexp}, rows, nkb, dig, scale, s);
 }
-cudaError_t i8_digits_gather(const I8Gather &g, int nkb, uint8_t *dig, double *scale, cudaStream_t s) {
+cudaError_t i8_digits_gather(const I8Gather &g, int nkb, uint8_t *dig, int *scale, cudaStream_t s) {
     return launch_digits(GatherLoad{g}, 8ll << g.lg, nkb, dig, scale, s);
 }
 
@@ -774,8 +815,8 @@ int i8_gemm_parts(long long M, long long N, int nkb) {
     return (int)std::max<long long>(1, std::min<long long>(148 / nt, nkb / 16));
 }
 
-cudaError_t i8_gemm(int M, int N, I8Operand A, I8Operand B, double alpha, int add, double *C, long long ldc,
-                    const int *cols, double *parts, int *err, cudaStream_t s) {
+cudaError_t i8_gemm(int M, int N, I8Operand A, I8Operand B, int add, double *C, long long ldc, const int *cols,
+                    double *parts, int *err, cudaStream_t s) {
     if (M <= 0 || N <= 0) return cudaSuccess;
     if (!operand_ok(A) || !operand_ok(B) || A.nkb != B.nkb || !C || !err || ldc < M) return cudaErrorInvalidValue;
     const int gm = (M + kBM - 1) / kBM, gn = (N + kBN - 1) / kBN;
@@ -785,7 +826,7 @@ cudaError_t i8_gemm(int M, int N, I8Operand A, I8Operand B, double alpha, int ad
     const long long nt = (long long)gm * gn * np;
     if (nt > 0x7fffffff) return cudaErrorInvalidValue;
     // the operand with fewer blocks is walked fastest: it stays in L2 while the other streams
-    DenseJob job{M, N, add, gm, gn, (int)nt, seg, A.nkb, gm <= gn, alpha, C, ldc, 0, cols};
+    DenseJob job{M, N, add, gm, gn, (int)nt, seg, A.nkb, gm <= gn, C, ldc, 0, cols};
     if (np > 1) {
         job.add = 0;
         job.C = parts;
@@ -804,7 +845,7 @@ cudaError_t i8_grouped(I8Operand A, I8Operand B, const I8Tile *tiles, int ntiles
                        cudaStream_t s) {
     if (ntiles <= 0) return cudaSuccess;
     if (!operand_ok(A) || !operand_ok(B) || !tiles || !C || !err) return cudaErrorInvalidValue;
-    return launch_gemm(A, B, GroupJob<false>{tiles, ntiles, add, 1.0, C, nullptr}, err, s);
+    return launch_gemm(A, B, GroupJob<false>{tiles, ntiles, add, C, nullptr}, err, s);
 }
 
 cudaError_t i8_grouped_gather(I8Operand A, I8Rows B, const int *rows, const I8Tile *tiles, int ntiles, int add, double *C,
@@ -812,7 +853,7 @@ cudaError_t i8_grouped_gather(I8Operand A, I8Rows B, const int *rows, const I8Ti
     if (ntiles <= 0) return cudaSuccess;
     const I8Operand b{B.dig, B.scale, B.nkb};
     if (!operand_ok(A) || !operand_ok(b) || !rows || !tiles || !C || !err) return cudaErrorInvalidValue;
-    return launch_gemm(A, b, GroupJob<true>{tiles, ntiles, add, 1.0, C, rows}, err, s);
+    return launch_gemm(A, b, GroupJob<true>{tiles, ntiles, add, C, rows}, err, s);
 }
 
 }  // namespace stk

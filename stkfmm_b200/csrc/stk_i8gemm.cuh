@@ -30,14 +30,17 @@ constexpr int kI8MaxSegment = 512;  // K blocks summed before the accumulators a
 // core matrices (8 rows x 16 bytes): a pipeline stage is one contiguous copy.
 struct I8Operand {
     const uint8_t *dig = nullptr;
-    const double *scale = nullptr;  // per row (padded to 128): 2^(e - 35); 0: zero row, NaN: non-finite row
-    int nkb = 0;                    // K blocks per row block
+    const int *scale = nullptr;  // per row (padded to 128): the exponent e - 35, or kI8NonFinite
+    int nkb = 0;                 // K blocks per row block
 };
+// Scales are kept as exponents: 2^(e - 35) itself leaves the range of a double for rows below
+// 2^-987, and a product of two scales does long before the results they stand for.
+constexpr int kI8NonFinite = 1 << 20;  // a row with an infinity or NaN: its products are NaN
 // Rows of digits to gather from: row r is nkb x 7 x 32 bytes (K block, plane, K), so that a
 // tile's columns are any rows, fetched 16 bytes at a time.
 struct I8Rows {
     const uint8_t *dig = nullptr;
-    const double *scale = nullptr;  // per row
+    const int *scale = nullptr;  // per row
     int nkb = 0;
 };
 inline size_t i8_row_bytes(long long rows, int nkb) { return (size_t)rows * nkb * kI8Planes * kI8K; }
@@ -50,51 +53,52 @@ inline size_t i8_bytes(long long rows, int nkb) {
 // Scales along K.  The far field's operators and densities are written in singular-vector
 // coordinates whose sizes fall over eight decades, large where the other operand is small; a
 // common scale per row would spend its digits on the largest.  Products are therefore formed
-// as (A D^-1)(D B) with D_k a power of two, the largest |A_mk| over m rounded up: `kscale`
-// below multiplies the values of index k before they are split (null: 1).
-// up[k] = 2^e > max_m |src[k ld + m]| (1 for a zero column), down[k] = 1 / up[k]
-cudaError_t i8_column_scales(const double *src, long long ld, long long rows, int K, double *up, double *down,
+// as (A D^-1)(D B) with D_k a power of two, the largest |A_mk| over m rounded up: `kexp` below
+// are exponents, and the values of index k are multiplied by 2^kexp[k] before they are split
+// (null: 0).
+// up[k] = e, 2^e > max_m |src[k ld + m]| (0 for a zero column; within +-kI8KExp), down[k] = -e
+constexpr int kI8KExp = 100;
+cudaError_t i8_column_scales(const double *src, long long ld, long long rows, int K, int *up, int *down,
                              cudaStream_t s);
 // the same for rows of K contiguous values: max over r of |src[r ld + k]|; mag: K words of scratch
-cudaError_t i8_row_scales(const double *src, long long ld, long long rows, int K, unsigned long long *mag, double *up,
-                          double *down, cudaStream_t s);
+cudaError_t i8_row_scales(const double *src, long long ld, long long rows, int K, unsigned *mag, int *up, int *down,
+                          cudaStream_t s);
 
-// x(r, k) = src[(idx ? idx[r] : r) ld + k] kscale[k], K contiguous; idx[r] < 0 gives a zero row.
-// rmul (nullable): powers of two that multiply the rows' stored scales.
-cudaError_t i8_digits(const double *src, long long ld, const int *idx, long long rows, int K, int nkb,
-                      const double *kscale, const double *rmul, uint8_t *dig, double *scale, cudaStream_t s);
+// x(r, k) = src[(idx ? idx[r] : r) ld + k] 2^kexp[k], K contiguous; idx[r] < 0 gives a zero row.
+// rmul (nullable): powers of two that multiply the rows (through their stored scales).
+cudaError_t i8_digits(const double *src, long long ld, const int *idx, long long rows, int K, int nkb, const int *kexp,
+                      const double *rmul, uint8_t *dig, int *scale, cudaStream_t s);
 // the same as gatherable rows (I8Rows)
-cudaError_t i8_digits_rows(const double *src, long long ld, long long rows, int K, int nkb, const double *kscale,
-                           uint8_t *dig, double *scale, cudaStream_t s);
+cudaError_t i8_digits_rows(const double *src, long long ld, long long rows, int K, int nkb, const int *kexp,
+                           uint8_t *dig, int *scale, cudaStream_t s);
 // the same with, per block b of 128 rows, kof[b] values (<= 32 nkb, the rest zero), nof[b] rows
-// (the rest zero) and the scales kscale + kset[b] kld
+// (the rest zero) and the exponents kexp + kset[b] kld
 cudaError_t i8_digits_blocks(const double *src, long long ld, long long rows, const int *kof, const int *nof, int nkb,
-                             const double *kscale, const int *kset, int kld, uint8_t *dig, double *scale,
-                             cudaStream_t s);
-// x(r, k) = src[k ld + r] kscale[k]
-cudaError_t i8_digits_trans(const double *src, long long ld, long long rows, int K, int nkb, const double *kscale,
-                            uint8_t *dig, double *scale, cudaStream_t s);
+                             const int *kexp, const int *kset, int kld, uint8_t *dig, int *scale, cudaStream_t s);
+// x(r, k) = src[k ld + r] 2^kexp[k]
+cudaError_t i8_digits_trans(const double *src, long long ld, long long rows, int K, int nkb, const int *kexp,
+                            uint8_t *dig, int *scale, cudaStream_t s);
 // rows of a gathered operand, in eight types of 2^lg rows: row r = (c, j = r mod 2^lg) has
 // x(r, k) = z[pos ldz + srow[row_off[c] + k]], pos = tab[tab_off[c] + j nq[c] + rowq[row_off[c] + k]]
-// (0 where pos < 0) times kscale[row_off[c] + k], k < K[c]; row_off multiples of 4
+// (0 where pos < 0) times 2^kexp[row_off[c] + k], k < K[c]; row_off multiples of 4
 struct I8Gather {
     const double *z;
     const int *tab, *rowq, *srow;
-    const double *kscale;
+    const int *kexp;
     long long tab_off[8], row_off[8];
     int nq[8], K[8];
     int ldz, lg;
 };
-cudaError_t i8_digits_gather(const I8Gather &g, int nkb, uint8_t *dig, double *scale, cudaStream_t s);
+cudaError_t i8_digits_gather(const I8Gather &g, int nkb, uint8_t *dig, int *scale, cudaStream_t s);
 
-// C[m + ldc col(n)] (add = 0: =, 1: +=) alpha sum_k A[m][k] B[n][k], m < M, n < N;
+// C[m + ldc col(n)] (add = 0: =, 1: +=) sum_k A[m][k] B[n][k], m < M, n < N;
 // col(n) = cols ? cols[n] : n (no two n may share a column).  Products with few output tiles
 // are split along K into i8_gemm_parts(M, N, nkb) parts, written to `parts` (M x N each) and
 // summed in order; parts may be null when that is 1.  err: device int, set non-zero when a
 // pipeline wait gave up.
 int i8_gemm_parts(long long M, long long N, int nkb);
-cudaError_t i8_gemm(int M, int N, I8Operand A, I8Operand B, double alpha, int add, double *C, long long ldc,
-                    const int *cols, double *parts, int *err, cudaStream_t s);
+cudaError_t i8_gemm(int M, int N, I8Operand A, I8Operand B, int add, double *C, long long ldc, const int *cols,
+                    double *parts, int *err, cudaStream_t s);
 
 // One 128 x 128 output tile of a grouped product: rows of A block a_blk, columns of B
 // block b_blk (row blocks of the operands), the first nkb K blocks of both.  Written (or

@@ -81,3 +81,19 @@ def test_zero_and_non_finite_rows(torch_cuda):
     assert not np.isfinite(got[bad]).any()
     np.testing.assert_allclose(got[~bad], (A @ B.T)[~bad], rtol=0, atol=1e-13)
     assert (got[1, ~bad[1]] == 0).all()
+
+
+def test_rows_at_the_ends_of_the_double_range(torch_cuda):
+    """Rows from 2^-1060 to 2^1000, every pair of them in one tile: whole numbers below 2^20, so that
+    sums of 64 products are exact and the result is one rounding of them (none but where it is
+    subnormal: one unit of the smallest there, for a rounding before the last)."""
+    rng = np.random.default_rng(5)
+    exps = np.array([-1060, -1022, -1000, -988, -700, -536, -465, -300, 0, 300, 465, 536, 700, 970, 1000])
+    ia, ib = (rng.integers(-2 ** 20, 2 ** 20, size=(3 * len(exps), 64)).astype(float) for _ in range(2))
+    ea, eb = np.repeat(exps, 3), np.tile(exps, 3)
+    with np.errstate(over="ignore"):
+        ref = np.ldexp(ia @ ib.T, ea[:, None] + eb[None, :])
+    got = product(torch_cuda, np.ldexp(ia, ea[:, None]), np.ldexp(ib, eb[:, None]))
+    normal = ~(np.abs(ref) < 2.0 ** -1022)
+    np.testing.assert_array_equal(got[normal], ref[normal])
+    assert np.abs(got[~normal] - ref[~normal]).max() <= 2.0 ** -1074
