@@ -400,8 +400,8 @@ extern "C" int stk_gemm_3xtf32(int M, int N, int K, const float *d_A, int lda, c
 extern "C" int stk_gemm_f64_i8(int M, int N, int K, const double *d_A, int lda, const double *d_B, int ldb, double *d_C,
                                int ldc, int beta, void *stream) {
     if (M < 0 || N < 0 || K < 0 || (beta != 0 && beta != 1)) return STK_ERR_INVALID_ARG;
-    if (M == 0 || N == 0 || K == 0) return STK_OK;
-    if (!d_A || !d_B || !d_C || lda < K || ldb < K || ldc < M) return STK_ERR_INVALID_ARG;
+    if (M == 0 || N == 0) return STK_OK;
+    if ((K > 0 && (!d_A || !d_B)) || !d_C || lda < K || ldb < K || ldc < M) return STK_ERR_INVALID_ARG;
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
         cudaGetLastError();
@@ -409,6 +409,12 @@ extern "C" int stk_gemm_f64_i8(int M, int N, int K, const double *d_A, int lda, 
     }
     if (!umma_available()) return STK_ERR_NOT_SUPPORTED;
     cudaStream_t s = (cudaStream_t)stream;
+    if (K == 0) {  // empty sums
+        const bool ok = beta || (cudaMemset2DAsync(d_C, sizeof(double) * ldc, 0, sizeof(double) * M, N, s) == cudaSuccess &&
+                                 cudaStreamSynchronize(s) == cudaSuccess);
+        cudaGetLastError();
+        return ok ? STK_OK : STK_ERR_CUDA;
+    }
     const int nkb = i8_kblocks(K);
     const size_t ba = i8_bytes(M, nkb), bb = i8_bytes(N, nkb);
     const size_t sa = sizeof(int) * i8_pad_rows(M), sb = sizeof(int) * i8_pad_rows(N);  // multiples of 512 bytes

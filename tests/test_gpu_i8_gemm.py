@@ -97,3 +97,18 @@ def test_rows_at_the_ends_of_the_double_range(torch_cuda):
     normal = ~(np.abs(ref) < 2.0 ** -1022)
     np.testing.assert_array_equal(got[normal], ref[normal])
     assert np.abs(got[~normal] - ref[~normal]).max() <= 2.0 ** -1074
+
+
+@pytest.mark.parametrize("beta", [0, 1])
+def test_empty_sum(torch_cuda, beta):
+    """K = 0: zeros (beta 0) or C as it was, and nothing beyond its M rows."""
+    from stkfmm_b200 import lib
+    C = np.arange(1.0, 36.0).reshape(5, 7)  # 5 columns of M = 4 within ldc = 7
+    out = torch_cuda.as_tensor(C, device="cuda")
+    a = torch_cuda.zeros(8, dtype=torch_cuda.float64, device="cuda")
+    rc = lib().stk_gemm_f64_i8(4, 5, 0, a.data_ptr(), 0, a.data_ptr(), 0, out.data_ptr(), 7, beta,
+                               torch_cuda.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    want = C.copy()
+    want[:, :4] *= beta
+    np.testing.assert_array_equal(out.cpu().numpy(), want)
