@@ -224,9 +224,13 @@ int stk_gemm_3xtf32(int M, int N, int K, const float *d_A, int lda, const float 
  * B[n ldb + k] for m < M, n < N, FP64 in and out: every row of A and B scaled by a
  * power of two and split into seven balanced base-256 digits, 34 exact integer
  * products on the sm_100a tensor cores (tcgen05 kind::i8), put together in FP64.
- * Error below ~2^-56 |a||b| per element (row norms), less than an FP64 sum's
- * rounding.  A row with an infinity or NaN gives NaN.  Device pointers; the call
- * allocates its scratch and waits for the result.  STK_ERR_NOT_SUPPORTED off sm_100. */
+ * Error of an element c: at most 4.2 K 2^-56 max|a| max|b| (the two rows' largest
+ * values; about sqrt(K) instead of K where their signs are mixed) plus 2^-52 |c|.
+ * That is normwise: products far below the rows' largest are not kept to their own
+ * 53 bits, as an FP64 sum's are.  (The far field balances its operands along K.)
+ * A row with an infinity or NaN gives NaN; every finite magnitude is in range.
+ * Device pointers; the call allocates its scratch and waits for the result.
+ * STK_ERR_NOT_SUPPORTED off sm_100. */
 int stk_gemm_f64_i8(int M, int N, int K, const double *d_A, int lda, const double *d_B, int ldb, double *d_C, int ldc,
                     int beta, void *stream);
 

@@ -5,11 +5,13 @@
 // a' = sum_i d_i 256^(6 - i) with -128 <= d_i <= 127 (the splitting of the published Ozaki
 // scheme, with integer products).  A product of two rows is
 //   sum_k a'_k b'_k ~ sum_{g = 0..7} 256^(12 - g) sum_{i + j = g} sum_k d_ik e_jk,
-// 34 int8 dot products accumulated exactly in int32.  The dropped terms i + j >= 8 are below the
-// rounding of the values to 2^-56 of their row's scale, and that is below the rounding of an FP64
-// sum.  (Without i + j = 7, 28 products and 15% faster, the dropped terms showed where a row's
-// largest value is far above the others: the rounding noise of a triply periodic Laplace FMM's
-// potential rose from 1.3e-10 to 1.9e-8.)
+// 34 int8 dot products accumulated exactly in int32.  A value is rounded to 2^-56 of its row's
+// scale, 2^e <= 2.02 max |x|, and the dropped terms i + j >= 8 add 2% to that: an element is off by
+// at most 4.2 K 2^-56 max|a| max|b|, about sqrt(K) of it with mixed signs, and 2^-52 of itself (two
+// conversions).  On rows of one size that is below the rounding of an FP64 sum; on graded rows it is
+// not componentwise (hence the scales along K below).  (Without i + j = 7, 28 products and 15%
+// faster, the dropped terms showed where a row's largest value is far above the others: the
+// rounding noise of a triply periodic Laplace FMM's potential rose from 1.3e-10 to 1.9e-8.)
 #pragma once
 #include <cstdint>
 

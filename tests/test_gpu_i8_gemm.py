@@ -112,3 +112,20 @@ def test_empty_sum(torch_cuda, beta):
     want = C.copy()
     want[:, :4] *= beta
     np.testing.assert_array_equal(out.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("K", [1, 40, 3584])
+def test_error_bound_holds_for_graded_rows(torch_cuda, K):
+    """The stated bound, 4.2 K 2^-56 max|a| max|b| + 2^-52 |c|, where rows of A fall by nine decades and
+    those of B rise by as many (each product as large as any other), where only A is graded and B misses
+    its largest value, and on plain values."""
+    rng = np.random.default_rng(K)
+    g = np.logspace(0, -9, K)
+    rows = lambda: rng.uniform(0.5, 1.0, size=(20, K)) * rng.choice([-1.0, 1.0], size=(20, K))
+    A = np.concatenate([rows() * g, np.abs(rows()) * g, rows()])
+    miss = rows()
+    miss[:, 0] = 0.0
+    B = np.concatenate([rows() / g, miss, np.abs(rows()) / g, rows()])
+    ref = A.astype(np.longdouble) @ B.astype(np.longdouble).T
+    bound = 4.2 * K * 2.0 ** -56 * np.abs(A).max(1)[:, None] * np.abs(B).max(1) + 2.0 ** -52 * np.abs(ref)
+    assert (np.abs(product(torch_cuda, A, B) - ref) <= bound).all()
