@@ -917,11 +917,9 @@ int build_m2l_lowrank(FarField &F, const std::vector<double> &unit, const double
 }
 
 // ---- FP64 products on the int8 tensor cores ---------------------------------------
-// Operator digits, built with the operators and shared with them.
+// Digits of an operator set (the cache's entry F), those that it lacks: made for the first handle
+// that wants them, tried again for the next one where there was no memory.
 int build_i8_operators(FarField &F, cudaStream_t s) {
-    F.i8 = F.i8_pq = false;
-    const char *env = getenv("STKFMM_F64_I8");
-    if ((env && env[0] == '0') || !umma_available()) return STK_OK;
     const int N = F.n * F.ke, k = F.m2l_rank;
     // column-major M x K operators: row m's values are ld apart
     auto op = [&](I8Buf &b, const DevBuf &src, int M, int K) -> int {
@@ -932,17 +930,21 @@ int build_i8_operators(FarField &F, cudaStream_t s) {
         FCUDA(i8_digits_trans((const double *)src.ptr, M, M, K, b.nkb, b.down(), b.digits(), b.scales(), s));
         return STK_OK;
     };
-    int rc = op(F.i8_uc2ue, F.uc2ue, N, N);
-    if (!rc) rc = op(F.i8_dc2de, F.dc2de, N, N);
-    if (!rc) rc = op(F.i8_m2m, F.m2m, N, 8 * N);
-    if (!rc) rc = op(F.i8_l2l, F.l2l, 8 * N, N);
-    if (!rc) rc = op(F.i8_vt, F.m2l_vt, k, N);
-    if (!rc) rc = op(F.i8_e, F.m2l_e, N, k);
-    if (rc) {  // no memory for them: the products stay with cuBLAS
-        for (I8Buf *b : {&F.i8_uc2ue, &F.i8_dc2de, &F.i8_m2m, &F.i8_l2l, &F.i8_vt, &F.i8_e}) b->release();
-        return STK_OK;
+    int rc = STK_OK;
+    if (!F.i8) {
+        rc = op(F.i8_uc2ue, F.uc2ue, N, N);
+        if (!rc) rc = op(F.i8_dc2de, F.dc2de, N, N);
+        if (!rc) rc = op(F.i8_m2m, F.m2m, N, 8 * N);
+        if (!rc) rc = op(F.i8_l2l, F.l2l, 8 * N, N);
+        if (!rc) rc = op(F.i8_vt, F.m2l_vt, k, N);
+        if (!rc) rc = op(F.i8_e, F.m2l_e, N, k);
+        if (rc) {  // no memory for them: the products stay with cuBLAS
+            for (I8Buf *b : {&F.i8_uc2ue, &F.i8_dc2de, &F.i8_m2m, &F.i8_l2l, &F.i8_vt, &F.i8_e}) b->release();
+            return STK_OK;
+        }
+        F.i8 = true;
     }
-    F.i8 = true;
+    if (F.i8_pq) return STK_OK;
     // the factors of every offset, within 8 GiB
     const int nslot = (int)F.m2l_r.size(), kb = (k + kI8Rows - 1) / kI8Rows;
     F.i8_q_blk.assign(nslot, 0);
@@ -1152,7 +1154,6 @@ int build_operators(FarField &F, cudaStream_t s) {
     FBLAS(cublasDgemm(F.blas, CUBLAS_OP_N, CUBLAS_OP_T, N, k, N, &one, (const double *)F.dc2de.ptr, N,
                       (const double *)VTu.ptr, N, &zero, (double *)F.m2l_e.ptr, N));
     rc = build_m2l_lowrank(F, unit, (const double *)VTu.ptr, (const double *)VTv.ptr, offset_matrix, K, T, s);
-    if (!rc) rc = build_i8_operators(F, s);
     if (rc) return rc;
     FCUDA(cudaStreamSynchronize(s));
     return STK_OK;
@@ -1290,6 +1291,7 @@ FarField::~FarField() {
     if (blas) cublasDestroy(blas);
     if (solver) cusolverDnDestroy(solver);
     if (built) cudaEventDestroy(built);
+    if (i8_built) cudaEventDestroy(i8_built);
     for (int i = 0; i < 8; i++) {
         if (tc_stream[i]) cudaStreamDestroy(tc_stream[i]);
         if (tc_ev[i]) cudaEventDestroy(tc_ev[i]);
@@ -1331,6 +1333,9 @@ void cache_put(std::map<OpsKey, std::weak_ptr<FarField>> &m, const OpsKey &k, co
     m[k] = e;
 }
 
+I8Buf FarField::*const kI8Operators[] = {&FarField::i8_uc2ue, &FarField::i8_dc2de, &FarField::i8_m2m, &FarField::i8_l2l,
+                                         &FarField::i8_vt,    &FarField::i8_e,     &FarField::i8_q,   &FarField::i8_p};
+
 // dst aliases src's level-independent operators
 void share_operators(FarField &dst, const FarField &src) {
     dst.m2l_rank = src.m2l_rank;
@@ -1349,17 +1354,33 @@ void share_operators(FarField &dst, const FarField &src) {
     dst.m2l_q32.share(src.m2l_q32);
     dst.m2l_vt.share(src.m2l_vt);
     dst.m2l_e.share(src.m2l_e);
-    dst.i8 = src.i8;
-    dst.i8_pq = src.i8_pq;
-    dst.i8_q_blk = src.i8_q_blk;
-    dst.i8_uc2ue.share(src.i8_uc2ue);
-    dst.i8_dc2de.share(src.i8_dc2de);
-    dst.i8_m2m.share(src.i8_m2m);
-    dst.i8_l2l.share(src.i8_l2l);
-    dst.i8_vt.share(src.i8_vt);
-    dst.i8_e.share(src.i8_e);
-    dst.i8_q.share(src.i8_q);
-    dst.i8_p.share(src.i8_p);
+    dst.n = src.n;
+    dst.ke = src.ke;
+}
+
+// F's digits: those of its operator set where this handle wants them (STKFMM_F64_I8=0 at its
+// set-up, or no sm_100: cuBLAS), whatever other handles of the set do
+int attach_i8_operators(FarField &F, cudaStream_t s) {
+    F.i8 = F.i8_pq = false;
+    const char *env = getenv("STKFMM_F64_I8");
+    if ((env && env[0] == '0') || !umma_available()) {
+        for (I8Buf FarField::*b : kI8Operators) (F.*b).release();
+        return STK_OK;
+    }
+    FarField &E = *F.ops_ref;
+    std::lock_guard<std::mutex> lock(E.i8_mu);
+    if (E.i8_built) FCUDA(cudaStreamWaitEvent(s, E.i8_built, 0));
+    if (!E.i8 || !E.i8_pq) {
+        const int rc = build_i8_operators(E, s);
+        if (rc) return rc;
+        if (!E.i8_built) FCUDA(cudaEventCreateWithFlags(&E.i8_built, cudaEventDisableTiming));
+        FCUDA(cudaEventRecord(E.i8_built, s));
+    }
+    F.i8 = E.i8;
+    F.i8_pq = E.i8_pq;
+    F.i8_q_blk = E.i8_q_blk;
+    for (I8Buf FarField::*b : kI8Operators) (F.*b).share(E.*b);
+    return STK_OK;
 }
 
 // an event recorded on s after the work queued so far (the entry's build)
@@ -1863,6 +1884,7 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
         F.tcc_ops = false;
         F.m2c_p = 0;  // the periodic operator follows the (possibly new) operators
     }
+    if ((rc = attach_i8_operators(F, s))) return rc;
     F.periodic = f->pbc >= 1;
     const int far_field = f->enable_ff ? 1 : 0;
     if (F.periodic && (F.m2c_p != F.p || F.m2c_m2x != F.m2x || F.m2c_pbc != f->pbc || F.m2c_ff != far_field)) {

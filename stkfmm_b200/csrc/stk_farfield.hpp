@@ -8,6 +8,7 @@
 // equivalent at 2.95 times the box half-width, centred on the box.
 #pragma once
 #include <memory>
+#include <mutex>
 #include <vector>
 
 #include <cublas_v2.h>
@@ -232,6 +233,9 @@ struct FarField {
     bool split = false;
     bool dn_own[8] = {true, true, true, true, true, true, true, true};
     cudaEvent_t built = nullptr;
+    // of an entry: its digits are made under the lock, by the first handle that wants them
+    std::mutex i8_mu;
+    cudaEvent_t i8_built = nullptr;
     ~FarField();
 };
 
