@@ -291,7 +291,9 @@ int Stk3DFMM_show_active_kernels(Stk3DFMM *fmm);
 /* STKFMM::evaluateKernel through the handle (STKFMM.cpp:88-99) */
 int Stk3DFMM_evaluate_kernel(Stk3DFMM *fmm, unsigned kernel, int nThreads, unsigned p2p, int nSrc,
                              double *srcCoord, double *srcValue, int nTrg, double *trgCoord, double *trgValue);
-/* choose FP64 or MIXED for the P2P kernels of this handle (default FP64) */
+/* choose FP64 or MIXED for the P2P kernels of this handle (default FP64).  The far
+ * field is set up for the precision it is first evaluated in; the first FP64
+ * evaluate_fmm after mixed ones sets it up again (and synchronises). */
 int Stk3DFMM_set_precision(Stk3DFMM *fmm, int precision);
 /* Multi-GPU sharding of one problem: this handle evaluates only shard `rank` of
  * `nranks` of the target-side work (near-field P2P, L2T, M2T), dealt by cost;

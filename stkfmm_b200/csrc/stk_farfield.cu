@@ -918,8 +918,9 @@ int build_m2l_lowrank(FarField &F, const std::vector<double> &unit, const double
 
 // ---- FP64 products on the int8 tensor cores ---------------------------------------
 // Digits of an operator set (the cache's entry F), those that it lacks: made for the first handle
-// that wants them, tried again for the next one where there was no memory.
-int build_i8_operators(FarField &F, cudaStream_t s) {
+// that wants them (pq: those of the M2L's factors too), tried again for the next one where there
+// was no memory.
+int build_i8_operators(FarField &F, bool pq, cudaStream_t s) {
     const int N = F.n * F.ke, k = F.m2l_rank;
     // column-major M x K operators: row m's values are ld apart
     auto op = [&](I8Buf &b, const DevBuf &src, int M, int K) -> int {
@@ -944,7 +945,7 @@ int build_i8_operators(FarField &F, cudaStream_t s) {
         }
         F.i8 = true;
     }
-    if (F.i8_pq) return STK_OK;
+    if (F.i8_pq || !pq) return STK_OK;
     // the factors of every offset, within 8 GiB
     const int nslot = (int)F.m2l_r.size(), kb = (k + kI8Rows - 1) / kI8Rows;
     F.i8_q_blk.assign(nslot, 0);
@@ -1358,28 +1359,30 @@ void share_operators(FarField &dst, const FarField &src) {
     dst.ke = src.ke;
 }
 
-// F's digits: those of its operator set where this handle wants them (STKFMM_F64_I8=0 at its
-// set-up, or no sm_100: cuBLAS), whatever other handles of the set do
-int attach_i8_operators(FarField &F, cudaStream_t s) {
+// F's digits: those of its operator set that this handle's precision uses (farfield_evaluate: all
+// in FP64, of a mixed handle laplace_p's but the M2L's factors), none with STKFMM_F64_I8=0 at its
+// set-up or without sm_100, whatever other handles of the set do.  They take 0.1 GB (laplace_p, p = 8)
+// to several.
+int attach_i8_operators(FarField &F, int prec, cudaStream_t s) {
     F.i8 = F.i8_pq = false;
+    for (I8Buf FarField::*b : kI8Operators) (F.*b).release();
     const char *env = getenv("STKFMM_F64_I8");
-    if ((env && env[0] == '0') || !umma_available()) {
-        for (I8Buf FarField::*b : kI8Operators) (F.*b).release();
-        return STK_OK;
-    }
+    const bool pq = prec == PREC_FP64;
+    if ((env && env[0] == '0') || !umma_available() || !(pq || F.ke == 1)) return STK_OK;
     FarField &E = *F.ops_ref;
     std::lock_guard<std::mutex> lock(E.i8_mu);
     if (E.i8_built) FCUDA(cudaStreamWaitEvent(s, E.i8_built, 0));
-    if (!E.i8 || !E.i8_pq) {
-        const int rc = build_i8_operators(E, s);
+    if (!E.i8 || (pq && !E.i8_pq)) {
+        const int rc = build_i8_operators(E, pq, s);
         if (rc) return rc;
         if (!E.i8_built) FCUDA(cudaEventCreateWithFlags(&E.i8_built, cudaEventDisableTiming));
         FCUDA(cudaEventRecord(E.i8_built, s));
     }
     F.i8 = E.i8;
-    F.i8_pq = E.i8_pq;
+    F.i8_pq = pq && E.i8_pq;
     F.i8_q_blk = E.i8_q_blk;
-    for (I8Buf FarField::*b : kI8Operators) (F.*b).share(E.*b);
+    for (I8Buf FarField::*b : kI8Operators)
+        if (pq || (b != &FarField::i8_q && b != &FarField::i8_p)) (F.*b).share(E.*b);
     return STK_OK;
 }
 
@@ -1884,7 +1887,8 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
         F.tcc_ops = false;
         F.m2c_p = 0;  // the periodic operator follows the (possibly new) operators
     }
-    if ((rc = attach_i8_operators(F, s))) return rc;
+    F.fp64 = f->precision == PREC_FP64;
+    if ((rc = attach_i8_operators(F, f->precision, s))) return rc;
     F.periodic = f->pbc >= 1;
     const int far_field = f->enable_ff ? 1 : 0;
     if (F.periodic && (F.m2c_p != F.p || F.m2c_m2x != F.m2x || F.m2c_pbc != f->pbc || F.m2c_ff != far_field)) {
@@ -2251,7 +2255,7 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
         if (!rc) rc = setup_m2l_chunks_i8(F, chunk_slot, valid, nn, s);
         if (rc) return rc;
         F.m2l_seg.clear();
-        if (!F.tcc || !F.i8_chunks) {
+        if (!F.tcc || (F.fp64 && !F.i8_chunks)) {
             // Per group of columns and padded rank r: two batched GEMMs over that group's
             // chunks whose offset has rank r,
             //   Z_c = Q_d^T X_c (r x 256),  Y_c = P_d Z_c (k x 256).

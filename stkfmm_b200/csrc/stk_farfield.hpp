@@ -106,6 +106,7 @@ struct FarField {
     bool scaled = false;
     double pot_exp[4] = {0, 0, 0, 0}, den_exp[4] = {0, 0, 0, 0};
     bool ready = false;
+    bool fp64 = false;     // set up for FP64 evaluations (a mixed handle's set-up leaves their M2L out)
     cublasHandle_t blas = nullptr;
     cusolverDnHandle_t solver = nullptr;
     // level-independent operators (column-major, FP64)

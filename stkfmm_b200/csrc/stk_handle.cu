@@ -636,8 +636,12 @@ extern "C" int Stk3DFMM_get_ulist(Stk3DFMM *fmm, unsigned kernel, int *sizes, in
 // The KIFMM operators and per-tree far-field data are built at the first
 // evaluation after setupTree (the reference builds them in setupTree,
 // FMMData.cpp:107-167); evaluate_near never needs them.
+// A handle that was set up in mixed precision lacks the FP64 path's data: it is set up again at
+// its first FP64 evaluation, with the same lists, once the evaluations queued on it are through.
 static int ensure_far(Stk3DFMM *fmm, KernelData *kd) {
-    if (kd->far_ready) return STK_OK;
+    if (kd->far_ready && (fmm->precision != PREC_FP64 || kd->far->fp64)) return STK_OK;
+    if (kd->far_ready && cudaDeviceSynchronize() != cudaSuccess) return STK_ERR_CUDA;
+    kd->far_ready = false;
     const int rc = farfield_setup(fmm, kd);
     if (rc) return rc;
     kd->far_ready = true;

@@ -51,3 +51,42 @@ def test_every_handle_reads_the_switch(torch_cuda, monkeypatch, kernel, max_pts)
         out = np.zeros_like(res[0])
         handles[0].evaluate_fmm(kernel, slv, out, dlv)
         np.testing.assert_array_equal(out, res[want])
+
+
+def used_bytes(torch):
+    torch.cuda.synchronize()
+    free, total = torch.cuda.mem_get_info()
+    return total - free
+
+
+# Stokes' translations in mixed precision: no int8 products at all; LapPGrad: the M2L's factors stay out
+@pytest.mark.parametrize("kernel,extra", [(8, 0), (1, 64 << 20)])
+def test_mixed_handles_hold_no_digits_they_do_not_use(torch_cuda, monkeypatch, kernel, extra):
+    """Device memory of a handle's first mixed evaluation, with the int8 products on and off.  The
+    operators' digits are 7 bytes a value: m2m, l2l (N x 8N) and four of at most N x N, 20 N^2 values,
+    N = 296 for LapPGrad at p = 8 (12 MB), rounded up to blocks; the rest is the operand of a product."""
+    import gc
+    pts, slv, dlv, td = fmm_case(kernel, 6000, seed=110)
+    run_fmm(kernel, 8, 60, pts, slv, dlv, td, prec=1)  # libraries and kernels are loaded
+    used = {}
+    for mode in ("0", "1"):
+        monkeypatch.setenv("STKFMM_F64_I8", mode)
+        gc.collect()
+        before = used_bytes(torch_cuda)
+        f, _ = run_fmm(kernel, 8, 60, pts, slv, dlv, td, prec=1)
+        used[mode] = used_bytes(torch_cuda) - before
+        del f
+    assert used["1"] <= used["0"] + extra + (8 << 20), used
+
+
+@pytest.mark.parametrize("kernel,max_pts", [(1, 60), (8, 60), (128, 150)])
+def test_precision_switched_between_evaluations(torch_cuda, kernel, max_pts):
+    """One handle, mixed - FP64 - mixed - FP64: the bits of handles that were made in that precision."""
+    pts, slv, dlv, td = fmm_case(kernel, 6000, seed=120 + kernel)
+    f, _ = run_fmm(kernel, 8, max_pts, pts, slv, dlv, td, prec=1)
+    fresh = [run_fmm(kernel, 8, max_pts, pts, slv, dlv, td, prec=prec) for prec in (0, 1)]
+    for prec in (1, 0, 1, 0):
+        f.set_precision(prec)
+        out = np.zeros((len(pts), td))
+        f.evaluate_fmm(kernel, slv, out, dlv)
+        np.testing.assert_array_equal(out, fresh[prec][1])
