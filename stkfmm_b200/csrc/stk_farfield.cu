@@ -922,26 +922,24 @@ int build_m2l_lowrank(FarField &F, const std::vector<double> &unit, const double
 // was no memory.
 int build_i8_operators(FarField &F, bool pq, cudaStream_t s) {
     const int N = F.n * F.ke, k = F.m2l_rank;
-    // column-major M x K operators: row m's values are ld apart
-    auto op = [&](I8Buf &b, const DevBuf &src, int M, int K) -> int {
-        int rc = b.reserve(M, K);
-        if (!rc) rc = b.reserve_kscale(K);
-        if (rc) return rc;
-        FCUDA(i8_column_scales((const double *)src.ptr, M, M, K, b.up(), b.down(), s));
-        FCUDA(i8_digits_trans((const double *)src.ptr, M, M, K, b.nkb, b.down(), b.digits(), b.scales(), s));
-        return STK_OK;
-    };
-    int rc = STK_OK;
     if (!F.i8) {
-        rc = op(F.i8_uc2ue, F.uc2ue, N, N);
-        if (!rc) rc = op(F.i8_dc2de, F.dc2de, N, N);
-        if (!rc) rc = op(F.i8_m2m, F.m2m, N, 8 * N);
-        if (!rc) rc = op(F.i8_l2l, F.l2l, 8 * N, N);
-        if (!rc) rc = op(F.i8_vt, F.m2l_vt, k, N);
-        if (!rc) rc = op(F.i8_e, F.m2l_e, N, k);
-        if (rc) {  // no memory for them: the products stay with cuBLAS
-            for (I8Buf *b : {&F.i8_uc2ue, &F.i8_dc2de, &F.i8_m2m, &F.i8_l2l, &F.i8_vt, &F.i8_e}) b->release();
+        // column-major M x K operators: row m's values are M apart
+        struct Op {
+            I8Buf &b;
+            const DevBuf &src;
+            int M, K;
+        } ops[] = {{F.i8_uc2ue, F.uc2ue, N, N}, {F.i8_dc2de, F.dc2de, N, N}, {F.i8_m2m, F.m2m, N, 8 * N},
+                   {F.i8_l2l, F.l2l, 8 * N, N}, {F.i8_vt, F.m2l_vt, k, N},   {F.i8_e, F.m2l_e, N, k}};
+        bool room = true;
+        for (Op &o : ops) room = room && !o.b.reserve(o.M, o.K) && !o.b.reserve_kscale(o.K);
+        if (!room) {  // the products stay with cuBLAS
+            for (Op &o : ops) o.b.release();
             return STK_OK;
+        }
+        for (Op &o : ops) {
+            FCUDA(i8_column_scales((const double *)o.src.ptr, o.M, o.M, o.K, o.b.up(), o.b.down(), s));
+            FCUDA(i8_digits_trans((const double *)o.src.ptr, o.M, o.M, o.K, o.b.nkb, o.b.down(), o.b.digits(),
+                                  o.b.scales(), s));
         }
         F.i8 = true;
     }
@@ -959,7 +957,7 @@ int build_i8_operators(FarField &F, bool pq, cudaStream_t s) {
     if (bytes > (8ull << 30)) return STK_OK;
     // scales along K: of Q over all offsets (one set of k), of P_d per offset (rmax each)
     const int rmax = F.m2l_rmax;
-    rc = F.i8_q.reserve((long long)qb * kI8Rows, k);
+    int rc = F.i8_q.reserve((long long)qb * kI8Rows, k);
     if (!rc) rc = F.i8_p.reserve((long long)nslot * kb * kI8Rows, rmax);
     if (!rc) rc = F.i8_q.reserve_kscale(k);
     if (!rc) rc = F.i8_p.reserve_kscale(nslot * rmax);
@@ -1363,12 +1361,12 @@ void share_operators(FarField &dst, const FarField &src) {
 // in FP64, of a mixed handle laplace_p's but the M2L's factors), none with STKFMM_F64_I8=0 at its
 // set-up or without sm_100, whatever other handles of the set do.  They take 0.1 GB (laplace_p, p = 8)
 // to several.
-int attach_i8_operators(FarField &F, int prec, cudaStream_t s) {
+int attach_i8_operators(FarField &F, int prec, bool allowed, cudaStream_t s) {
     F.i8 = F.i8_pq = false;
     for (I8Buf FarField::*b : kI8Operators) (F.*b).release();
     const char *env = getenv("STKFMM_F64_I8");
     const bool pq = prec == PREC_FP64;
-    if ((env && env[0] == '0') || !umma_available() || !(pq || F.ke == 1)) return STK_OK;
+    if (!allowed || (env && env[0] == '0') || !umma_available() || !(pq || F.ke == 1)) return STK_OK;
     FarField &E = *F.ops_ref;
     std::lock_guard<std::mutex> lock(E.i8_mu);
     if (E.i8_built) FCUDA(cudaStreamWaitEvent(s, E.i8_built, 0));
@@ -1504,7 +1502,11 @@ static int setup_m2l_chunks_i8(FarField &F, const std::vector<int> &chunk_slot, 
     F.i8_x.nkb = i8_kblocks(k);
     F.i8_chunks = !(F.i8_z.reserve(gcols, rmax) || F.i8_x.dig.reserve(i8_row_bytes(nn, F.i8_x.nkb)) ||
                     F.i8_x.scale.reserve(sizeof(int) * (size_t)nn));
-    if (!F.i8_chunks) return STK_OK;
+    if (!F.i8_chunks) {
+        F.i8_x.release();
+        F.i8_z.release();
+        return STK_OK;
+    }
     int rc = F.i8_valid.upload(valid.data(), sizeof(int) * nc, s);
     if (!rc) rc = F.i8_rank.upload(rank.data(), sizeof(int) * nc, s);
     if (!rc) rc = F.i8_slot.upload(chunk_slot.data(), sizeof(int) * nc, s);
@@ -1650,6 +1652,8 @@ static int setup_m2l_dense(FarField &F, const Octree &T, int nslot, cudaStream_t
     F.dn_i8 = F.i8_pq && dig_bytes <= (16ull << 30) &&
               !(F.dn_q8.reserve((long long)std::max(qb, 1) * kI8Rows, k) || F.dn_p8.reserve(64LL * kb * kI8Rows, rcc_all) ||
                 F.dn_phi8.reserve(nmax, k) || F.dn_zc8.reserve(nmax, rcc_all));
+    if (!F.dn_i8)
+        for (I8Buf *b : {&F.dn_q8, &F.dn_p8, &F.dn_phi8, &F.dn_zc8}) b->release();
     // tensor-core operands of the mixed path (3xTF32 hi / lo, K-major rows of a multiple
     // of 4 floats): Qs_c'^T per source type and Pv_{c,c'}^T per block, within 4 GiB
     F.tc = false;
@@ -1828,7 +1832,7 @@ static int setup_m2l_dense(FarField &F, const Octree &T, int nslot, cudaStream_t
     return STK_OK;
 }
 
-int farfield_setup(Stk3DFMM *f, KernelData *kd) {
+static int setup_far(Stk3DFMM *f, KernelData *kd, bool i8) {
     const KernelInfo *ki = kd->info;
     // free space, or periodic in x (PX), x and y (PXY) or all axes (PXYZ): the far
     // images through the root's M2C operator
@@ -1888,7 +1892,7 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
         F.m2c_p = 0;  // the periodic operator follows the (possibly new) operators
     }
     F.fp64 = f->precision == PREC_FP64;
-    if ((rc = attach_i8_operators(F, f->precision, s))) return rc;
+    if ((rc = attach_i8_operators(F, f->precision, i8, s))) return rc;
     F.periodic = f->pbc >= 1;
     const int far_field = f->enable_ff ? 1 : 0;
     if (F.periodic && (F.m2c_p != F.p || F.m2c_m2x != F.m2x || F.m2c_pbc != f->pbc || F.m2c_ff != far_field)) {
@@ -2332,9 +2336,39 @@ int farfield_setup(Stk3DFMM *f, KernelData *kd) {
         if (!rc) rc = F.tmp1.reserve(sizeof(double) * (size_t)std::max(maxm, 1) * N);
         if (rc) return rc;
     }
+    // the evaluation's records
+    for (int k = 0; k < 2; k++) {
+        int rs = 0;
+        for (const ListPass *P : {&F.s2m[k], &F.s2l[k]})
+            if (P->uk >= 0) rs = std::max(rs, uk_record_stride(P->uk));
+        if (rs) rc = F.rec_pts[k].reserve(sizeof(double) * (size_t)std::max(T.sets[k].n, 1) * rs);
+        if (rc) return rc;
+    }
+    rc = F.rec_surf.reserve(sizeof(double) * (size_t)nn * n *
+                            std::max(uk_record_stride(F.l2t.uk), F.m2t.n_items ? uk_record_stride(F.m2t.uk) : 0));
+    if (rc) return rc;
     FCUDA(cudaStreamSynchronize(s));
     F.ready = true;
     return STK_OK;
+}
+
+// The digits of the int8 products are taken where there is room: a set-up that fails with them is
+// tried once more without.
+int farfield_setup(Stk3DFMM *f, KernelData *kd) {
+    const int rc = setup_far(f, kd, true);
+    if (rc != STK_ERR_CUDA || !kd->far->i8) return rc;
+    FarField &F = *kd->far;
+    cudaGetLastError();
+    for (I8Buf *b : {&F.i8_b, &F.i8_x, &F.i8_z, &F.dn_q8, &F.dn_p8, &F.dn_phi8, &F.dn_zc8}) b->release();
+    F.i8_parts.release();
+    for (I8Buf FarField::*b : kI8Operators) (F.*b).release();
+    {
+        FarField &E = *F.ops_ref;
+        std::lock_guard<std::mutex> lock(E.i8_mu);
+        E.i8 = E.i8_pq = false;
+        for (I8Buf FarField::*b : kI8Operators) (E.*b).release();
+    }
+    return setup_far(f, kd, false);
 }
 
 // The mixed path's dense M2L of one complete level on the tensor cores

@@ -90,3 +90,35 @@ def test_precision_switched_between_evaluations(torch_cuda, kernel, max_pts):
         out = np.zeros((len(pts), td))
         f.evaluate_fmm(kernel, slv, out, dlv)
         np.testing.assert_array_equal(out, fresh[prec][1])
+
+
+# all digits but few, the operators' but not the factors', and somewhat more
+@pytest.mark.parametrize("slack_mb", [40, 130, 250])
+def test_set_up_where_the_digits_leave_no_room(torch_cuda, monkeypatch, slack_mb):
+    """With the device memory that a handle needs without digits, and some of what they would take, a
+    handle is set up and gives the sums: what runs without the int8 products runs with them on.  Their
+    difference from cuBLAS is below the noise of such an FMM, 1e-9 (its error at p = 8 is 1e-6)."""
+    import gc
+    torch = torch_cuda
+    pts, slv, _, td = fmm_case(8, 6000, seed=130)
+    monkeypatch.setenv("STKFMM_F64_I8", "0")
+    keep, ref = run_fmm(8, 8, 60, pts, slv, None, td)  # the operators stay
+    gc.collect()
+    torch.cuda.empty_cache()
+    before = used_bytes(torch)
+    f, _ = run_fmm(8, 8, 60, pts, slv, None, td)
+    need = used_bytes(torch) - before
+    del f
+    gc.collect()
+    monkeypatch.setenv("STKFMM_F64_I8", "1")
+    hog = torch.empty(torch.cuda.mem_get_info()[0] - need - (slack_mb << 20), dtype=torch.uint8, device="cuda")
+    try:
+        f, out = run_fmm(8, 8, 60, pts, slv, None, td)
+        assert rel_l2(out, ref) < 1e-9
+        del f
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    # with room again the digits are made
+    f, out = run_fmm(8, 8, 60, pts, slv, None, td)
+    assert (out != ref).any() and rel_l2(out, ref) < 1e-9
