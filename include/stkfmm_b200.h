@@ -337,7 +337,11 @@ int Stk3DFMM_evaluate_near_device(Stk3DFMM *fmm, unsigned kernel, const double *
 /* evaluate_fmm on device buffers in the caller's order (values as given, unit
  * box only: STK_ERR_NOT_SUPPORTED otherwise), queued on `stream` without a host
  * synchronisation: d_trg_value += near field + KIFMM far field.  The first call
- * after setup_tree builds the far-field operators and synchronises. */
+ * after setup_tree builds the far-field operators and synchronises.  The far
+ * field's tensor-core kernels bound their waits; one that gave up (a fault of the
+ * device or of this library) leaves results unwritten and an error code, which
+ * evaluate_fmm returns by itself and Stk3DFMM_last_kernel_ms after device
+ * evaluations: STK_ERR_CUDA, once.  setup_tree's next evaluation clears it. */
 int Stk3DFMM_evaluate_fmm_device(Stk3DFMM *fmm, unsigned kernel, const double *d_src_SL_value, double *d_trg_value,
                                  const double *d_src_DL_value, void *stream);
 /* Device time (ms, CUDA events on the launching stream) of the kernel launches
@@ -404,7 +408,8 @@ int StkWallFMM_show_active_kernels(StkWallFMM *fmm);
  * sub-FMM (the Laplace sub-FMMs, whose terms cancel near the sources, stay FP64); the
  * evaluation on device buffers in the caller's order queued on `stream` (null: the
  * handle's stream; the first call after setup_tree builds the sub-FMMs' far-field
- * operators and synchronises); device time (ms) of the last evaluation */
+ * operators and synchronises); device time (ms) of the last evaluation, or
+ * STK_ERR_CUDA as from Stk3DFMM_last_kernel_ms */
 int StkWallFMM_set_precision(StkWallFMM *fmm, int precision);
 /* Stk3DFMM_set_far_field for every sub-FMM (the reference's StkWallFMM enableFF,
  * STKFMM.hpp:233-234); takes effect at the next setup_tree */

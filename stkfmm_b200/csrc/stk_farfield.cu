@@ -1919,12 +1919,11 @@ static int setup_far(Stk3DFMM *f, KernelData *kd, bool i8) {
     }
     const Octree &T = kd->tree;
     const int nn = T.num_nodes(), n = F.n, N = n * ke;
-    // set by a tensor-core product whose pipeline wait gave up
-    if (!F.tc_err.ptr) {
-        rc = F.tc_err.reserve(sizeof(int) * 4);
-        if (rc) return rc;
-        FCUDA(cudaMemsetAsync(F.tc_err.ptr, 0, sizeof(int) * 4, s));
-    }
+    // set by a tensor-core product whose pipeline wait gave up; a code that was left by an
+    // evaluation on the tree before is not this one's
+    rc = F.tc_err.reserve(sizeof(int) * 4);
+    if (rc) return rc;
+    FCUDA(cudaMemsetAsync(F.tc_err.ptr, 0, sizeof(int) * 4, s));
     std::vector<double> unit = unit_surface(p);
     rc = upload_points(F.unit_surf, unit, s);
     // node levels and centres on the device

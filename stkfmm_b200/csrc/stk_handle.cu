@@ -353,6 +353,27 @@ extern "C" int Stk3DFMM_set_precision(Stk3DFMM *fmm, int precision) {
     return STK_OK;
 }
 
+int stk::handle_status(Stk3DFMM *f) {
+    int rc = STK_OK;
+    for (auto &kv : f->pool)
+        if (kv.second->last_far) {
+            const int r = farfield_status(kv.second.get());
+            if (r) rc = r;
+        }
+    return rc;
+}
+
+// Test hook (not in the header): leaves the code that a tensor-core product leaves when a pipeline
+// wait gives up, for the evaluations of `kernel` queued so far.
+extern "C" int stk_test_post_wait_error(Stk3DFMM *fmm, unsigned kernel) {
+    auto it = fmm->pool.find(kernel);
+    if (it == fmm->pool.end() || !it->second->far || !it->second->far->tc_err.ptr) return STK_ERR_STATE;
+    const int code = 1;
+    HCUDA(cudaDeviceSynchronize());
+    HCUDA(cudaMemcpy(it->second->far->tc_err.ptr, &code, sizeof(int), cudaMemcpyHostToDevice));
+    return STK_OK;
+}
+
 // Near-field (and with far = true, the KIFMM far-field) evaluation on device
 // buffers in the caller's order.  d_sl / d_dl hold values already scaled
 // (scaleSrc); d_out_user receives trg += sF^k * result (scaleTrg) in the

@@ -121,4 +121,7 @@ namespace stk {
 // callers upload the target array there, overlapping the kernels.
 int near_device(Stk3DFMM *f, KernelData *kd, const double *d_sl, const double *d_dl, double *d_out_user,
                 cudaStream_t s, bool far, const std::function<int()> &before_scatter = nullptr);
+// farfield_status of every kernel of a handle whose last evaluation had a far field (after the
+// evaluations have completed)
+int handle_status(Stk3DFMM *f);
 }

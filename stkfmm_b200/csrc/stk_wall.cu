@@ -202,6 +202,8 @@ struct StkWallFMM {
     }
 };
 
+extern "C" int stk_test_post_wait_error(Stk3DFMM *fmm, unsigned kernel);
+
 static int family_of(unsigned kernel) {
     return kernel == STK_Stokes ? 0 : kernel == STK_RPY ? 1 : -1;
 }
@@ -418,6 +420,17 @@ static int run_subs(StkWallFMM *w, int f, const double *const *sv, const double 
     return rc;
 }
 
+// After the evaluation has completed: STK_ERR_CUDA when a tensor-core product of a sub-FMM gave up at
+// a pipeline wait.
+static int subs_status(StkWallFMM *w, int f) {
+    int rc = STK_OK;
+    for (Stk3DFMM *h : w->sub[f]) {
+        const int r = h ? handle_status(h) : STK_OK;
+        if (r) rc = r;
+    }
+    return rc;
+}
+
 // The wall evaluation on device buffers: d_trg_value (caller's order, kdimTrg per
 // target) += wall FMM of d_src_SL_value (caller's order, kdimSL per source).
 static int wall_eval(StkWallFMM *w, int f, const double *d_sl, double *d_out, cudaStream_t s) {
@@ -513,7 +526,14 @@ extern "C" int StkWallFMM_evaluate_fmm(StkWallFMM *fmm, unsigned kernel, const i
     if (rc) return rc;
     if (nout) WCUDA(cudaMemcpyAsync(trg_value, fmm->d_out.ptr, nout * sizeof(double), cudaMemcpyDeviceToHost, s));
     WCUDA(cudaStreamSynchronize(s));
-    return STK_OK;
+    return subs_status(fmm, f);
+}
+
+// Test hook (not in the header): stk_test_post_wait_error of sub-FMM `sub`
+extern "C" int stk_test_post_wall_wait_error(StkWallFMM *fmm, unsigned kernel, int sub) {
+    const int f = family_of(kernel);
+    if (f < 0 || sub < 0 || sub >= kSubs || !fmm->sub[f][sub]) return STK_ERR_INVALID_ARG;
+    return stk_test_post_wait_error(fmm->sub[f][sub], kSubKernel[f][sub]);
 }
 
 // this library's kernels launched by the last evaluation: the sub-FMMs' plus staging and assembly
@@ -541,5 +561,6 @@ extern "C" int StkWallFMM_last_kernel_ms(StkWallFMM *fmm, float *ms) {
         cudaGetLastError();
         return STK_ERR_CUDA;
     }
-    return STK_OK;
+    const int a = subs_status(fmm, 0), b = subs_status(fmm, 1);
+    return a ? a : b;
 }

@@ -1,5 +1,7 @@
 """GPU: the FP64 far field on the int8 tensor cores in whole FMMs: strengths at the ends of the double
 range, and the switch between them and cuBLAS."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -122,3 +124,54 @@ def test_set_up_where_the_digits_leave_no_room(torch_cuda, monkeypatch, slack_mb
     # with room again the digits are made
     f, out = run_fmm(8, 8, 60, pts, slv, None, td)
     assert (out != ref).any() and rel_l2(out, ref) < 1e-9
+
+
+def test_a_given_up_wait_is_an_error(torch_cuda):
+    """The code that a tensor-core kernel leaves when a pipeline wait gives up, put there by a hook: the
+    next call that looks (a host evaluation, last_kernel_ms) fails once, of the wall for every sub-FMM;
+    set_up of a new tree clears it."""
+    import stkfmm_b200 as S
+    from stkfmm_b200 import lib
+    from stkfmm_b200._lib import StkError
+    L = lib()
+    post, post_wall = L.stk_test_post_wait_error, L.stk_test_post_wall_wait_error
+    post.argtypes = [ctypes.c_void_p, ctypes.c_uint]
+    post_wall.argtypes = [ctypes.c_void_p, ctypes.c_uint, ctypes.c_int]
+    pts, slv, _, td = fmm_case(8, 4000, seed=140)
+    f, ref = run_fmm(8, 6, 60, pts, slv, None, td)
+
+    def again():
+        out = np.zeros_like(ref)
+        f.evaluate_fmm(8, slv, out, None)
+        return out
+
+    for look in (again, lambda: f.last_kernel_ms(8)):
+        assert post(f.fmm, 8) == 0
+        with pytest.raises(StkError):
+            look()
+        look()
+    assert post(f.fmm, 8) == 0
+    f.setup_tree(8)
+    np.testing.assert_array_equal(again(), ref)
+
+    for kernel, nsub in ((8, 3), (16, 4)):
+        pw = pts * [1, 1, 0.45] + [0, 0, 0.01]
+        vw = np.concatenate([slv[:, :3], np.full((len(pw), 1), 1e-4)], axis=1)[:, :3 if kernel == 8 else 4]
+        w = S.StkWallFMM(6, 60, 0, kernel)
+        w.set_box(np.zeros(3), 1.0)
+        w.set_points(pw, pw, None)
+        w.setup_tree(kernel)
+
+        def wall():
+            out = np.zeros((len(pw), 3 if kernel == 8 else 6))
+            w.evaluate_fmm(kernel, vw, out)
+            return out
+
+        ref_w = wall()
+        for look in (wall, w.last_kernel_ms):
+            for sub in range(nsub):
+                assert post_wall(w.fmm, kernel, sub) == 0
+                with pytest.raises(StkError):
+                    look()
+                look()
+        np.testing.assert_array_equal(wall(), ref_w)
