@@ -73,9 +73,15 @@ template <class K> struct NtvOf<K, std::void_t<decltype(K::NTV)>> {
 
 template <int UK> struct Rec {
     static constexpr int SDIM = Uk<UK>::SDIM;
-    static constexpr int RS = (3 + Uk<UK>::NV + 1) & ~1;  // doubles per global record (16-byte multiple)
-    // landing slot: a record, or a direct sum's raw values before they are staged in place
-    static constexpr int SLOT = (3 + (SDIM > Uk<UK>::NV ? SDIM : Uk<UK>::NV) + 1) & ~1;
+    // doubles (16-byte multiples) of a record with the source's values, and with its staged values
+    static constexpr int RAW = (3 + SDIM + 1) & ~1, STAGED = (3 + Uk<UK>::NV + 1) & ~1;
+    // Records carry staged values unless that makes them larger (laplace_pgrad, the Hessian and
+    // gradient kernels); those, and a direct sum's sources, are staged in every tile that reads
+    // them (262k points, lists of 1728 sources, mixed: laplace_dipolepgradgrad 10 doubles staged
+    // 1032 us, 6 raw 970; stokes_pvellaplacian 10 857, 8 814; FP64 the same to 1%).
+    static constexpr bool kStaged = STAGED <= RAW;
+    static constexpr int RS = kStaged ? STAGED : RAW;  // doubles per record
+    static constexpr int SLOT = STAGED > RAW ? STAGED : RAW;  // landing slot of values staged in place
 };
 
 // Resident CTAs per SM requested from the register allocator (1: no
@@ -191,7 +197,8 @@ __global__ void __launch_bounds__(Cta<MIXED>::threads, MinBlocks<UK, MIXED>::val
     constexpr int TV = K::TV;  // per-output-point values (adjoint kernels)
     constexpr int NTV = NtvOf<K>::value;
     constexpr int RS = Rec<UK>::RS;
-    constexpr int RSS = RawStride<DIRECT ? Rec<UK>::SLOT : RS>::value;
+    constexpr bool STAGE = DIRECT || !Rec<UK>::kStaged;  // values are staged here
+    constexpr int RSS = RawStride<STAGE ? Rec<UK>::SLOT : RS>::value;
     constexpr int TPL = TargetsPerLane<K>::value;
     constexpr bool HILO = MIXED && kMixedDisp == kDispHiLo;
     // shared tile, one row per component: coordinates (FP64, or FP32 hi x3 + lo x3)
@@ -347,10 +354,15 @@ __global__ void __launch_bounds__(Cta<MIXED>::threads, MinBlocks<UK, MIXED>::val
                 code = ent & 31;
                 sbeg = a.src_box_begin[sb];
                 sz = a.src_box_end[sb] - sbeg;
-                if (ec + lane == w.e1 - 1) sz = min(sz, w.stop);
-                if (ec + lane == w.e0) {
-                    sbeg += w.skip;
-                    sz -= w.skip;
+                // mixed items hold whole entries; looking for parts of them cost 4 registers, and
+                // the adjoint and dipole kernels a CTA per SM (262k points: regvel_adjoint_trg 777 ->
+                // 824 us)
+                if constexpr (!MIXED) {
+                    if (ec + lane == w.e1 - 1) sz = min(sz, w.stop);
+                    if (ec + lane == w.e0) {
+                        sbeg += w.skip;
+                        sz -= w.skip;
+                    }
                 }
                 // bit 5: the segment may hold a source at a target's position (always,
                 // unless the lists guarantee coincidence only in the unshifted own box)
@@ -414,14 +426,15 @@ __global__ void __launch_bounds__(Cta<MIXED>::threads, MinBlocks<UK, MIXED>::val
                     cp_async_wait_group<0>();
                     if (lane < n) {  // fix up this lane's own record in place
                         double *raw = traw[wid][zone][lane];
-                        if constexpr (DIRECT) {
+                        if constexpr (STAGE) {
                             double f[K::SDIM], v[NV];
 #pragma unroll
                             for (int q = 0; q < K::SDIM; q++) f[q] = raw[3 + q];
                             K::stage(f, v);
 #pragma unroll
                             for (int q = 0; q < NV; q++) raw[3 + q] = v[q];
-                        } else {
+                        }
+                        if constexpr (!DIRECT) {
                             const int cd = s_code[zseg[0]] & 31;
                             if (cd != kShiftNoneCode) {  // periodic image
                                 raw[0] += (cd % 3 - 1) * a.period;
@@ -435,9 +448,10 @@ __global__ void __launch_bounds__(Cta<MIXED>::threads, MinBlocks<UK, MIXED>::val
                     const double(*tile)[RSS] = traw[wid][zone];
 STK_UNROLL(STK_P2P_UNROLL_FP64)
                     for (int j = sub; j < n; j += g) {
-                        double rn[RS];
+                        constexpr int RN = Rec<UK>::STAGED;
+                        double rn[RN];
 #pragma unroll
-                        for (int q = 0; q < RS / 2; q++) {
+                        for (int q = 0; q < RN / 2; q++) {
                             const double2 t2 = *reinterpret_cast<const double2 *>(&tile[j][2 * q]);
                             rn[2 * q] = t2.x;
                             rn[2 * q + 1] = t2.y;
@@ -465,7 +479,7 @@ STK_UNROLL(STK_P2P_UNROLL_FP64)
                     double x[3];
                     if (lane < n) {
                         const double *raw = traw[wid][zone][lane];
-                        constexpr int RR = DIRECT ? Rec<UK>::SLOT : RS;
+                        constexpr int RR = STAGE ? Rec<UK>::RAW : RS;
                         double rn[RR];
 #pragma unroll
                         for (int q = 0; q < RR / 2; q++) {
@@ -488,7 +502,7 @@ STK_UNROLL(STK_P2P_UNROLL_FP64)
                                 x[2] += (cd / 9 - 1) * a.period;
                             }
                         }
-                        if constexpr (DIRECT) {
+                        if constexpr (STAGE) {
                             K::stage(rn + 3, v);
                         } else {
 #pragma unroll
@@ -611,16 +625,19 @@ STK_UNROLL(STK_P2P_UNROLL_MIXED)
                 if constexpr (DIRECT) {
                     store = a.atomic_out == 0;
                     if (a.parts) dst = a.parts + ((size_t)w.e0 * a.ntrg + tt[h]) * TDIM;
-                } else if (w.part >= 0) {
-                    store = true;
-                    dst = a.parts + (size_t)(w.part + tt[h] - w.t0) * TDIM;
+                } else if constexpr (!MIXED) {
+                    if (w.part >= 0) {
+                        store = true;
+                        dst = a.parts + (size_t)(w.part + tt[h] - w.t0) * TDIM;
+                    }
                 }
 #pragma unroll
                 for (int k = 0; k < TDIM; k++) {
                     const double val = K::SCALE * K::comp_scale(k) * o[h][k];
                     if (store)
                         dst[k] = val;
-                    else if (a.atomic_out == 2)
+                    else if (DIRECT && a.atomic_out == 2)  // (in lists, unused, it cost kernels of 7 to 16
+                                                           // components 2 to 3%)
                         atomicAdd(dst + k, val);
                     else
                         dst[k] += val;
@@ -725,7 +742,23 @@ __global__ void sum_chunks_kernel(const double *__restrict__ parts, int n_chunk,
     }
 }
 
-// One thread per source: its values staged once here instead of in every tile that reads it.
+// a record's values from its source's: staged or as they are, zeros behind
+template <int UK> __device__ __forceinline__ void record_values(const double (&f)[Uk<UK>::SDIM], double (&r)[Rec<UK>::RS]) {
+    using K = Uk<UK>;
+    constexpr int n = Rec<UK>::kStaged ? K::NV : K::SDIM;
+    double v[n];
+    if constexpr (Rec<UK>::kStaged) {
+        K::stage(f, v);
+    } else {
+#pragma unroll
+        for (int k = 0; k < n; k++) v[k] = f[k];
+    }
+#pragma unroll
+    for (int k = 3; k < Rec<UK>::RS; k++) r[k] = k - 3 < n ? v[k - 3 < n ? k - 3 : 0] : 0.0;
+}
+
+// One thread per source: its values staged once here instead of in every tile that reads it
+// (Rec<>::kStaged).
 template <int UK>
 __global__ void pack_records_kernel(int n, const int *__restrict__ perm, const double *__restrict__ xyz,
                                     const double *__restrict__ v1, int d1, const double *__restrict__ v2,
@@ -734,15 +767,13 @@ __global__ void pack_records_kernel(int n, const int *__restrict__ perm, const d
     constexpr int RS = Rec<UK>::RS;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int p = perm ? perm[i] : i;
-        double f[K::SDIM], r[RS], v[K::NV];
+        double f[K::SDIM], r[RS];
 #pragma unroll
         for (int k = 0; k < K::SDIM; k++)
             f[k] = k < d1 ? v1[(size_t)p * d1 + k] : v2[(size_t)p * (K::SDIM - d1) + k - d1];
-        K::stage(f, v);
+        record_values<UK>(f, r);
 #pragma unroll
         for (int k = 0; k < 3; k++) r[k] = xyz[3 * (size_t)i + k];
-#pragma unroll
-        for (int k = 3; k < RS; k++) r[k] = k - 3 < K::NV ? v[k - 3 < K::NV ? k - 3 : 0] : 0.0;
         double2 *o = reinterpret_cast<double2 *>(rec + (size_t)i * RS);
 #pragma unroll
         for (int k = 0; k < RS / 2; k++) o[k] = make_double2(r[2 * k], r[2 * k + 1]);
@@ -764,7 +795,7 @@ __global__ void pack_surface_kernel(const int *__restrict__ nodes, int m, int n,
          idx += (long long)gridDim.x * blockDim.x) {
         const int i = (int)(idx / n), j = (int)(idx - (long long)i * n), b = nodes[i];
         const size_t p = (size_t)b * n + j;
-        double f[K::SDIM], r[RS], v[K::NV];
+        double f[K::SDIM], r[RS];
 #pragma unroll
         for (int k = 0; k < K::SDIM; k++) f[k] = dens[p * K::SDIM + k];
         if (level) {
@@ -772,11 +803,9 @@ __global__ void pack_surface_kernel(const int *__restrict__ nodes, int m, int n,
             for (int k = 0; k < K::SDIM; k++)
                 if (e.v[k & 3] != 0.0) f[k] *= exp2(-(double)level[b] * e.v[k & 3]);
         }
-        K::stage(f, v);
+        record_values<UK>(f, r);
 #pragma unroll
         for (int k = 0; k < 3; k++) r[k] = xyz[3 * p + k];
-#pragma unroll
-        for (int k = 3; k < RS; k++) r[k] = k - 3 < K::NV ? v[k - 3 < K::NV ? k - 3 : 0] : 0.0;
         double2 *o = reinterpret_cast<double2 *>(rec + p * RS);
 #pragma unroll
         for (int k = 0; k < RS / 2; k++) o[k] = make_double2(r[2 * k], r[2 * k + 1]);
@@ -813,7 +842,7 @@ int uk_record_stride(int uk) {
 cudaError_t launch_list_p2p(int uk, int prec, const ListP2PArgs &a, int num_sms, cudaStream_t stream) {
     if (a.n_items <= 0) return cudaSuccess;
     if (uk >= 0 && uk < UK_COUNT && uk_tvdim(uk) > 0 && !a.trg_aux) return cudaErrorInvalidValue;
-    if (a.n_groups > 0 && (!a.groups || !a.parts)) return cudaErrorInvalidValue;
+    if (a.atomic_out != 0 || (a.n_groups > 0 && (!a.groups || !a.parts))) return cudaErrorInvalidValue;
     const cudaError_t e = with_uk(uk, [&](auto id) {
         constexpr int UK = decltype(id)::value;
         return prec == PREC_MIXED ? launch_impl<UK, true, false>(a, num_sms, stream)

@@ -33,7 +33,7 @@ struct PartGroup {
 
 // Device-resident description of one list evaluation.
 struct ListP2PArgs {
-    const double *src_rec;     // source records, RS doubles each: x, y, z, staged values..., padding
+    const double *src_rec;     // source records (launch_pack_records), uk_record_stride doubles each
     const int *src_box_begin;  // per source box: first record
     const int *src_box_end;    // per source box: one past the last record
     const int *list_ent;       // per entry: (source box << 5) | periodic shift code (0..26, 13 = none)
@@ -44,7 +44,7 @@ struct ListP2PArgs {
     double *trg_out;           // outputs, TDIM doubles each, accumulated
     const double *box_centre;  // per target box: local origin for the mixed path (3 doubles)
     double period;             // periodic image length (1 for the unit box)
-    int atomic_out;            // 1 when several items may write the same target
+    int atomic_out;            // direct sums only: 0 trg_out or parts =, 1 +=, 2 += by atomics (lists: 0, +=)
     const double *trg_aux;     // per-target values (TV doubles each) of the adjoint kernels, else null
     int coincident_own_box;    // 1: a source can sit at a target's position only in an unshifted
                                // entry of the target's own box (lists of one octree over both
@@ -59,8 +59,8 @@ struct ListP2PArgs {
     double *parts;           // outputs of each chunk, ntrg x TDIM each (null: one chunk)
 };
 
-// Record stride (doubles) for a micro-kernel: 3 coordinates + NV staged values,
-// rounded up to a 16-byte multiple.
+// Record stride (doubles) for a micro-kernel: 3 coordinates + its staged values (or the
+// source's SDIM, where those are fewer), rounded up to a 16-byte multiple; never above that of SDIM.
 int uk_record_stride(int uk);
 int uk_sdim_host(int uk);
 int uk_tdim_host(int uk);
@@ -79,8 +79,9 @@ void direct_chunks(int uk, int prec, int ntrg, int nsrc, int num_sms, int &chunk
 // trg_out; add = 0: trg_out = sum, 1: +=, 2: += by atomics, without parts
 cudaError_t launch_direct_p2p(int uk, int prec, const ListP2PArgs &a, int add, int num_sms, cudaStream_t stream);
 
-// Source records of micro-kernel uk: rec[i] = (xyz[i], stage(v1[perm[i]] (d1 values),
-// v2[perm[i]] (the rest of SDIM)), 0 padding); perm may be null (identity), v2 null.
+// Source records of micro-kernel uk: rec[i] = (xyz[i], values, 0 padding), values = those of v1[perm[i]]
+// (d1) and v2[perm[i]] (the rest of SDIM), staged where that makes no larger record; perm may be
+// null (identity), v2 null.
 cudaError_t launch_pack_records(int uk, int n, const int *perm, const double *xyz, const double *v1, int d1,
                                 const double *v2, double *rec, cudaStream_t stream);
 
