@@ -243,10 +243,13 @@ int stk_gemm_f64_i8(int M, int N, int K, const double *d_A, int lda, const doubl
  * (on the current device); *status gets STK_OK or the error, NULL is returned on
  * error.  stk_p2p_plan_execute queues one micro-kernel over the plan's list on
  * `stream` and returns without a host wait; outputs accumulate.  The plan's
- * scratch (the packed source records and the work counter) is shared by its
- * executions: executions of one plan must be ordered (one stream, or the caller
- * synchronises between streams).  The first execution with a larger record
- * stride allocates (and synchronises the device).  d_trg_aux: per-target values
+ * scratch (the packed source records, the sums of split items and the work
+ * counter) is shared by its executions: executions of one plan must be ordered
+ * (one stream, or the caller synchronises between streams).  It is allocated at
+ * creation for records of up to 8 doubles and 8 components; the first execution
+ * with a larger record stride (micro-kernels of 6 values and more) allocates and
+ * synchronises the device, and the first FP64 one of more than 8 components
+ * allocates.  d_trg_aux: per-target values
  * of the adjoint micro-kernels (stk_ukernel_aux_dim), else NULL.
  * stk_p2p_plan_destroy waits for the device before freeing. */
 typedef struct stk_p2p_plan stk_p2p_plan;

@@ -17,6 +17,7 @@
 
 #include "../../include/stkfmm_b200.h"
 #include "stk_p2p.cuh"
+#include "stk_tree.hpp"
 #include "stk_ukernels.cuh"
 #include "stk_work.hpp"
 
@@ -37,6 +38,7 @@ struct stk_p2p_plan {
     unsigned int *d_counter = nullptr;
     double *d_rec = nullptr;  // packed source records, grown to the largest record stride used (at least 8)
     size_t rec_cap = 0;       // doubles
+    size_t parts_bytes(int wide) const { return (size_t)part_targets * (wide ? 16 : 8) * sizeof(double); }
     ~stk_p2p_plan() {
         cudaFree(d_sbeg);
         cudaFree(d_send);
@@ -109,22 +111,44 @@ extern "C" stk_p2p_plan *stk_p2p_plan_create(int n_trg_box, const int *trg_begin
     p->period = period;
     const int nent = n_trg_box > 0 ? list_off[n_trg_box] : 0;
     bool ok = cudaGetDevice(&p->device) == cudaSuccess &&
-              cudaDeviceGetAttribute(&p->num_sms, cudaDevAttrMultiProcessorCount, p->device) == cudaSuccess &&
-              cudaMalloc(&p->d_counter, 64) == cudaSuccess && upload(&p->d_sbeg, src_begin, n_src_box) == cudaSuccess &&
-              upload(&p->d_send, src_end, n_src_box) == cudaSuccess && upload(&p->d_ent, list_ent, nent) == cudaSuccess;
-    if (ok && n_trg_box > 0) {
-        std::vector<stk::WorkItem> items;
-        std::vector<stk::PartGroup> groups;
-        stk::build_list_items(n_trg_box, trg_begin, trg_end, list_off, list_ent, src_begin, src_end, items, p->pairs);
-        p->n_items[1] = (int)items.size();
-        ok = upload(&p->d_items[1], items.data(), items.size()) == cudaSuccess;
-        stk::build_split_items(n_trg_box, trg_begin, trg_end, list_off, list_ent, src_begin, src_end, p->num_sms * 15,
-                               items, groups, p->part_targets);
-        p->n_items[0] = (int)items.size();
-        p->n_groups = (int)groups.size();
-        ok = ok && upload(&p->d_items[0], items.data(), items.size()) == cudaSuccess &&
-             upload(&p->d_groups, groups.data(), groups.size()) == cudaSuccess;
+              cudaDeviceGetAttribute(&p->num_sms, cudaDevAttrMultiProcessorCount, p->device) == cudaSuccess;
+    // The two item lists on host threads of their own, and meanwhile, on this one, the device's
+    // arrays and the records of most executions (eight doubles a source).  One after the other the
+    // lists alone took 2.6 ms for 262k points, and buffers that the first execution allocated made it
+    // wait: creation and first FP64 pass 4.3 ms, 2.8 before there were two lists.
+    std::vector<stk::WorkItem> items[2];
+    std::vector<stk::PartGroup> groups;
+    const size_t records = (size_t)std::max(nsrc, 1) * 8;
+    bool host_ok = true;
+    try {
+        stk::parallel_ranges(ok ? 3 : 0, 1, [&](size_t i0, size_t i1) {
+            for (size_t i = i0; i < i1; i++) {
+                if (i == 0) {
+                    ok = cudaMalloc(&p->d_counter, 64) == cudaSuccess && upload(&p->d_sbeg, src_begin, n_src_box) == cudaSuccess &&
+                         upload(&p->d_send, src_end, n_src_box) == cudaSuccess && upload(&p->d_ent, list_ent, nent) == cudaSuccess;
+                    if (ok && nent > 0 && cudaMalloc(&p->d_rec, records * sizeof(double)) == cudaSuccess) p->rec_cap = records;
+                } else if (n_trg_box > 0 && i == 1) {
+                    stk::build_list_items(n_trg_box, trg_begin, trg_end, list_off, list_ent, src_begin, src_end, items[1],
+                                          p->pairs);
+                } else if (n_trg_box > 0) {
+                    stk::build_split_items(n_trg_box, trg_begin, trg_end, list_off, list_ent, src_begin, src_end,
+                                           p->num_sms * 15, items[0], groups, p->part_targets);
+                }
+            }
+        });
+    } catch (...) {  // host memory
+        host_ok = false;
     }
+    ok = ok && host_ok;
+    p->n_items[0] = (int)items[0].size();
+    p->n_items[1] = (int)items[1].size();
+    p->n_groups = (int)groups.size();
+    ok = ok && upload(&p->d_items[0], items[0].data(), items[0].size()) == cudaSuccess &&
+         upload(&p->d_items[1], items[1].data(), items[1].size()) == cudaSuccess &&
+         upload(&p->d_groups, groups.data(), groups.size()) == cudaSuccess;
+    // the slots of FP64 sums of up to eight components (an execution without them tries again)
+    if (ok && p->n_groups > 0 && cudaMalloc(&p->d_parts[0], p->parts_bytes(0)) != cudaSuccess) p->d_parts[0] = nullptr;
+    cudaGetLastError();
     if (!ok) {
         cudaGetLastError();
         delete p;
@@ -160,8 +184,7 @@ extern "C" int stk_p2p_plan_execute(stk_p2p_plan *plan, int ukernel, int precisi
     if (cudaGetDevice(&dev) != cudaSuccess || dev != plan->device) return STK_ERR_INVALID_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     const int sd = stk::uk_sdim_host(ukernel), rs = stk::uk_record_stride(ukernel);
-    // records, at least eight doubles each where they can be had, so that a forward pass and its
-    // adjoints (3 to 5 staged values) allocate once
+    // records: the plan's own hold eight doubles each (a forward pass and its adjoints: 3 to 5 values)
     const size_t n = std::max(plan->nsrc, 1), need = n * rs;
     if (plan->rec_cap < need) {
         // grow the record buffer: earlier executions may still read it on any stream
@@ -192,7 +215,7 @@ extern "C" int stk_p2p_plan_execute(stk_p2p_plan *plan, int ukernel, int precisi
     if (!mixed && plan->n_groups > 0 && !*parts) {
         cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
         cudaThreadExchangeStreamCaptureMode(&mode);
-        if (cudaMalloc(parts, (size_t)plan->part_targets * (td > 8 ? 16 : 8) * sizeof(double)) != cudaSuccess) {
+        if (cudaMalloc(parts, plan->parts_bytes(td > 8)) != cudaSuccess) {
             cudaGetLastError();
             *parts = nullptr;
             list = 1;
