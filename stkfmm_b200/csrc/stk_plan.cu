@@ -115,13 +115,13 @@ extern "C" stk_p2p_plan *stk_p2p_plan_create(int n_trg_box, const int *trg_begin
     // The two item lists on host threads of their own, and meanwhile, on this one, the device's
     // arrays and the records of most executions (eight doubles a source).  One after the other the
     // lists alone took 2.6 ms for 262k points, and buffers that the first execution allocated made it
-    // wait: creation and first FP64 pass 4.3 ms, 2.8 before there were two lists.
+    // wait: creation and first FP64 pass 4.3 ms, 2.8 before there were two lists.  (Small lists: here.)
     std::vector<stk::WorkItem> items[2];
     std::vector<stk::PartGroup> groups;
     const size_t records = (size_t)std::max(nsrc, 1) * 8;
     bool host_ok = true;
     try {
-        stk::parallel_ranges(ok ? 3 : 0, 1, [&](size_t i0, size_t i1) {
+        stk::parallel_ranges(ok ? 3 : 0, nent > 16384 ? 1 : 3, [&](size_t i0, size_t i1) {
             for (size_t i = i0; i < i1; i++) {
                 if (i == 0) {
                     ok = cudaMalloc(&p->d_counter, 64) == cudaSuccess && upload(&p->d_sbeg, src_begin, n_src_box) == cudaSuccess &&
