@@ -133,7 +133,10 @@ static int direct_device(int uk, int nsrc, const double *d_src, const double *d_
     a.ntrg = ntrg;
     direct_chunks(uk, prec, ntrg, nsrc, ws.num_sms(), a.src_chunk, a.n_chunk);
     if ((rc = ws.begin(stream))) return rc;
-    if (a.n_chunk > 1 && !(a.parts = ws.buf<double>(Workspace::kParts, (size_t)a.n_chunk * ntrg * uk_tdim_host(uk)))) {
+    const bool in_place = direct_in_place(uk, a, d_out);
+    if ((a.n_chunk > 1 || in_place) &&
+        !(a.parts = ws.buf<double>(Workspace::kParts, (size_t)a.n_chunk * ntrg * uk_tdim_host(uk)))) {
+        if (in_place) return STK_ERR_CUDA;
         a.n_chunk = 1;  // no memory for the chunks' sums: one chunk of all sources
         a.src_chunk = (nsrc + 31) / 32 * 32;
     }

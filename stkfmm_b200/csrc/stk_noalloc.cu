@@ -114,7 +114,17 @@ extern "C" int stk_ukernel_direct_device_noalloc(int ukernel, int nsrc, const do
     a.trg_xyz = d_trg_coord;
     a.trg_out = d_trg_value;
     const bool fits = (size_t)a.n_chunk * ntrg * tdim * sizeof(double) <= kNoAllocScratchBytes;
-    if (fits) a.parts = static_cast<double *>(base);
+    const bool in_place = stk::direct_in_place(ukernel, a, d_trg_value);
+    if (fits && (a.n_chunk > 1 || in_place)) {
+        a.parts = static_cast<double *>(base);
+    } else if (in_place) {  // a copy of the sources, which fits by the limit above
+        double *x = static_cast<double *>(base), *v = x + 3 * (size_t)nsrc;
+        if (cudaMemcpyAsync(x, d_src_coord, sizeof(double) * 3 * nsrc, cudaMemcpyDefault, (cudaStream_t)stream) != cudaSuccess ||
+            cudaMemcpyAsync(v, d_src_value, sizeof(double) * sdim * nsrc, cudaMemcpyDefault, (cudaStream_t)stream) != cudaSuccess)
+            return STK_ERR_CUDA;
+        a.src_xyz = x;
+        a.src_val = v;
+    }
     if (stk::launch_direct_p2p(ukernel, precision, a, fits ? 1 : 2, sms, (cudaStream_t)stream) != cudaSuccess)
         return STK_ERR_CUDA;
     return STK_OK;

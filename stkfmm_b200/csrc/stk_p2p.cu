@@ -2,6 +2,7 @@
 // stk_p2p_kernel.cuh).
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 
 #include "stk_p2p_kernel.cuh"
 #include "stk_ukernels.cuh"
@@ -213,15 +214,22 @@ void direct_chunks(int uk, int prec, int ntrg, int nsrc, int num_sms, int &chunk
     }
 }
 
+bool direct_in_place(int uk, const ListP2PArgs &a, const double *out) {
+    auto meets = [&](const double *p, size_t n) {
+        const uintptr_t b = reinterpret_cast<uintptr_t>(p), o = reinterpret_cast<uintptr_t>(out);
+        return b < o + sizeof(double) * (size_t)a.ntrg * uk_tdim(uk) && o < b + sizeof(double) * n;
+    };
+    return meets(a.src_xyz, 3 * (size_t)a.nsrc) || meets(a.src_val, (size_t)uk_sdim(uk) * a.nsrc);
+}
+
 cudaError_t launch_direct_p2p(int uk, int prec, const ListP2PArgs &args, int add, int num_sms, cudaStream_t stream) {
     if (args.nsrc <= 0 || args.ntrg <= 0) return cudaSuccess;
     if (uk < 0 || uk >= UK_COUNT || (uk_tvdim(uk) > 0) != (args.trg_aux != nullptr)) return cudaErrorInvalidValue;
-    const bool split = args.n_chunk > 1;
+    const bool split = args.parts != nullptr;  // (one chunk too: targets written over the sources)
     const long long items = (long long)((args.ntrg + 63) / 64) * args.n_chunk;
-    if ((split && add != 2 && !args.parts) || items > 0x7fffffffll) return cudaErrorInvalidValue;
+    if ((args.n_chunk > 1 && add != 2 && !split) || items > 0x7fffffffll) return cudaErrorInvalidValue;
     ListP2PArgs a = args;
     a.n_items = (int)items;
-    if (!split) a.parts = nullptr;
     a.atomic_out = split && add != 2 ? 0 : add;
     if (add == 2) a.parts = nullptr;
     cudaError_t e = prec == PREC_MIXED ? direct_p2p_mixed(uk, a, num_sms, stream) : direct_p2p_fp64(uk, a, num_sms, stream);

@@ -186,3 +186,27 @@ def test_fp64_rsqrt_pointwise():
     # the gradient, -r / (4 pi r^3)
     g = -trg / (r2 * np.sqrt(r2))[:, None] / (4 * np.pi)
     assert np.max(np.abs(out[:, 1:] - g) / np.linalg.norm(g, axis=1)[:, None]) < 2e-15
+
+
+# few sources and many targets (one chunk of sources, later waves of items read what the first have
+# written; 400k: the sums fit no scratch of the entry without allocation), many chunks
+@pytest.mark.parametrize("entry", ["", "_noalloc"])
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("over", ["values", "coordinates"])
+@pytest.mark.parametrize("ns,nt", [(32, 200000), (32, 400000), (3000, 3000)])
+def test_direct_in_place(torch_cuda, L, ns, nt, over, prec, entry):
+    """Results added over the sources' values, or over their coordinates (points moved by their own
+    velocities): the sum is that of the sources as they were."""
+    rng = np.random.default_rng(ns + nt)
+    src, val, trg = rng.random((ns, 3)), uk_values(rng, 4, ns), rng.random((nt, 3))
+    out0 = rng.random((nt, 3))
+    out0[:ns] = val if over == "values" else src
+    o = dev(torch_cuda, out0)
+    s = dev(torch_cuda, src) if over == "values" else o
+    v = dev(torch_cuda, val) if over == "coordinates" else o
+    t = dev(torch_cuda, trg)
+    rc = getattr(L, "stk_ukernel_direct_device" + entry)(4, ns, s.data_ptr(), v.data_ptr(), nt, t.data_ptr(), o.data_ptr(),
+                                                         prec, torch_cuda.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    torch_cuda.cuda.synchronize()
+    assert rel_l2(o.cpu().numpy() - out0, O.direct(4, src, val, trg)) < TOL[prec]
