@@ -143,6 +143,7 @@ static int direct_device(int uk, int nsrc, const double *d_src, const double *d_
     a.trg_xyz = d_trg;
     a.trg_out = d_out;
     a.box_centre = nullptr;  // per-item origin: the item's first target
+    a.counter = ws.counter();
     a.trg_aux = d_trg_aux;
     STK_CUDA(launch_direct_p2p(uk, prec, a, add, ws.num_sms(), stream));
     return ws.end(stream);

@@ -113,7 +113,10 @@ extern "C" int stk_ukernel_direct_device_noalloc(int ukernel, int nsrc, const do
     stk::direct_chunks(ukernel, precision, ntrg, nsrc, sms, a.src_chunk, a.n_chunk);
     a.trg_xyz = d_trg_coord;
     a.trg_out = d_trg_value;
-    const bool fits = (size_t)a.n_chunk * ntrg * tdim * sizeof(double) <= kNoAllocScratchBytes;
+    // the work counter of mixed items: the array's end (the limit above leaves room for it)
+    constexpr size_t room = kNoAllocScratchBytes - 256;
+    a.counter = reinterpret_cast<unsigned int *>(static_cast<unsigned char *>(base) + room);
+    const bool fits = (size_t)a.n_chunk * ntrg * tdim * sizeof(double) <= room;
     const bool in_place = stk::direct_in_place(ukernel, a, d_trg_value);
     if (fits && (a.n_chunk > 1 || in_place)) {
         a.parts = static_cast<double *>(base);

@@ -227,7 +227,7 @@ cudaError_t launch_direct_p2p(int uk, int prec, const ListP2PArgs &args, int add
     if (uk < 0 || uk >= UK_COUNT || (uk_tvdim(uk) > 0) != (args.trg_aux != nullptr)) return cudaErrorInvalidValue;
     const bool split = args.parts != nullptr;  // (one chunk too: targets written over the sources)
     const long long items = (long long)((args.ntrg + 63) / 64) * args.n_chunk;
-    if ((args.n_chunk > 1 && add != 2 && !split) || items > 0x7fffffffll) return cudaErrorInvalidValue;
+    if ((prec == PREC_MIXED && !args.counter) || (args.n_chunk > 1 && add != 2 && !split) || items > 0x7fffffffll) return cudaErrorInvalidValue;
     ListP2PArgs a = args;
     a.n_items = (int)items;
     a.atomic_out = split && add != 2 ? 0 : add;

@@ -78,8 +78,8 @@ cudaError_t launch_list_p2p(int uk, int prec, const ListP2PArgs &a, int num_sms,
 // through parts then, or the sources are copied.
 bool direct_in_place(int uk, const ListP2PArgs &a, const double *out);
 void direct_chunks(int uk, int prec, int ntrg, int nsrc, int num_sms, int &chunk, int &n_chunk);
-// a: src_xyz, src_val, nsrc, ntrg, src_chunk, n_chunk, parts (n_chunk > 1, or in place), trg_xyz,
-// trg_aux and trg_out; add = 0: trg_out = sum, 1: +=, 2: += by atomics, without parts
+// a: src_xyz, src_val, nsrc, ntrg, src_chunk, n_chunk, parts (n_chunk > 1, or in place), counter
+// (mixed), trg_xyz, trg_aux and trg_out; add = 0: trg_out = sum, 1: +=, 2: += by atomics, without parts
 cudaError_t launch_direct_p2p(int uk, int prec, const ListP2PArgs &a, int add, int num_sms, cudaStream_t stream);
 
 // Source records of micro-kernel uk: rec[i] = (xyz[i], values, 0 padding), values = those of v1[perm[i]]

@@ -230,7 +230,15 @@ __global__ void __launch_bounds__(Cta<MIXED>::threads, MinBlocks<UK, MIXED>::val
         int it = 0;
         WorkItem w;
         if constexpr (DIRECT) {
-            it = (turn * gridDim.x + blockIdx.x) * kWarpsPerCta + wid;  // equal items: dealt in turn
+            // Equal items.  FP64: dealt in turn (direct_chunks fills whole turns).  Mixed: taken from the
+            // counter, as their number fills the last turn anyhow (50k x 50k points, dealt: rpy_u 3.30
+            // ms, 3.02 taken; stokes_regftvel 4.73, 4.49).
+            if constexpr (MIXED) {
+                if (lane == 0) it = (int)atomicAdd(a.counter, 1u);
+                it = __shfl_sync(kFull, it, 0);
+            } else {
+                it = (turn * gridDim.x + blockIdx.x) * kWarpsPerCta + wid;
+            }
             if (it >= a.n_items) break;
             const int nc = (a.ntrg + 63) >> 6, c = it % nc;
             w.trg_box = c;
@@ -670,7 +678,7 @@ cudaError_t launch_impl(const ListP2PArgs &a, int num_sms, cudaStream_t stream) 
     constexpr int kWarpsPerCta = Cta<MIXED>::warps;
     long long want = ((long long)a.n_items + kWarpsPerCta - 1) / kWarpsPerCta;
     int grid = (int)std::max(1LL, std::min<long long>((long long)num_sms * blocks_per_sm, want));
-    if (!DIRECT && (err = cudaMemsetAsync(a.counter, 0, sizeof(unsigned int), stream)) != cudaSuccess) return err;
+    if ((!DIRECT || MIXED) && (err = cudaMemsetAsync(a.counter, 0, sizeof(unsigned int), stream)) != cudaSuccess) return err;
     list_p2p_kernel<UK, MIXED, DIRECT><<<grid, Cta<MIXED>::threads, 0, stream>>>(a);
     return cudaGetLastError();
 }
