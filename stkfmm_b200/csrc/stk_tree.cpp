@@ -7,7 +7,6 @@
 #include <exception>
 #include <mutex>
 #include <numeric>
-#include <system_error>
 #include <thread>
 
 namespace stk {
@@ -61,7 +60,7 @@ void parallel_ranges(size_t n, size_t grain, const std::function<void(size_t, si
     size_t started = 1;
     try {
         for (; started < nt; started++) th.emplace_back(run, started);
-    } catch (const std::system_error &) {  // no more threads: the rest runs here
+    } catch (...) {  // no more threads, or no memory for one: the rest runs here
     }
     run(0);
     for (size_t i = started; i < nt; i++) run(i);

@@ -178,3 +178,55 @@ def test_point_order_is_a_stable_morton_sort(dup, n):
     np.testing.assert_array_equal(perm, np.argsort(key, kind="stable"))
     np.testing.assert_array_equal(t.point_set(2)[0], perm)
     np.testing.assert_array_equal(t.point_set(1)[0], np.concatenate([[n - 1], perm[perm != n - 1]]))
+
+
+def test_parallel_ranges_without_memory_for_a_thread(tmp_path):
+    """Every allocation of a parallel loop failing in turn: it throws bad_alloc before its first thread
+    starts, or runs every range once; the program is never ended."""
+    import os
+    import shutil
+    import subprocess
+    cxx = shutil.which("g++") or shutil.which("c++")
+    if not cxx:
+        pytest.skip("no C++ compiler")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    src = tmp_path / "ranges.cpp"
+    src.write_text(r"""
+#include <atomic>
+#include <cstdlib>
+#include <new>
+#include "stk_tree.hpp"
+static std::atomic<long> left(-1);
+void *operator new(std::size_t n) {
+    if (left >= 0 && left-- == 0) throw std::bad_alloc();
+    return std::malloc(n);
+}
+void operator delete(void *p) noexcept { std::free(p); }
+void operator delete(void *p, std::size_t) noexcept { std::free(p); }
+int main() {
+    for (long k = 0; k < 64; k++) {
+        std::atomic<int> ran[8] = {};
+        const std::function<void(size_t, size_t)> f = [&](size_t a, size_t b) {
+            for (; a < b; a++) ran[a]++;
+        };
+        left = k;
+        try {
+            stk::parallel_ranges(8, 1, f);
+        } catch (const std::bad_alloc &) {
+            left = -1;
+            for (auto &r : ran)
+                if (r > 1) return 1;
+            continue;
+        }
+        left = -1;
+        for (auto &r : ran)
+            if (r != 1) return 2;
+    }
+    return 0;
+}
+""")
+    exe = tmp_path / "ranges"
+    csrc = os.path.join(root, "stkfmm_b200", "csrc")
+    subprocess.run([cxx, "-std=c++17", "-O1", "-pthread", "-I", csrc, str(src), os.path.join(csrc, "stk_tree.cpp"), "-o",
+                    str(exe)], check=True)
+    assert subprocess.run([str(exe)]).returncode == 0
