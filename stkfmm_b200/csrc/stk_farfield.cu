@@ -1243,6 +1243,7 @@ int setup_pass(ListPass &P, int uk, const std::vector<int> &tb, const std::vecto
                int n_src_box, bool own_src, const std::vector<double> &centres, int balance_warps, bool check,
                cudaStream_t s, int shard_rank = 0, int shard_n = 1) {
     P.uk = uk;
+    P.check = check;
     std::vector<WorkItem> items;
     std::vector<PartGroup> groups;
     long long slots = 0;
@@ -1250,9 +1251,7 @@ int setup_pass(ListPass &P, int uk, const std::vector<int> &tb, const std::vecto
                      P.pairs, balance_warps, shard_rank, shard_n);
     P.n_items = (int)items.size();
     int rc = P.items[1].upload(items, groups, 0, s);
-    if (check) {
-        if (!rc) P.items[0].share(P.items[1]);
-    } else {
+    if (!check) {
         build_split_items((int)tb.size(), tb.data(), te.data(), off.data(), ent.data(), h_src_beg, h_src_end,
                           balance_warps * 5 / 4, items, groups, slots, shard_rank, shard_n);
         if (!rc) rc = P.items[0].upload(items, groups, slots, s);
@@ -1266,13 +1265,13 @@ int setup_pass(ListPass &P, int uk, const std::vector<int> &tb, const std::vecto
 
 int run_pass(const ListPass &P, int prec, const double *rec, const int *src_beg, const int *src_end,
              const double *trg_xyz, double *out, unsigned int *counter, DevBuf &parts, int sms, cudaStream_t s) {
-    if (P.items[prec].n_items == 0) return STK_OK;
+    if (P.list(prec).n_items == 0) return STK_OK;
     ListP2PArgs a{};
     a.src_rec = rec;
     a.src_box_begin = src_beg;
     a.src_box_end = src_end;
     a.list_ent = (const int *)P.ent.ptr;
-    list_args(P.items, prec, uk_tdim_host(P.uk), parts, a);
+    list_args(P.items, P.check ? PREC_MIXED : prec, uk_tdim_host(P.uk), parts, a);
     t_launches += a.n_groups ? 2 : 1;
     a.counter = counter;
     a.trg_xyz = trg_xyz;

@@ -32,10 +32,13 @@ struct ListPass {
     int n_items = 0;    // 0: nothing to do (the mixed path's count)
     long long pairs = 0;
     ItemList items[2];  // FP64, mixed
+    bool check = false;  // check potentials: the mixed path's items in both precisions
+    const ItemList &list(int prec) const { return items[check ? 1 : prec]; }
     DevBuf ent, src_beg, src_end, trg_box_centre;
     void reset() {
         uk = -1;
         n_items = items[0].n_items = items[1].n_items = 0;
+        items[0].part_targets = 0;
         pairs = 0;
     }
 };

@@ -111,6 +111,8 @@ Stk3DFMM::~Stk3DFMM() {
     if (ev_out) cudaEventDestroy(ev_out);
 }
 
+static void reserve_parts(const Stk3DFMM *f, KernelData *kd);
+
 extern "C" Stk3DFMM *Stk3DFMM_create(int mult_order, int max_pts, int pbc, unsigned kernelComb) {
     if (mult_order < 2 || max_pts < 1 || pbc < 0 || pbc > 3 || kernelComb == 0) return nullptr;
     if (stk_device_count() <= 0) return nullptr;
@@ -266,7 +268,7 @@ extern "C" int Stk3DFMM_setup_tree(Stk3DFMM *fmm, unsigned kernel) {
     const PointSet &tg = T.sets[2];
     kd->u_pairs[0] = kd->u_pairs[1] = 0;
     for (int k = 0; k < 2; k++) {
-        kd->u_items[k][0].n_items = kd->u_items[k][1].n_items = 0;
+        for (ItemList &l : kd->u_items[k]) l.n_items = l.part_targets = 0;
         if (k == 1 && (!dl || kd->fused)) continue;
         const PointSet &sp = T.sets[k];
         std::vector<WorkItem> items;
@@ -292,6 +294,7 @@ extern "C" int Stk3DFMM_setup_tree(Stk3DFMM *fmm, unsigned kernel) {
     if (!rc && cudaStreamSynchronize(s) != cudaSuccess) rc = STK_ERR_CUDA;
     if (rc) return rc;
     kd->tree_ready = true;
+    reserve_parts(fmm, kd);
     if (verbose())
         printf("tree: %d nodes, %zu leaves, depth %d, U entries %zu, U pairs SL %lld DL %lld\n", nn, T.leaves.size(),
                T.depth(), T.U.size(), kd->u_pairs[0], kd->u_pairs[1]);
@@ -347,9 +350,22 @@ extern "C" int Stk3DFMM_set_far_field(Stk3DFMM *fmm, int enable) {
     return STK_OK;
 }
 
+// The slots of a kernel's split FP64 sums, allocated with its lists and not by an evaluation.
+static void reserve_parts(const Stk3DFMM *f, KernelData *kd) {
+    if (f->precision != PREC_FP64 || !kd->tree_ready) return;
+    long long slots = 0;
+    for (int k = 0; k < 2; k++) slots = std::max(slots, kd->u_items[k][0].part_targets);
+    if (kd->far_ready)
+        for (const ListPass *P : {&kd->far->near[0], &kd->far->near[1], &kd->far->m2t, &kd->far->l2t})
+            slots = std::max(slots, P->items[0].part_targets);
+    if (slots > 0) (void)kd->d_parts.reserve(sizeof(double) * (size_t)slots * kd->info->kdim_trg);
+}
+
 extern "C" int Stk3DFMM_set_precision(Stk3DFMM *fmm, int precision) {
     if (!fmm || (precision != STK_FP64 && precision != STK_MIXED)) return STK_ERR_INVALID_ARG;
     fmm->precision = precision;
+    cudaSetDevice(fmm->device);
+    for (auto &kv : fmm->pool) reserve_parts(fmm, kv.second.get());
     return STK_OK;
 }
 
@@ -666,6 +682,7 @@ static int ensure_far(Stk3DFMM *fmm, KernelData *kd) {
     const int rc = farfield_setup(fmm, kd);
     if (rc) return rc;
     kd->far_ready = true;
+    reserve_parts(fmm, kd);
     return STK_OK;
 }
 

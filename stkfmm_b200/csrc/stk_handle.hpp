@@ -45,18 +45,11 @@ struct ItemList {
     int n_items = 0, n_groups = 0;
     long long part_targets = 0;  // target slots of split sums
     int upload(const std::vector<WorkItem> &it, const std::vector<PartGroup> &g, long long slots, cudaStream_t s);
-    void share(const ItemList &o) {
-        items.share(o.items);
-        groups.share(o.groups);
-        n_items = o.n_items;
-        n_groups = o.n_groups;
-        part_targets = o.part_targets;
-    }
 };
 
 // The items of a pass [FP64, mixed] for `prec`, its groups and the slots' buffer into the kernel's
 // arguments (tdim components).  Without memory for the slots an FP64 pass takes the mixed
-// path's items, which split no sources.
+// path's items, which split no sources.  (reserve_parts has allocated them at set-up.)
 void list_args(const ItemList (&lists)[2], int prec, int tdim, DevBuf &parts, ListP2PArgs &a);
 
 // One activated kernel: the reference's impl::FMMData (STKFMM_impl.hpp:19-174).

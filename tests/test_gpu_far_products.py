@@ -175,3 +175,26 @@ def test_a_given_up_wait_is_an_error(torch_cuda):
                     look()
                 look()
         np.testing.assert_array_equal(wall(), ref_w)
+
+
+@pytest.mark.parametrize("far", [False, True])
+def test_evaluations_allocate_no_slots_of_split_sums(torch_cuda, far):
+    """A handle evaluated in mixed precision and set to FP64: the slots of its split sums are allocated by
+    the switch (near field alone) or the far field's set-up, not by the evaluations that follow."""
+    pts, slv, dlv, td = fmm_case(1, 20000, seed=150)
+    keep, _ = run_fmm(1, 6, 200, pts, slv, dlv, td)  # libraries and kernels are loaded
+    keep.evaluate_near(1, slv, np.zeros((len(pts), td)), dlv)
+    f, _ = run_fmm(1, 6, 200, pts, slv, dlv, td, prec=1)
+
+    def evaluate():
+        (f.evaluate_fmm if far else f.evaluate_near)(1, slv, np.zeros((len(pts), td)), dlv)
+
+    evaluate()
+    before = used_bytes(torch_cuda)
+    f.set_precision(0)
+    if far:
+        evaluate()  # the far field's FP64 set-up
+    held = used_bytes(torch_cuda)
+    assert held > before, "no split sums in this case"
+    evaluate()
+    assert used_bytes(torch_cuda) == held
