@@ -174,9 +174,10 @@ int stk_ukernel_direct_aux_device(int ukernel, int nsrc, const double *d_src_coo
  * and cannot afford the device-wide synchronisation of cudaMalloc/cudaFree,
  * hosts that forbid run-time allocation.  No reference counterpart.
  * It calls no cudaMalloc/cudaFree: all scratch lives in one fixed 8 MiB array
- * that the library reserves on every GPU where it is loaded.  Sizes whose
- * scratch (work list + nsrc packed source records) exceeds 8 MiB are refused
- * with STK_ERR_SIZE (about 130k sources for 8-double records).  It takes every
+ * that the library reserves on every GPU where it is loaded.  Sizes are bounded:
+ * 24 bytes per 64 targets and chunk of sources (of at least 256) plus a padded
+ * record per source (3 coordinates and its values) must not exceed 8 MiB, else
+ * STK_ERR_SIZE (about 130k sources of 4 values).  It takes every
  * micro-kernel stk_ukernel_direct_device takes without per-target values; the
  * adjoint ids (13, 14) are refused with STK_ERR_INVALID_ARG.  The first call on
  * a device looks the array up (cudaGetSymbolAddress) and the first call of each
@@ -294,8 +295,11 @@ int Stk3DFMM_show_active_kernels(Stk3DFMM *fmm);
 /* STKFMM::evaluateKernel through the handle (STKFMM.cpp:88-99) */
 int Stk3DFMM_evaluate_kernel(Stk3DFMM *fmm, unsigned kernel, int nThreads, unsigned p2p, int nSrc,
                              double *srcCoord, double *srcValue, int nTrg, double *trgCoord, double *trgValue);
-/* choose FP64 or MIXED for the P2P kernels of this handle (default FP64).  The far
- * field is set up for the precision it is first evaluated in; the first FP64
+/* choose FP64 or MIXED for the P2P kernels of this handle (default FP64).  MIXED
+ * also runs the M2L's factors on the TF32 tensor cores (3-way split), but keeps
+ * the FP64 products of the Stokes translations (Stokes, RPY, RegVel, PVel, ...) on
+ * cuBLAS, for the same rounding; FP64 runs them on the int8 tensor cores and can
+ * be as fast (PVel, p = 12).  The far field is set up for the precision it is first evaluated in; the first FP64
  * evaluate_fmm after mixed ones sets it up again (and synchronises). */
 int Stk3DFMM_set_precision(Stk3DFMM *fmm, int precision);
 /* Multi-GPU sharding of one problem: this handle evaluates only shard `rank` of
@@ -370,7 +374,7 @@ int Stk3DFMM_get_fmm_stats(Stk3DFMM *fmm, unsigned kernel, long long *out);
 /* Floating-point work of one compressed M2L of `kernel` (after its first evaluate_fmm):
  * out[0] = 4 k r_d per V-list pair at the offsets' true ranks plus the two basis
  * products (4 N k per node), out[1] = the flops the GEMMs execute (ranks padded to
- * multiples of 32, columns to 256-pair chunks). */
+ * multiples of 32, columns to 128-pair chunks). */
 int Stk3DFMM_get_m2l_work(Stk3DFMM *fmm, unsigned kernel, double *out);
 /* Copy the U-list of the last setup_tree (leaf-sorted indices, same layout as
  * stk_p2p_lists).  Pass null arrays to query sizes: sizes = {n_leaf_boxes, n_entries, nSL, nDL, nTrg}. */

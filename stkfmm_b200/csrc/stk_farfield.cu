@@ -1393,9 +1393,9 @@ int record_built(FarField &e, cudaStream_t s) {
 
 // Tensor-core operands and tile tables of the mixed path's chunked M2L (the levels the
 // dense M2L does not take).  Per group of column chunks two grouped GEMM launches:
-//   stage 1  Z_c = Q_d^T X_c (r_d x 256 per chunk c of offset d), written split into
+//   stage 1  Z_c = Q_d^T X_c (r_d x 128 per chunk c of offset d), written split into
 //            TF32 hi / lo parts as the next stage's K-major operand (rows of rmax);
-//   stage 2  Y_c = P_d Z_c (k x 256), FP32, reduced per target as on the SIMT path.
+//   stage 2  Y_c = P_d Z_c (k x 128), FP32, reduced per target as on the SIMT path.
 // Every tile is 128 x 128 (rows of the factor x columns of the chunk) over the whole K.
 // The operands (~8 (sum_d r_d k + nslot k rmax) bytes) must fit in 4 GiB, else the
 // SIMT path stays; STKFMM_M2L_TC=0 turns both tensor-core paths off.
@@ -2260,7 +2260,7 @@ static int setup_far(Stk3DFMM *f, KernelData *kd, bool i8) {
         if (!F.tcc || (F.fp64 && !F.i8_chunks)) {
             // Per group of columns and padded rank r: two batched GEMMs over that group's
             // chunks whose offset has rank r,
-            //   Z_c = Q_d^T X_c (r x 256),  Y_c = P_d Z_c (k x 256).
+            //   Z_c = Q_d^T X_c (r x 128),  Y_c = P_d Z_c (k x 128).
             // Pointer arrays in (group, rank, chunk) order -- A: the offset's factor; B, C:
             // the chunk's slot in its group -- as FP64 and FP32 views of the same buffers.
             std::vector<int> order;
@@ -2548,9 +2548,9 @@ int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const dou
     t_launches = 0;
     // The mixed path rounds the densities to FP32 after the FP64 products.  Those of the Stokes
     // translations are larger than the fields they stand for by orders of magnitude, and
-    // products that round differently, however well, move the mixed result by up to 3.5e-8 (Stokes
-    // wall, 100k points; within its 3e-7 error, but no longer the same numbers); laplace_p's
-    // by 6e-13.  So the mixed path takes the int8 products for laplace_p alone.
+    // products that round differently, however well, move the mixed result by up to 7.8e-8 (drawn
+    // Stokes, RPY and PVel cases; within its 3e-7 error, but no longer the same numbers);
+    // laplace_p's by 6e-13.  So the mixed path takes the int8 products for laplace_p alone.
     const bool i8 = F.i8 && (prec == PREC_FP64 || F.ke == 1);
     FCUDA(cudaMemsetAsync(phi, 0, sizeof(double) * (size_t)nn * N, s));
     FCUDA(cudaMemsetAsync(psi, 0, sizeof(double) * (size_t)nn * N, s));
@@ -2722,7 +2722,7 @@ int farfield_evaluate(Stk3DFMM *f, KernelData *kd, const double *d_sl, const dou
         FCUDA(cudaGetLastError());
         for (const M2LSeg &sg : F.m2l_seg) {
             if (sg.group != c0 / gc) continue;
-            // Z = Q_d^T X (r x 256), then Y = P_d Z (k x 256), for the segment's chunks
+            // Z = Q_d^T X (r x 128), then Y = P_d Z (k x 128), for the segment's chunks
             FBLAS(cublasGemmBatchedEx(F.blas, CUBLAS_OP_T, CUBLAS_OP_N, sg.rank, kM2LChunk, k, alpha,
                                       (const void *const *)P[0].ptr + sg.start, dt, k,
                                       (const void *const *)P[1].ptr + sg.start, dt, k, beta,

@@ -83,8 +83,8 @@ extern "C" int stk_ukernel_direct_device_noalloc(int ukernel, int nsrc, const do
         cudaGetLastError();
         return STK_ERR_NO_DEVICE;
     }
-    // The sizes this entry takes, by its interface: the records and the work list of 64-target
-    // chunks x source chunks (>= 256 points) within the scratch.
+    // The sizes this entry takes are its interface's, not what is needed below: 24 bytes per 64
+    // targets x chunk of sources (>= 256 points), 12 per chunk, and a record per source.
     const long long nchunk = (ntrg + kItemTargets - 1) / kItemTargets;
     const long long want_items = (long long)(sms > 0 ? sms : 1) * 64;
     long long nsc = (want_items + nchunk - 1) / nchunk;

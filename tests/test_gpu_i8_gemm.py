@@ -129,3 +129,22 @@ def test_error_bound_holds_for_graded_rows(torch_cuda, K):
     ref = A.astype(np.longdouble) @ B.astype(np.longdouble).T
     bound = 4.2 * K * 2.0 ** -56 * np.abs(A).max(1)[:, None] * np.abs(B).max(1) + 2.0 ** -52 * np.abs(ref)
     assert (np.abs(product(torch_cuda, A, B) - ref) <= bound).all()
+
+
+def test_m2l_shape(torch_cuda):
+    """A product of the triply periodic RPY case's M2L (rank 636, 32,768 nodes, 3,584 stacked ranks) on
+    normal operands, 12 columns of it against long-double sums (also the profiled launch)."""
+    from stkfmm_b200 import lib
+    torch = torch_cuda
+    M, N, K = 636, 32768, 3584
+    gen = torch.Generator(device="cuda").manual_seed(11)
+    A = torch.randn((M, K), dtype=torch.float64, device="cuda", generator=gen)
+    B = torch.randn((N, K), dtype=torch.float64, device="cuda", generator=gen)
+    C = torch.empty((N, M), dtype=torch.float64, device="cuda")
+    rc = lib().stk_gemm_f64_i8(M, N, K, A.data_ptr(), K, B.data_ptr(), K, C.data_ptr(), M, 0,
+                               torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    cols = np.linspace(0, N - 1, 12).astype(int)
+    ref = B[cols].cpu().numpy().astype(np.longdouble) @ A.cpu().numpy().astype(np.longdouble).T
+    err = np.linalg.norm((C[cols].cpu().numpy() - ref).astype(float)) / np.linalg.norm(ref.astype(float))
+    assert err < 2.0 ** -53 * (1 + np.sqrt(K) / 4), err
