@@ -11,11 +11,11 @@
 // The eight digit groups i + j = 0 .. 7 need 8 x 128 TMEM columns and there are 512, so a
 // tile takes two passes over K: groups 0-3 (planes 0-3 of both operands, 10 products per K
 // block) drained into an int64 per output, then groups 4-7 (all planes, 24 products).
-// What bounds it (M = 636, N = 32768, K = 3584, B200): 1.55 ms, 97 TFLOP/s of FP64 work (cuBLAS:
-// 29.9); tensor pipe active 71% at 1.64 GHz (power), L2 7.1 TB/s.  By shared memory alone, the
+// What bounds it (M = 636, N = 32768, K = 3584, B200): 1.58 ms, 95 TFLOP/s of FP64 work (cuBLAS:
+// 29.9); tensor pipe active 80% of the time at 1.68 GHz (power), L2 6.2 TB/s.  By shared memory alone, the
 // 34 MMAs of a K block read 8 KB each and the copies write 88 KB: 2800 clocks for 34 x 64 of MMA.
 // 128 x 64 tiles (all groups resident, one pass) would read 6 KB per MMA of half the work; CTA
-// pairs (256 x 128 tiles, 2110 clocks by the same count) measured 1.71 ms.
+// pairs (256 x 128 tiles, 2110 clocks by the same count) measured 1.71 ms beside 1.55.
 // Short K (M2L's P_d, 4 K blocks): the chain of the two passes, 18000 clocks a tile, 5900 of
 // them MMA: the second pass's MMAs 6200, the drains 1800 and 6000, the wait for the first 2000;
 // a third of the L2 traffic less (blocks kept for the second pass, used rows only) changed nothing.
