@@ -294,7 +294,9 @@ extern "C" int Stk3DFMM_setup_tree(Stk3DFMM *fmm, unsigned kernel) {
     if (!rc && cudaStreamSynchronize(s) != cudaSuccess) rc = STK_ERR_CUDA;
     if (rc) return rc;
     kd->tree_ready = true;
-    reserve_parts(fmm, kd);
+    // (a handle whose FMM is evaluated takes its far field's, the larger, at that set-up; a new one
+    // allocates all its buffers at its first evaluation)
+    if (kd->timed && !kd->last_far) reserve_parts(fmm, kd);
     if (verbose())
         printf("tree: %d nodes, %zu leaves, depth %d, U entries %zu, U pairs SL %lld DL %lld\n", nn, T.leaves.size(),
                T.depth(), T.U.size(), kd->u_pairs[0], kd->u_pairs[1]);
