@@ -384,6 +384,7 @@ int stk::handle_status(Stk3DFMM *f) {
 // Test hook (not in the header): leaves the code that a tensor-core product leaves when a pipeline
 // wait gives up, for the evaluations of `kernel` queued so far.
 extern "C" int stk_test_post_wait_error(Stk3DFMM *fmm, unsigned kernel) {
+    if (!fmm) return STK_ERR_INVALID_ARG;
     auto it = fmm->pool.find(kernel);
     if (it == fmm->pool.end() || !it->second->far || !it->second->far->tc_err.ptr) return STK_ERR_STATE;
     const int code = 1;

@@ -532,7 +532,7 @@ extern "C" int StkWallFMM_evaluate_fmm(StkWallFMM *fmm, unsigned kernel, const i
 // Test hook (not in the header): stk_test_post_wait_error of sub-FMM `sub`
 extern "C" int stk_test_post_wall_wait_error(StkWallFMM *fmm, unsigned kernel, int sub) {
     const int f = family_of(kernel);
-    if (f < 0 || sub < 0 || sub >= kSubs || !fmm->sub[f][sub]) return STK_ERR_INVALID_ARG;
+    if (!fmm || f < 0 || sub < 0 || sub >= kSubs || !fmm->sub[f][sub]) return STK_ERR_INVALID_ARG;
     return stk_test_post_wait_error(fmm->sub[f][sub], kSubKernel[f][sub]);
 }
 
